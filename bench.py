@@ -266,6 +266,11 @@ def main():
         launches["n"] += per_call.get(name, 0)
         return orig_call(name, *a)
     _lib._call = counting_call
+    native = _lib.native()                  # the eager route calls the two composite entry points itself and counts them
+
+    def launch_count():
+        fwd, bwd = native.call_counts()
+        return launches["n"] + fwd * per_call["dm_attn_forward"] + bwd * per_call["dm_attn_backward"]
 
     scaling = args.scaling if world > 1 else "weak"     # one GPU: the whole config either way
     if scaling == "strong":
@@ -343,11 +348,11 @@ def main():
                 step()
             torch.cuda.current_stream().wait_stream(side)
             torch.cuda.synchronize()
-            launches["n"] = 0
+            before = launch_count()
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph):
                 step()
-            launches_per_step = launches["n"]
+            launches_per_step = launch_count() - before
             for _ in range(2):
                 graph.replay()
         except Exception as e:                      # noqa: BLE001
@@ -356,7 +361,7 @@ def main():
             torch.cuda.synchronize()
     run_step = graph.replay if graph is not None else step
     sync_all()
-    launches["n"] = 0
+    launches_before = launch_count()
 
     # The timed region: the K steps, repeated (same K steps again) until at least --min-seconds of GPU time have been timed, so
     # that the number is a sustained one and the clock sampler sees the GPU under load.  The first K steps alone are kept as
@@ -372,7 +377,7 @@ def main():
         for _ in range(repeats - 1):
             total_ms += max_over_ranks(timed_steps(run_step, args.steps))
     n_timed = args.steps * repeats
-    n_launch = launches["n"] if graph is None else launches_per_step * n_timed
+    n_launch = launch_count() - launches_before if graph is None else launches_per_step * n_timed
     ms_step = total_ms / n_timed
     value = world * flops / (ms_step * 1e-3) / 1e12       # every rank does `flops` (its whole config, or its equal shard)
     burst = {"value": world * flops / (burst_ms / args.steps * 1e-3) / 1e12, "unit": "TFLOP/s", "ms_per_step": burst_ms / args.steps,

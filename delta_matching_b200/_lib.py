@@ -14,6 +14,7 @@ import torch
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _LIB = None
 _LIB_PATH = None
+_NATIVE = None
 
 E4M3 = torch.float8_e4m3fn
 
@@ -103,6 +104,24 @@ def lib():
 
 def loaded_library():
     return _LIB_PATH
+
+
+def native():
+    """The module of the eager route (_dm_torch.so, csrc/dm_torch.cpp), bound to the loaded library's entry points on first use."""
+    global _NATIVE
+    if _NATIVE is None:
+        path = os.path.join(_HERE, "_dm_torch.so")
+        if not os.path.isfile(path):
+            raise RuntimeError("delta_matching_b200: _dm_torch.so is not built; run `python -m delta_matching_b200.build` in the checkout")
+        import importlib.util
+        spec = importlib.util.spec_from_file_location("delta_matching_b200._dm_torch", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        from . import split
+        mod.bind({n: C.cast(getattr(lib(), n), C.c_void_p).value
+                  for n in ("dm_attn_forward", "dm_attn_backward", "dm_bwd_workspace_bytes")}, split)
+        _NATIVE = mod
+    return _NATIVE
 
 
 def build_info() -> str:

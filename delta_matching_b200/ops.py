@@ -112,8 +112,7 @@ def _(x, Hk):
 
 def attn_fwd_eager(q: Tensor, k: Tensor, v: Tensor, causal: bool):
     """The whole forward as plain calls into the library: q (B, N, H, D), k / v (B, N, Hk, D) bf16 ->
-    O, LSE, Q8, Q8s, K8, K8s, V8, V8s.  The autograd route calls this directly in eager mode (the torch.library dispatcher
-    costs more host time per call than all the kernel launches together) and the custom op below under torch.compile."""
+    O, LSE, Q8, Q8s, K8, K8s, V8, V8s (the body of the custom op below; the eager route goes through the native module)."""
     return _lib.attn_forward(q, k, v, causal)
 
 
