@@ -187,7 +187,6 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         // Each runs its loop converged (all lanes wait and compute the same addresses, so they stay in uniform registers)
         // and lane 0 alone executes the asynchronous instruction.
         dm::reg_dec<40>();
-        const bool leader = lane == 0;
         if (warp == kSoftmaxWarps + 4) {
             // ---- S^T = K Q^T and dP^T = V dO^T of every m-block, as soon as the softmax warps have read the previous pair
             constexpr uint32_t idesc_sp = dm::idesc_e4m3(128, 64, false, false);
@@ -215,7 +214,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                     dm::tc_fence_after();
                     const uint32_t t_s = tmem, t_dp = tmem + 64;
                     const uint32_t qs = q_lo + st * kStageQ, dos = do_lo + st * kStageQ;
-                    if (leader) {
+                    if (dm::elect_one()) {
 #pragma unroll
                         for (int hh = 0; hh < kDH; ++hh) {
 #pragma unroll
@@ -258,12 +257,12 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                     const int t = gt + it, st = t % kStages, par = t & 1, pp = (t >> 1) & 1;
                     dm::mbar_wait(&s.bar_codes[t & 1], (t >> 1) & 1, wc);
                     // every softmax warp is past the row constants of this m-block: their ring slot may be refilled
-                    if (leader) dm::mbar_arrive(&s.bar_rows_free[t % 3]);
+                    if (dm::elect_one()) dm::mbar_arrive(&s.bar_rows_free[t % 3]);
                     if (t >= 1) dm::mbar_wait(&s.bar_dkv_free, (t - 1) & 1, wc);
                     dm::tc_fence_after();
                     const uint32_t qs = q_lo + st * kStageQ + zh * kSubQ, dos = do_lo + st * kStageQ + zh * kSubQ;
                     const uint32_t pa = pt_lo + 4 * par, da = ds_lo + pp * kSub + 4 * par;
-                    if (leader) {
+                    if (dm::elect_one()) {
                         // head_dim 128: dV_tmp accumulates the two m-blocks of a 128-row dO scale block; head_dim 256: one m-block
                         dm::umma_e4m3_lo_rt(t_dv, pa, dos, idesc_dkv, (kD == 128 && par != 0) ? 1u : 0u);
                         dm::umma_e4m3_lo<true>(t_dv, pa + 2, dos + 256, idesc_dkv);
@@ -288,7 +287,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             if (gt > 0) {
                 // the last products: wait so shared memory stays valid until the tensor pipe has read it
                 dm::mbar_wait(&s.bar_dkv_free, (gt - 1) & 1, wc);
-                if (leader) dm::tma_store_wait_all0();
+                if (dm::elect_one()) dm::tma_store_wait_all0();
             }
         } else if (warp == kSoftmaxWarps + 6) {
             // ---- TMA loads: an item's K / V once the previous item's last S^T / dP^T have read theirs, then the Q8 / dO8
@@ -301,7 +300,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                 const int q_row0 = w.hc.bh * p.rm.nq + w.m_lo * 64;
                 if (w.n_it > 0) {
                     if (kvn >= 1) dm::mbar_wait(&s.bar_kv_free, (kvn - 1) & 1, wc);
-                    if (leader) {
+                    if (dm::elect_one()) {
                         dm::mbar_expect_tx(&s.bar_kv, 2 * kDH * kTile);
                         for (int hh = 0; hh < kDH; ++hh) {
                             dm::tma_load_2d(s.k[hh], &tm_k, 128 * hh, kv_row0, &s.bar_kv);
@@ -313,7 +312,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                 for (int it = 0; it < w.n_it; ++it) {
                     const int t = gt + it, st = t % kStages;
                     if (t >= kStages) dm::mbar_wait(&s.bar_stage_free[st], (t / kStages - 1) & 1, wc);
-                    if (leader) {
+                    if (dm::elect_one()) {
                         dm::mbar_expect_tx(&s.bar_qdo[st], 2 * kDH * kHalf);
 #pragma unroll
                         for (int hh = 0; hh < kDH; ++hh) {
@@ -350,7 +349,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                         *reinterpret_cast<float2*>(&s.dlk[slot][gq][2 * lane]) = make_float2(-(d2.x * kk[gq]), -(d2.y * kk[gq]));
                     if (lane < 2) s.sc[slot][lane] = sc_v;
                     __syncwarp();
-                    if (leader) dm::mbar_arrive(&s.bar_rows_full[slot]);
+                    if (dm::elect_one()) dm::mbar_arrive(&s.bar_rows_full[slot]);
                 }
                 gt += w.n_it;
             }

@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kThreads128, 1)
 bwd2_d128_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_k, const Bwd2Params p) {
     extern __shared__ uint8_t smem_raw[];
     Bwd2Smem& s = *reinterpret_cast<Bwd2Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int nbn = p.N / 128;
     const int nq_blk = p.rm.nq / 128, nbm_l = p.rm.nq / 64;
     dm::WaitCtx wc{&s.abort_flag, p.status};
@@ -103,7 +103,6 @@ bwd2_d128_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
 
     if (warp == 8) {
         // ---- TMA loads
-        const bool leader = lane == 0;
         int gt = 0;
         for (int r = 0;; ++r) {
             const Bwd2Item w = bwd2_item(p, r);
@@ -113,7 +112,7 @@ bwd2_d128_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
             for (int it = 0; it < w.n_it; ++it) {
                 const int t = gt + it, st = t % kRing;
                 if (t >= kRing) dm::mbar_wait(&s.bar_free[st], (t / kRing - 1) & 1, wc);
-                if (leader) {
+                if (dm::elect_one()) {
                     dm::mbar_expect_tx(&s.bar_ld[st], 2 * kTile);
                     dm::tma_load_2d(s.a[st], &tm_ds, 0, (int)((tile0 + it) * 128), &s.bar_ld[st]);
                     dm::tma_load_2d(s.b[st], &tm_k, 0, kv_row0 + it * 128, &s.bar_ld[st]);
@@ -124,7 +123,6 @@ bwd2_d128_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
         }
     } else if (warp == 9) {
         // ---- MMA issue: both operands MN-major, one K step = 32 tile rows = 4096 bytes
-        const bool leader = lane == 0;
         constexpr uint32_t idesc = dm::idesc_e4m3(128, 128, true, true);
         constexpr uint32_t kSub = kTile >> 4;
         const uint32_t a_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.a[0])), b_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.b[0]));
@@ -138,7 +136,7 @@ bwd2_d128_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
                 if (t >= kAcc) dm::mbar_wait(&s.bar_acc_free[b], (t / kAcc - 1) & 1, wc);
                 dm::tc_fence_after();
                 const uint32_t aa = a_lo + st * kSub, ba = b_lo + st * kSub, d = tmem + b * 128;
-                if (leader) {
+                if (dm::elect_one()) {
                     dm::umma_e4m3_lo<false>(d, aa, ba, idesc);
 #pragma unroll
                     for (int k = 1; k < 4; ++k) dm::umma_e4m3_lo<true>(d, aa + 256 * k, ba + 256 * k, idesc);
@@ -238,7 +236,7 @@ __global__ void __launch_bounds__(256, 1)
 bwd2_d256_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_k, const Bwd2Params p) {
     extern __shared__ uint8_t smem_raw[];
     Bwd2Smem256& s = *reinterpret_cast<Bwd2Smem256*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = warp >> 2;                           // d half
     const int row = (warp & 3) * 32 + lane;
     const dm::HeadCoord hc = dm::head_coord(blockIdx.x, p.h0, p.hcount, p.H, p.Hk);
@@ -275,19 +273,22 @@ bwd2_d256_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
         const int st = it % kStages;
         dm::mbar_wait(&s.bar_ld[st], (it / kStages) & 1, wc);
         dm::tc_fence_after();
-        const uint64_t ad = dm::smem_desc_sw128(dm::smem_u32(s.a[st]));
+        const uint32_t ad = dm::smem_desc_lo_sw128(dm::smem_u32(s.a[st]));
 #pragma unroll
         for (int kh = 0; kh < 2; ++kh)
 #pragma unroll
             for (int dh = 0; dh < 2; ++dh) {
-                const uint64_t bd = dm::smem_desc_sw128(dm::smem_u32(s.b[st][dh]));
+                const uint32_t bd = dm::smem_desc_lo_sw128(dm::smem_u32(s.b[st][dh]));
 #pragma unroll
-                for (int k2 = 0; k2 < 2; ++k2)
-                    dm::umma_e4m3(tmem + kh * 256 + dh * 128, ad + 256 * (2 * kh + k2), bd + 256 * (2 * kh + k2), idesc, k2 > 0);
+                for (int k2 = 0; k2 < 2; ++k2) {
+                    const uint32_t a = ad + 256 * (2 * kh + k2), b = bd + 256 * (2 * kh + k2), d = tmem + kh * 256 + dh * 128;
+                    if (k2 == 0) dm::umma_e4m3_lo<false>(d, a, b, idesc);
+                    else dm::umma_e4m3_lo<true>(d, a, b, idesc);
+                }
             }
         dm::umma_commit(&s.bar_mma);
     };
-    if (tid == 0) {
+    if (warp == 0 && dm::elect_one()) {
         for (int i = 0; i < kStages && i < n_it; ++i) load(i);
         issue(0);
     }
@@ -303,7 +304,7 @@ bwd2_d256_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
         const float psi2[2] = {psi_row[2 * it], psi_row[2 * it + 1]};
         dm::mbar_wait(&s.bar_mma, it & 1, wc);
         dm::tc_fence_after();
-        if (tid == 0 && it + kStages < n_it) load(it + kStages);
+        if (warp == 0 && it + kStages < n_it && dm::elect_one()) load(it + kStages);
 #pragma unroll
         for (int kh = 0; kh < 2; ++kh) {
             const float psi_cur = psi2[kh];
@@ -322,7 +323,7 @@ bwd2_d256_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
         }
         dm::tc_fence_before();
         __syncthreads();
-        if (tid == 0 && it + 1 < n_it) issue(it + 1);
+        if (warp == 0 && it + 1 < n_it && dm::elect_one()) issue(it + 1);
     }
 
     const int n_glob = rb * 128 + row;

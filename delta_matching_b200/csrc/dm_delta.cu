@@ -59,7 +59,7 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     extern __shared__ uint8_t smem_raw[];
     constexpr int kDH = kD / 128;
     DeltaSmem<kD>& s = *reinterpret_cast<DeltaSmem<kD>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = warp >> 2;
     const int row = (warp & 3) * 32 + lane;
     const dm::HeadCoord hc = dm::head_coord(blockIdx.x, p.h0, p.hcount, p.H, p.Hk);
@@ -104,20 +104,26 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
         const uint32_t t_s = tmem, t_dp = t_s + 128;
 #pragma unroll
         for (int hh = 0; hh < kDH; ++hh) {
-            const uint64_t qd = dm::smem_desc_sw128(dm::smem_u32(s.q[hh])), kd = dm::smem_desc_sw128(dm::smem_u32(s.k[st][hh]));
+            const uint32_t qd = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[hh])), kd = dm::smem_desc_lo_sw128(dm::smem_u32(s.k[st][hh]));
 #pragma unroll
-            for (int k = 0; k < 4; ++k) dm::umma_e4m3(t_s, qd + 2 * k, kd + 2 * k, idesc, (hh | k) != 0);
+            for (int k = 0; k < 4; ++k) {
+                if ((hh | k) == 0) dm::umma_e4m3_lo<false>(t_s, qd, kd, idesc);
+                else dm::umma_e4m3_lo<true>(t_s, qd + 2 * k, kd + 2 * k, idesc);
+            }
         }
 #pragma unroll
         for (int hh = 0; hh < kDH; ++hh) {
-            const uint64_t dd = dm::smem_desc_sw128(dm::smem_u32(s.dO[hh])), vd = dm::smem_desc_sw128(dm::smem_u32(s.v[st][hh]));
+            const uint32_t dd = dm::smem_desc_lo_sw128(dm::smem_u32(s.dO[hh])), vd = dm::smem_desc_lo_sw128(dm::smem_u32(s.v[st][hh]));
 #pragma unroll
-            for (int k = 0; k < 4; ++k) dm::umma_e4m3(t_dp, dd + 2 * k, vd + 2 * k, idesc, (hh | k) != 0);
+            for (int k = 0; k < 4; ++k) {
+                if ((hh | k) == 0) dm::umma_e4m3_lo<false>(t_dp, dd, vd, idesc);
+                else dm::umma_e4m3_lo<true>(t_dp, dd + 2 * k, vd + 2 * k, idesc);
+            }
         }
         dm::umma_commit(&s.bar_mma[0]);
     };
 
-    if (tid == 0) {
+    if (warp == 0 && dm::elect_one()) {
         dm::mbar_expect_tx(&s.bar_qdo, 2 * kDH * kTile);
         for (int hh = 0; hh < kDH; ++hh) {
             dm::tma_load_2d(s.q[hh], &tm_q, 128 * hh, q_row0, &s.bar_qdo);
@@ -191,7 +197,7 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
         }
         dm::tc_fence_before();
         __syncthreads();                       // S | dP have been read; stage `st` tiles are free
-        if (tid == 0) {
+        if (warp == 0 && dm::elect_one()) {
             if (it + 1 < n_tiles) issue(it + 1);
             if (it + 2 < n_tiles) load_kv(it + 2);
         }

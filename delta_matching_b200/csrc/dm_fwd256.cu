@@ -47,7 +47,7 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 const __grid_constant__ CUtensorMap tm_v, const Fwd256Params p) {
     extern __shared__ uint8_t smem_raw[];
     Fwd256Smem& s = *reinterpret_cast<Fwd256Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = warp >> 2;
     const int row = (warp & 3) * 32 + lane;
     const dm::HeadCoord hc = dm::head_coord(blockIdx.x, p.h0, p.hcount, p.H, p.Hk);
@@ -91,14 +91,17 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         dm::tc_fence_after();
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
-            const uint64_t qd = dm::smem_desc_sw128(dm::smem_u32(s.q[hh])), kd = dm::smem_desc_sw128(dm::smem_u32(s.k[st][hh]));
+            const uint32_t qd = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[hh])), kd = dm::smem_desc_lo_sw128(dm::smem_u32(s.k[st][hh]));
 #pragma unroll
-            for (int k = 0; k < 4; ++k) dm::umma_e4m3(t_s, qd + 2 * k, kd + 2 * k, idesc_s, (hh | k) != 0);
+            for (int k = 0; k < 4; ++k) {
+                if ((hh | k) == 0) dm::umma_e4m3_lo<false>(t_s, qd, kd, idesc_s);
+                else dm::umma_e4m3_lo<true>(t_s, qd + 2 * k, kd + 2 * k, idesc_s);
+            }
         }
         dm::umma_commit(&s.bar_s);
     };
 
-    if (tid == 0) {
+    if (warp == 0 && dm::elect_one()) {
         dm::mbar_expect_tx(&s.bar_q, 2 * kTile);
         dm::tma_load_2d(s.q[0], &tm_q, 0, q_row0, &s.bar_q);
         dm::tma_load_2d(s.q[1], &tm_q, 128, q_row0, &s.bar_q);
@@ -159,7 +162,7 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         __syncthreads();
         // every thread holds its scores: S of the next tile may overwrite the buffer, under pass B and the products
-        if (tid == 0 && it + 1 < n_tiles) issue_s(it + 1);
+        if (warp == 0 && it + 1 < n_tiles && dm::elect_one()) issue_s(it + 1);
         const float tile_max = fmaxf(fmaxf(s.gmax[0][row], s.gmax[1][row]), fmaxf(s.gmax[2][row], s.gmax[3][row]));
         const float m_new = fmaxf(m_run, tile_max);
         const float m_cur = (m_new == -INFINITY) ? 0.f : m_new;
@@ -205,15 +208,15 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // while thread 0 issues the next group's products, so those form under the additions instead of after them.
         auto issue_pv = [&](int grp) {   // thread 0 only
             dm::tc_fence_after();
-            const uint64_t pd = dm::smem_desc_sw128(dm::smem_u32(s.p)) + 2 * grp;      // 32 bytes of keys per group
+            const uint32_t pd = dm::smem_desc_lo_sw128(dm::smem_u32(s.p)) + 2 * grp;      // 32 bytes of keys per group
 #pragma unroll
             for (int dh = 0; dh < 2; ++dh) {
-                const uint64_t vd = dm::smem_desc_sw128(dm::smem_u32(s.v[st][dh])) + 256 * grp;   // 32 key rows = 4096 bytes
-                dm::umma_e4m3(t_d + 128 * dh, pd, vd, idesc_pv, 0);
+                const uint32_t vd = dm::smem_desc_lo_sw128(dm::smem_u32(s.v[st][dh])) + 256 * grp;   // 32 key rows = 4096 bytes
+                dm::umma_e4m3_lo<false>(t_d + 128 * dh, pd, vd, idesc_pv);
             }
             dm::umma_commit(&s.bar_d);
         };
-        if (tid == 0) issue_pv(0);
+        if (warp == 0 && dm::elect_one()) issue_pv(0);
 #pragma unroll 1
         for (int grp = 0; grp < 4; ++grp) {
             dm::mbar_wait(&s.bar_d, d_phase & 1, wc);
@@ -240,11 +243,11 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             dm::tmem_ld_wait();
             dm::tc_fence_before();
             __syncthreads();                               // every thread holds its last two pieces: the buffer is free
-            if (tid == 0 && grp < 3) issue_pv(grp + 1);
+            if (warp == 0 && grp < 3 && dm::elect_one()) issue_pv(grp + 1);
             add32(2, sa);
             add32(3, sb);
         }
-        if (tid == 0 && it + 2 < n_tiles) load_kv(it + 2);
+        if (warp == 0 && it + 2 < n_tiles && dm::elect_one()) load_kv(it + 2);
     }
 
     // ---- epilogue

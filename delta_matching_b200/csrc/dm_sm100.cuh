@@ -85,6 +85,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
     return mbar_wait_limit(bar, parity, ctx, DM_WAIT_LIMIT);
 }
 
+// One lane of a converged warp (always the same one).  Under this predicate the compiler knows that a single lane executes the
+// asynchronous instruction and feeds its descriptors from uniform registers; under `lane == 0` it cannot, and every
+// tcgen05.mma costs the issuing warp more.  Pass 1: 1268 -> 1211 us (B4 N4096 H32 Hk8 causal), 1638 -> 1418 us at head_dim 256
+// (B2 N4096 H16 Hk4 full); pass 2: 236 -> 225 us.  The forward and pass 0's role kernel, whose issuing warps wait most of
+// their time, did not gain and keep `lane == 0`.
+// A warp index taken through __shfl_sync tells the compiler the same about the role branch; it is used where it measured
+// faster (pass 2: 225 -> 217 us, forward at head_dim 256: 714 -> 699 us), not in pass 1 (1211 -> 1268 us).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok));
+    return ok != 0;
+}
+
 // Warp-level arrive: every lane has finished its part (the caller fences as needed), lane 0 arrives once for the warp.
 __device__ __forceinline__ void mbar_arrive_warp(uint64_t* bar) {
     __syncwarp();
