@@ -174,6 +174,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
     dm::tc_fence_before();
     __syncthreads();
     dm::tc_fence_after();
+    dm::pdl_wait();
     // tensor memory: S^T | dP^T at columns [0, 64) | [64, 128), dV product [128, 256), dK product [256, 384), dV accumulator
     // [384, 512)
     const uint32_t tmem = s.tmem_base;
@@ -741,8 +742,6 @@ extern "C" int dm_bwd_fp8_pass1_cp(const void* q8, const void* k8, const void* v
     if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
     const int64_t items = (int64_t)sh.B * hcount * (sh.N / 128) * (sh.D / 128);
     const int grid = (int)(items < sms ? items : sms);
-    if (sh.D == 128) bwd1_kernel<128><<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(tq, td, tk, tv, ts, p);
-    else bwd1_kernel<256><<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(tq, td, tk, tv, ts, p);
-    DM_CUDA(cudaGetLastError());
+    DM_CUDA(dmh::launch_pdl(sh.D == 128 ? bwd1_kernel<128> : bwd1_kernel<256>, grid, kThreads, smem, stream, tq, td, tk, tv, ts, p));
     return DM_OK;
 }

@@ -97,6 +97,7 @@ bwd2_d128_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
     dm::tc_fence_before();
     __syncthreads();
     dm::tc_fence_after();
+    dm::pdl_wait();
     const uint32_t tmem = s.tmem_base;
     // Every role walks the same item list; `gt` counts the key tiles of the items before the current one, so ring stages,
     // buffer indices and mbarrier phases run on across items (t = gt + it).
@@ -256,6 +257,7 @@ bwd2_d256_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
     dm::tc_fence_before();
     __syncthreads();
     dm::tc_fence_after();
+    dm::pdl_wait();
     const uint32_t tmem = s.tmem_base;
     const uint32_t lane_base = (uint32_t)(warp & 3) * 32;
     const int64_t tile0 = ((int64_t)bhl * nbn + rb) * nbn;
@@ -388,8 +390,7 @@ extern "C" int dm_bwd_fp8_pass2_cp(const void* ds8_ws, const float* psi_ws, cons
                  dm::make_fastdiv(sh.H / sh.Hk)};
     if (sh.D == 256) {
         const int smem = (int)sizeof(Bwd2Smem256) + 1024;
-        bwd2_d256_kernel<<<dim3(sh.B * hcount, sh.N / 128), 256, smem, static_cast<cudaStream_t>(stream)>>>(ts, tk, p);
-        DM_CUDA(cudaGetLastError());
+        DM_CUDA(dmh::launch_pdl(bwd2_d256_kernel, dim3(sh.B * hcount, sh.N / 128), 256, smem, stream, ts, tk, p));
         return DM_OK;
     }
     const int smem = (int)sizeof(Bwd2Smem) + 1024;
@@ -397,7 +398,6 @@ extern "C" int dm_bwd_fp8_pass2_cp(const void* ds8_ws, const float* psi_ws, cons
     if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
     const int64_t items = (int64_t)sh.B * hcount * (cp.nq / 128);
     const int grid = (int)(items < sms ? items : sms);
-    bwd2_d128_kernel<<<grid, kThreads128, smem, static_cast<cudaStream_t>(stream)>>>(ts, tk, p);
-    DM_CUDA(cudaGetLastError());
+    DM_CUDA(dmh::launch_pdl(bwd2_d128_kernel, grid, kThreads128, smem, stream, ts, tk, p));
     return DM_OK;
 }

@@ -83,6 +83,7 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     dm::tc_fence_before();
     __syncthreads();
     dm::tc_fence_after();
+    dm::pdl_wait();
     const uint32_t tmem = s.tmem_base;
     const uint32_t lane_base = (uint32_t)(warp & 3) * 32;
     const int q_row0 = hc.bh * p.rm.nq + li * 128;
@@ -296,6 +297,7 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     dm::tc_fence_before();
     __syncthreads();
     dm::tc_fence_after();
+    dm::pdl_wait();
     const uint32_t tmem = s.tmem_base;
     constexpr uint32_t kSub = kTile >> 4;
     // `gt` counts the key tiles of the items before the current one: ring stages, buffers and phases run on across items
@@ -477,13 +479,11 @@ int launch(const void* q8, const void* k8, const void* v8, const void* do8, cons
     if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
     if (!kDebug && kD == 128 && items >= 2 * (int64_t)sms && tiles >= 24 * (int64_t)sms) {
         const DeltaDivs fd{dm::make_fastdiv(sh.B * p.hcount), dm::make_fastdiv(p.hcount), dm::make_fastdiv(sh.H / sh.Hk)};
-        delta_roles_kernel<<<sms, kDzThreads, (int)sizeof(DeltaRolesSmem) + 1024, static_cast<cudaStream_t>(stream)>>>(tq, td, tk, tv, p, fd);
-        DM_CUDA(cudaGetLastError());
+        DM_CUDA(dmh::launch_pdl(delta_roles_kernel, sms, kDzThreads, sizeof(DeltaRolesSmem) + 1024, stream, tq, td, tk, tv, p, fd));
         return DM_OK;
     }
     const int smem = (int)sizeof(DeltaSmem<kD>) + 1024;
-    delta_kernel<kDebug, kD><<<dim3(sh.B * p.hcount, p.rm.nq / 128), 256, smem, static_cast<cudaStream_t>(stream)>>>(tq, td, tk, tv, p);
-    DM_CUDA(cudaGetLastError());
+    DM_CUDA(dmh::launch_pdl(delta_kernel<kDebug, kD>, dim3(sh.B * p.hcount, p.rm.nq / 128), 256, smem, stream, tq, td, tk, tv, p));
     return DM_OK;
 }
 

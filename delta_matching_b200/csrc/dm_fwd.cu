@@ -117,6 +117,7 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     dm::tc_fence_before();
     __syncthreads();
     dm::tc_fence_after();
+    dm::pdl_wait();
     const uint32_t tmem = s.tmem_base;
     const uint32_t t_d0 = tmem + 256, t_d1 = tmem + 384;      // S buffers at columns [0, 128) and [128, 256)
     const uint32_t lane_base = (uint32_t)(warp & 3) * 32;
@@ -498,7 +499,6 @@ extern "C" int dm_fwd_fp8_cp(const void* q8, const void* k8, const void* v8, con
     // persistent: one CTA per SM walks the (head, row block) items, heaviest first
     const int64_t items = (int64_t)sh.B * hcount * (cp.nq / 128);
     const int grid = (int)(items < sms ? items : sms);
-    fwd_d128_kernel<<<grid, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(tq, tk, tv, p);
-    DM_CUDA(cudaGetLastError());
+    DM_CUDA(dmh::launch_pdl(fwd_d128_kernel, grid, kThreads, smem, stream, tq, tk, tv, p));
     return DM_OK;
 }

@@ -69,6 +69,7 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     dm::tc_fence_before();
     __syncthreads();
     dm::tc_fence_after();
+    dm::pdl_wait();
     const uint32_t tmem = s.tmem_base;
     const uint32_t t_s = tmem, t_d = tmem + 128;          // S: 128 columns; D_grp: 256 columns
     const uint32_t lane_base = (uint32_t)(warp & 3) * 32;
@@ -296,8 +297,7 @@ int launch_fwd_d256(const void* q8, const void* k8, const void* v8, const float*
     Fwd256Params p{q8s, k8s, v8s, static_cast<__nv_bfloat16*>(o), lse, sh.H, sh.Hk, sh.N, h0, hcount, sh.causal, status};
     const int smem = (int)sizeof(Fwd256Smem) + 1024;
     if ((rc = prepare_fwd256(err, errlen))) return rc;
-    fwd_d256_kernel<<<dim3(sh.B * hcount, sh.N / 128), 256, smem, static_cast<cudaStream_t>(stream)>>>(tq, tk, tv, p);
-    DM_CUDA(cudaGetLastError());
+    DM_CUDA(launch_pdl(fwd_d256_kernel, dim3(sh.B * hcount, sh.N / 128), 256, smem, stream, tq, tk, tv, p));
     return DM_OK;
 }
 }  // namespace dmh

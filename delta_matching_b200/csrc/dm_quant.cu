@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "dm_host.h"
+#include "dm_launch.cuh"
 
 namespace {
 
@@ -75,11 +76,13 @@ __device__ __forceinline__ void kmean_partial_block(int xblk, int bh, const __nv
 template <int D>
 __global__ void __launch_bounds__(256) kmean_partial_kernel(const __nv_bfloat16* __restrict__ k, int64_t sb, int64_t sn, int64_t sh,
                                                             int Hk, int N, float* __restrict__ partials) {
+    dm::pdl_wait();
     kmean_partial_block<D>(blockIdx.x, blockIdx.y, k, sb, sn, sh, Hk, N, partials);
 }
 
 template <int D>
 __global__ void kmean_fold_kernel(const float* __restrict__ partials, int N, float* __restrict__ km) {
+    dm::pdl_wait();
     const int bh = blockIdx.x, d = threadIdx.x;
     const float* p = partials + (int64_t)bh * (N / 64) * D + d;
     float acc = 0.f;
@@ -249,6 +252,7 @@ __global__ void __launch_bounds__(256) quant_kernel(const __nv_bfloat16* __restr
                                                     const __nv_bfloat16* __restrict__ o, int64_t ob, int64_t on, int64_t oh,
                                                     const float* __restrict__ km, uint8_t* __restrict__ codes,
                                                     float* __restrict__ scales, float* __restrict__ delta, int heads, int N, float sm) {
+    dm::pdl_wait();
     quant_block<D, MODE>(blockIdx.x, blockIdx.y, x, sb, sn, sh, o, ob, on, oh, km, codes, scales, delta, heads, N, sm);
 }
 
@@ -259,6 +263,7 @@ template <int D>
 __global__ void __launch_bounds__(256) quant_k_folded_kernel(const __nv_bfloat16* __restrict__ x, int64_t sb, int64_t sn, int64_t sh,
                                                              const float* __restrict__ partials, float* __restrict__ km_out,
                                                              uint8_t* __restrict__ codes, float* __restrict__ scales, int heads, int N) {
+    dm::pdl_wait();
     __shared__ float s_km[D];
     const int bh = blockIdx.y;
     if (threadIdx.x < D) {
@@ -287,6 +292,7 @@ struct PrologueArgs {
 };
 template <int D>
 __global__ void __launch_bounds__(256) prologue_kernel(const PrologueArgs a) {
+    dm::pdl_wait();
     int i = blockIdx.x;
     if (i < a.n_p) {
         kmean_partial_block<D>(i % a.pbx, i / a.pbx, a.k, a.ks.b, a.ks.n, a.ks.h, a.Hk, a.N, a.partials);
@@ -305,6 +311,7 @@ __global__ void __launch_bounds__(256) prologue_kernel(const PrologueArgs a) {
 // blockIdx.y picks one of up to two (input, output) pairs of the same shape: dK and dV of a backward fold in one launch.
 __global__ void __launch_bounds__(256) gqa_fold_kernel(const uint4* __restrict__ x0, uint4* __restrict__ out0, const uint4* __restrict__ x1,
                                                        uint4* __restrict__ out1, int64_t total_vec, int H, int Hk, int D) {
+    dm::pdl_wait();
     const uint4* __restrict__ x = blockIdx.y ? x1 : x0;
     uint4* __restrict__ out = blockIdx.y ? out1 : out0;
     const int vpr = D / 8;                                   // 16-byte vectors per head row
@@ -371,11 +378,11 @@ extern "C" int dm_kmean(const void* k, DmStrides ks, int32_t B, int32_t Hk, int3
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const __nv_bfloat16* kp = static_cast<const __nv_bfloat16*>(k);
     if (D == 128) {
-        kmean_partial_kernel<128><<<dim3(N / 64 / 4, B * Hk), 256, 0, st>>>(kp, ks.b, ks.n, ks.h, Hk, N, partials);
-        kmean_fold_kernel<128><<<B * Hk, 128, 0, st>>>(partials, N, km);
+        DM_CUDA(dmh::launch_pdl(kmean_partial_kernel<128>, dim3(N / 64 / 4, B * Hk), 256, 0, stream, kp, ks.b, ks.n, ks.h, Hk, N, partials));
+        DM_CUDA(dmh::launch_pdl(kmean_fold_kernel<128>, B * Hk, 128, 0, stream, partials, N, km));
     } else {
-        kmean_partial_kernel<256><<<dim3(N / 64 / 2, B * Hk), 256, 0, st>>>(kp, ks.b, ks.n, ks.h, Hk, N, partials);
-        kmean_fold_kernel<256><<<B * Hk, 256, 0, st>>>(partials, N, km);
+        DM_CUDA(dmh::launch_pdl(kmean_partial_kernel<256>, dim3(N / 64 / 2, B * Hk), 256, 0, stream, kp, ks.b, ks.n, ks.h, Hk, N, partials));
+        DM_CUDA(dmh::launch_pdl(kmean_fold_kernel<256>, B * Hk, 256, 0, stream, partials, N, km));
     }
     DM_CUDA(cudaGetLastError());
     return DM_OK;
@@ -407,10 +414,7 @@ extern "C" int dm_quant_qv_kpartials(const void* q, DmStrides qs, const void* k,
     a.sm = s.D == 128 ? 0.08838834764831845f : 0.0625f;
     const int64_t total = (int64_t)a.n_p + a.n_q + (int64_t)a.vbx * s.B * s.Hk;
     DM_REQUIRE(total < ((int64_t)1 << 31), DM_ERR_ARG, "problem too large for one launch");
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (s.D == 128) prologue_kernel<128><<<(unsigned)total, 256, 0, st>>>(a);
-    else prologue_kernel<256><<<(unsigned)total, 256, 0, st>>>(a);
-    DM_CUDA(cudaGetLastError());
+    DM_CUDA(dmh::launch_pdl(s.D == 128 ? prologue_kernel<128> : prologue_kernel<256>, (unsigned)total, 256, 0, stream, a));
     return DM_OK;
 }
 
@@ -426,8 +430,8 @@ extern "C" int dm_kmean_partials(const void* k, DmStrides ks, int32_t B, int32_t
     if ((rc = check_strides(k, ks, D, "k", err, errlen))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const __nv_bfloat16* kp = static_cast<const __nv_bfloat16*>(k);
-    if (D == 128) kmean_partial_kernel<128><<<dim3(N / 64 / 4, B * Hk), 256, 0, st>>>(kp, ks.b, ks.n, ks.h, Hk, N, partials);
-    else kmean_partial_kernel<256><<<dim3(N / 64 / 2, B * Hk), 256, 0, st>>>(kp, ks.b, ks.n, ks.h, Hk, N, partials);
+    if (D == 128) DM_CUDA(dmh::launch_pdl(kmean_partial_kernel<128>, dim3(N / 64 / 4, B * Hk), 256, 0, stream, kp, ks.b, ks.n, ks.h, Hk, N, partials));
+    else DM_CUDA(dmh::launch_pdl(kmean_partial_kernel<256>, dim3(N / 64 / 2, B * Hk), 256, 0, stream, kp, ks.b, ks.n, ks.h, Hk, N, partials));
     DM_CUDA(cudaGetLastError());
     return DM_OK;
 }
@@ -438,10 +442,7 @@ extern "C" int dm_kmean_fold(const float* partials, int32_t B, int32_t Hk, int32
     if (rc) return rc;
     if ((rc = dmh::check_device_ptr(partials, "partials", err, errlen))) return rc;
     if ((rc = dmh::check_device_ptr(km, "km", err, errlen))) return rc;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (D == 128) kmean_fold_kernel<128><<<B * Hk, 128, 0, st>>>(partials, N, km);
-    else kmean_fold_kernel<256><<<B * Hk, 256, 0, st>>>(partials, N, km);
-    DM_CUDA(cudaGetLastError());
+    DM_CUDA(dmh::launch_pdl(D == 128 ? kmean_fold_kernel<128> : kmean_fold_kernel<256>, B * Hk, D, 0, stream, partials, N, km));
     return DM_OK;
 }
 
@@ -551,9 +552,8 @@ static void launch_quant(const void* x, DmStrides xs, const void* o, DmStrides o
                          float* delta, int B, int heads, int N, cudaStream_t st) {
     constexpr int BLK = (MODE == 1 || MODE == 2) ? (D == 128 ? 64 : 32) : (D == 128 ? 128 : 64);
     const float sm = D == 128 ? 0.08838834764831845f : 0.0625f;
-    quant_kernel<D, MODE><<<dim3(N / BLK, B * heads), 256, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(x), xs.b, xs.n, xs.h, static_cast<const __nv_bfloat16*>(o), os.b, os.n, os.h, km,
-        static_cast<uint8_t*>(codes), scales, delta, heads, N, sm);
+    dmh::launch_pdl(quant_kernel<D, MODE>, dim3(N / BLK, B * heads), 256, 0, st, static_cast<const __nv_bfloat16*>(x), xs.b, xs.n, xs.h,
+                    static_cast<const __nv_bfloat16*>(o), os.b, os.n, os.h, km, static_cast<uint8_t*>(codes), scales, delta, heads, N, sm);
 }
 
 extern "C" int dm_quant(int32_t mode, const void* x, DmStrides xs, int32_t B, int32_t heads, int32_t N, int32_t D, const float* km,
@@ -593,9 +593,8 @@ int launch_kmean_fold_quant_k(const void* k, DmStrides ks, const float* partials
         if ((rc = check_device_ptr(ptrs[i], names[i], err, errlen))) return rc;
     if ((rc = check_strides(k, ks, s.D, "k", err, errlen))) return rc;
     DM_REQUIRE(aligned16(k8), DM_ERR_ARG, "codes is not 16-byte aligned");
-    quant_k_folded_kernel<128><<<dim3(s.N / 64, s.B * s.Hk), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(k), ks.b, ks.n, ks.h, partials, km, static_cast<uint8_t*>(k8), k8s, s.Hk, s.N);
-    DM_CUDA(cudaGetLastError());
+    DM_CUDA(launch_pdl(quant_k_folded_kernel<128>, dim3(s.N / 64, s.B * s.Hk), 256, 0, stream, static_cast<const __nv_bfloat16*>(k), ks.b, ks.n,
+                       ks.h, partials, km, static_cast<uint8_t*>(k8), k8s, s.Hk, s.N));
     return DM_OK;
 }
 }  // namespace dmh
@@ -643,9 +642,8 @@ int launch_gqa_fold(const void* x0, void* out0, const void* x1, void* out1, int 
     const int64_t total = (int64_t)B * N * Hk * (D / 8);
     int blocks = (int)((total + 255) / 256);
     if (blocks > 148 * 16) blocks = 148 * 16;
-    gqa_fold_kernel<<<dim3(blocks, x1 ? 2 : 1), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint4*>(x0), static_cast<uint4*>(out0), static_cast<const uint4*>(x1), static_cast<uint4*>(out1), total, H, Hk, D);
-    DM_CUDA(cudaGetLastError());
+    DM_CUDA(launch_pdl(gqa_fold_kernel, dim3(blocks, x1 ? 2 : 1), 256, 0, stream, static_cast<const uint4*>(x0), static_cast<uint4*>(out0),
+                       static_cast<const uint4*>(x1), static_cast<uint4*>(out1), total, H, Hk, D));
     return DM_OK;
 }
 }  // namespace dmh
@@ -704,11 +702,11 @@ extern "C" int dm_kmean_noalloc(const void* k, DmStrides ks, int32_t B, int32_t 
     // Every partial that the fold reads is written by the partial kernel of this same call first, so nothing in the
     // shared array has to start at zero; what the previous call left there is simply overwritten.
     if (D == 128) {
-        kmean_partial_kernel<128><<<dim3(N / 64 / 4, B * Hk), 256, 0, st>>>(kp, ks.b, ks.n, ks.h, Hk, N, partials);
-        kmean_fold_kernel<128><<<B * Hk, 128, 0, st>>>(partials, N, km);
+        DM_CUDA(dmh::launch_pdl(kmean_partial_kernel<128>, dim3(N / 64 / 4, B * Hk), 256, 0, stream, kp, ks.b, ks.n, ks.h, Hk, N, partials));
+        DM_CUDA(dmh::launch_pdl(kmean_fold_kernel<128>, B * Hk, 128, 0, stream, partials, N, km));
     } else {
-        kmean_partial_kernel<256><<<dim3(N / 64 / 2, B * Hk), 256, 0, st>>>(kp, ks.b, ks.n, ks.h, Hk, N, partials);
-        kmean_fold_kernel<256><<<B * Hk, 256, 0, st>>>(partials, N, km);
+        DM_CUDA(dmh::launch_pdl(kmean_partial_kernel<256>, dim3(N / 64 / 2, B * Hk), 256, 0, stream, kp, ks.b, ks.n, ks.h, Hk, N, partials));
+        DM_CUDA(dmh::launch_pdl(kmean_fold_kernel<256>, B * Hk, 256, 0, stream, partials, N, km));
     }
     DM_CUDA(cudaGetLastError());
     return DM_OK;

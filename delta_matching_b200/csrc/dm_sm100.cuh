@@ -16,6 +16,8 @@
 #include <cuda_fp8.h>
 #include <stdint.h>
 
+#include "dm_launch.cuh"
+
 namespace dm {
 
 #ifndef DM_WAIT_LIMIT
