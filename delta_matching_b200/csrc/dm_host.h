@@ -8,6 +8,7 @@
 #include <stdio.h>
 #include <stdarg.h>
 #include <string.h>
+#include <atomic>
 #include <mutex>
 
 #include "../../include/dm_b200.h"
@@ -39,8 +40,21 @@ inline int fail(char* err, size_t errlen, int code, const char* fmt, ...) {
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// A composite entry point (dm_compose.cu) checks its caller's pointers once and asks for the current device once; the entry
+// points it chains, entered inside the scope, skip both (each asked the driver eight to fourteen times before).
+struct CallScope {
+    static thread_local int device;       // -1 outside a scope
+    int outer;
+    explicit CallScope(int dev) : outer(device) { device = dev; }
+    ~CallScope() { device = outer; }
+    static bool active() { return device >= 0; }
+};
+// The current device: the scope's, else the runtime's.
+int current_device(int* dev, char* err, size_t errlen);
+
 // Requires the pointer to be device-accessible memory on the current device (rejects host pointers before any launch).
 int check_device_ptr(const void* p, const char* name, char* err, size_t errlen);
+int check_device_ptr_on(const void* p, const char* name, int dev, char* err, size_t errlen);      // with the current device at hand
 
 // 2-D uint8 tensor map: `rows` rows of `row_bytes` bytes (pitch = row_bytes), boxes of box_rows x 128 bytes, 128-byte swizzle.
 int make_tmap_u8(CUtensorMap* out, const void* base, uint64_t row_bytes, uint64_t rows, uint32_t box_rows, char* err, size_t errlen);
@@ -57,16 +71,17 @@ bool register_pool_ok(int compiled_regs_per_thread, int threads, int regs_needed
 // that device current, the first time an entry point that needs it is called there (or from dm_init).
 struct DeviceOnce {
     std::mutex mu;
-    bool done[64] = {};
+    std::atomic<bool> done[64] = {};
 };
 template <class F>
 int device_once(DeviceOnce& o, char* err, size_t errlen, F&& f) {
     int dev = 0;
-    DM_CUDA(cudaGetDevice(&dev));
+    if (int rc = current_device(&dev, err, errlen)) return rc;
+    if (dev >= 0 && dev < 64 && o.done[dev].load(std::memory_order_acquire)) return DM_OK;
     std::lock_guard<std::mutex> lk(o.mu);
-    if (dev >= 0 && dev < 64 && o.done[dev]) return DM_OK;
+    if (dev >= 0 && dev < 64 && o.done[dev].load(std::memory_order_relaxed)) return DM_OK;
     if (int rc = f()) return rc;
-    if (dev >= 0 && dev < 64) o.done[dev] = true;
+    if (dev >= 0 && dev < 64) o.done[dev].store(true, std::memory_order_release);
     return DM_OK;
 }
 // Number of SMs of the current device (cached per device).
