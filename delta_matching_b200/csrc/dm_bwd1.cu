@@ -26,8 +26,7 @@
 //                                  (columns [384, 512)); the fold warps read product and accumulator, add, and store it back
 // Q8 / dO8 m-block tiles serve twice: K-major as the B operand of S^T / dP^T and MN-major as the B operand of dK / dV.
 // The dS' tile layout in global memory is [key][row] (128 x 128 bytes), which pass 2 reads as an MN-major A operand.
-#include "dm_attn_common.cuh"
-#include "dm_host.h"
+#include "dm_bwd1.h"
 
 namespace dmh {
 int check_shape(const DmShape& s, int h0, int hcount, char* err, size_t errlen);
@@ -76,65 +75,11 @@ struct Bwd1Smem {
     int abort_flag;
 };
 
-struct Bwd1Params {
-    const float* q8s;
-    const float* k8s;
-    const float* v8s;
-    const float* do8s;
-    const float* lse;
-    const float* delta;
-    __nv_bfloat16* dk;
-    __nv_bfloat16* dv;
-    uint8_t* ds_ws;
-    float* psi;
-    int H, Hk, N, h0, hcount, causal;
-    int* status;
-    dm::RowMap rm;                                // which rows of the sequence the Q-side tensors hold
-    int out_fp32;                                 // dK / dV leave as fp32 (partials that another rank's are added to)
-    int n_heads;                                  // batch * hcount: (batch, query head) pairs of this call
-    dm::FastDiv fd_heads, fd_hcount, fd_rep, fd_nbn;   // divisions by n_heads, hcount, H / Hk and N / 128
-};
-
-// The work list: one item = one 128-key block J of one (batch, query head) (and one d half at head_dim 256), ordered by
-// key block, i.e. heaviest first when causal.  CTA c takes position c of the even rounds and G - 1 - c of the odd ones
-// (a snake), so the long and the short items of a round pair up.
-struct Bwd1Item {
-    dm::HeadCoord hc;
-    int J, zh, m_lo, n_it, bhl;
-    bool valid;
-};
-template <int kD>
-__device__ __forceinline__ Bwd1Item bwd1_item(const Bwd1Params& p, int round) {
-    Bwd1Item w;
-    const int G = gridDim.x, c = blockIdx.x;
-    const int nbn = p.N / 128;
-    const int idx = round * G + ((round & 1) ? G - 1 - c : c);
-    w.valid = idx < p.n_heads * nbn * (kD / 128);
-    const int jz = (int)dm::fdiv((uint32_t)idx, p.fd_heads);
-    w.hc = dm::head_coord(idx - jz * p.n_heads, p.h0, p.fd_hcount, p.H, p.Hk, p.fd_rep);
-    w.bhl = w.hc.b * p.hcount + (w.hc.h - p.h0);
-    w.zh = kD == 128 ? 0 : (int)dm::fdiv((uint32_t)jz, p.fd_nbn);   // d half whose dK / dV columns the item keeps
-    w.J = jz - w.zh * nbn;
-    // m-blocks are counted in the local rows; global position grows with the local index, and both chunks of a row map
-    // start on a 128-row pair, so local and global m-block parity agree.  Causal: start at the first local m-block that is
-    // not wholly above the diagonal of key block J; a rank may hold none (n_it == 0: dK = dV = 0 for this block).
-    const int nq_blk = p.rm.nq / 128, nbm = p.rm.nq / 64;
-    w.m_lo = 0;
-    if (p.causal) {
-        const int rest = nq_blk - p.rm.half;
-        if (w.J < p.rm.off0 + p.rm.half) w.m_lo = 2 * max(w.J - p.rm.off0, 0);
-        else if (w.J < p.rm.off1 + rest) w.m_lo = 2 * (p.rm.half + max(w.J - p.rm.off1, 0));
-        else w.m_lo = nbm;
-    }
-    w.n_it = nbm - w.m_lo;
-    return w;
-}
-
 template <int kD>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                 const __grid_constant__ CUtensorMap tm_ds, const Bwd1Params p) {
+                 const __grid_constant__ CUtensorMap tm_ds, const dm::Bwd1Params p) {
     extern __shared__ uint8_t smem_raw[];
     using G = Geo<kD>;
     constexpr int kDH = G::kDH, kStages = G::kStages, kGrp = G::kGrp, kKPS = G::kKeysPerScale;
@@ -196,7 +141,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             const uint32_t q_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[0][0])), do_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.dO[0][0]));
             int gt = 0, kvn = 0;
             for (int r = 0;; ++r) {
-                const Bwd1Item w = bwd1_item<kD>(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
                 if (!w.valid) break;
                 if (w.n_it > 0) dm::mbar_wait(&s.bar_kv, kvn & 1, wc);
                 for (int it = 0; it < w.n_it; ++it) {
@@ -251,7 +196,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             const uint32_t pt_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.pt)), ds_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.ds[0]));
             int gt = 0;
             for (int r = 0;; ++r) {
-                const Bwd1Item w = bwd1_item<kD>(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
                 if (!w.valid) break;
                 const int zh = w.zh;
                 const int ds_row0 = (int)((((int64_t)w.bhl * nq_blk + (w.m_lo >> 1)) * nbn + w.J) * 128);   // dS' tile of the first row pair
@@ -296,7 +241,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             // tiles of its m-blocks as far ahead as the ring allows
             int gt = 0, kvn = 0;
             for (int r = 0;; ++r) {
-                const Bwd1Item w = bwd1_item<kD>(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
                 if (!w.valid) break;
                 const int kv_row0 = w.hc.bhk * p.N + w.J * 128;
                 const int q_row0 = w.hc.bh * p.rm.nq + w.m_lo * 64;
@@ -332,7 +277,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             const int nsq = kD == 128 ? nq_blk : nbm;
             int gt = 0;
             for (int r = 0;; ++r) {
-                const Bwd1Item w = bwd1_item<kD>(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
                 if (!w.valid) break;
                 float kk[kGrp];
 #pragma unroll
@@ -361,7 +306,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         dm::reg_inc<184>();
         int gt = 0;
         for (int r = 0;; ++r) {
-        const Bwd1Item w = bwd1_item<kD>(p, r);
+        const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
         if (!w.valid) break;
         const int J = w.J, zh = w.zh, n_it = w.n_it;
         const dm::HeadCoord hc = w.hc;
@@ -540,7 +485,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         const int kgrp = key / kKPS;                  // K / V scale group inside the block
         int gt = 0;
         for (int r = 0;; ++r) {
-        const Bwd1Item w = bwd1_item<kD>(p, r);
+        const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
         if (!w.valid) break;
         // few values live across the m-block loop (these warps run on 64 registers): the item's psi column as a pointer,
         // and whether its first row pair is the diagonal block of this key block (it is the first one of the causal loop)
@@ -668,16 +613,18 @@ int check_cp(const DmShape& s, const DmCp& cp, char* err, size_t errlen);
 }
 
 namespace dmh {
+int prepare_bwd1_d128(char* err, size_t errlen);
+int launch_bwd1_d128(const CUtensorMap& tq, const CUtensorMap& td, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ts,
+                     const dm::Bwd1Params& p, int grid, void* stream, char* err, size_t errlen);
 int prepare_bwd1(char* err, size_t errlen) {
     static DeviceOnce once;
     return device_once(once, err, errlen, [&]() -> int {
-        DM_CUDA(cudaFuncSetAttribute(bwd1_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Bwd1Smem<128>) + 1024));
         DM_CUDA(cudaFuncSetAttribute(bwd1_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Bwd1Smem<256>) + 1024));
         // setmaxnreg requests: 16 softmax warps keep 64, 4 fold warps take 184, 4 service warps keep 40
         constexpr int kPool = kComputeThreads * 64 + 128 * 184 + 128 * 40;
         static_assert(kPool == kThreads * 80, "the roles' register requests must add up to the launch pool");
-        if (int rc = check_register_pool((const void*)bwd1_kernel<128>, kThreads, kPool, err, errlen)) return rc;
-        return check_register_pool((const void*)bwd1_kernel<256>, kThreads, kPool, err, errlen);
+        if (int rc = check_register_pool((const void*)bwd1_kernel<256>, kThreads, kPool, err, errlen)) return rc;
+        return prepare_bwd1_d128(err, errlen);
     });
 }
 }  // namespace dmh
@@ -724,24 +671,25 @@ extern "C" int dm_bwd_fp8_pass1_cp(const void* q8, const void* k8, const void* v
     DM_REQUIRE(ntiles * 128 < ((uint64_t)1 << 31), DM_ERR_ARG, "dS' workspace too large for one call: split the heads (got %llu tiles)",
                (unsigned long long)ntiles);
     CUtensorMap tq, td, tk, tv, ts;
-    if ((rc = dmh::make_tmap_u8(&tq, q8, sh.D, (uint64_t)sh.B * sh.H * cp.nq, 64, err, errlen))) return rc;
-    if ((rc = dmh::make_tmap_u8(&td, do8, sh.D, (uint64_t)sh.B * sh.H * cp.nq, 64, err, errlen))) return rc;
+    if ((rc = dmh::make_tmap_u8(&tq, q8, sh.D, (uint64_t)sh.B * sh.H * cp.nq, sh.D == 128 ? 128 : 64, err, errlen))) return rc;
+    if ((rc = dmh::make_tmap_u8(&td, do8, sh.D, (uint64_t)sh.B * sh.H * cp.nq, sh.D == 128 ? 128 : 64, err, errlen))) return rc;
     if ((rc = dmh::make_tmap_u8(&tk, k8, sh.D, (uint64_t)sh.B * sh.Hk * sh.N, 128, err, errlen))) return rc;
     if ((rc = dmh::make_tmap_u8(&tv, v8, sh.D, (uint64_t)sh.B * sh.Hk * sh.N, 128, err, errlen))) return rc;
     if ((rc = dmh::make_tmap_u8(&ts, ds8_ws, 128, ntiles * 128, 128, err, errlen))) return rc;
     int* status = dmh::device_status_word(err, errlen);
     if (!status) return DM_ERR_CUDA;
-    Bwd1Params p{q8s, k8s, v8s, do8s, lse, delta, static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), static_cast<uint8_t*>(ds8_ws), psi_ws,
+    dm::Bwd1Params p{q8s, k8s, v8s, do8s, lse, delta, static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), static_cast<uint8_t*>(ds8_ws), psi_ws,
                  sh.H, sh.Hk, sh.N, h0, hcount, sh.causal, status, dm::RowMap{cp.nq, cp.half_blocks, cp.off0, cp.off1}, out_fp32,
                  sh.B * hcount, dm::make_fastdiv(sh.B * hcount), dm::make_fastdiv(hcount), dm::make_fastdiv(sh.H / sh.Hk),
                  dm::make_fastdiv(sh.N / 128)};
     // persistent: one CTA per SM walks the (key block, head[, d half]) items, heaviest first
     if ((rc = dmh::prepare_bwd1(err, errlen))) return rc;
-    const int smem = (int)(sh.D == 128 ? sizeof(Bwd1Smem<128>) : sizeof(Bwd1Smem<256>)) + 1024;
+    const int smem = (int)sizeof(Bwd1Smem<256>) + 1024;
     int sms = 0;
     if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
     const int64_t items = (int64_t)sh.B * hcount * (sh.N / 128) * (sh.D / 128);
     const int grid = (int)(items < sms ? items : sms);
-    DM_CUDA(dmh::launch_pdl(sh.D == 128 ? bwd1_kernel<128> : bwd1_kernel<256>, grid, kThreads, smem, stream, tq, td, tk, tv, ts, p));
+    if (sh.D == 128) return dmh::launch_bwd1_d128(tq, td, tk, tv, ts, p, grid, stream, err, errlen);
+    DM_CUDA(dmh::launch_pdl(bwd1_kernel<256>, grid, kThreads, smem, stream, tq, td, tk, tv, ts, p));
     return DM_OK;
 }

@@ -183,6 +183,23 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
         : "r"(taddr)
         : "memory");
 }
+// 16 lanes x 256 bit x 4 (32 columns), the matrix-fragment layout: with lane base L (a multiple of 16 inside the warp's quarter),
+// register 4 j + 2 a + e of thread t is lane L + t / 4 + 8 a, column c + 8 j + 2 (t % 4) + e.
+__device__ __forceinline__ void tmem_ld16x256_x4(uint32_t taddr, uint32_t* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+// Four 16 x 8 byte matrices from that layout (register j = the four bytes of fragment j, in register order), stored transposed:
+// column i of matrix j becomes 16 consecutive bytes at the address that lane 8 j + i gives.
+__device__ __forceinline__ void stmatrix_t_b8_x4(uint32_t saddr, const uint32_t* r) {
+    asm volatile("stmatrix.sync.aligned.m16n8.x4.trans.shared.b8 [%0], {%1, %2, %3, %4};"
+                 ::"r"(saddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
+                 : "memory");
+}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -312,6 +329,12 @@ __device__ __forceinline__ void add2(float& y0, float& y1, float x0, float x1) {
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+// max(|a|, |b|, |c|)
+__device__ __forceinline__ float fmax3_abs(float a, float b, float c) {
+    float d;
+    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
 // two fp32 -> two e4m3 (round-to-nearest-even, saturate-to-finite), lo in bits 0..7
