@@ -34,7 +34,7 @@ constexpr int kTile = 128 * 128;
 constexpr int kSoftmaxThreads = 512;
 constexpr int kFoldWarp = 16, kServiceWarp = 24;
 constexpr int kThreads = 896;
-constexpr int kRegSoftmax = 64, kRegFold = 104, kRegService = 40;     // per thread after setmaxnreg: the sum is the launch pool
+constexpr int kRegSoftmax = 72, kRegFold = 96, kRegService = 24;     // per thread after setmaxnreg: the sum is the launch pool
 constexpr int kStages = 3;             // Q / dO ring, 128 rows each
 constexpr int kRows = 3;               // ring of row constants
 constexpr int kGf = 4;                 // ring of product scales between softmax and fold warps
@@ -42,10 +42,10 @@ constexpr int kGf = 4;                 // ring of product scales between softmax
 // Named barriers.  Warp-to-warp hand-offs cost a quarter of an mbarrier's; an arriving side is never a whole round ahead, because
 // its next arrival on the same barrier needs a product that is issued behind the synchronising side's.
 constexpr int kBarSpFree = 1;          // (S | dP) is in registers                          512 + 32
-constexpr int kBarAmax = 2;            // the warps' maxima are in shared memory            512
-constexpr int kBarCodes = 3;           // + tile parity: the tile's codes are               512 + 32
-constexpr int kBarXFree = 5;           // the fold warps hold the dK product                256 + 32
-constexpr int kBarDvFree = 6;          // dV's accumulator is in the next tile's unit       256 + 32
+constexpr int kBarAmax = 2;            // + row half: its warps' maxima are in shared memory  256
+constexpr int kBarCodes = 4;           // + tile parity: the tile's codes are               512 + 32
+constexpr int kBarXFree = 6;           // the fold warps hold the dK product                256 + 32
+constexpr int kBarDvFree = 7;          // dV's accumulator is in the next tile's unit       256 + 32
 
 struct Smem {
     alignas(1024) uint8_t k[kTile];
@@ -58,6 +58,7 @@ struct Smem {
     alignas(16) float2 rd[kRows][128];    // per row: 8 - lse * log2e, -delta
     alignas(16) float sc[kRows][4];       // q8sc, do8sc of the tile, what dV's accumulator is multiplied by before it, its unit
     alignas(16) float gf[kGf][4];         // dK scale of rows 0..63, of rows 64..127, dV's unit
+    float psi[kGf][2];                    // psi of the tile's two m-blocks, on its way to pass 2
     float amax[2][16];                    // [tile parity][8 * row half + warp of the half]
     uint64_t bar_kv, bar_kv_free, bar_qdo[kStages], bar_stage_free[kStages], bar_sp_full, bar_x_full, bar_done[2], bar_ds_free[2],
         bar_rows_full[kRows], bar_rows_free[kRows];
@@ -71,7 +72,7 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                  const __grid_constant__ CUtensorMap tm_ds, const dm::Bwd1Params p) {
     extern __shared__ uint8_t smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int nbn = p.N / 128, nq_blk = p.rm.nq / 128;
     // `t` counts the CTA's tiles (128 rows each) over its items, so ring stages, buffer parities and mbarrier phases run on across
     // items.  `kvn` counts the items that loaded K / V (those with tiles).
@@ -158,6 +159,7 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 const dm::Bwd1Item w = dm::bwd1_item<128>(p, r);
                 if (!w.valid) break;
                 int ds_row = (int)((((int64_t)w.bhl * nq_blk + (w.m_lo >> 1)) * nbn + w.J) * 128);   // dS' tile of the first row block
+                float* psi_out = p.psi + ((int64_t)w.bhl * (2 * nq_blk) + w.m_lo + (lane & 1)) * nbn + w.J;
                 for (int it = 0; it < w.n_it; it += 2, ++t, ds_row += nbn * 128) {
                     const int par = t & 1, st = t % kStages;
                     const uint32_t qs = q_lo + st * kSub, dos = do_lo + st * kSub, da = ds_lo + par * kSub, pa = pt_lo + par * kSub;
@@ -178,6 +180,7 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                         dm::tma_store_commit();
                     }
                     __syncwarp();
+                    if (lane < 2) psi_out[(int64_t)it * nbn] = s.psi[t % kGf][lane];
                     // dV += P-hat8^T dO8, in the accumulator itself
                     if (t > 0) dm::named_bar_sync(kBarDvFree, 256 + 32);
                     dm::tc_fence_after();
@@ -287,12 +290,12 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
             for (int i = 0; i < 64; ++i) dk_acc[i] = 0.f;
             const float ik = 1.0f / p.k8s[(int64_t)w.hc.bhk * (p.N / 64) + 2 * w.J + (key >> 6)];   // for the epilogue; read early
-            auto fold_dk = [&](int m) {                             // two products a tile
+            auto fold_dk = [&](const float* g, int m) {             // two products a tile
                 dm::mbar_wait(&s.bar_x_full, m, wc);                // also orders the ring slot written before the codes
                 dm::tc_fence_after();
                 uint32_t sa[16], sb[16];
                 dm::tmem_ld16(x_src, sa);
-                const float gk = s.gf[t % kGf][m];
+                const float gk = g[m];
                 // four 16-column pieces, the next one in flight while one is added
 #pragma unroll
                 for (int pc = 0; pc < 4; ++pc) {
@@ -312,8 +315,9 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 }
             };
             for (int it = 0; it < w.n_it; it += 2, ++t) {
-                fold_dk(0);
-                fold_dk(1);                                          // (its product was committed behind the tile's dV)
+                const float* g = s.gf[t % kGf];
+                fold_dk(g, 0);
+                fold_dk(g, 1);                                       // (its product was committed behind the tile's dV)
                 if (it + 2 < w.n_it) {
                     // dV's accumulator into the next tile's unit
                     const int slot = (t + 1) % kRows;
@@ -433,7 +437,6 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             const float k8s_t = p.k8s[(int64_t)w.hc.bhk * (p.N / 64) + 2 * w.J + (kq >> 1)];
             const float v8s_t = p.v8s[(int64_t)w.hc.bhk * (p.N / 64) + 2 * w.J + (kq >> 1)];
             const bool diag_item = p.causal && n_it > 0 && dm::global_block(p.rm, w.m_lo >> 1) == w.J;
-            float* psi_it = p.psi + ((int64_t)w.bhl * (2 * nq_blk) + w.m_lo) * nbn + w.J;
             float g_max = 0.f;
 
             for (int it = 0; it < n_it; ++it, ++t) {
@@ -492,28 +495,22 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 // the warp's maximum in one instruction: non-negative floats order like their bit patterns
                 const float am = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(am0, am1))));
                 if (lane == 0) s.amax[par][8 * rhalf + 2 * kq + (rq & 1)] = am;
-                dm::named_bar_sync(kBarAmax, kSoftmaxThreads);
-                // psi of both m-blocks in order (every thread: the second one's floor depends on the first one's scale):
-                // psi = max(psi_raw, g_max * 256e-8 / q8sc); the quotient can only win when its numerator exceeds psi_raw * q8sc,
-                // so the division is formed only then (the 1 % margin covers the rounding of both sides)
-                float psi[2], g[2];
+                dm::named_bar_sync(kBarAmax + rhalf, kSoftmaxThreads / 2);
+                // psi of the m-block: psi = max(psi_raw, g_max * 256e-8 / q8sc); the quotient can only win when its numerator
+                // exceeds psi_raw * q8sc, so the division is formed only then (the 1 % margin covers the rounding of both sides).
+                // g_max runs over the m-blocks of this row half: the floor acts only on a tile whose maximum lies eight decades
+                // below an earlier one's, and one barrier for both halves and both psi in every thread cost 3 %.
+                float psi_my;
                 {
-                    const uint32_t a = __float_as_uint(s.amax[par][lane & 15]);
-                    const uint32_t a0 = __reduce_max_sync(0xffffffffu, (lane & 8) ? 0u : a);
-                    const uint32_t a1 = __reduce_max_sync(0xffffffffu, (lane & 8) ? a : 0u);
-#pragma unroll
-                    for (int m = 0; m < 2; ++m) {
-                        const float amx = __uint_as_float(m ? a1 : a0) * (1.0f / 448.0f);
-                        const float psi_raw = fmaxf(amx, 1e-30f);
-                        psi[m] = psi_raw;
-                        const float fl_num = g_max * (256.0f * 1e-8f);
-                        if (fl_num > psi_raw * q8sc * 0.99f) psi[m] = fmaxf(psi_raw, fl_num / q8sc);
-                        if (amx < 1e-30f) psi[m] = 0.f;                          // a zero tile
-                        g[m] = psi[m] * dm::kMoInv * q8sc;
-                        g_max = fmaxf(g_max, g[m]);
-                    }
+                    const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(s.amax[par][8 * rhalf + (lane & 7)])));
+                    const float amx = mx * (1.0f / 448.0f);
+                    psi_my = fmaxf(amx, 1e-30f);
+                    const float fl_num = g_max * (256.0f * 1e-8f);
+                    if (fl_num > psi_my * q8sc * 0.99f) psi_my = fmaxf(psi_my, fl_num / q8sc);
+                    if (amx < 1e-30f) psi_my = 0.f;                          // a zero tile
                 }
-                const float psi_my = rhalf ? psi[1] : psi[0];
+                const float g_my = psi_my * dm::kMoInv * q8sc;
+                g_max = fmaxf(g_max, g_my);
                 const float psi_inv = psi_my == 0.f ? 0.f : __frcp_rn(psi_my);   // the correctly rounded reciprocal, as 1 / psi
 
                 // ---- phase 2: dS' codes, to shared memory for dK and for the tile that leaves to pass 2
@@ -530,11 +527,11 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     dm::stmatrix_t_b8_x4((addr ^ (16 * h)) + ds_off, c4);
                 }
                 // the scales of this tile's products for the fold warps (the ring slot was last read four tiles ago; S of this tile
-                // waited for the products of two tiles ago) and psi for pass 2
-                if (tid == 0) {
-                    *reinterpret_cast<float4*>(s.gf[t % kGf]) = make_float4(g[0], g[1], s.sc[rb][3], 0.f);
-                    psi_it[(int64_t)(2 * it) * nbn] = psi[0];
-                    psi_it[(int64_t)(2 * it + 1) * nbn] = psi[1];
+                // waited for the products of two tiles ago) and psi, which the product warp takes to global memory
+                if ((tid & ~64) == 0) {           // one thread of each row half
+                    s.gf[t % kGf][rhalf] = g_my;
+                    s.psi[t % kGf][rhalf] = psi_my;
+                    if (rhalf == 0) s.gf[t % kGf][2] = s.sc[rb][3];
                 }
                 dm::fence_proxy_async_smem();
                 dm::named_bar_arrive(kBarCodes + par, kSoftmaxThreads + 32);
