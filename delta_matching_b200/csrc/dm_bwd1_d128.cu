@@ -132,6 +132,7 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                         dm::mbar_wait(&s.bar_done[t & 1], ((t - 2) >> 1) & 1, wc);
                         dm::mbar_wait(&s.bar_ds_free[t & 1], ((t - 2) >> 1) & 1, wc);
                     }
+                    dm::mbar_wait(&s.bar_rows_full[t % kRows], (t / kRows) & 1, wc);      // saves the softmax warps a wait of their own
                     if (t >= 1) dm::named_bar_sync(kBarSpFree, kSoftmaxThreads + 32);
                     dm::tc_fence_after();
                     const uint32_t qs = q_lo + st * kSub, dos = do_lo + st * kSub;
@@ -429,7 +430,7 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // this lane's line of the transposed stores: key 32 kq + lane, the 16-byte chunk of rows [32 rq, +16) (the next chunk: ^ 16)
         const uint32_t st_addr = dm::smem_u32(s.pt[0]) + (32 * kq + lane) * 128 + (((2 * rq) ^ (lane & 7)) << 4);
         const uint32_t ds_off = dm::smem_u32(s.ds[0]) - dm::smem_u32(s.pt[0]);
-        int t = 0;
+        int t = 0, rb = 0;                            // tiles so far; ring slot of the row constants
         for (int r = 0;; ++r) {
             const dm::Bwd1Item w = dm::bwd1_item<128>(p, r);
             if (!w.valid) break;
@@ -439,15 +440,14 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             const bool diag_item = p.causal && n_it > 0 && dm::global_block(p.rm, w.m_lo >> 1) == w.J;
             float g_max = 0.f;
 
-            for (int it = 0; it < n_it; ++it, ++t) {
-                const int par = t & 1, rb = t % kRows;
-                dm::mbar_wait(&s.bar_rows_full[rb], (t / kRows) & 1, wc);
+            for (int it = 0; it < n_it; ++it, ++t, rb = rb == kRows - 1 ? 0 : rb + 1) {
+                const int par = t & 1;
+                dm::mbar_wait(&s.bar_sp_full, par, wc);
                 const float q8sc = s.sc[rb][0], do8sc = s.sc[rb][1];
                 const float dsc = dm::descale_log2(q8sc, k8s_t);
                 const float dpk = do8sc * v8s_t * k8s_t;
                 const float2* rd = &s.rd[rb][row_t];
                 const uint32_t addr = st_addr + par * kTile;
-                dm::mbar_wait(&s.bar_sp_full, par, wc);
                 dm::tc_fence_after();
 
                 // ---- phase 1: P-hat, dS', tile amax; P-hat codes to shared memory.  Two halves of 16 rows; S first: the
