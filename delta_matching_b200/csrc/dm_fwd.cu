@@ -26,22 +26,26 @@ namespace {
 
 constexpr int kTile = 128 * 128;   // bytes of one e4m3 tile (128 rows x 128 bytes)
 constexpr int kStages = 3;
-constexpr int kThreads = 512;
-constexpr int kSoftmaxThreads = 256;
+constexpr int kThreads = 896;
+constexpr int kSoftmaxThreads = 512;
+constexpr int kFoldWarp = 16, kServiceWarp = 24;
+constexpr int kRegSoftmax = 72, kRegFold = 96, kRegService = 24;      // per thread after setmaxnreg; the sum is the launch pool
+// Named barriers (a warp-to-warp hand-off costs a quarter of an mbarrier's; an arriving side is never a whole round ahead, because
+// its next arrival on the same barrier needs a product that is issued behind the synchronising side's).
+constexpr int kBarCodes = 1;       // + 2 * team + key group: the group's codes are in tensor memory     128 + 32
+constexpr int kBarDFree = 5;       // + key group: the fold warps hold the group's product              256 + 32
+constexpr int kItems = 8;          // a team without a tile in a one-tile item can be four items ahead of the fold warps
 constexpr int kRing = 4;           // depth of the per-tile row-constant ring between softmax and fold warps
 
 struct FwdSmem {
     alignas(1024) uint8_t q[2][kTile];             // by work item parity: the next item's Q arrives under this item's tail
     alignas(1024) uint8_t k[kStages][kTile];
     alignas(1024) uint8_t v[kStages][kTile];
-    float gmax[2][2][128];            // [tile parity][key group][row]
-    float wgt[kRing][2][128];         // [tile % kRing][key group][row]
-    float alpha[kRing][128];
-    float lsum[4][2][128];            // [work item % 4][key group][row]: with one-tile items the softmax warps can be three
-                                      // items ahead of the fold warps
-    alignas(16) uint8_t stg[4][32 * 256];   // per fold warp: its 32 bf16 O rows on their way out (16-byte chunks XOR-swizzled by the row)
-    uint64_t bar_q[2], bar_q_free[2], bar_kv[kStages], bar_kv_free[kStages], bar_s_full[2], bar_s_free[2], bar_codes[2],
-        bar_d_full[2], bar_d_free, bar_l[4];
+    float ms[kRing][2][128];          // [tile % kRing][key group][row]: the basis of the row's codes, log2 units
+    float vs[kRing][2];               // the group's V scale
+    float2 lsum[kItems][4][128];      // [work item % kItems][2 * (tile parity in the item) + key group][row]: part of the denominator and its unit (log2)
+    alignas(16) uint8_t stg[8][32 * 128];   // per fold warp: its 32 bf16 half rows of O on their way out (16-byte chunks XOR-swizzled by the row)
+    uint64_t bar_q[2], bar_q_free[2], bar_kv[kStages], bar_kv_free[kStages], bar_s_full[2], bar_d_full[2][2], bar_l[kItems];   // bar_d_full: [tile parity][key group]
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -86,7 +90,7 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
     extern __shared__ uint8_t smem_raw[];
     FwdSmem& s = *reinterpret_cast<FwdSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int nq_blk = p.rm.nq / 128;
     dm::WaitCtx wc{&s.abort_flag, p.status};
     // Every role walks the same list of work items; `gt` counts the key tiles of the items before the current one, so
@@ -96,18 +100,16 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         s.abort_flag = 0;
         for (int i = 0; i < kStages; ++i) {
             dm::mbar_init(&s.bar_kv[i], 1);
-            dm::mbar_init(&s.bar_kv_free[i], 1);
+            dm::mbar_init(&s.bar_kv_free[i], 2);
         }
         for (int i = 0; i < 2; ++i) {
             dm::mbar_init(&s.bar_s_full[i], 1);
-            dm::mbar_init(&s.bar_s_free[i], 8);
-            dm::mbar_init(&s.bar_codes[i], 8);
-            dm::mbar_init(&s.bar_d_full[i], 1);
+            dm::mbar_init(&s.bar_d_full[i][0], 1);
+            dm::mbar_init(&s.bar_d_full[i][1], 1);
             dm::mbar_init(&s.bar_q[i], 1);
             dm::mbar_init(&s.bar_q_free[i], 1);
         }
-        dm::mbar_init(&s.bar_d_free, 4);
-        for (int i = 0; i < 4; ++i) dm::mbar_init(&s.bar_l[i], 8);
+        for (int i = 0; i < kItems; ++i) dm::mbar_init(&s.bar_l[i], kSoftmaxThreads / 32);
         dm::fence_mbar_init();
         dm::tma_prefetch_desc(&tm_q);
         dm::tma_prefetch_desc(&tm_k);
@@ -122,15 +124,13 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const uint32_t t_d0 = tmem + 256, t_d1 = tmem + 384;      // S buffers at columns [0, 128) and [128, 256)
     const uint32_t lane_base = (uint32_t)(warp & 3) * 32;
 
-    if (warp >= 12) {
+    if (warp >= kServiceWarp) {
         // =============================================================== service warps
-        dm::reg_dec<40>();
-        const bool leader = lane == 0;
+        dm::reg_dec<kRegService>();
         constexpr uint32_t kSub = kTile >> 4;
-        if (warp == 12) {
-            // ---- S = Q K^T of tile t into buffer t & 1.  The code tile of the same parity is rewritten by the softmax of
-            // this tile, so the products of tile t - 2, which read it, must be complete: waiting for them here gates the
-            // softmax warps through S.
+        if (warp == kServiceWarp) {
+            // ---- S = Q K^T of tile t into buffer t & 1, once the products of tile t - 2 are complete: they read their codes from
+            // that buffer, and their codes came after the softmax warps had read its scores.
             constexpr uint32_t idesc_s = dm::idesc_e4m3(128, 128, false, false);
             const uint32_t q_lo0 = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[0])), k_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.k[0]));
             int gt = 0;
@@ -144,12 +144,12 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     const int t = gt + it, st = t % kStages, b = t & 1;
                     dm::mbar_wait(&s.bar_kv[st], (t / kStages) & 1, wc);
                     if (t >= 2) {
-                        dm::mbar_wait(&s.bar_s_free[b], ((t - 2) >> 1) & 1, wc);
-                        dm::mbar_wait(&s.bar_d_full[b], ((t - 2) >> 1) & 1, wc);
+                        dm::mbar_wait(&s.bar_d_full[b][0], ((t - 2) >> 1) & 1, wc);
+                        dm::mbar_wait(&s.bar_d_full[b][1], ((t - 2) >> 1) & 1, wc);
                     }
                     dm::tc_fence_after();
                     const uint32_t ks = k_lo + st * kSub, ts = tmem + b * 128;
-                    if (leader) {
+                    if (dm::elect_one()) {
                         dm::umma_e4m3_lo<false>(ts, q_lo, ks, idesc_s);
 #pragma unroll
                         for (int k = 1; k < 4; ++k) dm::umma_e4m3_lo<true>(ts, q_lo + 2 * k, ks + 2 * k, idesc_s);
@@ -160,36 +160,35 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 }
                 gt += w.n_tiles;
             }
-        } else if (warp == 13) {
-            // ---- D_g = C_g V_g for both key groups once the codes of tile t are in shared memory and the fold warps
-            // have read the products of tile t - 1
+        } else if (warp <= kServiceWarp + 2) {
+            // ---- D_g = C_g V_g, one warp per key group, once the group's codes are in tensor memory and the fold warps hold its product
+            // of the tile before
+            const int g = warp - kServiceWarp - 1;
             constexpr uint32_t idesc_pv = dm::idesc_e4m3(128, 128, false, true);
-            const uint32_t v_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.v[0]));
-            int gt = 0;
+            const uint32_t v_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.v[0])) + 512 * g;      // V rows of the group (MN-major: 32 rows = +256)
+            const uint32_t t_d = g ? t_d1 : t_d0;
+            int t = 0, st = 0;
             for (int r = 0;; ++r) {
                 const FwdItem w = fwd_item(p, r);
                 if (!w.valid) break;
-                for (int it = 0; it < w.n_tiles; ++it) {
-                    const int t = gt + it, st = t % kStages, b = t & 1;
-                    dm::mbar_wait(&s.bar_kv[st], (t / kStages) & 1, wc);
-                    dm::mbar_wait(&s.bar_codes[b], (t >> 1) & 1, wc);
-                    if (t >= 1) dm::mbar_wait(&s.bar_d_free, (t - 1) & 1, wc);
+                for (int it = 0; it < w.n_tiles; ++it, ++t) {
+                    const int b = t & 1;
+                    const uint32_t pa = tmem + b * 128 + 64 * g, va = v_lo + st * kSub;     // codes: columns [64 g, 64 g + 16) of S buffer b
+                    if (t >= 1) dm::named_bar_sync(kBarDFree + g, 256 + 32);
+                    dm::named_bar_sync(kBarCodes + 2 * b + g, 128 + 32);       // (V came with the K that S was made of)
                     dm::tc_fence_after();
-                    const uint32_t pa = tmem + b * 128, va = v_lo + st * kSub;     // codes of group g: columns [64 g, 64 g + 16) of S buffer b
-                    if (leader) {
-                        // group gg: codes columns [64 gg, 64 gg + 64) (K-major, +4 per 64 bytes), V rows [64 gg, +64) (MN-major, +512)
-                        dm::umma_e4m3_ts<false>(t_d0, pa, va, idesc_pv);
-                        dm::umma_e4m3_ts<true>(t_d0, pa + 8, va + 256, idesc_pv);
-                        dm::umma_e4m3_ts<false>(t_d1, pa + 64, va + 512, idesc_pv);
-                        dm::umma_e4m3_ts<true>(t_d1, pa + 72, va + 768, idesc_pv);
-                        dm::umma_commit(&s.bar_d_full[b]);
+                    if (dm::elect_one()) {
+                        dm::umma_e4m3_ts<false>(t_d, pa, va, idesc_pv);
+                        dm::umma_e4m3_ts<true>(t_d, pa + 8, va + 256, idesc_pv);
+                        dm::umma_commit(&s.bar_d_full[b][g]);
                         dm::umma_commit(&s.bar_kv_free[st]);       // K was read by S long ago, V just now
                     }
                     __syncwarp();
+                    if (++st == kStages) st = 0;
                 }
-                gt += w.n_tiles;
             }
-        } else if (warp == 14) {
+            if (t > 0) dm::named_bar_sync(kBarDFree + g, 256 + 32);      // the last release: no arrival is left over
+        } else {
             // ---- TMA loads: every item's Q, then its K / V tiles, as far ahead as the rings allow (across items too)
             int gt = 0;
             for (int r = 0;; ++r) {
@@ -198,14 +197,14 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 const int qb = r & 1;
                 const int q_row0 = w.hc.bh * p.rm.nq + w.li * 128, kv_row0 = w.hc.bhk * p.N;
                 if (r >= 2) dm::mbar_wait(&s.bar_q_free[qb], ((r - 2) >> 1) & 1, wc);
-                if (leader) {
+                if (dm::elect_one()) {
                     dm::mbar_expect_tx(&s.bar_q[qb], kTile);
                     dm::tma_load_2d(s.q[qb], &tm_q, 0, q_row0, &s.bar_q[qb]);
                 }
                 for (int it = 0; it < w.n_tiles; ++it) {
                     const int t = gt + it, st = t % kStages, j = w.n_tiles - 1 - it;
                     if (t >= kStages) dm::mbar_wait(&s.bar_kv_free[st], (t / kStages - 1) & 1, wc);
-                    if (leader) {
+                    if (dm::elect_one()) {
                         dm::mbar_expect_tx(&s.bar_kv[st], 2 * kTile);
                         dm::tma_load_2d(s.k[st], &tm_k, 0, kv_row0 + j * 128, &s.bar_kv[st]);
                         dm::tma_load_2d(s.v[st], &tm_v, 0, kv_row0 + j * 128, &s.bar_kv[st]);
@@ -215,75 +214,94 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 gt += w.n_tiles;
             }
         }
-    } else if (warp >= 8) {
-        // =============================================================== fold warps: thread = row, all 128 columns of O
-        dm::reg_inc<208>();
-        const int row = (warp & 3) * 32 + lane;
+    } else if (warp >= kFoldWarp) {
+        // =============================================================== fold warps: thread = (row, 64 of O's 128 columns)
+        dm::reg_inc<kRegFold>();
+        const int row = (warp & 3) * 32 + lane, half = (warp >> 2) & 1;
+        const uint32_t src = dm::tmem_addr(t_d0, lane_base, 64 * half);      // group 1's products: + 128
         int gt = 0;
         for (int r = 0;; ++r) {
             const FwdItem w = fwd_item(p, r);
             if (!w.valid) break;
-            float o_acc[128];
+            float o_acc[64];
 #pragma unroll
-            for (int i = 0; i < 128; ++i) o_acc[i] = 0.f;
+            for (int i = 0; i < 64; ++i) o_acc[i] = 0.f;
+            float ref = -INFINITY;                     // o_acc's basis, log2 units: O = o_acc * 2^ref / denominator
             for (int it = 0; it < w.n_tiles; ++it) {
                 const int t = gt + it, b = t & 1, rg = t % kRing;
-                dm::mbar_wait(&s.bar_d_full[b], (t >> 1) & 1, wc);      // also orders the ring slot written before the codes
-                dm::tc_fence_after();
-                const float alpha = s.alpha[rg][row], w0 = s.wgt[rg][0][row], w1 = s.wgt[rg][1][row];
-                uint32_t sa[32], sb[32];
-                dm::tmem_ld32(dm::tmem_addr(t_d0, lane_base, 0), sa);
-                if (__any_sync(0xffffffffu, alpha != 1.0f)) {
 #pragma unroll
-                    for (int i = 0; i < 128; i += 2) dm::mul2(o_acc[i], o_acc[i + 1], o_acc[i], o_acc[i + 1], alpha, alpha);
+                for (int g = 0; g < 2; ++g) {
+                    dm::mbar_wait(&s.bar_d_full[b][g], (t >> 1) & 1, wc);      // also orders the ring slot written before the codes
+                    dm::tc_fence_after();
+                    uint32_t sa[16], sb[16];
+                    dm::tmem_ld16(src + 128 * g, sa);
+                    const float ms = s.ms[rg][g][row], vs = s.vs[rg][g];
+                    // The basis moves only when a group's basis has grown 8 binades past it (a weight stays below 2^8 times its V scale,
+                    // far inside fp32), so O is rescaled a few times per item instead of at every new maximum.
+                    const bool grow = ms > ref + 8.0f;
+                    if (__any_sync(0xffffffffu, grow)) {
+                        const float alpha = grow ? dm::ex2(ref - ms) : 1.0f;
+                        if (grow) ref = ms;
+#pragma unroll
+                        for (int i = 0; i < 64; i += 2) dm::mul2(o_acc[i], o_acc[i + 1], o_acc[i], o_acc[i + 1], alpha, alpha);
+                    }
+                    const float wg = ms == -INFINITY ? 0.f : vs * dm::ex2(ms - ref);      // (a group without a visible key)
+                    // four 16-column pieces, the next one in flight while one is added
+#pragma unroll
+                    for (int pc = 0; pc < 4; ++pc) {
+                        uint32_t* cur = (pc & 1) ? sb : sa;
+                        uint32_t* nxt = (pc & 1) ? sa : sb;
+                        dm::tmem_ld_wait();
+                        if (pc < 3) {
+                            dm::tmem_ld16(src + 128 * g + 16 * (pc + 1), nxt);
+                        } else {
+                            dm::tc_fence_before();
+                            dm::named_bar_arrive(kBarDFree + g, 256 + 32);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 16; i += 2)
+                            dm::fma2(o_acc[16 * pc + i], o_acc[16 * pc + i + 1], __uint_as_float(cur[i]), __uint_as_float(cur[i + 1]), wg,
+                                     o_acc[16 * pc + i], o_acc[16 * pc + i + 1]);
+                    }
                 }
-                // eight 32-column pieces (group 0 columns 0..127, then group 1), the next one in flight while one is added
-#pragma unroll
-                for (int pc = 0; pc < 8; ++pc) {
-                    uint32_t* cur = (pc & 1) ? sb : sa;
-                    uint32_t* nxt = (pc & 1) ? sa : sb;
-                    dm::tmem_ld_wait();
-                    if (pc < 7) dm::tmem_ld32(dm::tmem_addr((pc + 1 < 4) ? t_d0 : t_d1, lane_base, 32 * ((pc + 1) & 3)), nxt);
-                    const float wg = (pc < 4) ? w0 : w1;
-                    const int c0 = 32 * (pc & 3);
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2)
-                        dm::fma2(o_acc[c0 + i], o_acc[c0 + i + 1], __uint_as_float(cur[i]), __uint_as_float(cur[i + 1]), wg,
-                                 o_acc[c0 + i], o_acc[c0 + i + 1]);
-                }
-                dm::tc_fence_before();
-                dm::mbar_arrive_warp(&s.bar_d_free);
             }
             gt += w.n_tiles;
-            // ---- the item's epilogue: the softmax warps have left both halves of the denominator
-            dm::mbar_wait(&s.bar_l[r & 3], (r >> 2) & 1, wc);
-            const float l = s.lsum[r & 3][0][row] + s.lsum[r & 3][1][row];
-            const bool dead = (l == 0.f) || (l != l);
-            const float inv = dead ? 0.f : 1.0f / l;
-            // The bf16 rows leave through shared memory: a thread holds a whole row, so stored directly every 16-byte store
-            // instruction would touch 32 different rows; from the warp's staging slice each instruction writes two whole 256-byte
-            // rows.  A warp's 32 rows are its own, so the hand-over needs no more than the warp.
-            uint8_t* stg = s.stg[warp & 3];
+            // ---- the item's epilogue: the softmax warps have left the denominator's four parts
+            dm::mbar_wait(&s.bar_l[r % kItems], (r / kItems) & 1, wc);
+            float2 lp[4];
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
+            for (int i = 0; i < 4; ++i) lp[i] = s.lsum[r % kItems][i][row];
+            const float unit = fmaxf(fmaxf(lp[0].y, lp[1].y), fmaxf(lp[2].y, lp[3].y));
+            float l = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) l += lp[i].x * dm::ex2(lp[i].y - unit);
+            const bool dead = (l == 0.f) || (l != l);
+            const float inv = dead ? 0.f : dm::ex2(ref - unit) / l;
+            if (half == 0) p.lse[(int64_t)w.hc.bh * p.rm.nq + w.li * 128 + row] = dead ? -INFINITY : unit * dm::kLn2 + logf(l);
+            // The bf16 half rows leave through shared memory: stored directly every 16-byte store instruction would touch 32 different
+            // rows; from the warp's staging slice each instruction writes four whole 128-byte half rows.  A warp's slice is its own, so
+            // the hand-over needs no more than the warp.
+            uint8_t* stg = s.stg[warp & 7];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
                 uint32_t w4[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     __nv_bfloat162 tt = __floats2bfloat162_rn(o_acc[8 * c + 2 * e] * inv, o_acc[8 * c + 2 * e + 1] * inv);
                     w4[e] = *reinterpret_cast<uint32_t*>(&tt);
                 }
-                *reinterpret_cast<uint4*>(stg + lane * 256 + ((c ^ (lane & 15)) << 4)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+                *reinterpret_cast<uint4*>(stg + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
             }
             __syncwarp();
             {
                 const int row0 = w.li * 128 + (warp & 3) * 32;          // first of the warp's rows inside the (local) Q-side tensors
-                uint8_t* obase = reinterpret_cast<uint8_t*>(p.o + (((int64_t)w.hc.b * p.rm.nq + row0) * p.H + w.hc.h) * 128);
+                uint8_t* obase = reinterpret_cast<uint8_t*>(p.o + (((int64_t)w.hc.b * p.rm.nq + row0) * p.H + w.hc.h) * 128) + 128 * half;
                 const int64_t row_bytes = (int64_t)p.H * 128 * 2;
-                const int j = lane & 15;
+                const int j = lane & 7;
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int rr = 2 * i + (lane >> 4);
-                    const uint4 val = *reinterpret_cast<const uint4*>(stg + rr * 256 + ((j ^ (rr & 15)) << 4));
+                for (int i = 0; i < 8; ++i) {
+                    const int rr = 4 * i + (lane >> 3);
+                    const uint4 val = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((j ^ (rr & 7)) << 4));
                     *reinterpret_cast<uint4*>(obase + rr * row_bytes + (j << 4)) = val;
                 }
             }
@@ -291,116 +309,119 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
     } else {
         // =============================================================== softmax warps
-        const int g = warp >> 2;                  // warpgroup = key group inside the tile
+        dm::reg_dec<kRegSoftmax>();
+        const int team = warp >> 3, g = (warp >> 2) & 1;      // parity of the tiles (= the S buffer), 64-key group of the tile
         const int row = (warp & 3) * 32 + lane;   // query row inside the block = tensor-memory lane
+        const uint32_t t_s = dm::tmem_addr(tmem + team * 128, lane_base, g * 64);
         int gt = 0;
-        // An item's Q scale and the K / V scales of its first key tile are read one item ahead: read at the item's start
-        // they would be three exposed global loads in front of its first tile.
+        // What an item's first tile needs from global memory is read one item ahead: read at the item's start it would be three
+        // exposed loads.
         float q8sc_nx = 0.f, ks_nx = 0.f, vs_nx = 0.f;
-        auto first_scales = [&](const FwdItem& wi) {
+        auto first_scales = [&](const FwdItem& wi, int gt_at) {
             if (!wi.valid) return;
-            const int64_t ko = (int64_t)wi.hc.bhk * (p.N / 64) + g + 2 * (wi.n_tiles - 1);
             q8sc_nx = p.q8s[(int64_t)wi.hc.bh * nq_blk + wi.li];
-            ks_nx = p.k8s[ko];
-            vs_nx = p.v8s[ko];
+            const int first = (gt_at ^ team) & 1;
+            if (first < wi.n_tiles) {
+                const int64_t ko = (int64_t)wi.hc.bhk * (p.N / 64) + g + 2 * (wi.n_tiles - 1 - first);
+                ks_nx = p.k8s[ko];
+                vs_nx = p.v8s[ko];
+            }
         };
-        first_scales(fwd_item(p, 0));
-        for (int r = 0;; ++r) {
-        const FwdItem w = fwd_item(p, r);
-        if (!w.valid) break;
-        const int n_tiles = w.n_tiles, I = w.I;
-        const float q8sc = q8sc_nx;
-        const float* ksp = p.k8s + (int64_t)w.hc.bhk * (p.N / 64) + g;
-        const float* vsp = p.v8s + (int64_t)w.hc.bhk * (p.N / 64) + g;
-        float m_run = -INFINITY, l_part = 0.f;
-
-        float ks_n = ks_nx, vs_n = vs_nx;
-        first_scales(fwd_item(p, r + 1));
-        for (int it = 0; it < n_tiles; ++it) {
-            const int t = gt + it, j = n_tiles - 1 - it, b = t & 1, rg = t % kRing;
-            const float ks = ks_n, vs = vs_n;
-            if (it + 1 < n_tiles) {
-                ks_n = ksp[2 * (j - 1)];
-                vs_n = vsp[2 * (j - 1)];
-            }
-
-            // ---- S for this thread's (row, key group): 64 fp32 values
-            dm::mbar_wait(&s.bar_s_full[b], (t >> 1) & 1, wc);
-            dm::tc_fence_after();
-            float sv[64];
-            dm::tmem_ld32(dm::tmem_addr(tmem + b * 128, lane_base, g * 64), reinterpret_cast<uint32_t*>(sv));
-            dm::tmem_ld32(dm::tmem_addr(tmem + b * 128, lane_base, g * 64 + 32), reinterpret_cast<uint32_t*>(sv) + 32);
-            dm::tmem_ld_wait();
-            dm::tc_fence_before();
-            dm::mbar_arrive_warp(&s.bar_s_free[b]);            // this S buffer may be overwritten
-
-            // The group maximum is taken on the raw products: the group's scale is positive, so scaling the maximum gives the
-            // maximum of the scaled scores bit for bit, and the scores themselves are scaled inside the exponent's one
-            // multiply-add below (x = raw * (dsc * log2 e) - ms).  The scale is kept a normal number (it underflows only when a Q
-            // block and a K group are both all zero, where every product is zero anyway), so that a masked -inf stays -inf.
-            const float dsc = fmaxf(q8sc * ks, 1.2e-38f);
-            if (p.causal && j == I) {
-#pragma unroll
-                for (int c = 0; c < 64; ++c)
-                    if (g * 64 + c > row) sv[c] = -INFINITY;
-            }
-            float gm;
-            {
-                float m0 = fmaxf(sv[0], sv[1]), m1 = fmaxf(sv[2], sv[3]);
-#pragma unroll
-                for (int c = 4; c < 64; c += 4) {
-                    m0 = dm::fmax3(m0, sv[c], sv[c + 1]);
-                    m1 = dm::fmax3(m1, sv[c + 2], sv[c + 3]);
+        FwdItem w = fwd_item(p, 0);
+        first_scales(w, 0);
+        for (int r = 0; w.valid; ++r) {
+            const int n_tiles = w.n_tiles, I = w.I;
+            const float q8sc = q8sc_nx;
+            const float* ksp = p.k8s + (int64_t)w.hc.bhk * (p.N / 64) + g;
+            const float* vsp = p.v8s + (int64_t)w.hc.bhk * (p.N / 64) + g;
+            // The thread's own running maximum (its group, its team's tiles): it only places the floor of the basis, 12 binades below
+            // it.  The denominator's part is kept in a unit of its own that moves like the fold warps' basis.
+            float m_run = -INFINITY, l_part = 0.f, l_ref = -INFINITY;
+            float ks_n = ks_nx, vs_n = vs_nx;
+            w = fwd_item(p, r + 1);
+            first_scales(w, gt + n_tiles);
+            for (int it = (gt ^ team) & 1; it < n_tiles; it += 2) {
+                const int t = gt + it, j = n_tiles - 1 - it, rg = t % kRing;
+                const float ks = ks_n, vs = vs_n;
+                if (it + 2 < n_tiles) {
+                    ks_n = ksp[2 * (j - 2)];
+                    vs_n = vsp[2 * (j - 2)];
                 }
-                gm = fmaxf(m0, m1) * dsc;
-            }
-            s.gmax[b][g][row] = gm;
-            dm::named_bar_sync(1, kSoftmaxThreads);
-            const float tile_max = fmaxf(s.gmax[b][0][row], s.gmax[b][1][row]);
-            const float m_new = fmaxf(m_run, tile_max);
-            const float m_cur = (m_new == -INFINITY) ? 0.f : m_new;
-            const float alpha = dm::ex2((m_run - m_cur) * dm::kLog2e);
-            const float ml2 = m_cur * dm::kLog2e;
-            const float ms = fmaxf(gm * dm::kLog2e, ml2 - dm::kPhatFloorB) - dm::kLog2_448;
-            const float sigma = dm::ex2(ms - ml2);
-            // the ring slot of tile it - kRing has been read: its fold came before the fold of tile it - 3, whose release
-            // of the product buffers came before the products of tile it - 2, which S of this tile waited for
-            s.wgt[rg][g][row] = vs * sigma;
-            if (g == 0) s.alpha[rg][row] = alpha;
-            float part0 = 0.f, part1 = 0.f;
-            uint32_t codes[16];
-            const float nms = -ms, cl = __fmul_rn(dsc, dm::kLog2e);
-#pragma unroll
-            for (int c = 0; c < 64; c += 4) {
-                float x0, x1, x2, x3;
-                dm::fma2(x0, x1, sv[c], sv[c + 1], cl, nms, nms);
-                dm::fma2(x2, x3, sv[c + 2], sv[c + 3], cl, nms, nms);
-                const float p0 = dm::ex2(x0), p1 = dm::ex2(x1), p2 = dm::ex2(x2), p3 = dm::ex2(x3);
-                dm::add2(part0, part1, p0, p1);
-                dm::add2(part0, part1, p2, p3);
-                codes[c >> 2] = dm::cvt_e4m3x4(p0, p1, p2, p3);
-            }
-            const float part = part0 + part1;
-            l_part = fmaf(l_part, alpha, sigma * part);
-            // the codes go back into tensor memory, over the first 16 columns of this thread's own 64 scores (all read by
-            // now): the P V products take them from there as their A operand, four e4m3 per column, lane = row
-            dm::tmem_st16(dm::tmem_addr(tmem + b * 128, lane_base, g * 64), codes);
-            m_run = m_new;
-            dm::tmem_st_wait();
-            dm::tc_fence_before();
-            dm::mbar_arrive_warp(&s.bar_codes[b]);
-        }
+                // The group maximum is taken on the raw products: the group's scale is positive, so scaling the maximum gives the
+                // maximum of the scaled scores bit for bit, and the scores themselves are scaled inside the exponent's one
+                // multiply-add below (x = raw * (dsc * log2 e) - ms).  The scale is kept a normal number (it underflows only when a Q
+                // block and a K group are both all zero, where every product is zero anyway), so that a masked -inf stays -inf.
+                const float dsc = fmaxf(q8sc * ks, 1.2e-38f);
+                const bool diag = p.causal && j == I;
 
-        gt += n_tiles;
-        // ---- the item's epilogue: denominator halves to the fold warps, LSE
-        s.lsum[r & 3][g][row] = l_part;
-        dm::mbar_arrive_warp(&s.bar_l[r & 3]);
-        dm::named_bar_sync(1, kSoftmaxThreads);
-        if (g == 0) {
-            const float l = s.lsum[r & 3][0][row] + s.lsum[r & 3][1][row];
-            const bool dead = (l == 0.f) || (l != l);
-            p.lse[(int64_t)w.hc.bh * p.rm.nq + w.li * 128 + row] = dead ? -INFINITY : m_run + logf(l);
-        }
+                // ---- S for this thread's (row, key group): 64 fp32 values, 32 at a time.  The second half stays in registers from its
+                // maximum to its codes, the first is read again.
+                dm::mbar_wait(&s.bar_s_full[team], (t >> 1) & 1, wc);
+                dm::tc_fence_after();
+                float sv[32];
+                float m0 = -INFINITY, m1 = -INFINITY;
+                auto load = [&](int h) {
+                    dm::tmem_ld32(t_s + 32 * h, reinterpret_cast<uint32_t*>(sv));
+                    dm::tmem_ld_wait();
+                    if (diag) {                                    // the diagonal tile only: keys above the row
+#pragma unroll
+                        for (int c = 0; c < 32; ++c)
+                            if (g * 64 + 32 * h + c > row) sv[c] = -INFINITY;
+                    }
+                };
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    load(h);
+#pragma unroll
+                    for (int c = 0; c < 32; c += 4) {
+                        m0 = dm::fmax3(m0, sv[c], sv[c + 1]);
+                        m1 = dm::fmax3(m1, sv[c + 2], sv[c + 3]);
+                    }
+                }
+                const float gm = fmaxf(m0, m1) * dsc;
+                m_run = fmaxf(m_run, gm);
+                const bool some = m_run != -INFINITY;              // a key has been visible
+                const float ms = fmaxf(gm * dm::kLog2e, (some ? m_run * dm::kLog2e : 0.f) - dm::kPhatFloorB) - dm::kLog2_448;
+                // the ring slot of tile t - kRing has been read: its fold released the group's product before the product of tile t - 3,
+                // and S of this tile waited for the product of tile t - 2.  A group without a visible key weighs nothing.
+                s.ms[rg][g][row] = some ? ms : -INFINITY;
+                if (lane == 0) s.vs[rg][g] = vs;
+                float part0 = 0.f, part1 = 0.f;
+                uint32_t codes[16];
+                const float nms = -ms, cl = __fmul_rn(dsc, dm::kLog2e);
+#pragma unroll
+                for (int h = 1; h >= 0; --h) {
+                    if (h == 0) load(0);
+#pragma unroll
+                    for (int c = 0; c < 32; c += 4) {
+                        float x0, x1, x2, x3;
+                        dm::fma2(x0, x1, sv[c], sv[c + 1], cl, nms, nms);
+                        dm::fma2(x2, x3, sv[c + 2], sv[c + 3], cl, nms, nms);
+                        const float p0 = dm::ex2(x0), p1 = dm::ex2(x1), p2 = dm::ex2(x2), p3 = dm::ex2(x3);
+                        dm::add2(part0, part1, p0, p1);
+                        dm::add2(part0, part1, p2, p3);
+                        codes[8 * h + (c >> 2)] = dm::cvt_e4m3x4(p0, p1, p2, p3);
+                    }
+                }
+                // the codes go back into tensor memory, over the first 16 columns of this thread's own 64 scores (all read by now): the
+                // P V products take them from there as their A operand, four e4m3 per column, lane = row
+                dm::tmem_st16(t_s, codes);
+                dm::tmem_st_wait();
+                dm::tc_fence_before();
+                dm::named_bar_arrive(kBarCodes + 2 * team + g, 128 + 32);
+                if (some) {
+                    if (ms > l_ref + 8.0f) {
+                        l_part *= dm::ex2(l_ref - ms);
+                        l_ref = ms;
+                    }
+                    l_part = fmaf(dm::ex2(ms - l_ref), part0 + part1, l_part);
+                }
+            }
+            // ---- the item's epilogue: this part of the denominator to the fold warps, which write O and LSE.  The parts are numbered by
+            // the parity of the tile inside the item: the order of their sum does not depend on the CTA's walk.
+            s.lsum[r % kItems][2 * ((gt ^ team) & 1) + g][row] = make_float2(l_part, l_ref);
+            gt += n_tiles;
+            dm::mbar_arrive_warp(&s.bar_l[r % kItems]);
         }
     }
     dm::tc_fence_before();
@@ -431,9 +452,8 @@ int launch_fwd_d256(const void* q8, const void* k8, const void* v8, const float*
 }
 
 namespace dmh {
-// setmaxnreg requests of the forward's roles: 8 softmax warps keep 128, 4 fold warps take 208, 4 service warps keep 40
-constexpr int kFwdRegPool = 256 * 128 + 128 * 208 + 128 * 40;
-static_assert(kFwdRegPool <= kThreads * 128, "the roles' register requests must fit the launch pool");
+constexpr int kFwdRegPool = kSoftmaxThreads * kRegSoftmax + 256 * kRegFold + 128 * kRegService;
+static_assert(kFwdRegPool == kThreads * 72, "the roles' register requests must add up to the launch pool");
 
 int prepare_fwd(char* err, size_t errlen) {
     static DeviceOnce once;
