@@ -294,26 +294,27 @@ bwd1_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             auto fold_dk = [&](const float* g, int m) {             // two products a tile
                 dm::mbar_wait(&s.bar_x_full, m, wc);                // also orders the ring slot written before the codes
                 dm::tc_fence_after();
+                // four 16-column pieces, two in flight
                 uint32_t sa[16], sb[16];
                 dm::tmem_ld16(x_src, sa);
+                dm::tmem_ld16(x_src + 16, sb);
                 const float gk = g[m];
-                // four 16-column pieces, the next one in flight while one is added
-#pragma unroll
-                for (int pc = 0; pc < 4; ++pc) {
-                    uint32_t* cur = (pc & 1) ? sb : sa;
-                    uint32_t* nxt = (pc & 1) ? sa : sb;
-                    dm::tmem_ld_wait();
-                    if (pc < 3) {
-                        dm::tmem_ld16(x_src + 16 * (pc + 1), nxt);
-                    } else {
-                        dm::tc_fence_before();
-                        dm::named_bar_arrive(kBarXFree, 256 + 32);
-                    }
+                auto add16 = [&](int pc, const uint32_t* x) {
 #pragma unroll
                     for (int i = 0; i < 16; i += 2)
-                        dm::fma2(dk_acc[16 * pc + i], dk_acc[16 * pc + i + 1], __uint_as_float(cur[i]), __uint_as_float(cur[i + 1]), gk,
+                        dm::fma2(dk_acc[16 * pc + i], dk_acc[16 * pc + i + 1], __uint_as_float(x[i]), __uint_as_float(x[i + 1]), gk,
                                  dk_acc[16 * pc + i], dk_acc[16 * pc + i + 1]);
-                }
+                };
+                dm::tmem_ld_wait();
+                add16(0, sa);
+                dm::tmem_ld16(x_src + 32, sa);
+                add16(1, sb);
+                dm::tmem_ld16(x_src + 48, sb);
+                dm::tmem_ld_wait();
+                dm::tc_fence_before();
+                dm::named_bar_arrive(kBarXFree, 256 + 32);
+                add16(2, sa);
+                add16(3, sb);
             };
             for (int it = 0; it < w.n_it; it += 2, ++t) {
                 const float* g = s.gf[t % kGf];

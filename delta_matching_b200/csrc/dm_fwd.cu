@@ -29,7 +29,7 @@ constexpr int kStages = 3;
 constexpr int kThreads = 896;
 constexpr int kSoftmaxThreads = 512;
 constexpr int kFoldWarp = 16, kServiceWarp = 24;
-constexpr int kRegSoftmax = 72, kRegFold = 96, kRegService = 24;      // per thread after setmaxnreg; the sum is the launch pool
+constexpr int kRegSoftmax = 64, kRegFold = 104, kRegService = 40;      // per thread after setmaxnreg; the sum is the launch pool
 // Named barriers (a warp-to-warp hand-off costs a quarter of an mbarrier's; an arriving side is never a whole round ahead, because
 // its next arrival on the same barrier needs a product that is issued behind the synchronising side's).
 constexpr int kBarCodes = 1;       // + 2 * team + key group: the group's codes are in tensor memory     128 + 32
@@ -221,20 +221,28 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const uint32_t src = dm::tmem_addr(t_d0, lane_base, 64 * half);      // group 1's products: + 128
         int gt = 0;
         for (int r = 0;; ++r) {
-            const FwdItem w = fwd_item(p, r);
-            if (!w.valid) break;
+            int n_tiles;                               // all that the tile loop keeps of the item: it has no registers to spare
+            {
+                const FwdItem w = fwd_item(p, r);
+                if (!w.valid) break;
+                n_tiles = w.n_tiles;
+            }
             float o_acc[64];
 #pragma unroll
             for (int i = 0; i < 64; ++i) o_acc[i] = 0.f;
             float ref = -INFINITY;                     // o_acc's basis, log2 units: O = o_acc * 2^ref / denominator
-            for (int it = 0; it < w.n_tiles; ++it) {
+            for (int it = 0; it < n_tiles; ++it) {
                 const int t = gt + it, b = t & 1, rg = t % kRing;
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
                     dm::mbar_wait(&s.bar_d_full[b][g], (t >> 1) & 1, wc);      // also orders the ring slot written before the codes
                     dm::tc_fence_after();
-                    uint32_t sa[16], sb[16];
-                    dm::tmem_ld16(src + 128 * g, sa);
+                    // eight 8-column pieces, two in flight (16-column pieces spill beside the 64 accumulators: 1904 against 1832 us at
+                    // B1 N16384 H32); the first pair arrives while the weight is worked out
+                    uint32_t sa[8], sb[8];
+                    auto ld8 = [&](int pc, uint32_t* x) { dm::tmem_ld8(src + 128 * g + 8 * pc, x); };
+                    ld8(0, sa);
+                    ld8(1, sb);
                     const float ms = s.ms[rg][g][row], vs = s.vs[rg][g];
                     // The basis moves only when a group's basis has grown 8 binades past it (a weight stays below 2^8 times its V scale,
                     // far inside fp32), so O is rescaled a few times per item instead of at every new maximum.
@@ -246,26 +254,31 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                         for (int i = 0; i < 64; i += 2) dm::mul2(o_acc[i], o_acc[i + 1], o_acc[i], o_acc[i + 1], alpha, alpha);
                     }
                     const float wg = ms == -INFINITY ? 0.f : vs * dm::ex2(ms - ref);      // (a group without a visible key)
-                    // four 16-column pieces, the next one in flight while one is added
+                    auto add8 = [&](int pc, const uint32_t* x) {
 #pragma unroll
-                    for (int pc = 0; pc < 4; ++pc) {
-                        uint32_t* cur = (pc & 1) ? sb : sa;
-                        uint32_t* nxt = (pc & 1) ? sa : sb;
+                        for (int i = 0; i < 8; i += 2)
+                            dm::fma2(o_acc[8 * pc + i], o_acc[8 * pc + i + 1], __uint_as_float(x[i]), __uint_as_float(x[i + 1]), wg,
+                                     o_acc[8 * pc + i], o_acc[8 * pc + i + 1]);
+                    };
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
                         dm::tmem_ld_wait();
-                        if (pc < 3) {
-                            dm::tmem_ld16(src + 128 * g + 16 * (pc + 1), nxt);
-                        } else {
-                            dm::tc_fence_before();
-                            dm::named_bar_arrive(kBarDFree + g, 256 + 32);
-                        }
-#pragma unroll
-                        for (int i = 0; i < 16; i += 2)
-                            dm::fma2(o_acc[16 * pc + i], o_acc[16 * pc + i + 1], __uint_as_float(cur[i]), __uint_as_float(cur[i + 1]), wg,
-                                     o_acc[16 * pc + i], o_acc[16 * pc + i + 1]);
+                        add8(2 * q, sa);
+                        ld8(2 * q + 2, sa);
+                        add8(2 * q + 1, sb);
+                        ld8(2 * q + 3, sb);
                     }
+                    dm::tmem_ld_wait();
+                    dm::tc_fence_before();
+                    dm::named_bar_arrive(kBarDFree + g, 256 + 32);
+                    add8(6, sa);
+                    add8(7, sb);
                 }
             }
-            gt += w.n_tiles;
+            gt += n_tiles;
+            int r_again = r;
+            asm volatile("" : "+r"(r_again));
+            const FwdItem w = fwd_item(p, r_again);
             // ---- the item's epilogue: the softmax warps have left the denominator's four parts
             dm::mbar_wait(&s.bar_l[r % kItems], (r / kItems) & 1, wc);
             float2 lp[4];
