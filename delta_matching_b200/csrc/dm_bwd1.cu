@@ -1,76 +1,152 @@
-// Pass 1 of the backward, head_dim 128: dK and dV per query head, plus the e4m3 dS' code tiles and their psi scales for
-// pass 2 (csrc/mainloop_bwd_sm90_fp8r.hpp:695-952 of the reference, restated for tcgen05).
+// Pass 1 of the backward: dK and dV per query head, plus the e4m3 dS' code tiles and their psi scales for pass 2
+// (csrc/mainloop_bwd_sm90_fp8r.hpp:695-952 of the reference, restated for tcgen05).
 //
-// One work item = one 128-key block of one (batch, query head); 64-row m-blocks ascending from the causal start.  The
-// kernel is persistent: one CTA per SM walks its share of the items, and the next item starts under the tail of the
-// current one.  768 threads in three roles that meet only through mbarriers:
-//   warps 0..15  softmax, four per scheduler: thread = (key, 16-row quarter of the m-block); P-hat, dS', the tile amax, psi
-//                and the two code tiles of every m-block; they hold no accumulator (64 registers each)
-//   warps 16..19 fold: thread = key; they own dK (128 fp32 columns in registers) and drive dV's accumulator in tensor memory
-//   warps 20..23 service, one per scheduler, loops converged with one issuing lane: the S^T / dP^T tcgen05.mma, the dK / dV
-//                tcgen05.mma and the dS' TMA store, the TMA loads, the per-row constants
-// Registers move between the roles by setmaxnreg; the CTA's pool is what it was launched with (768 x 80), so what the
-// softmax and service warps give up (16 x 16 + 4 x 40 per lane) is exactly what the fold warps take (4 x 104).
-// Everything is computed transposed (keys x rows): tensor-memory lane = key, so the per-key scales are per-thread
-// constants.  Per m-block:
-//   S^T = K Q^T, dP^T = V dO^T     tcgen05.mma M128 N64 K32 x 4 each into the (S | dP) tensor-memory buffer, issued as soon
-//                                  as the softmax warps have read the previous m-block's
-//   softmax warps                  P-hat, dS' = P-hat (dP descaled - delta k8s), tile amax over the 64 x 128 tile (one named
-//                                  barrier among the softmax threads), psi by the F2 / F2b rules, codes
-//                                  P-hat8 = e4m3(P-hat), dS'8 = e4m3(dS' / psi) into two swizzled K-major tiles [key][row];
-//                                  the finished 128 x 128 dS' tile of a row pair leaves by one TMA store
-//   dV_tmp (+)= P-hat8^T dO8       M128 N128 K32 x 2, zero-initialised on the first m-block of a 128-row dO scale block
-//   dK_tmp  = dS'8^T Q8            M128 N128 K32 x 2, zero-initialised
-//   dK += dK_tmp * (psi 2^-8 q8sc)   by the fold warps, in registers, while the softmax warps are on the next m-block
-//   dV += dV_tmp * (2^-8 do8sc)       once per 128-row dO scale block: dV's fp32 accumulator lives in tensor memory
-//                                  (columns [384, 512)); the fold warps read product and accumulator, add, and store it back
-// Q8 / dO8 m-block tiles serve twice: K-major as the B operand of S^T / dP^T and MN-major as the B operand of dK / dV.
-// The dS' tile layout in global memory is [key][row] (128 x 128 bytes), which pass 2 reads as an MN-major A operand.
-#include "dm_bwd1.h"
+// One work item = one 128-key block of one (batch, query head), walked in tiles of 128 rows (two 64-row m-blocks) from the causal
+// start; at head_dim 256 one of its two d halves (Geo below).  The kernel is persistent: one CTA per SM walks its share of the items, every
+// role keeps its own place in the list, and the next item starts under the tail of the current one.  896 threads:
+//   warps 0..15  softmax: P-hat, dS', the tile maxima, psi and both code tiles
+//   warps 16..23 fold: thread = (key, 64 d columns); dK in registers, and dV's accumulator kept in the unit of the next dO block
+//   warps 24..27 service, one per scheduler: the S / dP MMAs, the dK / dV MMAs and the dS' store, the TMA loads, the row constants
+// Per tile:
+//   S = Q K^T, dP = dO V^T   M128 N128 K32 x 4 each (x 8 at head_dim 256), tensor-memory lane = row, as soon as the softmax warps hold
+//                            the previous pair
+//   softmax warps            codes P-hat8 = e4m3(P-hat), dS'8 = e4m3(dS' / psi), psi by the F2 / F2b rules from the tile maxima
+//   X = dS'8(m0)^T Q8        fold: dK += X * (psi 2^-8 q8sc)
+//   dV += P-hat8^T dO8       into the accumulator itself (tensor memory), which is in units of this block's dO scale
+//   X = dS'8(m1)^T Q8        fold: dK += X * (psi 2^-8 q8sc); then dV's accumulator times (this block's / the next one's dO scale)
+// (head_dim 256 has a dO scale per m-block: dV's product is formed m-block by m-block, its accumulator moved after each.)
+// Q8 / dO8 tiles serve twice: K-major as the A operand of S / dP and MN-major as the B operand of dK / dV.
+//
+// Why this shape.  The kernel before this one held S^T / dP^T (lane = key) for one 64-row m-block at a time: N = 64 MMAs run the
+// tensor pipe at half rate, the row constants came from shared memory in every thread (8 x 16 bytes per 16 elements), and each of
+// the two m-blocks of 128 rows was a serial chain of its own (products, exponentials, maximum over a barrier, psi, codes:
+// about 2600 clocks).  Here a chain of about 3800 clocks, which is what bounds the kernel, serves 128 x 128.  S / dP are read in the
+// matrix-fragment layout (tcgen05.ld 16x256b): a thread has four rows and eight keys of each, so the row constants are registers, and
+// a fragment of four codes is what stmatrix stores transposed, so the [key][row] code tiles (A operand of dK / dV, and the tile pass 2
+// reads) still leave as whole 16-byte chunks.  With both m-blocks in one step dV's product would be a third use of the one product
+// buffer X (tensor memory is full: S 128, dP 128, X 128, dV 128 columns), and X's round trip (MMA, commit, fold, release) sets the
+// pace then; so dV accumulates in place and only its unit is moved, off that path.
+// Measured at B4 N4096 H32 causal: 1235 us before; 1290 with dV through X; 1206 with dV in place; 1037 with the unit moved in
+// 16-column pieces (fewer spills in the fold warps, which need 64 accumulators and two 16-register pieces); 960 with 72 / 96 / 24
+// registers per role and a maximum barrier per row half; 900 with the hardware warps in the order service, fold, softmax.
+// head_dim 256 (B2 N4096 H16 full): 1350 us with the kernel before this one, 1217 with this.
+#include "dm_attn_common.cuh"
+#include "dm_host.h"
 
-namespace dmh {
-int check_shape(const DmShape& s, int h0, int hcount, char* err, size_t errlen);
+namespace dm {
+
+struct Bwd1Params {
+    const float* q8s;
+    const float* k8s;
+    const float* v8s;
+    const float* do8s;
+    const float* lse;
+    const float* delta;
+    __nv_bfloat16* dk;
+    __nv_bfloat16* dv;
+    uint8_t* ds_ws;
+    float* psi;
+    int H, Hk, N, h0, hcount, causal;
+    int* status;
+    RowMap rm;                                    // which rows of the sequence the Q-side tensors hold
+    int out_fp32;                                 // dK / dV leave as fp32 (partials that another rank's are added to)
+    int n_heads;                                  // batch * hcount: (batch, query head) pairs of this call
+    FastDiv fd_heads, fd_hcount, fd_rep, fd_nbn;  // divisions by n_heads, hcount, H / Hk and N / 128
+};
+
+// The work list: one item = one 128-key block J of one (batch, query head) (and one d half at head_dim 256), ordered by
+// key block, i.e. heaviest first when causal.  CTA c takes position c of the even rounds and G - 1 - c of the odd ones
+// (a snake), so the long and the short items of a round pair up.
+struct Bwd1Item {
+    HeadCoord hc;
+    int J, zh, m_lo, n_it, bhl;                   // m_lo, n_it: first 64-row m-block and their count, both even
+    bool valid;
+};
+template <int kD>
+__device__ __forceinline__ Bwd1Item bwd1_item(const Bwd1Params& p, int round) {
+    Bwd1Item w;
+    const int G = gridDim.x, c = blockIdx.x;
+    const int nbn = p.N / 128;
+    const int idx = round * G + ((round & 1) ? G - 1 - c : c);
+    w.valid = idx < p.n_heads * nbn * (kD / 128);
+    const int jz = (int)fdiv((uint32_t)idx, p.fd_heads);
+    w.hc = head_coord(idx - jz * p.n_heads, p.h0, p.fd_hcount, p.H, p.Hk, p.fd_rep);
+    w.bhl = w.hc.b * p.hcount + (w.hc.h - p.h0);
+    w.zh = kD == 128 ? 0 : (int)fdiv((uint32_t)jz, p.fd_nbn);   // d half whose dK / dV columns the item keeps
+    w.J = jz - w.zh * nbn;
+    // m-blocks are counted in the local rows; global position grows with the local index, and both chunks of a row map
+    // start on a 128-row pair, so local and global m-block parity agree.  Causal: start at the first local m-block that is
+    // not wholly above the diagonal of key block J; a rank may hold none (n_it == 0: dK = dV = 0 for this block).
+    const int nq_blk = p.rm.nq / 128, nbm = p.rm.nq / 64;
+    w.m_lo = 0;
+    if (p.causal) {
+        const int rest = nq_blk - p.rm.half;
+        if (w.J < p.rm.off0 + p.rm.half) w.m_lo = 2 * max(w.J - p.rm.off0, 0);
+        else if (w.J < p.rm.off1 + rest) w.m_lo = 2 * (p.rm.half + max(w.J - p.rm.off1, 0));
+        else w.m_lo = nbm;
+    }
+    w.n_it = nbm - w.m_lo;
+    return w;
 }
+
+}  // namespace dm
+
 
 namespace {
 
 constexpr int kTile = 128 * 128;
-constexpr int kHalf = 64 * 128;
-constexpr int kSoftmaxWarps = 16;      // four per scheduler: key quarter (warp & 3) x 16-row quarter of the m-block (warp >> 2)
-constexpr int kComputeThreads = 32 * kSoftmaxWarps;
-constexpr int kThreads = kComputeThreads + 256;   // + one fold warpgroup + one service warpgroup
-constexpr int kRing = 4;               // depth of the per-m-block scale ring between softmax and fold warps
+constexpr int kSoftmaxThreads = 512;
+constexpr int kFoldWarp = 16, kServiceWarp = 24;
+constexpr int kThreads = 896;
+constexpr int kRegSoftmax = 72, kRegFold = 96, kRegService = 24;     // per thread after setmaxnreg: the sum is the launch pool
+constexpr int kRows = 3;               // ring of row constants
+constexpr int kGf = 4;                 // ring of product scales between softmax and fold warps
+
+// Named barriers.  Warp-to-warp hand-offs cost a quarter of an mbarrier's; an arriving side is never a whole round ahead, because
+// its next arrival on the same barrier needs a product that is issued behind the synchronising side's.
+constexpr int kBarSpFree = 1;          // (S | dP) is in registers                          512 + 32
+constexpr int kBarAmax = 2;            // + psi tile: its warps' maxima are in shared memory  256 (head_dim 256: 128)
+constexpr int kBarCodes = 6;           // + tile parity: the tile's codes are               512 + 32
+constexpr int kBarXFree = 8;           // the fold warps hold the dK product                256 + 32
+constexpr int kBarDvFree = 9;          // dV's accumulator is in the next block's unit      256 + 32
 
 // Geometry per head dim.  head_dim 256 (csrc/mainloop_bwd_sm90_fp8v10.hpp:1674-1761 of the reference): a code row is two
-// 128-byte sub-tiles, K / V scales per 32 keys, Q / dO scales per 64-row m-block, psi per 64 rows x 64 keys (so a CTA's 128
-// keys carry two psi tiles per m-block, one per lane half), dV folded every m-block.  The dK / dV accumulators of 128 keys x
-// 256 columns do not fit the registers, so two work items (d half 0 and 1) share a key block: both form S^T / dP^T, each
-// keeps its 128 columns of dK / dV, and only d half 0 writes the dS' tiles and psi.
+// 128-byte sub-tiles, K / V scales per 32 keys, Q / dO scales per 64-row m-block (so dV's unit moves at every m-block), psi per
+// 64 rows x 64 keys.  The accumulators of 128 keys x 256 columns do not fit, so two work items (d half 0 and 1) share a key block:
+// both form S / dP, each keeps its 128 columns of dK / dV, and only d half 0 stores the dS' tiles and psi.  An item's own half of Q
+// and dO lives until the products have read it, the other half only until S / dP have: one stage of it is enough.
 template <int kD>
 struct Geo {
-    static constexpr int kDH = kD / 128;                 // 128-byte sub-tiles per code row
-    static constexpr int kStages = kD == 128 ? 4 : 3;    // Q / dO ring depth
+    static constexpr int kDH = kD / 128;
+    static constexpr int kOwn = kD == 128 ? 3 : 2;       // ring of the tiles of Q / dO that the products read (the item's d half)
+    static constexpr int kOth = kD == 128 ? 0 : 1;       // stage of the other d half
+    static constexpr int kDs = kD == 128 ? 2 : 1;        // dS' code tiles
+    static constexpr int kStgCols = kD == 128 ? 32 : 16; // columns of the output staging
     static constexpr int kKeysPerScale = kD == 128 ? 64 : 32;
-    static constexpr int kGrp = 128 / kKeysPerScale;     // K / V scale groups per key block
+    static constexpr int kGrp = 128 / kKeysPerScale;     // K / V scales per key block
+    static constexpr int kPsiKeys = kD == 128 ? 1 : 2;   // psi tiles along the keys of a key block
+    static constexpr int kPsiWarps = 8 / kPsiKeys;       // softmax warps of a psi tile
 };
 
 template <int kD>
-struct Bwd1Smem {
-    static constexpr int kDH = Geo<kD>::kDH, kStages = Geo<kD>::kStages, kGrp = Geo<kD>::kGrp;
-    alignas(1024) uint8_t k[kDH][kTile];
-    alignas(1024) uint8_t v[kDH][kTile];
-    alignas(1024) uint8_t q[kStages][kDH][kHalf];
-    alignas(1024) uint8_t dO[kStages][kDH][kHalf];
-    alignas(1024) uint8_t pt[kTile];      // P-hat codes, [key][row of the 128-row pair]; an m-block owns one 64-byte half
-    alignas(1024) uint8_t ds[2][kTile];   // dS' codes, same layout, one tile per 128-row pair parity (a TMA store drains the other)
-    alignas(1024) uint8_t stg[kD == 128 ? 2 * kTile : 16];   // head_dim 128: the epilogue's 128 rows x 256 bytes of bf16 dK / dV
-    alignas(16) float rc[3][64];                      // 8 - lse * log2e per row of the m-block (ring of 3 m-blocks)
-    alignas(16) float dlk[3][kGrp][64];               // -delta * k8s(group) per row
-    float sc[3][2];                                   // q8sc, do8sc of the m-block (same ring)
-    float gf[kRing][4];                               // per m-block: dK scale of key half 0, of key half 1, dV scale
-    float amax[2][kSoftmaxWarps];
-    uint64_t bar_kv, bar_qdo[kStages], bar_stage_free[kStages], bar_sp_full, bar_sp_free, bar_codes[2], bar_dkv_full[2],
-        bar_dkv_free, bar_ds_free[2], bar_rows_full[3], bar_rows_free[3], bar_kv_free;
+struct Smem {
+    using G = Geo<kD>;
+    alignas(1024) uint8_t k[G::kDH][kTile];
+    alignas(1024) uint8_t v[G::kDH][kTile];
+    alignas(1024) uint8_t q[G::kOwn + G::kOth][kTile];      // the own half's stages, then the other half's
+    alignas(1024) uint8_t dO[G::kOwn + G::kOth][kTile];
+    alignas(1024) uint8_t pt[2][kTile];       // P-hat codes, [key][row], by tile parity
+    alignas(1024) uint8_t ds[G::kDs][kTile];  // dS' codes, same layout
+    alignas(16) uint8_t stg[8][32 * 2 * G::kStgCols];  // per fold warp: 32 keys of bf16 columns on their way out (chunks XOR-swizzled)
+    alignas(16) float2 rd[kRows][128];        // per row: 8 - lse * log2e, -delta
+    alignas(16) float sc[kRows][8];                       // of m-block m: [m] q8sc, [2 + m] do8sc, [4 + m] what dV's accumulator is multiplied by
+                                              // before it, [6 + m] dV's unit
+    float gf[kGf][4];                         // dK scale of m-block m, 64-key half h at [2 m + h]
+    float fv[kGf];                            // dV's unit after the tile
+    float psi[kGf][4];                        // psi of m-block m (psi tile h along the keys: [2 m + h]), on its way to pass 2
+    float amax[2][16];                        // [tile parity][psi tile, warp of it]
+    uint64_t bar_kv, bar_kv_free, bar_own[3], bar_own_free[3], bar_oth, bar_oth_free, bar_sp_full, bar_x_full, bar_dv_full, bar_done[2],
+        bar_ds_free[2], bar_rows_full[kRows], bar_rows_free[kRows];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -78,41 +154,42 @@ struct Bwd1Smem {
 template <int kD>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
-                 const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                 const __grid_constant__ CUtensorMap tm_ds, const dm::Bwd1Params p) {
+            const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
+            const __grid_constant__ CUtensorMap tm_ds, const dm::Bwd1Params p) {
     extern __shared__ uint8_t smem_raw[];
     using G = Geo<kD>;
-    constexpr int kDH = G::kDH, kStages = G::kStages, kGrp = G::kGrp, kKPS = G::kKeysPerScale;
-    Bwd1Smem<kD>& s = *reinterpret_cast<Bwd1Smem<kD>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nbn = p.N / 128;
-    const int nq_blk = p.rm.nq / 128, nbm = p.rm.nq / 64;   // local 128-row blocks and 64-row m-blocks
-    // Persistent: one CTA per SM walks its items (bwd1_item).  Every role keeps its own place in the list; `gt` counts the
-    // m-blocks of the items before the current one (always even), so ring stages, buffer parities and mbarrier phases
-    // run on across items (t = gt + it below) and the next item's loads, S^T / dP^T and first m-blocks run under the
-    // current item's last folds and its epilogue.  `kvn` counts the items that loaded K / V (those with m-blocks).
+    constexpr int kDH = G::kDH, kOwn = G::kOwn;
+    Smem<kD>& s = *reinterpret_cast<Smem<kD>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    // The hardware warps are taken in the order service, fold, softmax (the role numbers below keep their tensor-memory quarter,
+    // warp mod 4): 949 -> 900 us against softmax first (B4 N4096 H32 causal).
+    const int tid = threadIdx.x, lane = tid & 31, hw_warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int warp = hw_warp < 4 ? hw_warp + kServiceWarp : (hw_warp < 12 ? hw_warp + kFoldWarp - 4 : hw_warp - 12);
+    const int nbn = p.N / 128, nq_blk = p.rm.nq / 128;
+    // `t` counts the CTA's tiles (128 rows each) over its items, so ring stages, buffer parities and mbarrier phases run on across
+    // items.  `kvn` counts the items that loaded K / V (those with tiles).
     dm::WaitCtx wc{&s.abort_flag, p.status};
 
     if (tid == 0) {
         s.abort_flag = 0;
         dm::mbar_init(&s.bar_kv, 1);
-        for (int i = 0; i < kStages; ++i) {
-            dm::mbar_init(&s.bar_qdo[i], 1);
-            dm::mbar_init(&s.bar_stage_free[i], 1);
+        dm::mbar_init(&s.bar_kv_free, 1);
+        dm::mbar_init(&s.bar_sp_full, 1);
+        dm::mbar_init(&s.bar_x_full, 1);
+        dm::mbar_init(&s.bar_dv_full, 1);
+        dm::mbar_init(&s.bar_oth, 1);
+        dm::mbar_init(&s.bar_oth_free, 1);
+        for (int i = 0; i < kOwn; ++i) {
+            dm::mbar_init(&s.bar_own[i], 1);
+            dm::mbar_init(&s.bar_own_free[i], 1);
         }
-        for (int i = 0; i < 3; ++i) {
+        for (int i = 0; i < kRows; ++i) {
             dm::mbar_init(&s.bar_rows_full[i], 1);
             dm::mbar_init(&s.bar_rows_free[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
-            dm::mbar_init(&s.bar_codes[i], kSoftmaxWarps);
-            dm::mbar_init(&s.bar_ds_free[i], 1);
-            dm::mbar_init(&s.bar_dkv_full[i], 1);
+            dm::mbar_init(&s.bar_done[i], 1);
+            dm::mbar_init(&s.bar_ds_free[i], kD == 128 ? 1 : 2);
         }
-        dm::mbar_init(&s.bar_sp_full, 1);
-        dm::mbar_init(&s.bar_sp_free, kSoftmaxWarps);
-        dm::mbar_init(&s.bar_dkv_free, 4);
-        dm::mbar_init(&s.bar_kv_free, 1);
         dm::fence_mbar_init();
     }
     if (warp == 0) dm::tmem_alloc(&s.tmem_base, 512);
@@ -120,485 +197,500 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
     __syncthreads();
     dm::tc_fence_after();
     dm::pdl_wait();
-    // tensor memory: S^T | dP^T at columns [0, 64) | [64, 128), dV product [128, 256), dK product [256, 384), dV accumulator
-    // [384, 512)
+    // tensor memory: S [0, 128) | dP [128, 256) (lane = row), product X [256, 384), dV accumulator [384, 512) (lane = key)
     const uint32_t tmem = s.tmem_base;
-    const uint32_t t_dv = tmem + 128, t_dk = tmem + 256, t_dva = tmem + 384;
+    const uint32_t t_x = tmem + 256, t_dva = tmem + 384;
     const uint32_t lane_base = (uint32_t)(warp & 3) * 32;
-    const int key = (warp & 3) * 32 + lane;       // tensor-memory lane of the softmax and fold threads
-    const int khalf = key >> 6;                   // 64-key half (the psi tile at head_dim 256)
 
-    if (warp >= kSoftmaxWarps + 4) {
-        // =============================================================== service warps (the last warpgroup), one per scheduler
-        // Each runs its loop converged (all lanes wait and compute the same addresses, so they stay in uniform registers)
-        // and lane 0 alone executes the asynchronous instruction.
-        dm::reg_dec<40>();
-        if (warp == kSoftmaxWarps + 4) {
-            // ---- S^T = K Q^T and dP^T = V dO^T of every m-block, as soon as the softmax warps have read the previous pair
-            constexpr uint32_t idesc_sp = dm::idesc_e4m3(128, 64, false, false);
-            constexpr uint32_t kSub = kTile >> 4, kSubQ = kHalf >> 4, kStageQ = (kDH * kHalf) >> 4;   // descriptor strides
-            const uint32_t k_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.k[0])), v_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.v[0]));
-            const uint32_t q_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[0][0])), do_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.dO[0][0]));
-            int gt = 0, kvn = 0;
+    if (warp >= kServiceWarp) {
+        // =============================================================== service warps: loops converged, one elected lane issues
+        dm::reg_dec<kRegService>();
+        constexpr uint32_t kSub = kTile >> 4;
+        if (warp == kServiceWarp) {
+            // ---- S = Q K^T and dP = dO V^T of every tile
+            constexpr uint32_t idesc_sp = dm::idesc_e4m3(128, 128, false, false);
+            const uint32_t k_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.k)), v_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.v));
+            const uint32_t q_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[0])), do_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.dO[0]));
+            int t = 0, kvn = 0;
             for (int r = 0;; ++r) {
                 const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
                 if (!w.valid) break;
-                if (w.n_it > 0) dm::mbar_wait(&s.bar_kv, kvn & 1, wc);
-                for (int it = 0; it < w.n_it; ++it) {
-                    const int t = gt + it, st = t % kStages;
-                    dm::mbar_wait(&s.bar_qdo[st], (t / kStages) & 1, wc);
-                    // the softmax warps read the row constants of this m-block once its products are there: waiting here
-                    // saves them a wait of their own
-                    dm::mbar_wait(&s.bar_rows_full[t % 3], (t / 3) & 1, wc);
-                    // The softmax warps rewrite, in this m-block, the P-hat half tile that the dV product of m-block t - 2 read,
-                    // and (first m-block of a row pair) the dS' tile that the TMA store of the pair two back drains: both
-                    // must be done.  Gating the products gates the softmax warps.
-                    if (t >= 2) dm::mbar_wait(&s.bar_dkv_full[t & 1], ((t - 2) >> 1) & 1, wc);
-                    const int pair = t >> 1;         // gt and m_lo are even: pairs start at even t
-                    if ((t & 1) == 0 && pair >= 2) dm::mbar_wait(&s.bar_ds_free[pair & 1], ((pair - 2) >> 1) & 1, wc);
-                    if (t >= 1) dm::mbar_wait(&s.bar_sp_free, (t - 1) & 1, wc);      // the last of them to come: nothing
-                    // else stands between it and the products (1426 -> 1355 us at head_dim 256, B2 N4096 H16 Hk4 full)
+                const int n = w.n_it >> 1;
+                if (n > 0) dm::mbar_wait(&s.bar_kv, kvn++ & 1, wc);
+                for (int it = 0; it < n; ++it, ++t) {
+                    const int st = t % kOwn;
+                    dm::mbar_wait(&s.bar_own[st], (t / kOwn) & 1, wc);
+                    if (kD == 256) dm::mbar_wait(&s.bar_oth, t & 1, wc);
+                    // The softmax warps rewrite the code tiles of tile t - 2: its products and its dS' store must be done.  Gating the
+                    // products gates the softmax warps.  (head_dim 256 has one dS' tile: they wait for tile t - 1 themselves.)
+                    if (t >= 2) {
+                        dm::mbar_wait(&s.bar_done[t & 1], ((t - 2) >> 1) & 1, wc);
+                        if (kD == 128) dm::mbar_wait(&s.bar_ds_free[t & 1], ((t - 2) >> 1) & 1, wc);
+                    }
+                    dm::mbar_wait(&s.bar_rows_full[t % kRows], (t / kRows) & 1, wc);      // saves the softmax warps a wait of their own
+                    if (t >= 1) dm::named_bar_sync(kBarSpFree, kSoftmaxThreads + 32);
                     dm::tc_fence_after();
-                    const uint32_t t_s = tmem, t_dp = tmem + 64;
-                    const uint32_t qs = q_lo + st * kStageQ, dos = do_lo + st * kStageQ;
                     if (dm::elect_one()) {
 #pragma unroll
-                        for (int hh = 0; hh < kDH; ++hh) {
+                        for (int m = 0; m < 2; ++m) {              // S, then dP; the d halves in order, whichever is the item's own
 #pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                if ((hh | k) == 0) dm::umma_e4m3_lo<false>(t_s, k_lo, qs, idesc_sp);
-                                else dm::umma_e4m3_lo<true>(t_s, k_lo + hh * kSub + 2 * k, qs + hh * kSubQ + 2 * k, idesc_sp);
-                            }
-                        }
+                            for (int hh = 0; hh < kDH; ++hh) {
+                                const uint32_t a = (m ? do_lo : q_lo) + (kD == 128 || hh == w.zh ? st : kOwn) * kSub;
+                                const uint32_t b = (m ? v_lo : k_lo) + hh * kSub, d = tmem + 128 * m;
 #pragma unroll
-                        for (int hh = 0; hh < kDH; ++hh) {
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) {
-                                if ((hh | k) == 0) dm::umma_e4m3_lo<false>(t_dp, v_lo, dos, idesc_sp);
-                                else dm::umma_e4m3_lo<true>(t_dp, v_lo + hh * kSub + 2 * k, dos + hh * kSubQ + 2 * k, idesc_sp);
+                                for (int k = 0; k < 4; ++k) {
+                                    if ((hh | k) == 0) dm::umma_e4m3_lo<false>(d, a, b, idesc_sp);
+                                    else dm::umma_e4m3_lo<true>(d, a + 2 * k, b + 2 * k, idesc_sp);
+                                }
                             }
                         }
                         dm::umma_commit(&s.bar_sp_full);
-                        // K / V have been read for the last time: the loader may bring the next item's
-                        if (it == w.n_it - 1) dm::umma_commit(&s.bar_kv_free);
+                        if (kD == 256) dm::umma_commit(&s.bar_oth_free);
+                        if (it == n - 1) dm::umma_commit(&s.bar_kv_free);     // the loader may bring the next item's K / V
                     }
                     __syncwarp();
                 }
-                if (w.n_it > 0) ++kvn;
-                gt += w.n_it;
             }
-        } else if (warp == kSoftmaxWarps + 5) {
-            // ---- dV_tmp (+)= P-hat8^T dO8 and dK_tmp = dS'8^T Q8 once the codes of an m-block are in shared memory and the
-            // fold warps have read the previous products; the finished dS' tile of a row pair leaves by one TMA store
-            constexpr uint32_t idesc_dkv = dm::idesc_e4m3(128, 128, false, true);
-            constexpr uint32_t kSub = kTile >> 4, kSubQ = kHalf >> 4, kStageQ = (kDH * kHalf) >> 4;
-            const uint32_t q_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[0][0])), do_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.dO[0][0]));
-            const uint32_t pt_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.pt)), ds_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.ds[0]));
-            int gt = 0;
+            if (t > 0) dm::named_bar_sync(kBarSpFree, kSoftmaxThreads + 32);      // the last release: no arrival is left over
+        } else if (warp == kServiceWarp + 1) {
+            // ---- dK's two products of a tile through X, dV's into its accumulator; the dS' store
+            constexpr uint32_t idesc_x = dm::idesc_e4m3(128, 128, false, true);
+            const uint32_t q_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[0])), do_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.dO[0]));
+            const uint32_t pt_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.pt[0])), ds_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.ds[0]));
+            int t = 0;
             for (int r = 0;; ++r) {
                 const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
                 if (!w.valid) break;
-                const int zh = w.zh;
-                const int ds_row0 = (int)((((int64_t)w.bhl * nq_blk + (w.m_lo >> 1)) * nbn + w.J) * 128);   // dS' tile of the first row pair
-                for (int it = 0; it < w.n_it; ++it) {
-                    const int t = gt + it, st = t % kStages, par = t & 1, pp = (t >> 1) & 1;
-                    dm::mbar_wait(&s.bar_codes[t & 1], (t >> 1) & 1, wc);
-                    // every softmax warp is past the row constants of this m-block: their ring slot may be refilled
-                    if (dm::elect_one()) dm::mbar_arrive(&s.bar_rows_free[t % 3]);
-                    if (t >= 1) dm::mbar_wait(&s.bar_dkv_free, (t - 1) & 1, wc);
-                    dm::tc_fence_after();
-                    const uint32_t qs = q_lo + st * kStageQ + zh * kSubQ, dos = do_lo + st * kStageQ + zh * kSubQ;
-                    const uint32_t pa = pt_lo + 4 * par, da = ds_lo + pp * kSub + 4 * par;
-                    if (dm::elect_one()) {
-                        // head_dim 128: dV_tmp accumulates the two m-blocks of a 128-row dO scale block; head_dim 256: one m-block
-                        dm::umma_e4m3_lo_rt(t_dv, pa, dos, idesc_dkv, (kD == 128 && par != 0) ? 1u : 0u);
-                        dm::umma_e4m3_lo<true>(t_dv, pa + 2, dos + 256, idesc_dkv);
-                        dm::umma_e4m3_lo<false>(t_dk, da, qs, idesc_dkv);
-                        dm::umma_e4m3_lo<true>(t_dk, da + 2, qs + 256, idesc_dkv);
-                        dm::umma_commit(&s.bar_dkv_full[t & 1]);
-                        dm::umma_commit(&s.bar_stage_free[st]);      // the Q / dO stage has been read for the last time
-                        if (par == 1) {
-                            // d half 1 (head_dim 256) stores nothing but arrives all the same: the phases run on across items
-                            if (zh == 0) {
-                                dm::tma_store_2d(&tm_ds, 0, ds_row0 + (it >> 1) * (nbn * 128), s.ds[pp]);
+                int ds_row = (int)((((int64_t)w.bhl * nq_blk + (w.m_lo >> 1)) * nbn + w.J) * 128);   // dS' tile of the first row block
+                const int psi_stride = nbn * G::kPsiKeys;
+                float* psi_out = p.psi + ((int64_t)w.bhl * (2 * nq_blk) + w.m_lo + (lane >> 1)) * psi_stride + G::kPsiKeys * w.J + (lane & 1);
+                const bool psi_lane = w.zh == 0 && lane < 4 && (lane & 1) < G::kPsiKeys;
+                for (int it = 0; it < w.n_it; it += 2, ++t, ds_row += nbn * 128) {
+                    const int par = t & 1, st = t % kOwn, dt = kD == 128 ? par : 0;
+                    const uint32_t qs = q_lo + st * kSub, dos = do_lo + st * kSub, da = ds_lo + dt * kSub, pa = pt_lo + par * kSub;
+                    if (kD == 128 && t >= 1 && dm::elect_one()) {       // the previous tile has left shared memory
+                        dm::tma_store_wait_read0();
+                        dm::mbar_arrive(&s.bar_ds_free[par ^ 1]);
+                    }
+                    __syncwarp();
+                    dm::named_bar_sync(kBarCodes + par, kSoftmaxThreads + 32);
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {          // the two m-blocks
+                        // dK_tmp
+                        if (t > 0 || m > 0) dm::named_bar_sync(kBarXFree, 256 + 32);
+                        dm::tc_fence_after();
+                        if (dm::elect_one()) {
+                            dm::umma_e4m3_lo<false>(t_x, da + 4 * m, qs + 512 * m, idesc_x);
+                            dm::umma_e4m3_lo<true>(t_x, da + 4 * m + 2, qs + 512 * m + 256, idesc_x);
+                            dm::umma_commit(&s.bar_x_full);
+                            if (m == 0 && w.zh == 0) {     // (d half 1 stores nothing but arrives all the same)
+                                dm::tma_store_2d(&tm_ds, 0, ds_row, s.ds[dt]);
                                 dm::tma_store_commit();
-                                dm::tma_store_wait_read0();
                             }
-                            dm::mbar_arrive(&s.bar_ds_free[pp]);
+                            if (kD == 128 && m == 1) {
+                                dm::umma_commit(&s.bar_own_free[st]);       // the stage's Q / dO have been read for the last time
+                                dm::umma_commit(&s.bar_done[par]);
+                            }
+                            if (kD == 256 && m == 1) {     // the one dS' tile has been read by both products, and has left
+                                dm::umma_commit(&s.bar_ds_free[0]);
+                                dm::tma_store_wait_read0();
+                                dm::mbar_arrive(&s.bar_ds_free[0]);
+                            }
+                        }
+                        __syncwarp();
+                        if (m == 0 && psi_lane) psi_out[(int64_t)it * psi_stride] = s.psi[t % kGf][lane];
+                        // dV += P-hat8^T dO8 of a whole dO scale block, in the accumulator itself
+                        if (kD == 256 || m == 0) {
+                            if (t > 0 || m > 0) dm::named_bar_sync(kBarDvFree, 256 + 32);
+                            dm::tc_fence_after();
+                            if (dm::elect_one()) {
+                                dm::umma_e4m3_lo_rt(t_dva, pa + 4 * m, dos + 512 * m, idesc_x, it > 0 || m > 0);
+#pragma unroll
+                                for (int k = 1; k < (kD == 128 ? 4 : 2); ++k)
+                                    dm::umma_e4m3_lo<true>(t_dva, pa + 4 * m + 2 * k, dos + 512 * m + 256 * k, idesc_x);
+                                if (kD == 256) dm::umma_commit(&s.bar_dv_full);
+                                if (kD == 128 || m == 1) dm::mbar_arrive(&s.bar_rows_free[t % kRows]);
+                                if (kD == 256 && m == 1) {
+                                    dm::umma_commit(&s.bar_own_free[st]);
+                                    dm::umma_commit(&s.bar_done[par]);
+                                }
+                            }
+                            __syncwarp();
                         }
                     }
-                    __syncwarp();
                 }
-                gt += w.n_it;
             }
-            if (gt > 0) {
-                // the last products: wait so shared memory stays valid until the tensor pipe has read it
-                dm::mbar_wait(&s.bar_dkv_free, (gt - 1) & 1, wc);
+            if (t > 0) {
+                dm::named_bar_sync(kBarXFree, 256 + 32);           // the last products: shared memory has been read
+                dm::named_bar_sync(kBarDvFree, 256 + 32);
                 if (dm::elect_one()) dm::tma_store_wait_all0();
+                __syncwarp();
             }
-        } else if (warp == kSoftmaxWarps + 6) {
-            // ---- TMA loads: an item's K / V once the previous item's last S^T / dP^T have read theirs, then the Q8 / dO8
-            // tiles of its m-blocks as far ahead as the ring allows
-            int gt = 0, kvn = 0;
+        } else if (warp == kServiceWarp + 2) {
+            // ---- TMA loads: an item's K / V once the previous item's last S / dP have read theirs, then the Q8 / dO8 tiles as far
+            // ahead as the ring allows
+            int t = 0, kvn = 0;
             for (int r = 0;; ++r) {
                 const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
                 if (!w.valid) break;
+                const int n = w.n_it >> 1;
                 const int kv_row0 = w.hc.bhk * p.N + w.J * 128;
                 const int q_row0 = w.hc.bh * p.rm.nq + w.m_lo * 64;
-                if (w.n_it > 0) {
+                if (n > 0) {
                     if (kvn >= 1) dm::mbar_wait(&s.bar_kv_free, (kvn - 1) & 1, wc);
                     if (dm::elect_one()) {
                         dm::mbar_expect_tx(&s.bar_kv, 2 * kDH * kTile);
+#pragma unroll
                         for (int hh = 0; hh < kDH; ++hh) {
                             dm::tma_load_2d(s.k[hh], &tm_k, 128 * hh, kv_row0, &s.bar_kv);
                             dm::tma_load_2d(s.v[hh], &tm_v, 128 * hh, kv_row0, &s.bar_kv);
                         }
                     }
+                    __syncwarp();
                     ++kvn;
                 }
-                for (int it = 0; it < w.n_it; ++it) {
-                    const int t = gt + it, st = t % kStages;
-                    if (t >= kStages) dm::mbar_wait(&s.bar_stage_free[st], (t / kStages - 1) & 1, wc);
+                for (int it = 0; it < n; ++it, ++t) {
+                    const int st = t % kOwn;
+                    if (t >= kOwn) dm::mbar_wait(&s.bar_own_free[st], (t / kOwn - 1) & 1, wc);
                     if (dm::elect_one()) {
-                        dm::mbar_expect_tx(&s.bar_qdo[st], 2 * kDH * kHalf);
-#pragma unroll
-                        for (int hh = 0; hh < kDH; ++hh) {
-                            dm::tma_load_2d(s.q[st][hh], &tm_q, 128 * hh, q_row0 + it * 64, &s.bar_qdo[st]);
-                            dm::tma_load_2d(s.dO[st][hh], &tm_do, 128 * hh, q_row0 + it * 64, &s.bar_qdo[st]);
-                        }
+                        dm::mbar_expect_tx(&s.bar_own[st], 2 * kTile);
+                        dm::tma_load_2d(s.q[st], &tm_q, 128 * w.zh, q_row0 + it * 128, &s.bar_own[st]);
+                        dm::tma_load_2d(s.dO[st], &tm_do, 128 * w.zh, q_row0 + it * 128, &s.bar_own[st]);
                     }
                     __syncwarp();
+                    if (kD == 256) {
+                        if (t >= 1) dm::mbar_wait(&s.bar_oth_free, (t - 1) & 1, wc);
+                        if (dm::elect_one()) {
+                            dm::mbar_expect_tx(&s.bar_oth, 2 * kTile);
+                            dm::tma_load_2d(s.q[kOwn], &tm_q, 128 * (w.zh ^ 1), q_row0 + it * 128, &s.bar_oth);
+                            dm::tma_load_2d(s.dO[kOwn], &tm_do, 128 * (w.zh ^ 1), q_row0 + it * 128, &s.bar_oth);
+                        }
+                        __syncwarp();
+                    }
                 }
-                gt += w.n_it;
             }
         } else {
-            // ---- per-row constants of the m-blocks, three ahead: 8 - lse * log2e and -delta * k8s(group) for the 64 rows
-            // (two per lane), and the Q / dO scales of the m-block
-            const int nsq = kD == 128 ? nq_blk : nbm;
-            int gt = 0;
+            // ---- the rows' constants (four per lane) and the Q / dO scales of the tile, kRows ahead
+            int t = 0;
             for (int r = 0;; ++r) {
                 const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
                 if (!w.valid) break;
-                float kk[kGrp];
+                float unit = 0.f, top = 0.f;
+                for (int it = 0; it < w.n_it; it += 2, ++t) {
+                    const int slot = t % kRows, li = (w.m_lo + it) >> 1;
+                    const int64_t gi = (int64_t)w.hc.bh * p.rm.nq + (int64_t)li * 128 + 4 * lane;
+                    float l4[4], d4[4];
 #pragma unroll
-                for (int gq = 0; gq < kGrp; ++gq) kk[gq] = p.k8s[(int64_t)w.hc.bhk * (p.N / kKPS) + kGrp * w.J + gq];
-                for (int it = 0; it < w.n_it; ++it) {
-                    const int t = gt + it, slot = t % 3, mb = w.m_lo + it;
-                    const int64_t gi = (int64_t)w.hc.bh * p.rm.nq + (int64_t)mb * 64 + 2 * lane;
-                    const float2 l2 = *reinterpret_cast<const float2*>(p.lse + gi);
-                    const float2 d2 = *reinterpret_cast<const float2*>(p.delta + gi);
-                    const int sq = (int)((int64_t)w.hc.bh * nsq) + (kD == 128 ? (mb >> 1) : mb);
-                    const float sc_v = lane == 0 ? p.q8s[sq] : (lane == 1 ? p.do8s[sq] : 0.f);
-                    if (t >= 3) dm::mbar_wait(&s.bar_rows_free[slot], (t / 3 - 1) & 1, wc);
-                    *reinterpret_cast<float2*>(&s.rc[slot][2 * lane]) = make_float2(dm::phat_row_const(l2.x), dm::phat_row_const(l2.y));
+                    for (int i = 0; i < 4; ++i) {
+                        l4[i] = p.lse[gi + i];
+                        d4[i] = p.delta[gi + i];
+                    }
+                    // Q / dO scales: of the tile's 128-row block, or of its two m-blocks
+                    const int64_t sq = kD == 128 ? (int64_t)w.hc.bh * nq_blk + li : ((int64_t)w.hc.bh * nq_blk + li) * 2;
+                    float q8sc[2], do8sc[2], mult[2], un[2];
 #pragma unroll
-                    for (int gq = 0; gq < kGrp; ++gq)
-                        *reinterpret_cast<float2*>(&s.dlk[slot][gq][2 * lane]) = make_float2(-(d2.x * kk[gq]), -(d2.y * kk[gq]));
-                    if (lane < 2) s.sc[slot][lane] = sc_v;
+                    for (int m = 0; m < 2; ++m) {
+                        q8sc[m] = kD == 256 || m == 0 ? p.q8s[sq + m] : q8sc[0];
+                        do8sc[m] = kD == 256 || m == 0 ? p.do8s[sq + m] : do8sc[0];
+                        // dV's accumulator is kept in units of the current dO scale block's scale, so that the MMAs add to it directly.
+                        // A block more than 2^-80 below the item's largest so far (an all-zero one) takes the unit at that bound: the
+                        // accumulator stays finite, and zero codes add nothing whatever the unit is.
+                        top = fmaxf(top, do8sc[m]);
+                        const float unit_new = kD == 256 || m == 0 ? fmaxf(do8sc[m], top * 0x1p-80f) : unit;
+                        mult[m] = unit / unit_new;
+                        unit = unit_new;
+                        un[m] = dm::kMoInv * unit;
+                    }
+                    if (t >= kRows) dm::mbar_wait(&s.bar_rows_free[slot], (t / kRows - 1) & 1, wc);
+#pragma unroll
+                    for (int i = 0; i < 4; i += 2)
+                        *reinterpret_cast<float4*>(&s.rd[slot][4 * lane + i]) =
+                            make_float4(dm::phat_row_const(l4[i]), -d4[i], dm::phat_row_const(l4[i + 1]), -d4[i + 1]);
+                    if (lane == 0) {
+                        *reinterpret_cast<float4*>(s.sc[slot]) = make_float4(q8sc[0], q8sc[1], do8sc[0], do8sc[1]);
+                        *reinterpret_cast<float4*>(s.sc[slot] + 4) = make_float4(mult[0], mult[1], un[0], un[1]);
+                    }
                     __syncwarp();
                     if (dm::elect_one()) dm::mbar_arrive(&s.bar_rows_full[slot]);
                 }
-                gt += w.n_it;
             }
         }
-    } else if (warp >= kSoftmaxWarps) {
-        // =============================================================== fold warps: thread = key, all 128 columns
-        dm::reg_inc<184>();
-        int gt = 0;
+    } else if (warp >= kFoldWarp) {
+        // =============================================================== fold warps: thread = (key, 64 d columns)
+        dm::reg_inc<kRegFold>();
+        const int key = (warp & 3) * 32 + lane, half = (warp >> 2) & 1;
+        const uint32_t x_src = dm::tmem_addr(t_x, lane_base, 64 * half), dva = dm::tmem_addr(t_dva, lane_base, 64 * half);
+        int t = 0;
         for (int r = 0;; ++r) {
-        const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
-        if (!w.valid) break;
-        const int J = w.J, zh = w.zh, n_it = w.n_it;
-        const dm::HeadCoord hc = w.hc;
-        const int kgrp = key / kKPS;
-        float dk_acc[128];
+            const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
+            if (!w.valid) break;
+            float dk_acc[64];
 #pragma unroll
-        for (int i = 0; i < 128; ++i) dk_acc[i] = 0.f;
-        bool dv_started = false;                  // the tensor-memory accumulator holds something of this item
-        const float ik = 1.0f / p.k8s[(int64_t)hc.bhk * (p.N / kKPS) + kGrp * J + kgrp];   // for the epilogue; read early
-        for (int it = 0; it < n_it; ++it) {
-            const int t = gt + it, r4 = t % kRing;
-            dm::mbar_wait(&s.bar_dkv_full[t & 1], (t >> 1) & 1, wc);   // also orders the ring slot written before the codes
-            dm::tc_fence_after();
-            const float gk = s.gf[r4][kD == 128 ? 0 : khalf], fv = s.gf[r4][2];
-            uint32_t sa[16], sb[16];
-            // dK: eight 16-column pieces, the next one in flight while one is added
-#define DM_DK_PIECE(PC, CUR, NXT)                                                                                       \
-            dm::tmem_ld_wait();                                                                                         \
-            if ((PC) < 7) dm::tmem_ld16(dm::tmem_addr(t_dk, lane_base, 16 * ((PC) + 1)), NXT);                           \
-            _Pragma("unroll") for (int i = 0; i < 16; i += 2)                                                            \
-                dm::fma2(dk_acc[16 * (PC) + i], dk_acc[16 * (PC) + i + 1], __uint_as_float(CUR[i]), __uint_as_float(CUR[i + 1]), gk, \
-                         dk_acc[16 * (PC) + i], dk_acc[16 * (PC) + i + 1]);
-            dm::tmem_ld16(dm::tmem_addr(t_dk, lane_base, 0), sa);
-            DM_DK_PIECE(0, sa, sb)
-            DM_DK_PIECE(1, sb, sa)
-            DM_DK_PIECE(2, sa, sb)
-            DM_DK_PIECE(3, sb, sa)
-            DM_DK_PIECE(4, sa, sb)
-            DM_DK_PIECE(5, sb, sa)
-            DM_DK_PIECE(6, sa, sb)
-            DM_DK_PIECE(7, sb, sa)
-#undef DM_DK_PIECE
-            // dV: the product of a whole dO scale block (two m-blocks at head_dim 128, one at 256) into the accumulator
-            if (kD == 256 || (t & 1) == 1) {
+            for (int i = 0; i < 64; ++i) dk_acc[i] = 0.f;
+            const float ik = 1.0f / p.k8s[(int64_t)w.hc.bhk * (p.N / G::kKeysPerScale) + G::kGrp * w.J + key / G::kKeysPerScale];   // for the epilogue; read early
+            auto fold_dk = [&](const float* g, int m) {             // two products a tile
+                dm::mbar_wait(&s.bar_x_full, m, wc);                // also orders the ring slot written before the codes
+                dm::tc_fence_after();
+                // four 16-column pieces, two in flight
+                uint32_t sa[16], sb[16];
+                dm::tmem_ld16(x_src, sa);
+                dm::tmem_ld16(x_src + 16, sb);
+                const float gk = g[2 * m];
+                auto add16 = [&](int pc, const uint32_t* x) {
 #pragma unroll
-                for (int pc = 0; pc < 8; ++pc) {
-                    dm::tmem_ld16(dm::tmem_addr(t_dv, lane_base, 16 * pc), sa);
-                    if (dv_started) dm::tmem_ld16(dm::tmem_addr(t_dva, lane_base, 16 * pc), sb);
+                    for (int i = 0; i < 16; i += 2)
+                        dm::fma2(dk_acc[16 * pc + i], dk_acc[16 * pc + i + 1], __uint_as_float(x[i]), __uint_as_float(x[i + 1]), gk,
+                                 dk_acc[16 * pc + i], dk_acc[16 * pc + i + 1]);
+                };
+                dm::tmem_ld_wait();
+                add16(0, sa);
+                dm::tmem_ld16(x_src + 32, sa);
+                add16(1, sb);
+                dm::tmem_ld16(x_src + 48, sb);
+                dm::tmem_ld_wait();
+                dm::tc_fence_before();
+                dm::named_bar_arrive(kBarXFree, 256 + 32);
+                add16(2, sa);
+                add16(3, sb);
+            };
+            auto rescale_dv = [&](float mult) {                     // dV's accumulator into the unit of the next dO scale block
+#pragma unroll
+                for (int pc = 0; pc < 4; ++pc) {
+                    uint32_t sa[16];
+                    dm::tmem_ld16(dva + 16 * pc, sa);
                     dm::tmem_ld_wait();
-                    if (dv_started) {
 #pragma unroll
-                        for (int i = 0; i < 16; i += 2) {
-                            float y0, y1;
-                            dm::fma2(y0, y1, __uint_as_float(sa[i]), __uint_as_float(sa[i + 1]), fv, __uint_as_float(sb[i]),
-                                     __uint_as_float(sb[i + 1]));
-                            sa[i] = __float_as_uint(y0);
-                            sa[i + 1] = __float_as_uint(y1);
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 16; i += 2) {
-                            float y0, y1;
-                            dm::fma2(y0, y1, __uint_as_float(sa[i]), __uint_as_float(sa[i + 1]), fv, 0.f, 0.f);
-                            sa[i] = __float_as_uint(y0);
-                            sa[i + 1] = __float_as_uint(y1);
-                        }
+                    for (int i = 0; i < 16; i += 2) {
+                        float y0, y1;
+                        dm::mul2(y0, y1, __uint_as_float(sa[i]), __uint_as_float(sa[i + 1]), mult, mult);
+                        sa[i] = __float_as_uint(y0);
+                        sa[i + 1] = __float_as_uint(y1);
                     }
-                    dm::tmem_st16(dm::tmem_addr(t_dva, lane_base, 16 * pc), sa);
+                    dm::tmem_st16(dva + 16 * pc, sa);
                 }
                 dm::tmem_st_wait();
-                dv_started = true;
-            }
-            dm::tc_fence_before();
-            dm::mbar_arrive_warp(&s.bar_dkv_free);
-        }
-
-        // ---- epilogue: dK *= 1 / k8s, dV from its accumulator, per query head.  A thread holds one row of 128 columns, and a
-        // store of 16 bytes per lane to 32 different rows costs the load/store unit one pass per row; so the bf16 rows go
-        // through shared memory (a buffer of their own, since the next item's tiles are already arriving; 16-byte chunks
-        // XOR-swizzled by the row so both sides are conflict-free) and leave as whole 256-byte rows, two per instruction.
-        // head_dim 256 has no room for that buffer and stores its rows directly, as the fp32 partials do.
-        const int n_glob = J * 128 + key;
-        const int64_t off = (((int64_t)hc.b * p.N + n_glob) * p.H + hc.h) * kD + zh * 128;
-        if (p.out_fp32) {
-#pragma unroll
-            for (int pc = 0; pc < 8; ++pc) {
-                float dvv[16];
-                if (dv_started) {
-                    dm::tmem_ld16(dm::tmem_addr(t_dva, lane_base, 16 * pc), reinterpret_cast<uint32_t*>(dvv));
-                    dm::tmem_ld_wait();
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) dvv[i] = 0.f;
-                }
-                float4* ok = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dk) + off + 16 * pc);
-                float4* ov = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dv) + off + 16 * pc);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    ok[c] = make_float4(dk_acc[16 * pc + 4 * c] * ik, dk_acc[16 * pc + 4 * c + 1] * ik, dk_acc[16 * pc + 4 * c + 2] * ik,
-                                        dk_acc[16 * pc + 4 * c + 3] * ik);
-                    ov[c] = make_float4(dvv[4 * c], dvv[4 * c + 1], dvv[4 * c + 2], dvv[4 * c + 3]);
-                }
-            }
-        } else if (kD == 256) {
-#pragma unroll
-            for (int pc = 0; pc < 8; ++pc) {
-                float dvv[16];
-                if (dv_started) {
-                    dm::tmem_ld16(dm::tmem_addr(t_dva, lane_base, 16 * pc), reinterpret_cast<uint32_t*>(dvv));
-                    dm::tmem_ld_wait();
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) dvv[i] = 0.f;
-                }
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    uint32_t wk[4], wv[4];
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const int i = 16 * pc + 8 * c + 2 * e;
-                        __nv_bfloat162 a2 = __floats2bfloat162_rn(dk_acc[i] * ik, dk_acc[i + 1] * ik);
-                        __nv_bfloat162 b2 = __floats2bfloat162_rn(dvv[8 * c + 2 * e], dvv[8 * c + 2 * e + 1]);
-                        wk[e] = *reinterpret_cast<uint32_t*>(&a2);
-                        wv[e] = *reinterpret_cast<uint32_t*>(&b2);
-                    }
-                    reinterpret_cast<uint4*>(p.dk + off + 16 * pc)[c] = make_uint4(wk[0], wk[1], wk[2], wk[3]);
-                    reinterpret_cast<uint4*>(p.dv + off + 16 * pc)[c] = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-                }
-            }
-        } else {
-            uint8_t* stg = s.stg;                                   // 128 rows x 256 bytes
-            const int wq = warp & 3;
-            const int64_t row_stride = (int64_t)p.H * kD;           // elements between consecutive keys
-            const int64_t off0 = (((int64_t)hc.b * p.N + J * 128) * p.H + hc.h) * kD + zh * 128;
-            auto rows_out = [&](__nv_bfloat16* dst) {
-                dm::named_bar_sync(2, 128);
-#pragma unroll 4
-                for (int j = 0; j < 16; ++j) {
-                    const int row = 8 * j + 2 * wq + (lane >> 4), c = lane & 15;
-                    const uint4 w = *reinterpret_cast<const uint4*>(stg + row * 256 + ((c ^ (row & 15)) << 4));
-                    *reinterpret_cast<uint4*>(dst + off0 + row * row_stride + 8 * c) = w;
-                }
-                dm::named_bar_sync(2, 128);
+                dm::tc_fence_before();
+                dm::named_bar_arrive(kBarDvFree, 256 + 32);
             };
-#pragma unroll
-            for (int c = 0; c < 16; ++c) {
-                uint32_t wk[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    __nv_bfloat162 a = __floats2bfloat162_rn(dk_acc[8 * c + 2 * e] * ik, dk_acc[8 * c + 2 * e + 1] * ik);
-                    wk[e] = *reinterpret_cast<uint32_t*>(&a);
+            for (int it = 0; it < w.n_it; it += 2, ++t) {
+                const float* g = s.gf[t % kGf] + (kD == 128 ? 0 : key >> 6);
+                fold_dk(g, 0);
+                if (kD == 256) {
+                    dm::mbar_wait(&s.bar_dv_full, 0, wc);            // two commits a tile, as for X
+                    dm::tc_fence_after();
+                    rescale_dv(s.sc[t % kRows][5]);
                 }
-                *reinterpret_cast<uint4*>(stg + key * 256 + ((c ^ (key & 15)) << 4)) = make_uint4(wk[0], wk[1], wk[2], wk[3]);
+                fold_dk(g, 1);                                       // (head_dim 128: its product was committed behind the tile's dV)
+                if (kD == 256) {
+                    dm::mbar_wait(&s.bar_dv_full, 1, wc);
+                    dm::tc_fence_after();
+                }
+                if (it + 2 < w.n_it) {
+                    const int slot = (t + 1) % kRows;
+                    dm::mbar_wait(&s.bar_rows_full[slot], ((t + 1) / kRows) & 1, wc);
+                    rescale_dv(s.sc[slot][4]);
+                }
             }
-            rows_out(p.dk);
-#pragma unroll
-            for (int pc = 0; pc < 8; ++pc) {
-                float dvv[16];
-                if (dv_started) {
-                    dm::tmem_ld16(dm::tmem_addr(t_dva, lane_base, 16 * pc), reinterpret_cast<uint32_t*>(dvv));
+
+            // ---- epilogue: dK *= 1 / k8s, dV from its accumulator, per query head
+            const bool have_dv = w.n_it > 0;
+            const float fv = have_dv ? s.fv[(t + kGf - 1) % kGf] : 0.f;      // dV's last unit
+            const int64_t row_stride = (int64_t)p.H * kD;            // elements between consecutive keys
+            const int64_t off = (((int64_t)w.hc.b * p.N + w.J * 128) * p.H + w.hc.h) * kD + 128 * w.zh + 64 * half;   // key 0 of the block
+            auto dv16 = [&](int pc, float* y) {
+                if (have_dv) {
+                    dm::tmem_ld16(dva + 16 * pc, reinterpret_cast<uint32_t*>(y));
                     dm::tmem_ld_wait();
                 } else {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) dvv[i] = 0.f;
+                    for (int i = 0; i < 16; ++i) y[i] = 0.f;
                 }
+            };
+            if (p.out_fp32) {
+                float4* ok = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dk) + off + key * row_stride);
+                float4* ov = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dv) + off + key * row_stride);
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    uint32_t wv[4];
+                for (int c = 0; c < 16; ++c)
+                    ok[c] = make_float4(dk_acc[4 * c] * ik, dk_acc[4 * c + 1] * ik, dk_acc[4 * c + 2] * ik, dk_acc[4 * c + 3] * ik);
+#pragma unroll
+                for (int pc = 0; pc < 4; ++pc) {
+                    float y[16];
+                    dv16(pc, y);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        ov[4 * pc + c] = make_float4(y[4 * c] * fv, y[4 * c + 1] * fv, y[4 * c + 2] * fv, y[4 * c + 3] * fv);
+                }
+            } else {
+                // The bf16 rows leave through the warp's own staging slice, kStgCols columns at a time: a thread holds one key, so
+                // stored directly every 16-byte store instruction would touch 32 rows; from the slice it writes 8 pieces of 64 bytes
+                // (head_dim 256: 16 of 32, whole sectors).
+                constexpr int kCh = G::kStgCols / 8;                   // 16-byte chunks per key
+                uint8_t* stg = s.stg[warp & 7];
+                auto chunk = [&](int row, int c) { return stg + row * (16 * kCh) + ((c ^ ((kCh == 4 ? row >> 1 : row >> 2) & (kCh - 1))) << 4); };
+                auto put8 = [&](int c, const float* y, float f) {      // 8 columns = one 16-byte chunk
+                    uint32_t w4[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        __nv_bfloat162 b2 = __floats2bfloat162_rn(dvv[8 * c + 2 * e], dvv[8 * c + 2 * e + 1]);
-                        wv[e] = *reinterpret_cast<uint32_t*>(&b2);
+                        __nv_bfloat162 a = __floats2bfloat162_rn(y[2 * e] * f, y[2 * e + 1] * f);
+                        w4[e] = *reinterpret_cast<uint32_t*>(&a);
                     }
-                    *reinterpret_cast<uint4*>(stg + key * 256 + (((2 * pc + c) ^ (key & 15)) << 4)) = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+                    *reinterpret_cast<uint4*>(chunk(lane, c)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+                };
+                auto out = [&](__nv_bfloat16* dst, int h) {            // 32 keys from the slice
+                    __syncwarp();
+                    const int c = lane & (kCh - 1);
+#pragma unroll
+                    for (int i = 0; i < kCh; ++i) {
+                        const int row = (32 / kCh) * i + lane / kCh;
+                        const uint4 val = *reinterpret_cast<const uint4*>(chunk(row, c));
+                        *reinterpret_cast<uint4*>(dst + off + (lane_base + row) * row_stride + G::kStgCols * h + 8 * c) = val;
+                    }
+                    __syncwarp();
+                };
+#pragma unroll
+                for (int h = 0; h < 64 / G::kStgCols; ++h) {
+#pragma unroll
+                    for (int c = 0; c < kCh; ++c) put8(c, dk_acc + G::kStgCols * h + 8 * c, ik);
+                    out(p.dk, h);
+                }
+#pragma unroll
+                for (int h = 0; h < 64 / G::kStgCols; ++h) {
+#pragma unroll
+                    for (int pc = 0; pc < kCh / 2; ++pc) {
+                        float y[16];
+                        dv16((kCh / 2) * h + pc, y);
+                        put8(2 * pc, y, fv);
+                        put8(2 * pc + 1, y + 8, fv);
+                    }
+                    out(p.dv, h);
                 }
             }
-            rows_out(p.dv);
-        }
-        dm::tc_fence_before();
-        gt += n_it;
+            if (have_dv) {
+                dm::tc_fence_before();
+                dm::named_bar_arrive(kBarDvFree, 256 + 32);
+            }
         }
     } else {
         // =============================================================== softmax warps
-        dm::reg_dec<64>();
-        const int g = warp >> 2;                      // row quarter: rows [16 g, 16 g + 16) of the m-block
-        const int kgrp = key / kKPS;                  // K / V scale group inside the block
-        int gt = 0;
+        dm::reg_dec<kRegSoftmax>();
+        const int rq = warp & 3, kq = warp >> 2;      // rows [32 rq, +32) and keys [32 kq, +32) of the tile
+        const int rhalf = rq >> 1;                    // the 64-row m-block
+        const int psi_tile = kD == 128 ? rhalf : 2 * rhalf + (kq >> 1);
+        const bool leader = (warp & (kD == 128 ? 13 : 5)) == 0;      // one warp of each psi tile
+        const int row_t = 32 * rq + (lane >> 2);      // the thread's rows: row_t + {0, 8, 16, 24}
+        const int key_t = 32 * kq + 2 * (lane & 3);   // its keys: key_t + 8 j + {0, 1}
+        const uint32_t t_s = dm::tmem_addr(tmem, lane_base, 32 * kq);
+        // this lane's line of the transposed stores: key 32 kq + lane, the 16-byte chunk of rows [32 rq, +16) (the next chunk: ^ 16)
+        const uint32_t st_addr = dm::smem_u32(s.pt[0]) + (32 * kq + lane) * 128 + (((2 * rq) ^ (lane & 7)) << 4);
+        const uint32_t ds_off = dm::smem_u32(s.ds[0]) - dm::smem_u32(s.pt[0]);
+        int t = 0, rb = 0;                            // tiles so far; ring slot of the row constants
         for (int r = 0;; ++r) {
-        const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
-        if (!w.valid) break;
-        // few values live across the m-block loop (these warps run on 64 registers): the item's psi column as a pointer,
-        // and whether its first row pair is the diagonal block of this key block (it is the first one of the causal loop)
-        const int n_it = w.n_it;
-        const float k8s_t = p.k8s[(int64_t)w.hc.bhk * (p.N / kKPS) + kGrp * w.J + kgrp];
-        const float v8s_t = p.v8s[(int64_t)w.hc.bhk * (p.N / kKPS) + kGrp * w.J + kgrp];
-        const bool diag_item = p.causal && n_it > 0 && dm::global_block(p.rm, w.m_lo >> 1) == w.J;
-        constexpr bool kHalfPsi = kD == 256;     // psi per 64 keys: [heads, N/64, N/64]; else [heads, N/64, N/128]
-        const int psi_stride = kHalfPsi ? nbm : nbn;
-        float* psi_it = w.zh == 0 ? p.psi + ((int64_t)w.bhl * nbm + w.m_lo) * psi_stride + (kHalfPsi ? 2 * w.J + khalf : w.J) : nullptr;
-        float g_max = 0.f;
+            const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
+            if (!w.valid) break;
+            const int n_it = w.n_it >> 1;
+            const float k8s_t = p.k8s[(int64_t)w.hc.bhk * (p.N / G::kKeysPerScale) + G::kGrp * w.J + 32 * kq / G::kKeysPerScale];
+            const float v8s_t = p.v8s[(int64_t)w.hc.bhk * (p.N / G::kKeysPerScale) + G::kGrp * w.J + 32 * kq / G::kKeysPerScale];
+            const bool diag_item = p.causal && n_it > 0 && dm::global_block(p.rm, w.m_lo >> 1) == w.J;
+            float g_max = 0.f;
 
-        for (int it = 0; it < n_it; ++it) {
-            const int t = gt + it, par = t & 1, sb = t & 1, rb = t % 3;     // gt and m_lo are even: t has the m-block's parity
-            dm::mbar_wait(&s.bar_sp_full, t & 1, wc);
-            dm::tc_fence_after();
-            // the ring slot of this m-block's row constants and scales was complete before S^T / dP^T were issued
-            const float q8sc = s.sc[rb][0], do8sc = s.sc[rb][1];
-            const float dsc = dm::descale_log2(q8sc, k8s_t);
-            const float dpk = do8sc * v8s_t * k8s_t;
+            for (int it = 0; it < n_it; ++it, ++t, rb = rb == kRows - 1 ? 0 : rb + 1) {
+                const int par = t & 1;
+                dm::mbar_wait(&s.bar_sp_full, par, wc);
+                const float q8sc = s.sc[rb][rhalf], do8sc = s.sc[rb][2 + rhalf];
+                const float dsc = dm::descale_log2(q8sc, k8s_t);
+                const float dpk = do8sc * v8s_t * k8s_t;
+                const float2* rd = &s.rd[rb][row_t];
+                const uint32_t addr = st_addr + par * kTile, ds_addr = st_addr + ds_off + (kD == 128 ? par * kTile : 0);
+                dm::tc_fence_after();
 
-            // ---- phase 1: P-hat, dS', tile amax; P-hat codes to shared memory.  S^T first: the exponentials run while
-            // dP^T is still on its way from tensor memory.
-            float sv[16], ds[16];
-            dm::tmem_ld16(dm::tmem_addr(tmem, lane_base, g * 16), reinterpret_cast<uint32_t*>(sv));
-            dm::tmem_ld_wait();
-            dm::tmem_ld16(dm::tmem_addr(tmem + 64, lane_base, g * 16), reinterpret_cast<uint32_t*>(ds));
-            const bool diag = diag_item && it < 2;
-            const int row_in_pair = par * 64 + g * 16;     // row offset of column 0 inside the 128-row pair
-            const float4* rc4 = reinterpret_cast<const float4*>(&s.rc[rb][g * 16]);
-            const float4* dl4 = reinterpret_cast<const float4*>(&s.dlk[rb][kgrp][g * 16]);
+                // ---- phase 1: P-hat, dS', tile amax; P-hat codes to shared memory.  Two halves of 16 rows; S first: the
+                // exponentials run while dP is still on its way from tensor memory.
+                float ds[32], am0 = 0.f, am1 = 0.f;
 #pragma unroll
-            for (int c4 = 0; c4 < 4; ++c4) {                // P-hat = 2^min(S dsc + rc, 12), the exponent two at a time
-                const float4 r4 = rc4[c4];
-                const int c = 4 * c4;
-                dm::fma2(sv[c], sv[c + 1], sv[c], sv[c + 1], dsc, r4.x, r4.y);
-                dm::fma2(sv[c + 2], sv[c + 3], sv[c + 2], sv[c + 3], dsc, r4.z, r4.w);
+                for (int h = 0; h < 2; ++h) {
+                    float sv[16], *dp = ds + 16 * h;
+                    dm::tmem_ld16x256_x4(t_s + (16u << 16) * h, reinterpret_cast<uint32_t*>(sv));
+                    const float2 ra = rd[16 * h], rb2 = rd[16 * h + 8];
+                    dm::tmem_ld_wait();
+                    dm::tmem_ld16x256_x4(t_s + 128 + (16u << 16) * h, reinterpret_cast<uint32_t*>(dp));
 #pragma unroll
-                for (int e = 0; e < 4; ++e) sv[c + e] = dm::ex2(fminf(sv[c + e], dm::kMoE + 4.0f));
-            }
-            if (diag) {                                     // the diagonal 128 x 128 block only: keys above the row
+                    for (int j = 0; j < 16; j += 4) {           // P-hat = 2^min(S dsc + rc, 12), the exponent two at a time
+                        dm::fma2(sv[j], sv[j + 1], sv[j], sv[j + 1], dsc, ra.x, ra.x);
+                        dm::fma2(sv[j + 2], sv[j + 3], sv[j + 2], sv[j + 3], dsc, rb2.x, rb2.x);
 #pragma unroll
-                for (int c = 0; c < 16; ++c)
-                    if (key > row_in_pair + c) sv[c] = 0.f;
-            }
-            dm::tmem_ld_wait();
-            dm::tc_fence_before();
-            dm::mbar_arrive_warp(&s.bar_sp_free);          // the (S | dP) buffer may be overwritten
-            float am4[4] = {0.f, 0.f, 0.f, 0.f};
+                        for (int e = 0; e < 4; ++e) sv[j + e] = dm::ex2(fminf(sv[j + e], dm::kMoE + 4.0f));
+                    }
+                    if (diag_item && it == 0) {                 // the diagonal 128 x 128 block only: keys above the row
 #pragma unroll
-            for (int c4 = 0; c4 < 4; ++c4) {
-                const float4 d4 = dl4[c4];                  // -delta * k8s per row
-                const int c = 4 * c4;
-                dm::fma2(ds[c], ds[c + 1], ds[c], ds[c + 1], dpk, d4.x, d4.y);
-                dm::fma2(ds[c + 2], ds[c + 3], ds[c + 2], ds[c + 3], dpk, d4.z, d4.w);
-                dm::mul2(ds[c], ds[c + 1], ds[c], ds[c + 1], sv[c], sv[c + 1]);
-                dm::mul2(ds[c + 2], ds[c + 3], ds[c + 2], ds[c + 3], sv[c + 2], sv[c + 3]);
+                        for (int j = 0; j < 16; ++j)
+                            if (key_t + 2 * (j & ~3) + (j & 1) > row_t + 16 * h + 4 * (j & 2)) sv[j] = 0.f;
+                    }
+                    dm::tmem_ld_wait();
+                    if (h == 1) {
+                        dm::tc_fence_before();
+                        dm::named_bar_arrive(kBarSpFree, kSoftmaxThreads + 32);     // (S | dP) may be overwritten
+                    }
+                    const float da = ra.y * k8s_t, db = rb2.y * k8s_t;              // -delta * k8s
 #pragma unroll
-                for (int e = 0; e < 4; ++e) am4[e] = fmaxf(am4[e], fabsf(ds[c + e]));
-            }
-            float amax = fmaxf(fmaxf(am4[0], am4[1]), fmaxf(am4[2], am4[3]));
-            {
-                uint32_t w[4];
+                    for (int j = 0; j < 16; j += 4) {
+                        dm::fma2(dp[j], dp[j + 1], dp[j], dp[j + 1], dpk, da, da);
+                        dm::fma2(dp[j + 2], dp[j + 3], dp[j + 2], dp[j + 3], dpk, db, db);
+                        dm::mul2(dp[j], dp[j + 1], dp[j], dp[j + 1], sv[j], sv[j + 1]);
+                        dm::mul2(dp[j + 2], dp[j + 3], dp[j + 2], dp[j + 3], sv[j + 2], sv[j + 3]);
+                        am0 = dm::fmax3_abs(am0, dp[j], dp[j + 1]);
+                        am1 = dm::fmax3_abs(am1, dp[j + 2], dp[j + 3]);
+                    }
+                    uint32_t c4[4];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) w[c] = dm::cvt_e4m3x4(sv[4 * c], sv[4 * c + 1], sv[4 * c + 2], sv[4 * c + 3]);
-                *reinterpret_cast<uint4*>(s.pt + dm::sw128(key, row_in_pair)) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-            // the warp's maximum in one instruction: non-negative floats order like their bit patterns
-            amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
-            if (lane == 0) s.amax[sb][warp] = amax;
-            dm::named_bar_sync(1, kComputeThreads);
-            // the tile maximum over the warps' maxima: one load per lane and one warp reduction.  head_dim 256: the psi tile is
-            // this thread's 64-key half, i.e. the warps of key quarters 2h and 2h+1 (warp & 2 selects the half)
-            {
-                const float a = s.amax[sb][lane & (kSoftmaxWarps - 1)];
-                const bool mine = kD == 128 || (((lane & 3) >> 1) == khalf);
-                amax = __uint_as_float(__reduce_max_sync(0xffffffffu, mine ? __float_as_uint(a) : 0u));
-            }
-            const bool tile_zero = amax * (1.0f / 448.0f) < 1e-30f;
-            const float psi_raw = fmaxf(amax * (1.0f / 448.0f), 1e-30f);
-            // psi = max(psi_raw, g_max * 256e-8 / q8sc); the quotient can only win when its numerator exceeds
-            // psi_raw * q8sc, so the division is formed only then (the 1 % margin covers the rounding of both sides)
-            float psi = psi_raw;
-            const float fl_num = g_max * (256.0f * 1e-8f);
-            if (fl_num > psi_raw * q8sc * 0.99f) psi = fmaxf(psi_raw, fl_num / q8sc);
-            const float psi_inv = tile_zero ? 0.f : __frcp_rn(psi);     // the correctly rounded reciprocal, as 1 / psi
-            const float g_cur = tile_zero ? 0.f : psi * dm::kMoInv * q8sc;
-            g_max = fmaxf(g_max, g_cur);
-            // psi for pass 2 and the scales of this m-block's products for the fold warps.  The ring slot was last read by
-            // the fold of m-block it - kRing, which came before the products of m-block it - 2 that S^T of this one waited for.
-            if (tid == 0 || (kD == 256 && tid == 64)) {
-                s.gf[t % kRing][khalf] = g_cur;
-                if (tid == 0) s.gf[t % kRing][2] = dm::kMoInv * do8sc;
-                if (psi_it) psi_it[(int64_t)it * psi_stride] = tile_zero ? 0.f : psi;
-            }
-
-            // ---- phase 2: dS' codes, to shared memory for dK and to the workspace tile for pass 2
-            uint8_t* dst = s.ds[(t >> 1) & 1];        // gt and m_lo are even: t >> 1 counts this CTA's row pairs
-            {
-                uint32_t w[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    float a0, a1, a2, a3;
-                    dm::mul2(a0, a1, ds[4 * c], ds[4 * c + 1], psi_inv, psi_inv);
-                    dm::mul2(a2, a3, ds[4 * c + 2], ds[4 * c + 3], psi_inv, psi_inv);
-                    w[c] = dm::cvt_e4m3x4(a0, a1, a2, a3);
+                    for (int j = 0; j < 4; ++j) c4[j] = dm::cvt_e4m3x4(sv[4 * j], sv[4 * j + 1], sv[4 * j + 2], sv[4 * j + 3]);
+                    dm::stmatrix_t_b8_x4(addr ^ (16 * h), c4);
                 }
-                *reinterpret_cast<uint4*>(dst + dm::sw128(key, row_in_pair)) = make_uint4(w[0], w[1], w[2], w[3]);
+                // the warp's maximum in one instruction: non-negative floats order like their bit patterns
+                const float am = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(am0, am1))));
+                if (lane == 0) s.amax[par][8 * rhalf + 2 * kq + (rq & 1)] = am;
+                if (kD == 256 && leader && t >= 1) dm::mbar_wait(&s.bar_ds_free[0], (t - 1) & 1, wc);   // one dS' tile: it is free
+                dm::named_bar_sync(kBarAmax + psi_tile, 32 * G::kPsiWarps);
+                // psi of the tile: psi = max(psi_raw, g_max * 256e-8 / q8sc); the quotient can only win when its numerator
+                // exceeds psi_raw * q8sc, so the division is formed only then (the 1 % margin covers the rounding of both sides).
+                // g_max runs over the psi tiles of this row half: the floor acts only on a tile whose maximum lies eight decades
+                // below an earlier one's, and one barrier for both halves and both psi in every thread cost 3 %.
+                float psi_my;
+                {
+                    const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(s.amax[par][psi_tile * G::kPsiWarps + (lane & (G::kPsiWarps - 1))])));
+                    const float amx = mx * (1.0f / 448.0f);
+                    psi_my = fmaxf(amx, 1e-30f);
+                    const float fl_num = g_max * (256.0f * 1e-8f);
+                    if (fl_num > psi_my * q8sc * 0.99f) psi_my = fmaxf(psi_my, fl_num / q8sc);
+                    if (amx < 1e-30f) psi_my = 0.f;                          // a zero tile
+                }
+                const float g_my = psi_my * dm::kMoInv * q8sc;
+                g_max = fmaxf(g_max, g_my);
+                const float psi_inv = psi_my == 0.f ? 0.f : __frcp_rn(psi_my);   // the correctly rounded reciprocal, as 1 / psi
+
+                // ---- phase 2: dS' codes, to shared memory for dK and for the tile that leaves to pass 2
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t c4[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float a0, a1, a2, a3;
+                        dm::mul2(a0, a1, ds[16 * h + 4 * j], ds[16 * h + 4 * j + 1], psi_inv, psi_inv);
+                        dm::mul2(a2, a3, ds[16 * h + 4 * j + 2], ds[16 * h + 4 * j + 3], psi_inv, psi_inv);
+                        c4[j] = dm::cvt_e4m3x4(a0, a1, a2, a3);
+                    }
+                    dm::stmatrix_t_b8_x4((ds_addr ^ (16 * h)), c4);
+                }
+                // the scales of this tile's products for the fold warps (the ring slot was last read four tiles ago; S of this tile
+                // waited for the products of two tiles ago) and psi, which the product warp takes to global memory
+                if (leader && lane == 0) {
+                    const int i = kD == 128 ? 2 * rhalf : psi_tile;
+                    s.gf[t % kGf][i] = g_my;
+                    s.psi[t % kGf][i] = psi_my;
+                    if (warp == 0) s.fv[t % kGf] = s.sc[rb][7];
+                }
+                dm::fence_proxy_async_smem();
+                dm::named_bar_arrive(kBarCodes + par, kSoftmaxThreads + 32);
             }
-            dm::fence_proxy_async_smem();
-            dm::mbar_arrive_warp(&s.bar_codes[sb]);
-        }
-        gt += n_it;
         }
     }
     dm::tc_fence_before();
@@ -609,22 +701,20 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
 }  // namespace
 
 namespace dmh {
+int check_shape(const DmShape& s, int h0, int hcount, char* err, size_t errlen);
 int check_cp(const DmShape& s, const DmCp& cp, char* err, size_t errlen);
 }
 
 namespace dmh {
-int prepare_bwd1_d128(char* err, size_t errlen);
-int launch_bwd1_d128(const CUtensorMap& tq, const CUtensorMap& td, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& ts,
-                     const dm::Bwd1Params& p, int grid, void* stream, char* err, size_t errlen);
 int prepare_bwd1(char* err, size_t errlen) {
     static DeviceOnce once;
     return device_once(once, err, errlen, [&]() -> int {
-        DM_CUDA(cudaFuncSetAttribute(bwd1_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Bwd1Smem<256>) + 1024));
-        // setmaxnreg requests: 16 softmax warps keep 64, 4 fold warps take 184, 4 service warps keep 40
-        constexpr int kPool = kComputeThreads * 64 + 128 * 184 + 128 * 40;
-        static_assert(kPool == kThreads * 80, "the roles' register requests must add up to the launch pool");
-        if (int rc = check_register_pool((const void*)bwd1_kernel<256>, kThreads, kPool, err, errlen)) return rc;
-        return prepare_bwd1_d128(err, errlen);
+        DM_CUDA(cudaFuncSetAttribute(bwd1_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<128>) + 1024));
+        DM_CUDA(cudaFuncSetAttribute(bwd1_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<256>) + 1024));
+        constexpr int kPool = kSoftmaxThreads * kRegSoftmax + 256 * kRegFold + 128 * kRegService;
+        static_assert(kPool == kThreads * 72, "the roles' register requests must add up to the launch pool");
+        if (int rc = check_register_pool((const void*)bwd1_kernel<128>, kThreads, kPool, err, errlen)) return rc;
+        return check_register_pool((const void*)bwd1_kernel<256>, kThreads, kPool, err, errlen);
     });
 }
 }  // namespace dmh
@@ -671,8 +761,8 @@ extern "C" int dm_bwd_fp8_pass1_cp(const void* q8, const void* k8, const void* v
     DM_REQUIRE(ntiles * 128 < ((uint64_t)1 << 31), DM_ERR_ARG, "dS' workspace too large for one call: split the heads (got %llu tiles)",
                (unsigned long long)ntiles);
     CUtensorMap tq, td, tk, tv, ts;
-    if ((rc = dmh::make_tmap_u8(&tq, q8, sh.D, (uint64_t)sh.B * sh.H * cp.nq, sh.D == 128 ? 128 : 64, err, errlen))) return rc;
-    if ((rc = dmh::make_tmap_u8(&td, do8, sh.D, (uint64_t)sh.B * sh.H * cp.nq, sh.D == 128 ? 128 : 64, err, errlen))) return rc;
+    if ((rc = dmh::make_tmap_u8(&tq, q8, sh.D, (uint64_t)sh.B * sh.H * cp.nq, 128, err, errlen))) return rc;
+    if ((rc = dmh::make_tmap_u8(&td, do8, sh.D, (uint64_t)sh.B * sh.H * cp.nq, 128, err, errlen))) return rc;
     if ((rc = dmh::make_tmap_u8(&tk, k8, sh.D, (uint64_t)sh.B * sh.Hk * sh.N, 128, err, errlen))) return rc;
     if ((rc = dmh::make_tmap_u8(&tv, v8, sh.D, (uint64_t)sh.B * sh.Hk * sh.N, 128, err, errlen))) return rc;
     if ((rc = dmh::make_tmap_u8(&ts, ds8_ws, 128, ntiles * 128, 128, err, errlen))) return rc;
@@ -684,12 +774,11 @@ extern "C" int dm_bwd_fp8_pass1_cp(const void* q8, const void* k8, const void* v
                  dm::make_fastdiv(sh.N / 128)};
     // persistent: one CTA per SM walks the (key block, head[, d half]) items, heaviest first
     if ((rc = dmh::prepare_bwd1(err, errlen))) return rc;
-    const int smem = (int)sizeof(Bwd1Smem<256>) + 1024;
     int sms = 0;
     if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
     const int64_t items = (int64_t)sh.B * hcount * (sh.N / 128) * (sh.D / 128);
     const int grid = (int)(items < sms ? items : sms);
-    if (sh.D == 128) return dmh::launch_bwd1_d128(tq, td, tk, tv, ts, p, grid, stream, err, errlen);
-    DM_CUDA(dmh::launch_pdl(bwd1_kernel<256>, grid, kThreads, smem, stream, tq, td, tk, tv, ts, p));
+    if (sh.D == 128) DM_CUDA(dmh::launch_pdl(bwd1_kernel<128>, grid, kThreads, sizeof(Smem<128>) + 1024, stream, tq, td, tk, tv, ts, p));
+    else DM_CUDA(dmh::launch_pdl(bwd1_kernel<256>, grid, kThreads, sizeof(Smem<256>) + 1024, stream, tq, td, tk, tv, ts, p));
     return DM_OK;
 }

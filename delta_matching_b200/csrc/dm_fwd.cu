@@ -2,23 +2,32 @@
 // faithful P basis (per row, per 64-key group) -- csrc/softmax_fq8f.h and csrc/mainloop_fwd_sm90_fp8f.hpp of the
 // reference, restated for tcgen05.
 //
-// One CTA = 128 query rows of one (batch, head).  512 threads in four roles:
-//   warps 0..7   softmax: thread (quarter q, lane, warpgroup g) owns row 32q+lane and key group g of every key tile
-//   warps 8..11  fold: thread = row; they own O (128 fp32 columns per thread) and nothing else
-//   warps 12..14 service (one issuing lane each, loops converged): 12 issues S, 13 issues the P V products, 14 the TMA loads
+// One work item = 128 query rows of one (batch, head); the kernel is persistent, one CTA per SM walks a list of items, and since
+// every role keeps its own place in the list, the loads and S of the next item start while the current one is finished.  896 threads:
+//   warps 0..15   softmax, two teams of eight on alternating key tiles: thread = (row, 64-key group of its team's tiles)
+//   warps 16..23  fold: thread = (row, 64 of O's 128 columns); they own O, the LSE and nothing else
+//   warps 24..27  service (converged loops, one elected lane issues): S; the products of key group 0; of key group 1; the TMA loads
 // Key tiles of 128 keys (two 64-key groups) are visited from the diagonal tile downwards.  Per tile:
-//   S = Q K^T            4 x tcgen05.mma (M128 N128 K32) into one of two tensor-memory buffers, up to two tiles ahead
-//   softmax              group max, running max exchanged through shared memory, basis
-//                        ms_g = max(gm_g*l2, m*l2 - 12) - log2(448), codes = e4m3(2^(S*l2 - ms_g)) written back into tensor
-//                        memory over the scores they came from (four codes per column, lane = row); the denominator is
-//                        summed from the unrounded p; the tile's alpha and the two weights w_g = v8sc_g * 2^(ms_g - m*l2)
-//                        per row go to a small ring for the fold warps
+//   S = Q K^T            4 x tcgen05.mma (M128 N128 K32) into the tensor-memory buffer of the tile's parity, i.e. of its team
+//   softmax              basis ms_g = max(gm_g*l2, m*l2 - 12) - log2(448) (gm: the group's maximum in this tile, m: the thread's own
+//                        running one), codes = e4m3(2^(S*l2 - ms_g)) written back into tensor memory over the scores they came from
+//                        (four codes per column, lane = row); the denominator's part is summed from the unrounded p.  ms_g goes to a
+//                        ring; nothing is exchanged between softmax threads
 //   D_g = C_g V_g        2 x tcgen05.mma per group (A = the codes in tensor memory, B = the V tile) into zero-initialised
-//                        tensor-memory temporaries, issued when the codes are stored and the previous products have been read
-//   O = O * alpha + D_0 w_0 + D_1 w_1   by the fold warps, in that order, while the softmax warps are on the next tile
-// K / V tiles arrive by TMA into a 3-stage ring.  The kernel is persistent: one CTA per SM walks a list of (head, row
-// block) items, and since every role keeps its own place in the list, the loads and S of the next item start while the
-// softmax and fold warps finish the current one.  Every mbarrier wait is bounded.
+//                        tensor-memory temporaries, issued when the codes are stored and the previous product has been read
+//   O += D_g * v8sc_g 2^(ms_g - ref)    by the fold warps; ref, O's basis, moves only when ms_g has passed it by 8 binades, and O is
+//                        divided by the denominator (the sum of the four threads' parts of a row) once, at the item's end
+// K / V tiles arrive by TMA into a 3-stage ring.  Every mbarrier wait is bounded.
+//
+// Why this shape.  A 128 x 128 tile holds 1024 clocks of exponentials and 512 of MMAs; with one set of softmax warps the wait for
+// S, the maxima, the exchange of the running maximum and the codes (about 1200 clocks a tile) ran with the exponential unit idle.  Two
+// teams half a tile apart overlap them, which needs two things gone: the running maximum handed from tile to tile (a serial chain
+// through both teams: measured slower than one set) and the rescaling of O at every new maximum.  A running maximum of the
+// thread's own only lowers the 12-binade floor of a group's basis (never the precision of its codes), and the bases, all powers
+// of two's arguments kept in fp32, meet in the fold.  The kernel is now bound by the fold (about 1950 clocks a tile: 2 x 64
+// tensor-memory columns and 128 multiply-adds per thread next to the MMAs' traffic); its 64 accumulators leave room for 8-column pieces only.
+// Measured (us, before -> two teams -> 8-column pieces): B1 N16384 H32 causal 2023 -> 1904 -> 1835; B4 N4096 H32 causal
+// 577 -> 560 -> 535; B2 N2048 H16 causal 51.2 -> 49.5.
 #include "dm_attn_common.cuh"
 #include "dm_host.h"
 
