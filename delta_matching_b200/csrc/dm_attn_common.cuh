@@ -7,7 +7,6 @@
 namespace dm {
 
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kLog2_448 = 8.8073549220576042f;   // csrc/softmax_fq8f.h:153 of the reference
 constexpr float kPhatFloorB = 12.0f;               // P-hat basis floor in binades below the running max (softmax_fq8f.h:147)
 constexpr float kMoE = 8.0f;                       // backward P-hat offset 2^8 (mainloop_bwd_sm90_fp8r.hpp:664)

@@ -52,7 +52,7 @@ struct FwdSmem {
     alignas(1024) uint8_t v[kStages][kTile];
     float ms[kRing][2][128];          // [tile % kRing][key group][row]: the basis of the row's codes, log2 units
     float vs[kRing][2];               // the group's V scale
-    float2 lsum[kItems][4][128];      // [work item % kItems][2 * (tile parity in the item) + key group][row]: part of the denominator and its unit (log2)
+    float2 lsum[kItems][4][128];      // [work item % kItems][2 * (tile parity in the item) + key group][row]: part of the denominator and its unit (the maximum it was taken against)
     alignas(16) uint8_t stg[8][32 * 128];   // per fold warp: its 32 bf16 half rows of O on their way out (16-byte chunks XOR-swizzled by the row)
     uint64_t bar_q[2], bar_q_free[2], bar_kv[kStages], bar_kv_free[kStages], bar_s_full[2], bar_d_full[2][2], bar_l[kItems];   // bar_d_full: [tile parity][key group]
     uint32_t tmem_base;
@@ -293,13 +293,13 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             float2 lp[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) lp[i] = s.lsum[r % kItems][i][row];
-            const float unit = fmaxf(fmaxf(lp[0].y, lp[1].y), fmaxf(lp[2].y, lp[3].y));
+            const float m = fmaxf(fmaxf(lp[0].y, lp[1].y), fmaxf(lp[2].y, lp[3].y));
             float l = 0.f;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) l += lp[i].x * dm::ex2(lp[i].y - unit);
+            for (int i = 0; i < 4; ++i) l += lp[i].x * dm::ex2((lp[i].y - m) * dm::kLog2e);
             const bool dead = (l == 0.f) || (l != l);
-            const float inv = dead ? 0.f : dm::ex2(ref - unit) / l;
-            if (half == 0) p.lse[(int64_t)w.hc.bh * p.rm.nq + w.li * 128 + row] = dead ? -INFINITY : unit * dm::kLn2 + logf(l);
+            const float inv = dead ? 0.f : dm::ex2(ref - m * dm::kLog2e) / l;
+            if (half == 0) p.lse[(int64_t)w.hc.bh * p.rm.nq + w.li * 128 + row] = dead ? -INFINITY : m + logf(l);
             // The bf16 half rows leave through shared memory: stored directly every 16-byte store instruction would touch 32 different
             // rows; from the warp's staging slice each instruction writes four whole 128-byte half rows.  A warp's slice is its own, so
             // the hand-over needs no more than the warp.
@@ -441,7 +441,9 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
             // ---- the item's epilogue: this part of the denominator to the fold warps, which write O and LSE.  The parts are numbered by
             // the parity of the tile inside the item: the order of their sum does not depend on the CTA's walk.
-            s.lsum[r % kItems][2 * ((gt ^ team) & 1) + g][row] = make_float2(l_part, l_ref);
+            // It leaves in units of 2^(maximum * log2 e): LSE = maximum + log(sum) then has one rounding at its own size.
+            s.lsum[r % kItems][2 * ((gt ^ team) & 1) + g][row] =
+                make_float2(m_run == -INFINITY ? 0.f : l_part * dm::ex2(l_ref - __fmul_rn(m_run, dm::kLog2e)), m_run);
             gt += n_tiles;
             dm::mbar_arrive_warp(&s.bar_l[r % kItems]);
         }
