@@ -29,7 +29,7 @@
 // Measured at B4 N4096 H32 causal: 1235 us before; 1290 with dV through X; 1206 with dV in place; 1037 with the unit moved in
 // 16-column pieces (fewer spills in the fold warps, which need 64 accumulators and two 16-register pieces); 960 with 72 / 96 / 24
 // registers per role and a maximum barrier per row half; 900 with the hardware warps in the order service, fold, softmax.
-// head_dim 256 (B2 N4096 H16 full): 1350 us with the kernel before this one, 1217 with this.
+// head_dim 256 (B2 N4096 H16 full): 1350 us with the kernel before this one, 1109 with this.
 #include "dm_attn_common.cuh"
 #include "dm_host.h"
 
@@ -114,7 +114,11 @@ constexpr int kBarDvFree = 9;          // dV's accumulator is in the next block'
 // 128-byte sub-tiles, K / V scales per 32 keys, Q / dO scales per 64-row m-block (so dV's unit moves at every m-block), psi per
 // 64 rows x 64 keys.  The accumulators of 128 keys x 256 columns do not fit, so two work items (d half 0 and 1) share a key block:
 // both form S / dP, each keeps its 128 columns of dK / dV, and only d half 0 stores the dS' tiles and psi.  An item's own half of Q
-// and dO lives until the products have read it, the other half only until S / dP have: one stage of it is enough.
+// and dO lives until the products have read it, the other half only until S / dP have: one stage of it is enough.  S of the next
+// tile is late behind the own half's two stages (the products end about 2000 clocks after the codes, a load takes 1300 more), and
+// there is no room for a third; Q and dO are released apart, each behind the last product that reads it, and S does not wait for dO
+// (B2 N4096 H16 full: 1217 -> 1141 us; 1109 with the other half loaded first and without a wait for the products before S; a stage
+// of both halves for S / dP and one of the own half for the products: 1292).
 template <int kD>
 struct Geo {
     static constexpr int kDH = kD / 128;
@@ -145,8 +149,8 @@ struct Smem {
     float fv[kGf];                            // dV's unit after the tile
     float psi[kGf][4];                        // psi of m-block m (psi tile h along the keys: [2 m + h]), on its way to pass 2
     float amax[2][16];                        // [tile parity][psi tile, warp of it]
-    uint64_t bar_kv, bar_kv_free, bar_own[3], bar_own_free[3], bar_oth, bar_oth_free, bar_sp_full, bar_x_full, bar_dv_full, bar_done[2],
-        bar_ds_free[2], bar_rows_full[kRows], bar_rows_free[kRows];
+    uint64_t bar_kv, bar_kv_free, bar_own[3], bar_own_free[3], bar_dov[2], bar_dov_free[2], bar_oth, bar_oth_free, bar_sp_full, bar_x_full,
+        bar_dv_full, bar_done[2], bar_ds_free[2], bar_rows_full[kRows], bar_rows_free[kRows];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -188,6 +192,8 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         }
         for (int i = 0; i < 2; ++i) {
             dm::mbar_init(&s.bar_done[i], 1);
+            dm::mbar_init(&s.bar_dov[i], 1);
+            dm::mbar_init(&s.bar_dov_free[i], 1);
             dm::mbar_init(&s.bar_ds_free[i], kD == 128 ? 1 : 2);
         }
         dm::fence_mbar_init();
@@ -222,10 +228,11 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                     dm::mbar_wait(&s.bar_own[st], (t / kOwn) & 1, wc);
                     if (kD == 256) dm::mbar_wait(&s.bar_oth, t & 1, wc);
                     // The softmax warps rewrite the code tiles of tile t - 2: its products and its dS' store must be done.  Gating the
-                    // products gates the softmax warps.  (head_dim 256 has one dS' tile: they wait for tile t - 1 themselves.)
-                    if (t >= 2) {
+                    // products gates the softmax warps.  (head_dim 256: dO's stage was refilled behind the last product of tile t - 2, and
+                    // the softmax warps wait for the one dS' tile themselves.)
+                    if (kD == 128 && t >= 2) {
                         dm::mbar_wait(&s.bar_done[t & 1], ((t - 2) >> 1) & 1, wc);
-                        if (kD == 128) dm::mbar_wait(&s.bar_ds_free[t & 1], ((t - 2) >> 1) & 1, wc);
+                        dm::mbar_wait(&s.bar_ds_free[t & 1], ((t - 2) >> 1) & 1, wc);
                     }
                     dm::mbar_wait(&s.bar_rows_full[t % kRows], (t / kRows) & 1, wc);      // saves the softmax warps a wait of their own
                     if (t >= 1) dm::named_bar_sync(kBarSpFree, kSoftmaxThreads + 32);
@@ -233,6 +240,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                     if (dm::elect_one()) {
 #pragma unroll
                         for (int m = 0; m < 2; ++m) {              // S, then dP; the d halves in order, whichever is the item's own
+                            if (kD == 256 && m == 1) dm::mbar_wait(&s.bar_dov[st], (t / kOwn) & 1, wc);
 #pragma unroll
                             for (int hh = 0; hh < kDH; ++hh) {
                                 const uint32_t a = (m ? do_lo : q_lo) + (kD == 128 || hh == w.zh ? st : kOwn) * kSub;
@@ -292,6 +300,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                                 dm::umma_commit(&s.bar_done[par]);
                             }
                             if (kD == 256 && m == 1) {     // the one dS' tile has been read by both products, and has left
+                                dm::umma_commit(&s.bar_own_free[st]);
                                 dm::umma_commit(&s.bar_ds_free[0]);
                                 dm::tma_store_wait_read0();
                                 dm::mbar_arrive(&s.bar_ds_free[0]);
@@ -310,10 +319,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                                     dm::umma_e4m3_lo<true>(t_dva, pa + 4 * m + 2 * k, dos + 512 * m + 256 * k, idesc_x);
                                 if (kD == 256) dm::umma_commit(&s.bar_dv_full);
                                 if (kD == 128 || m == 1) dm::mbar_arrive(&s.bar_rows_free[t % kRows]);
-                                if (kD == 256 && m == 1) {
-                                    dm::umma_commit(&s.bar_own_free[st]);
-                                    dm::umma_commit(&s.bar_done[par]);
-                                }
+                                if (kD == 256 && m == 1) dm::umma_commit(&s.bar_dov_free[st]);
                             }
                             __syncwarp();
                         }
@@ -351,19 +357,27 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                 }
                 for (int it = 0; it < n; ++it, ++t) {
                     const int st = t % kOwn;
-                    if (t >= kOwn) dm::mbar_wait(&s.bar_own_free[st], (t / kOwn - 1) & 1, wc);
-                    if (dm::elect_one()) {
-                        dm::mbar_expect_tx(&s.bar_own[st], 2 * kTile);
-                        dm::tma_load_2d(s.q[st], &tm_q, 128 * w.zh, q_row0 + it * 128, &s.bar_own[st]);
-                        dm::tma_load_2d(s.dO[st], &tm_do, 128 * w.zh, q_row0 + it * 128, &s.bar_own[st]);
-                    }
-                    __syncwarp();
                     if (kD == 256) {
                         if (t >= 1) dm::mbar_wait(&s.bar_oth_free, (t - 1) & 1, wc);
                         if (dm::elect_one()) {
                             dm::mbar_expect_tx(&s.bar_oth, 2 * kTile);
                             dm::tma_load_2d(s.q[kOwn], &tm_q, 128 * (w.zh ^ 1), q_row0 + it * 128, &s.bar_oth);
                             dm::tma_load_2d(s.dO[kOwn], &tm_do, 128 * (w.zh ^ 1), q_row0 + it * 128, &s.bar_oth);
+                        }
+                        __syncwarp();
+                    }
+                    if (t >= kOwn) dm::mbar_wait(&s.bar_own_free[st], (t / kOwn - 1) & 1, wc);
+                    if (dm::elect_one()) {
+                        dm::mbar_expect_tx(&s.bar_own[st], kD == 128 ? 2 * kTile : kTile);
+                        dm::tma_load_2d(s.q[st], &tm_q, 128 * w.zh, q_row0 + it * 128, &s.bar_own[st]);
+                        if (kD == 128) dm::tma_load_2d(s.dO[st], &tm_do, 128 * w.zh, q_row0 + it * 128, &s.bar_own[st]);
+                    }
+                    __syncwarp();
+                    if (kD == 256) {
+                        if (t >= kOwn) dm::mbar_wait(&s.bar_dov_free[st], (t / kOwn - 1) & 1, wc);
+                        if (dm::elect_one()) {
+                            dm::mbar_expect_tx(&s.bar_dov[st], kTile);
+                            dm::tma_load_2d(s.dO[st], &tm_do, 128 * w.zh, q_row0 + it * 128, &s.bar_dov[st]);
                         }
                         __syncwarp();
                     }
