@@ -1,4 +1,4 @@
-// Pass 0 of the backward, head_dim 128: the matched delta.  delta[row] = 2^-8 * sum over visible keys of
+// Pass 0 of the backward: the matched delta.  delta[row] = 2^-8 * sum over visible keys of
 // P-hat * dP, built from the backward's own fp8 operands with exactly the P-hat arithmetic pass 1 uses, so that
 // rowsum(P-hat * (dP - delta)) cancels to fp32 round-off (csrc/fp11_delta_v6.h:338-376,458-462 of the reference).
 //
@@ -215,8 +215,8 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
 }
 
 // ------------------------------------------------------------------------------------------------------------------------------
-// The production kernel at head_dim 128: the same sums as delta_kernel<false, 128>, as a persistent kernel in roles.
-// One CTA per SM walks the (head, row block) items, heaviest first; 640 threads:
+// The production kernel: the same sums as delta_kernel<false, kD>, as a persistent kernel in roles.
+// One CTA per SM walks the (head, row block) items, heaviest first; 576 threads:
 //   warps 0..15  compute, four per scheduler, in two teams of eight: team 0 takes the even key tiles and team 1 the odd ones
 //                (counted over the CTA's whole walk), so the two teams are half a tile apart in time and one team's waits
 //                and tensor-memory loads run under the other team's exponentials.  Thread (row, 64-key group g) does
@@ -228,17 +228,21 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
 // an mbarrier, and only the four warps that add them up and store the result (team 0, group 0) wait for it; the buffers
 // rotate over four items (the teams are never more than two tiles apart, because the MMAs are issued in tile order).  An
 // item's row constants and first scales are read one item ahead.
+// head_dim 256 has room for one Q8 / dO8 pair and two K8 / V8 stages; its products (1024 clocks a tile) run under the teams' exponentials
+// where the one-role kernel had them in turn: B2 N4096 H16 causal
+// 228 -> 158 us, full 414 -> 277, B1 N1920 H8 causal 35 -> 28.
 constexpr int kDzComputeWarps = 16;
 constexpr int kDzThreads = 32 * kDzComputeWarps + 64;
-constexpr int kDzStages = 3;
 
+template <int kD>
 struct DeltaRolesSmem {
-    alignas(1024) uint8_t q[2][kTile];
-    alignas(1024) uint8_t dO[2][kTile];
-    alignas(1024) uint8_t k[kDzStages][kTile];
-    alignas(1024) uint8_t v[kDzStages][kTile];
+    static constexpr int kDH = kD / 128, kQ = kD == 128 ? 2 : 1, kStages = kD == 128 ? 3 : 2;
+    alignas(1024) uint8_t q[kQ][kDH][kTile];
+    alignas(1024) uint8_t dO[kQ][kDH][kTile];
+    alignas(1024) uint8_t k[kStages][kDH][kTile];
+    alignas(1024) uint8_t v[kStages][kDH][kTile];
     double part[4][4][128];          // [item % 4][2 * team + group][row]
-    uint64_t bar_qdo[2], bar_qdo_free[2], bar_kv[kDzStages], bar_kv_free[kDzStages], bar_sp[2], bar_part[4];
+    uint64_t bar_qdo[2], bar_qdo_free[2], bar_kv[kStages], bar_kv_free[kStages], bar_sp[2], bar_part[4];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -265,12 +269,15 @@ __device__ __forceinline__ DeltaItem delta_item(const DeltaParams& p, const Delt
     return w;
 }
 
+template <int kD>
 __global__ void __launch_bounds__(kDzThreads, 1)
 delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                    const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const DeltaParams p,
                    const DeltaDivs fd) {
     extern __shared__ uint8_t smem_raw[];
-    DeltaRolesSmem& s = *reinterpret_cast<DeltaRolesSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    using Smem = DeltaRolesSmem<kD>;
+    constexpr int kDH = Smem::kDH, kQ = Smem::kQ, kStages = Smem::kStages;
+    Smem& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nq_blk = p.rm.nq / 128;
     dm::WaitCtx wc{&s.abort_flag, p.status};
@@ -282,7 +289,7 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             dm::mbar_init(&s.bar_qdo_free[i], 1);
             dm::mbar_init(&s.bar_sp[i], 1);
         }
-        for (int i = 0; i < kDzStages; ++i) {
+        for (int i = 0; i < kStages; ++i) {
             dm::mbar_init(&s.bar_kv[i], 1);
             dm::mbar_init(&s.bar_kv_free[i], 1);
         }
@@ -309,23 +316,33 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         for (int r = 0;; ++r) {
             const DeltaItem w = delta_item(p, fd, r);
             if (!w.valid) break;
-            const int qb = r & 1;
+            const int qb = r % kQ;
             const int q_row0 = w.hc.bh * p.rm.nq + w.li * 128, kv_row0 = w.hc.bhk * p.N;
-            if (r >= 2) dm::mbar_wait(&s.bar_qdo_free[qb], ((r - 2) >> 1) & 1, wc);
-            if (leader) {
-                dm::mbar_expect_tx(&s.bar_qdo[qb], 2 * kTile);
-                dm::tma_load_2d(s.q[qb], &tm_q, 0, q_row0, &s.bar_qdo[qb]);
-                dm::tma_load_2d(s.dO[qb], &tm_do, 0, q_row0, &s.bar_qdo[qb]);
-            }
-            for (int it = 0; it < w.n_tiles; ++it) {
-                const int t = gt + it, st = t % kDzStages;
-                if (t >= kDzStages) dm::mbar_wait(&s.bar_kv_free[st], (t / kDzStages - 1) & 1, wc);
+            auto load_qdo = [&] {
+                if (r >= kQ) dm::mbar_wait(&s.bar_qdo_free[qb], (r / kQ - 1) & 1, wc);
                 if (leader) {
-                    dm::mbar_expect_tx(&s.bar_kv[st], 2 * kTile);
-                    dm::tma_load_2d(s.k[st], &tm_k, 0, kv_row0 + it * 128, &s.bar_kv[st]);
-                    dm::tma_load_2d(s.v[st], &tm_v, 0, kv_row0 + it * 128, &s.bar_kv[st]);
+                    dm::mbar_expect_tx(&s.bar_qdo[qb], 2 * kDH * kTile);
+#pragma unroll
+                    for (int hh = 0; hh < kDH; ++hh) {
+                        dm::tma_load_2d(s.q[qb][hh], &tm_q, 128 * hh, q_row0, &s.bar_qdo[qb]);
+                        dm::tma_load_2d(s.dO[qb][hh], &tm_do, 128 * hh, q_row0, &s.bar_qdo[qb]);
+                    }
+                }
+            };
+            if (kQ == 2) load_qdo();
+            for (int it = 0; it < w.n_tiles; ++it) {
+                const int t = gt + it, st = t % kStages;
+                if (t >= kStages) dm::mbar_wait(&s.bar_kv_free[st], (t / kStages - 1) & 1, wc);
+                if (leader) {
+                    dm::mbar_expect_tx(&s.bar_kv[st], 2 * kDH * kTile);
+#pragma unroll
+                    for (int hh = 0; hh < kDH; ++hh) {
+                        dm::tma_load_2d(s.k[st][hh], &tm_k, 128 * hh, kv_row0 + it * 128, &s.bar_kv[st]);
+                        dm::tma_load_2d(s.v[st][hh], &tm_v, 128 * hh, kv_row0 + it * 128, &s.bar_kv[st]);
+                    }
                 }
                 __syncwarp();
+                if (kQ == 1 && it == 0) load_qdo();      // the one Q / dO pair is free only behind the last item's last products
             }
             gt += w.n_tiles;
         }
@@ -333,30 +350,36 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         // ---- MMA issue
         const bool leader = lane == 0;
         constexpr uint32_t idesc = dm::idesc_e4m3(128, 128, false, false);
-        const uint32_t q_lo0 = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[0])), do_lo0 = dm::smem_desc_lo_sw128(dm::smem_u32(s.dO[0]));
-        const uint32_t k_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.k[0])), v_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.v[0]));
+        const uint32_t q_lo0 = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[0][0])), do_lo0 = dm::smem_desc_lo_sw128(dm::smem_u32(s.dO[0][0]));
+        const uint32_t k_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.k[0][0])), v_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.v[0][0]));
         int gt = 0;
         for (int r = 0;; ++r) {
             const DeltaItem w = delta_item(p, fd, r);
             if (!w.valid) break;
-            const int qb = r & 1;
-            dm::mbar_wait(&s.bar_qdo[qb], (r >> 1) & 1, wc);
-            const uint32_t q_lo = q_lo0 + qb * kSub, do_lo = do_lo0 + qb * kSub;
+            const int qb = r % kQ;
+            dm::mbar_wait(&s.bar_qdo[qb], (r / kQ) & 1, wc);
+            const uint32_t q_lo = q_lo0 + qb * kDH * kSub, do_lo = do_lo0 + qb * kDH * kSub;
             for (int it = 0; it < w.n_tiles; ++it) {
-                const int t = gt + it, st = t % kDzStages, b = t & 1;
-                dm::mbar_wait(&s.bar_kv[st], (t / kDzStages) & 1, wc);
+                const int t = gt + it, st = t % kStages, b = t & 1;
+                dm::mbar_wait(&s.bar_kv[st], (t / kStages) & 1, wc);
                 // a team says through a named barrier that it holds its buffer's values: a hand-off between warps costs a fifth
                 // of what an mbarrier's does
                 if (t >= 2) dm::named_bar_sync(2 + b, 16 * kDzComputeWarps + 32);
                 dm::tc_fence_after();
-                const uint32_t ks = k_lo + st * kSub, vs = v_lo + st * kSub, t_s = tmem + b * 256, t_dp = t_s + 128;
+                const uint32_t ks = k_lo + st * kDH * kSub, vs = v_lo + st * kDH * kSub, t_s = tmem + b * 256;
                 if (leader) {
-                    dm::umma_e4m3_lo<false>(t_s, q_lo, ks, idesc);
 #pragma unroll
-                    for (int k = 1; k < 4; ++k) dm::umma_e4m3_lo<true>(t_s, q_lo + 2 * k, ks + 2 * k, idesc);
-                    dm::umma_e4m3_lo<false>(t_dp, do_lo, vs, idesc);
+                    for (int m = 0; m < 2; ++m) {
 #pragma unroll
-                    for (int k = 1; k < 4; ++k) dm::umma_e4m3_lo<true>(t_dp, do_lo + 2 * k, vs + 2 * k, idesc);
+                        for (int hh = 0; hh < kDH; ++hh) {
+                            const uint32_t x = (m ? do_lo : q_lo) + hh * kSub, y = (m ? vs : ks) + hh * kSub, d = t_s + 128 * m;
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                if ((hh | k) == 0) dm::umma_e4m3_lo<false>(d, x, y, idesc);
+                                else dm::umma_e4m3_lo<true>(d, x + 2 * k, y + 2 * k, idesc);
+                            }
+                        }
+                    }
                     dm::umma_commit(&s.bar_sp[b]);
                     dm::umma_commit(&s.bar_kv_free[st]);
                     if (it == w.n_tiles - 1) dm::umma_commit(&s.bar_qdo_free[qb]);
@@ -374,18 +397,22 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
         int gt = 0;
         // what the item's first tile needs from global memory is read one item ahead
         int64_t rowi_nx = 0;
-        float q8sc_nx = 0.f, do8sc_nx = 0.f, lse_nx = 0.f, ks_nx = 0.f, vs_nx = 0.f;
+        float q8sc_nx = 0.f, do8sc_nx = 0.f, lse_nx = 0.f, ks_nx[kDH] = {}, vs_nx[kDH] = {};
         auto prefetch = [&](const DeltaItem& wi, int gt_at) {
             if (!wi.valid) return;
             rowi_nx = (int64_t)wi.hc.bh * p.rm.nq + wi.li * 128 + row;
-            q8sc_nx = p.q8s[(int64_t)wi.hc.bh * nq_blk + wi.li];
-            do8sc_nx = p.do8s[(int64_t)wi.hc.bh * nq_blk + wi.li];
+            const int64_t sq = kD == 128 ? (int64_t)wi.hc.bh * nq_blk + wi.li : ((int64_t)wi.hc.bh * nq_blk + wi.li) * 2 + (row >> 6);
+            q8sc_nx = p.q8s[sq];
+            do8sc_nx = p.do8s[sq];
             lse_nx = p.lse[rowi_nx];
             const int first = (gt_at ^ team) & 1;
             if (first < wi.n_tiles) {
-                const int64_t so = (int64_t)wi.hc.bhk * (p.N / 64) + g + 2 * first;
-                ks_nx = p.k8s[so];
-                vs_nx = p.v8s[so];
+                const int64_t so = (int64_t)wi.hc.bhk * (p.N / 64) * kDH + (g + 2 * first) * kDH;
+#pragma unroll
+                for (int h = 0; h < kDH; ++h) {
+                    ks_nx[h] = p.k8s[so + h];
+                    vs_nx[h] = p.v8s[so + h];
+                }
             }
         };
         DeltaItem w = delta_item(p, fd, 0);
@@ -395,19 +422,30 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             const int64_t rowi = rowi_nx;
             const float q8sc = q8sc_nx, do8sc = do8sc_nx;
             const float rc = dm::phat_row_const(lse_nx);
-            const float* ksp = p.k8s + (int64_t)w.hc.bhk * (p.N / 64) + g;
-            const float* vsp = p.v8s + (int64_t)w.hc.bhk * (p.N / 64) + g;
+            // K / V scales of the thread's keys: one per 64 keys at head_dim 128, one per 32 keys (a half below) at head_dim 256
+            const float* ksp = p.k8s + ((int64_t)w.hc.bhk * (p.N / 64) + g) * kDH;
+            const float* vsp = p.v8s + ((int64_t)w.hc.bhk * (p.N / 64) + g) * kDH;
             double acc = 0.0;
             const int it0 = (gt ^ team) & 1;                   // this team's first tile of the item
-            float ks_n = ks_nx, vs_n = vs_nx;
+            float ks_n[kDH], vs_n[kDH];
+#pragma unroll
+            for (int h = 0; h < kDH; ++h) {
+                ks_n[h] = ks_nx[h];
+                vs_n[h] = vs_nx[h];
+            }
             const DeltaItem w_next = delta_item(p, fd, r + 1);
             prefetch(w_next, gt + n_tiles);
             for (int it = it0; it < n_tiles; it += 2) {
                 const int t = gt + it;
-                const float dsc = dm::descale_log2(q8sc, ks_n), dpsc = do8sc * vs_n;
-                if (it + 2 < n_tiles) {
-                    ks_n = ksp[2 * (it + 2)];
-                    vs_n = vsp[2 * (it + 2)];
+                float dsc2[kDH], dpsc2[kDH];
+#pragma unroll
+                for (int h = 0; h < kDH; ++h) {
+                    dsc2[h] = dm::descale_log2(q8sc, ks_n[h]);
+                    dpsc2[h] = do8sc * vs_n[h];
+                    if (it + 2 < n_tiles) {
+                        ks_n[h] = ksp[2 * (it + 2) * kDH + h];
+                        vs_n[h] = vsp[2 * (it + 2) * kDH + h];
+                    }
                 }
                 const bool diag = p.causal && it == I;
                 dm::mbar_wait(&s.bar_sp[team], (t >> 1) & 1, wc);
@@ -422,6 +460,7 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                         dm::tc_fence_before();
                         dm::named_bar_arrive(2 + team, 16 * kDzComputeWarps + 32);     // the team's buffer may be overwritten
                     }
+                    const float dsc = dsc2[half % kDH], dpsc = dpsc2[half % kDH];
 #pragma unroll
                     for (int c = 0; c < 32; c += 2) {           // P-hat = 2^min(S dsc + rc, 12), the exponent two at a time
                         dm::fma2(sv[c], sv[c + 1], sv[c], sv[c + 1], dsc, rc, rc);
@@ -471,19 +510,25 @@ int launch(const void* q8, const void* k8, const void* v8, const void* do8, cons
     if ((rc = dmh::make_tmap_u8(&tk, k8, kD, (uint64_t)sh.B * sh.Hk * sh.N, 128, err, errlen))) return rc;
     if ((rc = dmh::make_tmap_u8(&tv, v8, kD, (uint64_t)sh.B * sh.Hk * sh.N, 128, err, errlen))) return rc;
     if ((rc = dmh::prepare_delta(err, errlen))) return rc;
-    // head_dim 128, production: the persistent kernel once every CTA has a walk of at least 24 key tiles (measured: it wins at
-    // 29 tiles per CTA, 0.041 against 0.044 ms, and by more on longer walks); the one-item-per-CTA kernel below stays for small problems, the debug row sums and head_dim 256
-    const int64_t items = (int64_t)sh.B * p.hcount * (p.rm.nq / 128);
-    const int64_t tiles = items * (sh.causal ? (sh.N / 128 + 1) / 2 : sh.N / 128);      // about: exact for the identity row map
-    int sms = 0;
-    if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
-    if (!kDebug && kD == 128 && items >= 2 * (int64_t)sms && tiles >= 24 * (int64_t)sms) {
-        const DeltaDivs fd{dm::make_fastdiv(sh.B * p.hcount), dm::make_fastdiv(p.hcount), dm::make_fastdiv(sh.H / sh.Hk)};
-        DM_CUDA(dmh::launch_pdl(delta_roles_kernel, sms, kDzThreads, sizeof(DeltaRolesSmem) + 1024, stream, tq, td, tk, tv, p, fd));
-        return DM_OK;
+    // The roles kernel: at head_dim 256 always (both kernels fill an SM with one CTA); at head_dim 128 once every CTA has a walk of at
+    // least 24 key tiles (measured: it wins at 29 tiles per CTA, 0.041 against 0.044 ms, and by more on longer walks).  The
+    // one-item-per-CTA kernel, two CTAs per SM at head_dim 128, stays for its small problems and for the debug row sums.
+    if constexpr (!kDebug) {
+        const int64_t items = (int64_t)sh.B * p.hcount * (p.rm.nq / 128);
+        const int64_t tiles = items * (sh.causal ? (sh.N / 128 + 1) / 2 : sh.N / 128);      // about: exact for the identity row map
+        int sms = 0;
+        if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
+        if (kD == 256 || (items >= 2 * (int64_t)sms && tiles >= 24 * (int64_t)sms)) {
+            const DeltaDivs fd{dm::make_fastdiv(sh.B * p.hcount), dm::make_fastdiv(p.hcount), dm::make_fastdiv(sh.H / sh.Hk)};
+            DM_CUDA(dmh::launch_pdl(delta_roles_kernel<kD>, (int)(items < sms ? items : sms), kDzThreads, sizeof(DeltaRolesSmem<kD>) + 1024,
+                                    stream, tq, td, tk, tv, p, fd));
+            return DM_OK;
+        }
     }
-    const int smem = (int)sizeof(DeltaSmem<kD>) + 1024;
-    DM_CUDA(dmh::launch_pdl(delta_kernel<kDebug, kD>, dim3(sh.B * p.hcount, p.rm.nq / 128), 256, smem, stream, tq, td, tk, tv, p));
+    if constexpr (kDebug || kD == 128) {
+        const int smem = (int)sizeof(DeltaSmem<kD>) + 1024;
+        DM_CUDA(dmh::launch_pdl(delta_kernel<kDebug, kD>, dim3(sh.B * p.hcount, p.rm.nq / 128), 256, smem, stream, tq, td, tk, tv, p));
+    }
     return DM_OK;
 }
 
@@ -496,9 +541,9 @@ int prepare_delta(char* err, size_t errlen) {
     static DeviceOnce once;
     return device_once(once, err, errlen, [&]() -> int {
         DM_CUDA(cudaFuncSetAttribute(delta_kernel<false, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaSmem<128>) + 1024));
-        DM_CUDA(cudaFuncSetAttribute(delta_roles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaRolesSmem) + 1024));
+        DM_CUDA(cudaFuncSetAttribute(delta_roles_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaRolesSmem<128>) + 1024));
+        DM_CUDA(cudaFuncSetAttribute(delta_roles_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaRolesSmem<256>) + 1024));
         DM_CUDA(cudaFuncSetAttribute(delta_kernel<true, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaSmem<128>) + 1024));
-        DM_CUDA(cudaFuncSetAttribute(delta_kernel<false, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaSmem<256>) + 1024));
         DM_CUDA(cudaFuncSetAttribute(delta_kernel<true, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaSmem<256>) + 1024));
         return DM_OK;
     });
