@@ -229,8 +229,11 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
 // rotate over four items (the teams are never more than two tiles apart, because the MMAs are issued in tile order).  An
 // item's row constants and first scales are read one item ahead.
 // head_dim 256 has room for one Q8 / dO8 pair and two K8 / V8 stages; its products (1024 clocks a tile) run under the teams' exponentials
-// where the one-role kernel had them in turn: B2 N4096 H16 causal
-// 228 -> 158 us, full 414 -> 277, B1 N1920 H8 causal 35 -> 28.
+// where the one-role kernel had them in turn: B2 N4096 H16 causal 228 -> 158 us, full 414 -> 277, B1 N1920 H8 causal 35 -> 28.
+// What bounds it: per scheduler four warps' chains (tensor-memory load, exponentials, multiply-adds) at 1700 clocks a tile where the
+// exponentials alone are 1024.  The scores are taken 16 columns at a time: 32 at a time spilled, and a piece in flight ahead of the one
+// being worked on took the registers of the spills again (B4 N4096 H32 head_dim 128: 425 us with 32, 403 with 16, 462 with 16 and the
+// next in flight, 430 with 8; head_dim 256 as above: 158, 138, 162, 141).
 constexpr int kDzComputeWarps = 16;
 constexpr int kDzThreads = 32 * kDzComputeWarps + 64;
 
@@ -278,7 +281,7 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     using Smem = DeltaRolesSmem<kD>;
     constexpr int kDH = Smem::kDH, kQ = Smem::kQ, kStages = Smem::kStages;
     Smem& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int nq_blk = p.rm.nq / 128;
     dm::WaitCtx wc{&s.abort_flag, p.status};
 
@@ -452,33 +455,37 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 dm::tc_fence_after();
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
-                    float sv[32], dp[32];
-                    dm::tmem_ld32(t_s + half * 32, reinterpret_cast<uint32_t*>(sv));
-                    dm::tmem_ld32(t_dp + half * 32, reinterpret_cast<uint32_t*>(dp));
-                    dm::tmem_ld_wait();
-                    if (half == 1) {
-                        dm::tc_fence_before();
-                        dm::named_bar_arrive(2 + team, 16 * kDzComputeWarps + 32);     // the team's buffer may be overwritten
-                    }
                     const float dsc = dsc2[half % kDH], dpsc = dpsc2[half % kDH];
-#pragma unroll
-                    for (int c = 0; c < 32; c += 2) {           // P-hat = 2^min(S dsc + rc, 12), the exponent two at a time
-                        dm::fma2(sv[c], sv[c + 1], sv[c], sv[c + 1], dsc, rc, rc);
-                        sv[c] = dm::ex2(fminf(sv[c], dm::kMoE + 4.0f));
-                        sv[c + 1] = dm::ex2(fminf(sv[c + 1], dm::kMoE + 4.0f));
-                    }
-                    if (diag) {                                 // the diagonal tile only: keys above the row
-#pragma unroll
-                        for (int c = 0; c < 32; ++c)
-                            if (g * 64 + half * 32 + c > row) sv[c] = 0.f;
-                    }
                     float a = 0.f;
 #pragma unroll
-                    for (int c = 0; c < 32; c += 2) {
-                        float d0, d1;
-                        dm::mul2(d0, d1, dp[c], dp[c + 1], dpsc, dpsc);
-                        a = fmaf(sv[c], d0, a);
-                        a = fmaf(sv[c + 1], d1, a);
+                    for (int q = 0; q < 2; ++q) {
+                        const int c0 = half * 32 + q * 16;
+                        float sv[16], dp[16];
+                        dm::tmem_ld16(t_s + c0, reinterpret_cast<uint32_t*>(sv));
+                        dm::tmem_ld16(t_dp + c0, reinterpret_cast<uint32_t*>(dp));
+                        dm::tmem_ld_wait();
+                        if (half == 1 && q == 1) {
+                            dm::tc_fence_before();
+                            dm::named_bar_arrive(2 + team, 16 * kDzComputeWarps + 32);     // the team's buffer may be overwritten
+                        }
+#pragma unroll
+                        for (int c = 0; c < 16; c += 2) {           // P-hat = 2^min(S dsc + rc, 12), the exponent two at a time
+                            dm::fma2(sv[c], sv[c + 1], sv[c], sv[c + 1], dsc, rc, rc);
+                            sv[c] = dm::ex2(fminf(sv[c], dm::kMoE + 4.0f));
+                            sv[c + 1] = dm::ex2(fminf(sv[c + 1], dm::kMoE + 4.0f));
+                        }
+                        if (diag) {                                 // the diagonal tile only: keys above the row
+#pragma unroll
+                            for (int c = 0; c < 16; ++c)
+                                if (g * 64 + c0 + c > row) sv[c] = 0.f;
+                        }
+#pragma unroll
+                        for (int c = 0; c < 16; c += 2) {
+                            float d0, d1;
+                            dm::mul2(d0, d1, dp[c], dp[c + 1], dpsc, dpsc);
+                            a = fmaf(sv[c], d0, a);
+                            a = fmaf(sv[c + 1], d1, a);
+                        }
                     }
                     acc += (double)(a * dm::kMoInv);
                 }
