@@ -2,15 +2,8 @@
 // P-hat * dP, built from the backward's own fp8 operands with exactly the P-hat arithmetic pass 1 uses, so that
 // rowsum(P-hat * (dP - delta)) cancels to fp32 round-off (csrc/fp11_delta_v6.h:338-376,458-462 of the reference).
 //
-// One CTA = 128 query rows of one (batch, head); 256 threads; key tiles of 128 keys ascending; TWO CTAs per SM (256
-// tensor-memory columns, < 113 KB shared memory and <= 128 registers each), so one CTA's MMAs run under the other's
-// arithmetic.  Per tile
-//   S  = Q  K^T   and   dP = dO V^T      8 x tcgen05.mma into tensor memory (S | dP, 256 columns)
-// then thread (row, key group g) forms P-hat for its 64 keys, accumulates fma(P-hat, dP * (do8sc * v8sc), a) per 32-key
-// half in ascending key order, and folds each half's fp32 partial (times 2^-8) into an fp64 accumulator.  The two key
-// groups' fp64 sums are added at the end and rounded once.
-// Also the debug row-sum kernel: the same loop with delta subtracted, producing rowsum and abs-rowsum of
-// P-hat * (dP - delta) / 256.
+// Two kernels: delta_roles_kernel (persistent, the production one, below) and rowsum_kernel, the debug one: the same walk with delta
+// subtracted, producing rowsum and abs-rowsum of P-hat * (dP - delta) / 256 in one role, one item per CTA.
 #include "dm_attn_common.cuh"
 #include "dm_host.h"
 
@@ -22,10 +15,10 @@ namespace {
 
 constexpr int kTile = 128 * 128;
 
-// kD = 256: a code row is two 128-byte sub-tiles (8 MMA K steps), K / V scales per 32 keys (exactly the 32-key halves this
-// kernel already reduces separately), Q / dO scales per 64 rows; 192 KB of shared memory, so one CTA per SM.
+// kD = 256: a code row is two 128-byte sub-tiles (8 MMA K steps), K / V scales per 32 keys (exactly the 32-key halves that are
+// reduced separately anyway), Q / dO scales per 64 rows.
 template <int kD>
-struct DeltaSmem {
+struct RowsumSmem {
     static constexpr int kDH = kD / 128;
     alignas(1024) uint8_t q[kDH][kTile];
     alignas(1024) uint8_t dO[kDH][kTile];
@@ -52,13 +45,17 @@ struct DeltaParams {
     dm::RowMap rm;
 };
 
-template <bool kDebug, int kD>
+// Debug row sums.  One CTA = 128 query rows of one (batch, head); 256 threads; key tiles of 128 keys ascending.  Per tile
+//   S  = Q  K^T   and   dP = dO V^T      8 x tcgen05.mma (16 at head_dim 256) into tensor memory (S | dP, 256 columns)
+// then thread (row, key group g) forms P-hat for its 64 keys and adds P-hat * (dP - delta) and its magnitude, folding each 32-key
+// half's fp32 partial (times 2^-8) into fp64 accumulators.  The two key groups' fp64 sums are added at the end and rounded once.
+template <int kD>
 __global__ void __launch_bounds__(256, kD == 128 ? 2 : 1)
-delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
-                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const DeltaParams p) {
+rowsum_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
+              const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const DeltaParams p) {
     extern __shared__ uint8_t smem_raw[];
     constexpr int kDH = kD / 128;
-    DeltaSmem<kD>& s = *reinterpret_cast<DeltaSmem<kD>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    RowsumSmem<kD>& s = *reinterpret_cast<RowsumSmem<kD>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int g = warp >> 2;
     const int row = (warp & 3) * 32 + lane;
@@ -141,7 +138,7 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     const float do8sc = p.do8s[sq];
     const int n_glob = li * 128 + row;              // row inside the (local) Q-side tensors
     const float rc = dm::phat_row_const(p.lse[(int64_t)hc.bh * p.rm.nq + n_glob]);
-    const float dlt = kDebug ? p.delta_in[(int64_t)hc.bh * p.rm.nq + n_glob] : 0.f;
+    const float dlt = p.delta_in[(int64_t)hc.bh * p.rm.nq + n_glob];
     double acc = 0.0, acc_abs = 0.0;
 
     for (int it = 0; it < n_tiles; ++it) {
@@ -177,24 +174,14 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
                 for (int c = 0; c < 32; ++c)
                     if (g * 64 + half * 32 + c > row) sv[c] = 0.f;
             }
-            if (kDebug) {
 #pragma unroll
-                for (int c = 0; c < 32; ++c) {
-                    const float t = sv[c] * (dp[c] * dpsc - dlt);
-                    a += t;
-                    aa += fabsf(t);
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < 32; c += 2) {
-                    float d0, d1;
-                    dm::mul2(d0, d1, dp[c], dp[c + 1], dpsc, dpsc);
-                    a = fmaf(sv[c], d0, a);
-                    a = fmaf(sv[c + 1], d1, a);
-                }
+            for (int c = 0; c < 32; ++c) {
+                const float t = sv[c] * (dp[c] * dpsc - dlt);
+                a += t;
+                aa += fabsf(t);
             }
             acc += (double)(a * dm::kMoInv);
-            if (kDebug) acc_abs += (double)(aa * dm::kMoInv);
+            acc_abs += (double)(aa * dm::kMoInv);
         }
         dm::tc_fence_before();
         __syncthreads();                       // S | dP have been read; stage `st` tiles are free
@@ -205,37 +192,39 @@ delta_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ C
     }
 
     s.part[g][row] = acc;
-    if (kDebug) s.part_abs[g][row] = acc_abs;
+    s.part_abs[g][row] = acc_abs;
     __syncthreads();
     if (g == 0) {
         p.out[(int64_t)hc.bh * p.rm.nq + n_glob] = (float)(s.part[0][row] + s.part[1][row]);
-        if (kDebug) p.out_abs[(int64_t)hc.bh * p.rm.nq + n_glob] = (float)(s.part_abs[0][row] + s.part_abs[1][row]);
+        p.out_abs[(int64_t)hc.bh * p.rm.nq + n_glob] = (float)(s.part_abs[0][row] + s.part_abs[1][row]);
     }
     if (warp == 0) dm::tmem_dealloc(tmem, 256);
 }
 
 // ------------------------------------------------------------------------------------------------------------------------------
-// The production kernel: the same sums as delta_kernel<false, kD>, as a persistent kernel in roles.
+// The production kernel, persistent, in roles.
 // One CTA per SM walks the (head, row block) items, heaviest first; 576 threads:
 //   warps 0..15  compute, four per scheduler, in two teams of eight: team 0 takes the even key tiles and team 1 the odd ones
 //                (counted over the CTA's whole walk), so the two teams are half a tile apart in time and one team's waits
-//                and tensor-memory loads run under the other team's exponentials.  Thread (row, 64-key group g) does
-//                what a thread of delta_kernel does: per 32-key half, P-hat and a = fma(P-hat, dP * (do8sc v8sc), a) in
-//                ascending key order, then acc_fp64 += a * 2^-8
+//                and tensor-memory loads run under the other team's exponentials.  Thread (row, 64-key group g), per 32-key
+//                half: P-hat and a = fma(P-hat, dP * (do8sc v8sc), a) in ascending key order, then acc_fp64 += a * 2^-8
 //   warp 16      TMA loads: Q8 / dO8 of an item (double-buffered by item), K8 / V8 tiles in a three-stage ring
 //   warp 17      tcgen05.mma: S = Q K^T and dP = dO V^T of a tile (8 x M128 N128 K32) into one of two (S | dP) buffers
 // A row's four fp64 sums (team x group) meet in shared memory at the item's end: every warp leaves its sums and arrives on
 // an mbarrier, and only the four warps that add them up and store the result (team 0, group 0) wait for it; the buffers
-// rotate over four items (the teams are never more than two tiles apart, because the MMAs are issued in tile order).  An
+// rotate over kDzItems items (on items of one tile the other team can be four items ahead of the storing warps: it has computed tile
+// t + 3, which is issued behind their release of tile t, and passed item t + 4).  An
 // item's row constants and first scales are read one item ahead.
 // head_dim 256 has room for one Q8 / dO8 pair and two K8 / V8 stages; its products (1024 clocks a tile) run under the teams' exponentials
 // where the one-role kernel had them in turn: B2 N4096 H16 causal 228 -> 158 us, full 414 -> 277, B1 N1920 H8 causal 35 -> 28.
 // What bounds it: per scheduler four warps' chains (tensor-memory load, exponentials, multiply-adds) at 1700 clocks a tile where the
 // exponentials alone are 1024.  The scores are taken 16 columns at a time: 32 at a time spilled, and a piece in flight ahead of the one
 // being worked on took the registers of the spills again (B4 N4096 H32 head_dim 128: 425 us with 32, 403 with 16, 462 with 16 and the
-// next in flight, 430 with 8; head_dim 256 as above: 158, 138, 162, 141).
+// next in flight, 430 with 8; head_dim 256 as above: 158, 138, 162, 141).  Short walks take it too: against the kernel with one role
+// and one item per CTA, two CTAs per SM, B4 N768 H12 19.1 -> 17.3 us, B1 N4096 H8 55 -> 36, B1 N512 H8 12.9 -> 11.7.
 constexpr int kDzComputeWarps = 16;
 constexpr int kDzThreads = 32 * kDzComputeWarps + 64;
+constexpr int kDzItems = 8;
 
 template <int kD>
 struct DeltaRolesSmem {
@@ -244,8 +233,8 @@ struct DeltaRolesSmem {
     alignas(1024) uint8_t dO[kQ][kDH][kTile];
     alignas(1024) uint8_t k[kStages][kDH][kTile];
     alignas(1024) uint8_t v[kStages][kDH][kTile];
-    double part[4][4][128];          // [item % 4][2 * team + group][row]
-    uint64_t bar_qdo[2], bar_qdo_free[2], bar_kv[kStages], bar_kv_free[kStages], bar_sp[2], bar_part[4];
+    double part[kDzItems][4][128];   // [item % kDzItems][2 * team + group][row]
+    uint64_t bar_qdo[2], bar_qdo_free[2], bar_kv[kStages], bar_kv_free[kStages], bar_sp[2], bar_part[kDzItems];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -296,7 +285,7 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             dm::mbar_init(&s.bar_kv[i], 1);
             dm::mbar_init(&s.bar_kv_free[i], 1);
         }
-        for (int i = 0; i < 4; ++i) dm::mbar_init(&s.bar_part[i], kDzComputeWarps);
+        for (int i = 0; i < kDzItems; ++i) dm::mbar_init(&s.bar_part[i], kDzComputeWarps);
         dm::fence_mbar_init();
         dm::tma_prefetch_desc(&tm_q);
         dm::tma_prefetch_desc(&tm_do);
@@ -492,11 +481,11 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
             }
             gt += n_tiles;
             // the row's four sums meet in shared memory; only the four storing warps wait for the others
-            const int pb = r & 3;
+            const int pb = r % kDzItems;
             s.part[pb][2 * team + g][row] = acc;
             dm::mbar_arrive_warp(&s.bar_part[pb]);             // (lane 0 arrives after __syncwarp: the warp's stores are ordered before it)
             if (warp < 4) {
-                dm::mbar_wait(&s.bar_part[pb], (r >> 2) & 1, wc);
+                dm::mbar_wait(&s.bar_part[pb], (r / kDzItems) & 1, wc);
                 p.out[rowi] = (float)((s.part[pb][0][row] + s.part[pb][1][row]) + (s.part[pb][2][row] + s.part[pb][3][row]));
             }
             w = w_next;
@@ -507,7 +496,7 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
     if (warp == 0) dm::tmem_dealloc(tmem, 512);
 }
 
-template <bool kDebug, int kD>
+template <int kD>
 int launch(const void* q8, const void* k8, const void* v8, const void* do8, const DeltaParams& p, const DmShape& sh, void* stream,
            char* err, size_t errlen) {
     int rc;
@@ -517,25 +506,17 @@ int launch(const void* q8, const void* k8, const void* v8, const void* do8, cons
     if ((rc = dmh::make_tmap_u8(&tk, k8, kD, (uint64_t)sh.B * sh.Hk * sh.N, 128, err, errlen))) return rc;
     if ((rc = dmh::make_tmap_u8(&tv, v8, kD, (uint64_t)sh.B * sh.Hk * sh.N, 128, err, errlen))) return rc;
     if ((rc = dmh::prepare_delta(err, errlen))) return rc;
-    // The roles kernel: at head_dim 256 always (both kernels fill an SM with one CTA); at head_dim 128 once every CTA has a walk of at
-    // least 24 key tiles (measured: it wins at 29 tiles per CTA, 0.041 against 0.044 ms, and by more on longer walks).  The
-    // one-item-per-CTA kernel, two CTAs per SM at head_dim 128, stays for its small problems and for the debug row sums.
-    if constexpr (!kDebug) {
-        const int64_t items = (int64_t)sh.B * p.hcount * (p.rm.nq / 128);
-        const int64_t tiles = items * (sh.causal ? (sh.N / 128 + 1) / 2 : sh.N / 128);      // about: exact for the identity row map
-        int sms = 0;
-        if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
-        if (kD == 256 || (items >= 2 * (int64_t)sms && tiles >= 24 * (int64_t)sms)) {
-            const DeltaDivs fd{dm::make_fastdiv(sh.B * p.hcount), dm::make_fastdiv(p.hcount), dm::make_fastdiv(sh.H / sh.Hk)};
-            DM_CUDA(dmh::launch_pdl(delta_roles_kernel<kD>, (int)(items < sms ? items : sms), kDzThreads, sizeof(DeltaRolesSmem<kD>) + 1024,
-                                    stream, tq, td, tk, tv, p, fd));
-            return DM_OK;
-        }
+    if (p.delta_in) {
+        DM_CUDA(dmh::launch_pdl(rowsum_kernel<kD>, dim3(sh.B * p.hcount, p.rm.nq / 128), 256, (int)sizeof(RowsumSmem<kD>) + 1024, stream, tq, td,
+                                tk, tv, p));
+        return DM_OK;
     }
-    if constexpr (kDebug || kD == 128) {
-        const int smem = (int)sizeof(DeltaSmem<kD>) + 1024;
-        DM_CUDA(dmh::launch_pdl(delta_kernel<kDebug, kD>, dim3(sh.B * p.hcount, p.rm.nq / 128), 256, smem, stream, tq, td, tk, tv, p));
-    }
+    const int64_t items = (int64_t)sh.B * p.hcount * (p.rm.nq / 128);
+    int sms = 0;
+    if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
+    const DeltaDivs fd{dm::make_fastdiv(sh.B * p.hcount), dm::make_fastdiv(p.hcount), dm::make_fastdiv(sh.H / sh.Hk)};
+    DM_CUDA(dmh::launch_pdl(delta_roles_kernel<kD>, (int)(items < sms ? items : sms), kDzThreads, sizeof(DeltaRolesSmem<kD>) + 1024, stream, tq,
+                            td, tk, tv, p, fd));
     return DM_OK;
 }
 
@@ -547,11 +528,10 @@ int check_cp(const DmShape& s, const DmCp& cp, char* err, size_t errlen);
 int prepare_delta(char* err, size_t errlen) {
     static DeviceOnce once;
     return device_once(once, err, errlen, [&]() -> int {
-        DM_CUDA(cudaFuncSetAttribute(delta_kernel<false, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaSmem<128>) + 1024));
         DM_CUDA(cudaFuncSetAttribute(delta_roles_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaRolesSmem<128>) + 1024));
         DM_CUDA(cudaFuncSetAttribute(delta_roles_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaRolesSmem<256>) + 1024));
-        DM_CUDA(cudaFuncSetAttribute(delta_kernel<true, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaSmem<128>) + 1024));
-        DM_CUDA(cudaFuncSetAttribute(delta_kernel<true, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DeltaSmem<256>) + 1024));
+        DM_CUDA(cudaFuncSetAttribute(rowsum_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowsumSmem<128>) + 1024));
+        DM_CUDA(cudaFuncSetAttribute(rowsum_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RowsumSmem<256>) + 1024));
         return DM_OK;
     });
 }
@@ -580,8 +560,8 @@ extern "C" int dm_delta_fp8_cp(const void* q8, const void* k8, const void* v8, c
     if (!status) return DM_ERR_CUDA;
     DeltaParams p{q8s, k8s, v8s, do8s, lse, nullptr, delta, nullptr, sh.H, sh.Hk, sh.N, h0, hcount, sh.causal, status,
                   dm::RowMap{cp.nq, cp.half_blocks, cp.off0, cp.off1}};
-    return sh.D == 128 ? launch<false, 128>(q8, k8, v8, do8, p, sh, stream, err, errlen)
-                       : launch<false, 256>(q8, k8, v8, do8, p, sh, stream, err, errlen);
+    return sh.D == 128 ? launch<128>(q8, k8, v8, do8, p, sh, stream, err, errlen)
+                       : launch<256>(q8, k8, v8, do8, p, sh, stream, err, errlen);
 }
 
 extern "C" int dm_bwd_dbg_rowsum(const void* q8, const void* k8, const void* v8, const void* do8, const float* q8s, const float* k8s,
@@ -597,6 +577,6 @@ extern "C" int dm_bwd_dbg_rowsum(const void* q8, const void* k8, const void* v8,
     if (!status) return DM_ERR_CUDA;
     DeltaParams p{q8s, k8s, v8s, do8s, lse, delta, rows, rows_abs, sh.H, sh.Hk, sh.N, 0, sh.H, sh.causal, status,
                   dm::RowMap{sh.N, sh.N / 128, 0, 0}};
-    return sh.D == 128 ? launch<true, 128>(q8, k8, v8, do8, p, sh, stream, err, errlen)
-                       : launch<true, 256>(q8, k8, v8, do8, p, sh, stream, err, errlen);
+    return sh.D == 128 ? launch<128>(q8, k8, v8, do8, p, sh, stream, err, errlen)
+                       : launch<256>(q8, k8, v8, do8, p, sh, stream, err, errlen);
 }

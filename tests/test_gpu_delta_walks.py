@@ -1,4 +1,4 @@
-"""Pass 0 at head_dim 256: the persistent roles kernel over walks of one tile, of one item and of several items per CTA, against the
+"""Pass 0: the persistent roles kernel over walks of one tile, of one item and of several items per CTA, against the
 debug row sums: with delta subtracted the rows of P-hat * (dP - delta) cancel to round-off."""
 import pytest
 import torch
@@ -9,9 +9,12 @@ from oracle import dm_oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("B,N,H,Hk,causal", [(1, 128, 2, 1, True), (1, 384, 3, 1, False), (1, 640, 2, 2, True), (3, 1280, 16, 4, True)])
-def test_delta_d256_cancels_the_row_sums(B, N, H, Hk, causal):
-    q, k, v, dO = (t.cuda() for t in O.make_inputs(B, N, H, Hk, 256, 2011))
+@pytest.mark.parametrize("D,unit", [(128, 256), (256, 128)])      # the unit of a sequence's length
+@pytest.mark.parametrize("B,n,H,Hk,causal", [(1, 1, 2, 1, True), (1, 3, 3, 1, False), (1, 5, 2, 2, True), (2, 10, 16, 4, True),
+                                             (16, 1, 64, 8, True)])
+def test_delta_equals_and_cancels_the_row_sums(B, n, H, Hk, causal, D, unit):
+    N = n * unit
+    q, k, v, dO = (t.cuda() for t in O.make_inputs(B, N, H, Hk, D, 2011))
     Q8, Q8s = _lib.quant(0, q)
     K8, K8s = _lib.quant(1, k, _lib.kmean(k))
     V8, V8s = _lib.quant(2, v)
