@@ -469,18 +469,18 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             };
             auto rescale_dv = [&](float mult) {                     // dV's accumulator into the unit of the next dO scale block
 #pragma unroll
-                for (int pc = 0; pc < 4; ++pc) {
-                    uint32_t sa[16];
-                    dm::tmem_ld16(dva + 16 * pc, sa);
+                for (int pc = 0; pc < 8; ++pc) {
+                    uint32_t sa[8];
+                    dm::tmem_ld8(dva + 8 * pc, sa);
                     dm::tmem_ld_wait();
 #pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
+                    for (int i = 0; i < 8; i += 2) {
                         float y0, y1;
                         dm::mul2(y0, y1, __uint_as_float(sa[i]), __uint_as_float(sa[i + 1]), mult, mult);
                         sa[i] = __float_as_uint(y0);
                         sa[i + 1] = __float_as_uint(y1);
                     }
-                    dm::tmem_st16(dva + 16 * pc, sa);
+                    dm::tmem_st8(dva + 8 * pc, sa);
                 }
                 dm::tmem_st_wait();
                 dm::tc_fence_before();

@@ -23,11 +23,10 @@ struct Fwd256Smem {
     alignas(1024) uint8_t q[2][kTile];          // [d half][128 rows x 128 bytes]
     alignas(1024) uint8_t k[2][2][kTile];       // [stage][d half]
     alignas(1024) uint8_t v[2][2][kTile];
-    alignas(1024) uint8_t p[kTile];             // P codes [row][128 keys]
     float gmax[4][128];
     float wgt[4][128];
     float lsum[2][128];
-    uint64_t bar_q, bar_kv[2], bar_s, bar_d;
+    uint64_t bar_q, bar_k[2], bar_v[2], bar_s, bar_d[2];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -59,10 +58,12 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (tid == 0) {
         s.abort_flag = 0;
         dm::mbar_init(&s.bar_q, 1);
-        dm::mbar_init(&s.bar_kv[0], 1);
-        dm::mbar_init(&s.bar_kv[1], 1);
         dm::mbar_init(&s.bar_s, 1);
-        dm::mbar_init(&s.bar_d, 1);
+        for (int i = 0; i < 2; ++i) {
+            dm::mbar_init(&s.bar_k[i], 1);
+            dm::mbar_init(&s.bar_v[i], 1);
+            dm::mbar_init(&s.bar_d[i], 1);
+        }
         dm::fence_mbar_init();
     }
     if (warp == 0) dm::tmem_alloc(&s.tmem_base, 512);
@@ -71,24 +72,23 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     dm::tc_fence_after();
     dm::pdl_wait();
     const uint32_t tmem = s.tmem_base;
-    const uint32_t t_s = tmem, t_d = tmem + 128;          // S: 128 columns; D_grp: 256 columns
+    const uint32_t t_s = tmem, t_d = tmem + 128, t_c = tmem + 384;      // S: 128 columns; D_grp: 256; the tile's codes: 8 per group
     const uint32_t lane_base = (uint32_t)(warp & 3) * 32;
     const int q_row0 = hc.bh * p.N + I * 128;
     const int kv_row0 = hc.bhk * p.N;
     constexpr uint32_t idesc_s = dm::idesc_e4m3(128, 128, false, false);
     constexpr uint32_t idesc_pv = dm::idesc_e4m3(128, 128, false, true);
 
-    auto load_kv = [&](int it) {   // thread 0 only
-        const int j = n_tiles - 1 - it, st = it & 1;
-        dm::mbar_expect_tx(&s.bar_kv[st], 4 * kTile);
-        for (int hh = 0; hh < 2; ++hh) {
-            dm::tma_load_2d(s.k[st][hh], &tm_k, 128 * hh, kv_row0 + j * 128, &s.bar_kv[st]);
-            dm::tma_load_2d(s.v[st][hh], &tm_v, 128 * hh, kv_row0 + j * 128, &s.bar_kv[st]);
-        }
+    auto load = [&](const CUtensorMap* tm, uint8_t (*dst)[kTile], uint64_t* bar, int it) {   // one thread
+        const int j = n_tiles - 1 - it;
+        dm::mbar_expect_tx(bar, 2 * kTile);
+        for (int hh = 0; hh < 2; ++hh) dm::tma_load_2d(dst[hh], tm, 128 * hh, kv_row0 + j * 128, bar);
     };
+    auto load_k = [&](int it) { load(&tm_k, s.k[it & 1], &s.bar_k[it & 1], it); };
+    auto load_v = [&](int it) { load(&tm_v, s.v[it & 1], &s.bar_v[it & 1], it); };
     auto issue_s = [&](int it) {   // thread 0 only
         const int st = it & 1;
-        dm::mbar_wait(&s.bar_kv[st], (it >> 1) & 1, wc);
+        dm::mbar_wait(&s.bar_k[st], (it >> 1) & 1, wc);
         dm::tc_fence_after();
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
@@ -106,8 +106,12 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         dm::mbar_expect_tx(&s.bar_q, 2 * kTile);
         dm::tma_load_2d(s.q[0], &tm_q, 0, q_row0, &s.bar_q);
         dm::tma_load_2d(s.q[1], &tm_q, 128, q_row0, &s.bar_q);
-        load_kv(0);
-        if (n_tiles > 1) load_kv(1);
+        load_k(0);
+        load_v(0);
+        if (n_tiles > 1) {
+            load_k(1);
+            load_v(1);
+        }
         dm::mbar_wait(&s.bar_q, 0, wc);
         issue_s(0);
     }
@@ -117,7 +121,6 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     float o_acc[128];
 #pragma unroll
     for (int i = 0; i < 128; ++i) o_acc[i] = 0.f;
-    int d_phase = 0;
     // the K / V scales of a tile are read one tile ahead: read at the tile's top they are two exposed global loads
     const float* ksb = p.k8s + (int64_t)hc.bhk * (p.N / 32) + 2 * g;
     const float* vsb = p.v8s + (int64_t)hc.bhk * (p.N / 32) + 2 * g;
@@ -136,6 +139,7 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
         dm::mbar_wait(&s.bar_s, it & 1, wc);
         dm::tc_fence_after();
+        if (warp == 0 && it + 2 < n_tiles && dm::elect_one()) load_k(it + 2);      // S has read K
         // ---- pass A: maxima of this thread's two 32-key groups (true units)
         float gm[2];
         float s2[2][32];                                   // this thread's 64 scores, kept through both passes
@@ -163,7 +167,11 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         __syncthreads();
         // every thread holds its scores: S of the next tile may overwrite the buffer, under pass B and the products
-        if (warp == 0 && it + 1 < n_tiles && dm::elect_one()) issue_s(it + 1);
+        // (and every product of the tile before has been folded: its V stage is free)
+        if (warp == 0 && it + 1 < n_tiles && dm::elect_one()) {
+            issue_s(it + 1);
+            if (it >= 1) load_v(it + 1);
+        }
         const float tile_max = fmaxf(fmaxf(s.gmax[0][row], s.gmax[1][row]), fmaxf(s.gmax[2][row], s.gmax[3][row]));
         const float m_new = fmaxf(m_run, tile_max);
         const float m_cur = (m_new == -INFINITY) ? 0.f : m_new;
@@ -193,35 +201,33 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             const float sigma = dm::ex2(ms - ml2);
             lacc = fmaf(sigma, (acc[0] + acc[1]) + (acc[2] + acc[3]), lacc);
             s.wgt[2 * g + gg][row] = vs[gg] * sigma;
-            *reinterpret_cast<uint4*>(s.p + dm::sw128(row, g * 64 + gg * 32)) = make_uint4(codes[0], codes[1], codes[2], codes[3]);
-            *reinterpret_cast<uint4*>(s.p + dm::sw128(row, g * 64 + gg * 32 + 16)) = make_uint4(codes[4], codes[5], codes[6], codes[7]);
+            dm::tmem_st8(dm::tmem_addr(t_c, lane_base, 8 * (2 * g + gg)), codes);       // four codes per column, lane = row
         }
         l_part = fmaf(l_part, alpha, lacc);
         if (!__all_sync(0xffffffffu, alpha == 1.0f)) {
 #pragma unroll
             for (int i = 0; i < 128; ++i) o_acc[i] *= alpha;
         }
-        dm::fence_proxy_async_smem();
+        dm::tmem_st_wait();
         dm::tc_fence_before();
-        __syncthreads();                                   // S consumed, P codes and weights visible
+        __syncthreads();                                   // P codes and weights visible
 
-        // ---- the four groups through the one product buffer.  A group's last two 32-column pieces are held in registers
-        // while thread 0 issues the next group's products, so those form under the additions instead of after them.
-        auto issue_pv = [&](int grp) {   // thread 0 only
+        // ---- the four groups through the product buffer of the warpgroup's d half.  A group's last two 32-column pieces are held in
+        // registers while the warpgroup's first warp issues the next group's product, so it forms under the additions.
+        auto issue_pv = [&](int grp) {   // one thread of the warpgroup
             dm::tc_fence_after();
-            const uint32_t pd = dm::smem_desc_lo_sw128(dm::smem_u32(s.p)) + 2 * grp;      // 32 bytes of keys per group
-#pragma unroll
-            for (int dh = 0; dh < 2; ++dh) {
-                const uint32_t vd = dm::smem_desc_lo_sw128(dm::smem_u32(s.v[st][dh])) + 256 * grp;   // 32 key rows = 4096 bytes
-                dm::umma_e4m3_lo<false>(t_d + 128 * dh, pd, vd, idesc_pv);
-            }
-            dm::umma_commit(&s.bar_d);
+            const uint32_t vd = dm::smem_desc_lo_sw128(dm::smem_u32(s.v[st][g])) + 256 * grp;   // 32 key rows = 4096 bytes
+            dm::umma_e4m3_ts<false>(t_d + 128 * g, t_c + 8 * grp, vd, idesc_pv);
+            dm::umma_commit(&s.bar_d[g]);
         };
-        if (warp == 0 && dm::elect_one()) issue_pv(0);
+        const bool issuer = (warp & 3) == 0;
+        if (issuer && dm::elect_one()) {
+            dm::mbar_wait(&s.bar_v[st], (it >> 1) & 1, wc);
+            issue_pv(0);
+        }
 #pragma unroll 1
         for (int grp = 0; grp < 4; ++grp) {
-            dm::mbar_wait(&s.bar_d, d_phase & 1, wc);
-            ++d_phase;
+            dm::mbar_wait(&s.bar_d[g], grp & 1, wc);
             dm::tc_fence_after();
             const float w = s.wgt[grp][row];
             const uint32_t src = dm::tmem_addr(t_d, lane_base, g * 128);
@@ -243,12 +249,11 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             dm::tmem_ld32(src + 96, sb);
             dm::tmem_ld_wait();
             dm::tc_fence_before();
-            __syncthreads();                               // every thread holds its last two pieces: the buffer is free
-            if (warp == 0 && grp < 3 && dm::elect_one()) issue_pv(grp + 1);
+            dm::named_bar_sync(1 + g, 128);                // every thread holds its last two pieces: the buffer is free
+            if (issuer && grp < 3 && dm::elect_one()) issue_pv(grp + 1);
             add32(2, sa);
             add32(3, sb);
         }
-        if (warp == 0 && it + 2 < n_tiles && dm::elect_one()) load_kv(it + 2);
     }
 
     // ---- epilogue
