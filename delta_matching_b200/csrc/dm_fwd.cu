@@ -52,7 +52,10 @@ struct FwdSmem {
     alignas(1024) uint8_t v[kStages][kTile];
     float ms[kRing][2][128];          // [tile % kRing][key group][row]: the basis of the row's codes, log2 units
     float vs[kRing][2];               // the group's V scale
-    float2 lsum[kItems][4][128];      // [work item % kItems][2 * (tile parity in the item) + key group][row]: part of the denominator and its unit (the maximum it was taken against)
+    // [work item % kItems][2 * (tile parity in the item) + key group][row]: part of the denominator and its unit (log2), and the
+    // maximum of the part's scores
+    float2 lsum[kItems][4][128];
+    float lmax[kItems][4][128];
     alignas(16) uint8_t stg[8][32 * 128];   // per fold warp: its 32 bf16 half rows of O on their way out (16-byte chunks XOR-swizzled by the row)
     uint64_t bar_q[2], bar_q_free[2], bar_kv[kStages], bar_kv_free[kStages], bar_s_full[2], bar_d_full[2][2], bar_l[kItems];   // bar_d_full: [tile parity][key group]
     uint32_t tmem_base;
@@ -291,14 +294,27 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             // ---- the item's epilogue: the softmax warps have left the denominator's four parts
             dm::mbar_wait(&s.bar_l[r % kItems], (r / kItems) & 1, wc);
             float2 lp[4];
+            float mp[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) lp[i] = s.lsum[r % kItems][i][row];
-            const float m = fmaxf(fmaxf(lp[0].y, lp[1].y), fmaxf(lp[2].y, lp[3].y));
+            for (int i = 0; i < 4; ++i) {
+                lp[i] = s.lsum[r % kItems][i][row];
+                mp[i] = s.lmax[r % kItems][i][row];
+            }
+            const float m0 = fmaxf(mp[0], mp[1]), m = fmaxf(m0, fmaxf(mp[2], mp[3])), ml2 = __fmul_rn(m, dm::kLog2e);
             float l = 0.f;
+            if (w.n_tiles == 2) {        // one tile per part: the running sum over the tiles, as a row's softmax in order would form it
+                const float alpha = dm::ex2((m0 - m) * dm::kLog2e), m0l2 = __fmul_rn(m0, dm::kLog2e);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) l += lp[i].x * dm::ex2((lp[i].y - m) * dm::kLog2e);
+                for (int g = 0; g < 2; ++g) {
+                    const float l0 = mp[g] == -INFINITY ? 0.f : __fmul_rn(dm::ex2(lp[g].y - m0l2), lp[g].x);
+                    l += fmaf(l0, alpha, __fmul_rn(dm::ex2(lp[2 + g].y - ml2), lp[2 + g].x));
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) l += mp[i] == -INFINITY ? 0.f : __fmul_rn(lp[i].x, dm::ex2(lp[i].y - ml2));
+            }
             const bool dead = (l == 0.f) || (l != l);
-            const float inv = dead ? 0.f : dm::ex2(ref - m * dm::kLog2e) / l;
+            const float inv = dead ? 0.f : dm::ex2(ref - ml2) / l;
             if (half == 0) p.lse[(int64_t)w.hc.bh * p.rm.nq + w.li * 128 + row] = dead ? -INFINITY : m + logf(l);
             // The bf16 half rows leave through shared memory: stored directly every 16-byte store instruction would touch 32 different
             // rows; from the warp's staging slice each instruction writes four whole 128-byte half rows.  A warp's slice is its own, so
@@ -376,8 +392,8 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 const float dsc = fmaxf(q8sc * ks, 1.2e-38f);
                 const bool diag = p.causal && j == I;
 
-                // ---- S for this thread's (row, key group): 64 fp32 values, 32 at a time.  The second half stays in registers from its
-                // maximum to its codes, the first is read again.
+                // ---- S for this thread's (row, key group): 64 fp32 values, 32 at a time.  The first half stays in registers from its
+                // maximum to its codes, the second is read again.
                 dm::mbar_wait(&s.bar_s_full[team], (t >> 1) & 1, wc);
                 dm::tc_fence_after();
                 float sv[32];
@@ -392,7 +408,7 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     }
                 };
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
+                for (int h = 1; h >= 0; --h) {
                     load(h);
 #pragma unroll
                     for (int c = 0; c < 32; c += 4) {
@@ -412,8 +428,8 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 uint32_t codes[16];
                 const float nms = -ms, cl = __fmul_rn(dsc, dm::kLog2e);
 #pragma unroll
-                for (int h = 1; h >= 0; --h) {
-                    if (h == 0) load(0);
+                for (int h = 0; h < 2; ++h) {
+                    if (h == 1) load(1);
 #pragma unroll
                     for (int c = 0; c < 32; c += 4) {
                         float x0, x1, x2, x3;
@@ -441,9 +457,8 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             }
             // ---- the item's epilogue: this part of the denominator to the fold warps, which write O and LSE.  The parts are numbered by
             // the parity of the tile inside the item: the order of their sum does not depend on the CTA's walk.
-            // It leaves in units of 2^(maximum * log2 e): LSE = maximum + log(sum) then has one rounding at its own size.
-            s.lsum[r % kItems][2 * ((gt ^ team) & 1) + g][row] =
-                make_float2(m_run == -INFINITY ? 0.f : l_part * dm::ex2(l_ref - __fmul_rn(m_run, dm::kLog2e)), m_run);
+            s.lsum[r % kItems][2 * ((gt ^ team) & 1) + g][row] = make_float2(l_part, l_ref);
+            s.lmax[r % kItems][2 * ((gt ^ team) & 1) + g][row] = m_run;
             gt += n_tiles;
             dm::mbar_arrive_warp(&s.bar_l[r % kItems]);
         }
