@@ -28,7 +28,8 @@
 // pace then; so dV accumulates in place and only its unit is moved, off that path.
 // Measured at B4 N4096 H32 causal: 1235 us before; 1290 with dV through X; 1206 with dV in place; 1037 with the unit moved in
 // 16-column pieces (fewer spills in the fold warps, which need 64 accumulators and two 16-register pieces); 960 with 72 / 96 / 24
-// registers per role and a maximum barrier per row half; 900 with the hardware warps in the order service, fold, softmax.
+// registers per role and a maximum barrier per row half; 900 with the hardware warps in the order service, fold, softmax; 875 with
+// the unit moved in 8-column pieces (28 instead of 88 bytes spilled).
 // head_dim 256 (B2 N4096 H16 full): 1350 us with the kernel before this one, 1109 with this.
 #include "dm_attn_common.cuh"
 #include "dm_host.h"

@@ -5,9 +5,15 @@
 // One CTA = 128 query rows of one (batch, head); 256 threads.  A code row is 256 bytes = two 128-byte swizzled sub-tiles
 // (d 0..127 and d 128..255), so S = Q K^T is 8 tcgen05.mma K steps.  Thread (row, warpgroup g) owns key groups 2g and
 // 2g + 1 of the tile (its 64 scores stay in registers from the maxima to the codes, beside the 128 columns of O) and the
-// d columns [128 g, 128 g + 128) of O.  Per group: D_grp = C_grp V_grp as two M128 N128 K32 MMAs (one per d half) into a
-// zero-initialised 256-column temporary, then O += D_grp * w_grp.  The four groups of a tile go through that one temporary
-// in turn.  Every mbarrier wait is bounded.
+// d columns [128 g, 128 g + 128) of O.  Per group: D_grp = C_grp V_grp, one M128 N128 K32 MMA per d half, issued by a thread of the
+// warpgroup that owns the half into the half's zero-initialised temporary, then O += D_grp * w_grp.  The four groups of a tile go
+// through that temporary in turn; the codes lie in tensor memory (A operand), K and V have rings of their own.  Every mbarrier wait is
+// bounded.
+//
+// What bounds it: one thread holds scores and O (255 registers), so there are eight warps and the chain per tile (scores, maxima,
+// exponentials, four rounds of product and fold) is 5900 clocks where exponentials and MMAs are 1024 each.  With the codes through
+// shared memory (a proxy fence each tile) and all 256 threads meeting at every product: B2 N4096 H16 full 726 us, now 702; B1 N1920
+// H8 causal 57 -> 55.
 #include "dm_attn_common.cuh"
 #include "dm_host.h"
 
