@@ -23,11 +23,11 @@ int check_shape(const DmShape& s, int h0, int hcount, char* err, size_t errlen);
 namespace {
 
 constexpr int kTile = 128 * 128;
-constexpr int kStages = 3;        // head_dim 256 kernel
+constexpr int kRing256 = 4;       // head_dim 256 kernel: dS' + K8 stages
 constexpr int kRing = 6;          // head_dim 128 kernel: dS' + K8 stages
 constexpr int kAcc = 4;           // head_dim 128 kernel: product buffers in tensor memory
 constexpr int kFoldThreads = 256;
-constexpr int kThreads128 = kFoldThreads + 64;
+constexpr int kThreads = kFoldThreads + 64;
 
 struct Bwd2Smem {
     alignas(1024) uint8_t a[kRing][kTile];   // dS' tile [key][row]
@@ -70,7 +70,7 @@ __device__ __forceinline__ Bwd2Item bwd2_item(const Bwd2Params& p, int round) {
     return w;
 }
 
-__global__ void __launch_bounds__(kThreads128, 1)
+__global__ void __launch_bounds__(kThreads, 1)
 bwd2_d128_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_k, const Bwd2Params p) {
     extern __shared__ uint8_t smem_raw[];
     Bwd2Smem& s = *reinterpret_cast<Bwd2Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -224,34 +224,42 @@ bwd2_d128_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
 // ---- head_dim 256 ---------------------------------------------------------------------------------------------------------
 // psi is per 64 rows x 64 keys (csrc/fq8_dq_pass2.h:95-125,188 of the reference), so a 128-key tile is two reductions (keys
 // 0..63 and 64..127: two K steps each) times two d halves = four M128 N128 accumulators = all 512 tensor-memory columns;
-// a thread (row, d half) folds the two key halves in ascending order with its row's psi and the F2 / F2b skip rules.
+// a thread (row, d half) folds the two key halves in ascending order with its row's psi and the F2 / F2b skip rules.  The roles are
+// those of head_dim 128; the accumulators of a key half are released as soon as they are in registers, so one key half's products
+// form under the other's fold.  What bounds it: the folds (256 tensor-memory columns a thread and tile).  One role with a
+// __syncthreads per tile, one item per CTA: B2 N4096 H16 full 269 us, with
+// this 213 (537 MB of dS' = 82 us), causal 158 -> 121, B1 N1920 H8 24.7 -> 22.2.
 struct Bwd2Smem256 {
-    alignas(1024) uint8_t a[kStages][kTile];      // dS' tile [key][row]
-    alignas(1024) uint8_t b[kStages][2][kTile];   // K8 tile [d half][key][128 bytes]
-    uint64_t bar_ld[kStages], bar_mma;
+    alignas(1024) uint8_t a[kRing256][kTile];      // dS' tile [key][row]
+    alignas(1024) uint8_t b[kRing256][2][kTile];   // K8 tile [d half][key][128 bytes]
+    alignas(16) uint8_t stg[8][32 * 128];          // per fold warp: 64 bf16 columns of its 32 rows on their way out (chunks XOR-swizzled)
+    uint64_t bar_ld[kRing256], bar_free[kRing256], bar_acc[2], bar_acc_free[2];      // accumulators: by key half
     uint32_t tmem_base;
     int abort_flag;
 };
 
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(kThreads, 1)
 bwd2_d256_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_k, const Bwd2Params p) {
     extern __shared__ uint8_t smem_raw[];
     Bwd2Smem256& s = *reinterpret_cast<Bwd2Smem256*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    const int g = warp >> 2;                           // d half
-    const int row = (warp & 3) * 32 + lane;
-    const dm::HeadCoord hc = dm::head_coord(blockIdx.x, p.h0, p.hcount, p.H, p.Hk);
-    const int bhl = hc.b * p.hcount + (hc.h - p.h0);
-    const int nbn = p.N / 128, nbm = p.N / 64;
-    const int rb = nbn - 1 - (int)blockIdx.y;
-    const int n_it = p.causal ? rb + 1 : nbn;
+    const int nbn = p.N / 128;
+    const int nq_blk = p.rm.nq / 128, nbm_l = p.rm.nq / 64;
     dm::WaitCtx wc{&s.abort_flag, p.status};
 
     if (tid == 0) {
         s.abort_flag = 0;
-        for (int i = 0; i < kStages; ++i) dm::mbar_init(&s.bar_ld[i], 1);
-        dm::mbar_init(&s.bar_mma, 1);
+        for (int i = 0; i < kRing256; ++i) {
+            dm::mbar_init(&s.bar_ld[i], 1);
+            dm::mbar_init(&s.bar_free[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            dm::mbar_init(&s.bar_acc[i], 1);
+            dm::mbar_init(&s.bar_acc_free[i], kFoldThreads / 32);
+        }
         dm::fence_mbar_init();
+        dm::tma_prefetch_desc(&tm_ds);
+        dm::tma_prefetch_desc(&tm_k);
     }
     if (warp == 0) dm::tmem_alloc(&s.tmem_base, 512);
     dm::tc_fence_before();
@@ -259,87 +267,136 @@ bwd2_d256_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
     dm::tc_fence_after();
     dm::pdl_wait();
     const uint32_t tmem = s.tmem_base;
-    const uint32_t lane_base = (uint32_t)(warp & 3) * 32;
-    const int64_t tile0 = ((int64_t)bhl * nbn + rb) * nbn;
-    const int kv_row0 = hc.bhk * p.N;
-    constexpr uint32_t idesc = dm::idesc_e4m3(128, 128, true, true);
 
-    auto load = [&](int it) {
-        const int st = it % kStages;
-        dm::mbar_expect_tx(&s.bar_ld[st], 3 * kTile);
-        dm::tma_load_2d(s.a[st], &tm_ds, 0, (int)((tile0 + it) * 128), &s.bar_ld[st]);
-        dm::tma_load_2d(s.b[st][0], &tm_k, 0, kv_row0 + it * 128, &s.bar_ld[st]);
-        dm::tma_load_2d(s.b[st][1], &tm_k, 128, kv_row0 + it * 128, &s.bar_ld[st]);
-    };
-    auto issue = [&](int it) {
-        const int st = it % kStages;
-        dm::mbar_wait(&s.bar_ld[st], (it / kStages) & 1, wc);
-        dm::tc_fence_after();
-        const uint32_t ad = dm::smem_desc_lo_sw128(dm::smem_u32(s.a[st]));
-#pragma unroll
-        for (int kh = 0; kh < 2; ++kh)
-#pragma unroll
-            for (int dh = 0; dh < 2; ++dh) {
-                const uint32_t bd = dm::smem_desc_lo_sw128(dm::smem_u32(s.b[st][dh]));
-#pragma unroll
-                for (int k2 = 0; k2 < 2; ++k2) {
-                    const uint32_t a = ad + 256 * (2 * kh + k2), b = bd + 256 * (2 * kh + k2), d = tmem + kh * 256 + dh * 128;
-                    if (k2 == 0) dm::umma_e4m3_lo<false>(d, a, b, idesc);
-                    else dm::umma_e4m3_lo<true>(d, a, b, idesc);
+    if (warp == 8) {
+        // ---- TMA loads
+        int t = 0;
+        for (int r = 0;; ++r) {
+            const Bwd2Item w = bwd2_item(p, r);
+            if (!w.valid) break;
+            const int64_t tile0 = ((int64_t)w.bhl * nq_blk + w.rb) * nbn;
+            const int kv_row0 = w.hc.bhk * p.N;
+            for (int it = 0; it < w.n_it; ++it, ++t) {
+                const int st = t % kRing256;
+                if (t >= kRing256) dm::mbar_wait(&s.bar_free[st], (t / kRing256 - 1) & 1, wc);
+                if (dm::elect_one()) {
+                    dm::mbar_expect_tx(&s.bar_ld[st], 3 * kTile);
+                    dm::tma_load_2d(s.a[st], &tm_ds, 0, (int)((tile0 + it) * 128), &s.bar_ld[st]);
+                    dm::tma_load_2d(s.b[st][0], &tm_k, 0, kv_row0 + it * 128, &s.bar_ld[st]);
+                    dm::tma_load_2d(s.b[st][1], &tm_k, 128, kv_row0 + it * 128, &s.bar_ld[st]);
                 }
-            }
-        dm::umma_commit(&s.bar_mma);
-    };
-    if (warp == 0 && dm::elect_one()) {
-        for (int i = 0; i < kStages && i < n_it; ++i) load(i);
-        issue(0);
-    }
-
-    const int mb = 2 * rb + (row >> 6);
-    const float* psi_row = p.psi + ((int64_t)bhl * nbm + mb) * nbm;     // [heads, N/64, N/64]
-    float psi_max = 0.f;
-    float dq[128];
-#pragma unroll
-    for (int i = 0; i < 128; ++i) dq[i] = 0.f;
-
-    for (int it = 0; it < n_it; ++it) {
-        const float psi2[2] = {psi_row[2 * it], psi_row[2 * it + 1]};
-        dm::mbar_wait(&s.bar_mma, it & 1, wc);
-        dm::tc_fence_after();
-        if (warp == 0 && it + kStages < n_it && dm::elect_one()) load(it + kStages);
-#pragma unroll
-        for (int kh = 0; kh < 2; ++kh) {
-            const float psi_cur = psi2[kh];
-            const bool take = (psi_cur != 0.f) && !(psi_cur < psi_max * 1e-8f);
-            if (take) {                                            // warp-uniform
-#pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    float t[32];
-                    dm::tmem_ld32(dm::tmem_addr(tmem + kh * 256 + g * 128, lane_base, 32 * h), reinterpret_cast<uint32_t*>(t));
-                    dm::tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) dq[32 * h + i] = fmaf(t[i], psi_cur, dq[32 * h + i]);
-                }
-                psi_max = fmaxf(psi_max, psi_cur);
+                __syncwarp();
             }
         }
-        dm::tc_fence_before();
-        __syncthreads();
-        if (warp == 0 && it + 1 < n_it && dm::elect_one()) issue(it + 1);
-    }
-
-    const int n_glob = rb * 128 + row;
-    __nv_bfloat16* op = p.dq + (((int64_t)hc.b * p.N + n_glob) * p.H + hc.h) * 256 + g * 128;
+    } else if (warp == 9) {
+        // ---- MMA issue: both operands MN-major, one K step = 32 tile rows = 4096 bytes
+        constexpr uint32_t idesc = dm::idesc_e4m3(128, 128, true, true);
+        constexpr uint32_t kSub = kTile >> 4;
+        const uint32_t a_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.a[0])), b_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.b[0][0]));
+        int t = 0;
+        for (int r = 0;; ++r) {
+            const Bwd2Item w = bwd2_item(p, r);
+            if (!w.valid) break;
+            for (int it = 0; it < w.n_it; ++it, ++t) {
+                const int st = t % kRing256;
+                dm::mbar_wait(&s.bar_ld[st], (t / kRing256) & 1, wc);
 #pragma unroll
-    for (int c = 0; c < 16; ++c) {
-        uint32_t w4[4];
+                for (int kh = 0; kh < 2; ++kh) {
+                    if (t >= 1) dm::mbar_wait(&s.bar_acc_free[kh], (t - 1) & 1, wc);
+                    dm::tc_fence_after();
+                    const uint32_t aa = a_lo + st * kSub + 512 * kh, ba = b_lo + 2 * st * kSub + 512 * kh, d = tmem + 256 * kh;
+                    if (dm::elect_one()) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            __nv_bfloat162 t = __floats2bfloat162_rn(dq[8 * c + 2 * e] * p.final_scale, dq[8 * c + 2 * e + 1] * p.final_scale);
-            w4[e] = *reinterpret_cast<uint32_t*>(&t);
+                        for (int dh = 0; dh < 2; ++dh) {
+                            dm::umma_e4m3_lo<false>(d + 128 * dh, aa, ba + dh * kSub, idesc);
+                            dm::umma_e4m3_lo<true>(d + 128 * dh, aa + 256, ba + dh * kSub + 256, idesc);
+                        }
+                        dm::umma_commit(&s.bar_acc[kh]);
+                        if (kh == 1) dm::umma_commit(&s.bar_free[st]);
+                    }
+                    __syncwarp();
+                }
+            }
         }
-        reinterpret_cast<uint4*>(op)[c] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+    } else {
+        // ---- fold warps: thread = (row, d half g)
+        const int g = warp >> 2;
+        const int row = (warp & 3) * 32 + lane;
+        const uint32_t lane_base = (uint32_t)(warp & 3) * 32;
+        int t = 0;
+        for (int r = 0;; ++r) {
+            const Bwd2Item w = bwd2_item(p, r);
+            if (!w.valid) break;
+            const int mb = 2 * w.rb + (row >> 6);
+            const float2* psi_row = reinterpret_cast<const float2*>(p.psi + ((int64_t)w.bhl * nbm_l + mb) * (2 * nbn));   // [heads, N/64, N/64]
+            float psi_max = 0.f;
+            float dq[128];
+#pragma unroll
+            for (int i = 0; i < 128; ++i) dq[i] = 0.f;
+            float2 psi_n = psi_row[0];                                     // read a tile ahead
+            for (int it = 0; it < w.n_it; ++it, ++t) {
+                const float psi2[2] = {psi_n.x, psi_n.y};
+                if (it + 1 < w.n_it) psi_n = psi_row[it + 1];
+#pragma unroll
+                for (int kh = 0; kh < 2; ++kh) {
+                    const float psi_cur = psi2[kh];
+                    const bool take = (psi_cur != 0.f) && !(psi_cur < psi_max * 1e-8f);
+                    dm::mbar_wait(&s.bar_acc[kh], t & 1, wc);
+                    dm::tc_fence_after();
+                    if (take) {                                            // warp-uniform: a warp's 32 rows share one m-block
+                        // eight 16-column pieces, two in flight (pieces of 32 spill beside the 128 accumulators)
+                        uint32_t ta[16], tb[16];
+                        const uint32_t src = dm::tmem_addr(tmem + kh * 256 + g * 128, lane_base, 0);
+                        auto add16 = [&](int h, const uint32_t* x) {
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) dq[16 * h + i] = fmaf(__uint_as_float(x[i]), psi_cur, dq[16 * h + i]);
+                        };
+                        dm::tmem_ld16(src, ta);
+                        dm::tmem_ld16(src + 16, tb);
+#pragma unroll
+                        for (int h = 0; h < 8; h += 2) {
+                            dm::tmem_ld_wait();
+                            add16(h, ta);
+                            if (h < 6) dm::tmem_ld16(src + 16 * h + 32, ta);
+                            add16(h + 1, tb);
+                            if (h < 6) dm::tmem_ld16(src + 16 * h + 48, tb);
+                        }
+                        psi_max = fmaxf(psi_max, psi_cur);
+                    }
+                    dm::tc_fence_before();
+                    dm::mbar_arrive_warp(&s.bar_acc_free[kh]);
+                }
+            }
+            // the bf16 rows leave through the warp's own staging slice, 64 columns at a time: four whole 128-byte pieces per instruction
+            uint8_t* stg = s.stg[warp];
+            uint8_t* obase = reinterpret_cast<uint8_t*>(p.dq + (((int64_t)w.hc.b * p.rm.nq + w.rb * 128 + (warp & 3) * 32) * p.H + w.hc.h) * 256) + 256 * g;
+            const int64_t row_bytes = (int64_t)p.H * 256 * 2;
+            const int j = lane & 7;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    uint32_t w4[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int i = 64 * h + 8 * c + 2 * e;
+                        __nv_bfloat162 tt = __floats2bfloat162_rn(dq[i] * p.final_scale, dq[i + 1] * p.final_scale);
+                        w4[e] = *reinterpret_cast<uint32_t*>(&tt);
+                    }
+                    *reinterpret_cast<uint4*>(stg + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int rr = 4 * i + (lane >> 3);
+                    const uint4 val = *reinterpret_cast<const uint4*>(stg + rr * 128 + ((j ^ (rr & 7)) << 4));
+                    *reinterpret_cast<uint4*>(obase + rr * row_bytes + 128 * h + (j << 4)) = val;
+                }
+                __syncwarp();
+            }
+        }
     }
+    dm::tc_fence_before();
     __syncthreads();
     if (warp == 0) dm::tmem_dealloc(tmem, 512);
 }
@@ -388,16 +445,11 @@ extern "C" int dm_bwd_fp8_pass2_cp(const void* ds8_ws, const float* psi_ws, cons
     Bwd2Params p{psi_ws, static_cast<__nv_bfloat16*>(dq), sh.H, sh.Hk, sh.N, h0, hcount, sh.causal, sm / 256.0f, status,
                  dm::RowMap{cp.nq, cp.half_blocks, cp.off0, cp.off1}, sh.B * hcount, dm::make_fastdiv(sh.B * hcount), dm::make_fastdiv(hcount),
                  dm::make_fastdiv(sh.H / sh.Hk)};
-    if (sh.D == 256) {
-        const int smem = (int)sizeof(Bwd2Smem256) + 1024;
-        DM_CUDA(dmh::launch_pdl(bwd2_d256_kernel, dim3(sh.B * hcount, sh.N / 128), 256, smem, stream, ts, tk, p));
-        return DM_OK;
-    }
-    const int smem = (int)sizeof(Bwd2Smem) + 1024;
     int sms = 0;
     if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
     const int64_t items = (int64_t)sh.B * hcount * (cp.nq / 128);
     const int grid = (int)(items < sms ? items : sms);
-    DM_CUDA(dmh::launch_pdl(bwd2_d128_kernel, grid, kThreads128, smem, stream, ts, tk, p));
+    if (sh.D == 128) DM_CUDA(dmh::launch_pdl(bwd2_d128_kernel, grid, kThreads, (int)sizeof(Bwd2Smem) + 1024, stream, ts, tk, p));
+    else DM_CUDA(dmh::launch_pdl(bwd2_d256_kernel, grid, kThreads, (int)sizeof(Bwd2Smem256) + 1024, stream, ts, tk, p));
     return DM_OK;
 }
