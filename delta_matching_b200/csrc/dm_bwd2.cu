@@ -226,9 +226,9 @@ bwd2_d128_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
 // 0..63 and 64..127: two K steps each) times two d halves = four M128 N128 accumulators = all 512 tensor-memory columns;
 // a thread (row, d half) folds the two key halves in ascending order with its row's psi and the F2 / F2b skip rules.  The roles are
 // those of head_dim 128; the accumulators of a key half are released as soon as they are in registers, so one key half's products
-// form under the other's fold.  What bounds it: the folds (256 tensor-memory columns a thread and tile).  One role with a
-// __syncthreads per tile, one item per CTA: B2 N4096 H16 full 269 us, with
-// this 213 (537 MB of dS' = 82 us), causal 158 -> 121, B1 N1920 H8 24.7 -> 22.2.
+// form under the other's fold.  What bounds it: the folds (256 tensor-memory columns a thread and tile).  Against one role with a
+// __syncthreads per tile and one item per CTA: B2 N4096 H16 full 269 -> 191 us (537 MB of dS' = 82 us), causal 158 -> 110, B1 N1920
+// H8 24.7 -> 20.
 struct Bwd2Smem256 {
     alignas(1024) uint8_t a[kRing256][kTile];      // dS' tile [key][row]
     alignas(1024) uint8_t b[kRing256][2][kTile];   // K8 tile [d half][key][128 bytes]
@@ -344,22 +344,24 @@ bwd2_d256_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
                     dm::mbar_wait(&s.bar_acc[kh], t & 1, wc);
                     dm::tc_fence_after();
                     if (take) {                                            // warp-uniform: a warp's 32 rows share one m-block
-                        // eight 16-column pieces, two in flight (pieces of 32 spill beside the 128 accumulators)
-                        uint32_t ta[16], tb[16];
+                        // sixteen 8-column pieces, two in flight (pieces of 16 spill beside the 128 accumulators: 213 against 191 us)
+                        uint32_t ta[8], tb[8];
                         const uint32_t src = dm::tmem_addr(tmem + kh * 256 + g * 128, lane_base, 0);
-                        auto add16 = [&](int h, const uint32_t* x) {
+                        auto add8 = [&](int h, const uint32_t* x) {
 #pragma unroll
-                            for (int i = 0; i < 16; ++i) dq[16 * h + i] = fmaf(__uint_as_float(x[i]), psi_cur, dq[16 * h + i]);
+                            for (int i = 0; i < 8; i += 2)
+                                dm::fma2(dq[8 * h + i], dq[8 * h + i + 1], __uint_as_float(x[i]), __uint_as_float(x[i + 1]), psi_cur, dq[8 * h + i],
+                                         dq[8 * h + i + 1]);
                         };
-                        dm::tmem_ld16(src, ta);
-                        dm::tmem_ld16(src + 16, tb);
+                        dm::tmem_ld8(src, ta);
+                        dm::tmem_ld8(src + 8, tb);
 #pragma unroll
-                        for (int h = 0; h < 8; h += 2) {
+                        for (int h = 0; h < 16; h += 2) {
                             dm::tmem_ld_wait();
-                            add16(h, ta);
-                            if (h < 6) dm::tmem_ld16(src + 16 * h + 32, ta);
-                            add16(h + 1, tb);
-                            if (h < 6) dm::tmem_ld16(src + 16 * h + 48, tb);
+                            add8(h, ta);
+                            if (h < 14) dm::tmem_ld8(src + 8 * h + 16, ta);
+                            add8(h + 1, tb);
+                            if (h < 14) dm::tmem_ld8(src + 8 * h + 24, tb);
                         }
                         psi_max = fmaxf(psi_max, psi_cur);
                     }
