@@ -11,23 +11,28 @@
 //   S = Q K^T            4 x tcgen05.mma (M128 N128 K32) into the tensor-memory buffer of the tile's parity, i.e. of its team
 //   softmax              basis ms_g = max(gm_g*l2, m*l2 - 12) - log2(448) (gm: the group's maximum in this tile, m: the thread's own
 //                        running one), codes = e4m3(2^(S*l2 - ms_g)) written back into tensor memory over the scores they came from
-//                        (four codes per column, lane = row); the denominator's part is summed from the unrounded p.  ms_g goes to a
-//                        ring; nothing is exchanged between softmax threads
+//                        (four codes per column, lane = row).  ms_g, gm_g and the sum of the unrounded p go to a ring; nothing is
+//                        exchanged between softmax threads
 //   D_g = C_g V_g        2 x tcgen05.mma per group (A = the codes in tensor memory, B = the V tile) into zero-initialised
 //                        tensor-memory temporaries, issued when the codes are stored and the previous product has been read
-//   O += D_g * v8sc_g 2^(ms_g - ref)    by the fold warps; ref, O's basis, moves only when ms_g has passed it by 8 binades, and O is
-//                        divided by the denominator (the sum of the four threads' parts of a row) once, at the item's end
+//   fold                 the row's softmax in tile order: M = max(M, gm_0, gm_1), alpha = 2^((M_before - M)*l2), s_g = 2^(ms_g - M*l2),
+//                        l_g = l_g alpha + s_g sum_g, O = O alpha + D_0 (v8sc_0 s_0) + D_1 (v8sc_1 s_1); O / (l_0 + l_1) at the end
 // K / V tiles arrive by TMA into a 3-stage ring.  Every mbarrier wait is bounded.
 //
 // Why this shape.  A 128 x 128 tile holds 1024 clocks of exponentials and 512 of MMAs; with one set of softmax warps the wait for
 // S, the maxima, the exchange of the running maximum and the codes (about 1200 clocks a tile) ran with the exponential unit idle.  Two
-// teams half a tile apart overlap them, which needs two things gone: the running maximum handed from tile to tile (a serial chain
-// through both teams: measured slower than one set) and the rescaling of O at every new maximum.  A running maximum of the
-// thread's own only lowers the 12-binade floor of a group's basis (never the precision of its codes), and the bases, all powers
-// of two's arguments kept in fp32, meet in the fold.  The kernel is now bound by the fold (about 1950 clocks a tile: 2 x 64
-// tensor-memory columns and 128 multiply-adds per thread next to the MMAs' traffic); its 64 accumulators leave room for 8-column pieces only.
-// Measured (us, before -> two teams -> 8-column pieces): B1 N16384 H32 causal 2023 -> 1904 -> 1835; B4 N4096 H32 causal
-// 577 -> 560 -> 535; B2 N2048 H16 causal 51.2 -> 49.5.
+// teams half a tile apart overlap them, which needs the running maximum handed from tile to tile gone from the softmax warps (a serial
+// chain through both teams: measured slower than one set).  It lives in the fold warps, which see the tiles in order: a running
+// maximum of the softmax thread's own only lowers the 12-binade floor of a group's basis (never the precision of its codes).
+// Why O and l are kept against the row's maximum of the moment and not in a basis that moves only now and then: in a row of few keys
+// O is a code times a V scale, and where the scale has few significant bits (the block's maximum / 448, a maximum whose significand is a
+// multiple of 7) up to half of these products lie exactly half way between two bf16 values: the last bit of a weight decides dozens of
+// elements of O at once, and through rowsum(dO * O) a visible part of the row's dQ.  Both forms are equally accurate; this one
+// rounds as a plain row softmax does, and it costs nothing: the softmax warps lose their share of the denominator and the fold its
+// epilogue, which pays for the multiplications of O (lazy basis -> this, us: B4 N4096 H32 causal 500 -> 499, B1 N16384 H32 1776 -> 1783,
+// B4 N768 H12 22.5 -> 20.5, B64 N256 H16 59.4 -> 53.2).
+// 28 warps' chains at about 55 % issue utilisation bound the kernel, no single resource: of the lazy form's 531 us at B4 N4096 H32 (on a
+// slower clock) 526 were left without the exponentials and 508 without three quarters of the fold's loads.
 #include "dm_attn_common.cuh"
 #include "dm_host.h"
 
@@ -43,7 +48,6 @@ constexpr int kRegSoftmax = 64, kRegFold = 104, kRegService = 40;      // per th
 // its next arrival on the same barrier needs a product that is issued behind the synchronising side's).
 constexpr int kBarCodes = 1;       // + 2 * team + key group: the group's codes are in tensor memory     128 + 32
 constexpr int kBarDFree = 5;       // + key group: the fold warps hold the group's product              256 + 32
-constexpr int kItems = 8;          // a team without a tile in a one-tile item can be four items ahead of the fold warps
 constexpr int kRing = 4;           // depth of the per-tile row-constant ring between softmax and fold warps
 
 struct FwdSmem {
@@ -51,13 +55,10 @@ struct FwdSmem {
     alignas(1024) uint8_t k[kStages][kTile];
     alignas(1024) uint8_t v[kStages][kTile];
     float ms[kRing][2][128];          // [tile % kRing][key group][row]: the basis of the row's codes, log2 units
+    float2 gp[kRing][2][128];         // the group's maximum and the sum of its exponentials against ms
     float vs[kRing][2];               // the group's V scale
-    // [work item % kItems][2 * (tile parity in the item) + key group][row]: part of the denominator and its unit (log2), and the
-    // maximum of the part's scores
-    float2 lsum[kItems][4][128];
-    float lmax[kItems][4][128];
     alignas(16) uint8_t stg[8][32 * 128];   // per fold warp: its 32 bf16 half rows of O on their way out (16-byte chunks XOR-swizzled by the row)
-    uint64_t bar_q[2], bar_q_free[2], bar_kv[kStages], bar_kv_free[kStages], bar_s_full[2], bar_d_full[2][2], bar_l[kItems];   // bar_d_full: [tile parity][key group]
+    uint64_t bar_q[2], bar_q_free[2], bar_kv[kStages], bar_kv_free[kStages], bar_s_full[2], bar_d_full[2][2];   // bar_d_full: [tile parity][key group]
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -121,7 +122,6 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             dm::mbar_init(&s.bar_q[i], 1);
             dm::mbar_init(&s.bar_q_free[i], 1);
         }
-        for (int i = 0; i < kItems; ++i) dm::mbar_init(&s.bar_l[i], kSoftmaxThreads / 32);
         dm::fence_mbar_init();
         dm::tma_prefetch_desc(&tm_q);
         dm::tma_prefetch_desc(&tm_k);
@@ -242,30 +242,40 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             float o_acc[64];
 #pragma unroll
             for (int i = 0; i < 64; ++i) o_acc[i] = 0.f;
-            float ref = -INFINITY;                     // o_acc's basis, log2 units: O = o_acc * 2^ref / denominator
+            float m_run = -INFINITY, l0 = 0.f, l1 = 0.f;        // the row's running maximum, the denominator's part per key group
             for (int it = 0; it < n_tiles; ++it) {
                 const int t = gt + it, b = t & 1, rg = t % kRing;
-#pragma unroll
-                for (int g = 0; g < 2; ++g) {
-                    dm::mbar_wait(&s.bar_d_full[b][g], (t >> 1) & 1, wc);      // also orders the ring slot written before the codes
-                    dm::tc_fence_after();
-                    // eight 8-column pieces, two in flight (16-column pieces spill beside the 64 accumulators: 1904 against 1832 us at
-                    // B1 N16384 H32); the first pair arrives while the weight is worked out
-                    uint32_t sa[8], sb[8];
-                    auto ld8 = [&](int pc, uint32_t* x) { dm::tmem_ld8(src + 128 * g + 8 * pc, x); };
-                    ld8(0, sa);
-                    ld8(1, sb);
-                    const float ms = s.ms[rg][g][row], vs = s.vs[rg][g];
-                    // The basis moves only when a group's basis has grown 8 binades past it (a weight stays below 2^8 times its V scale,
-                    // far inside fp32), so O is rescaled a few times per item instead of at every new maximum.
-                    const bool grow = ms > ref + 8.0f;
-                    if (__any_sync(0xffffffffu, grow)) {
-                        const float alpha = grow ? dm::ex2(ref - ms) : 1.0f;
-                        if (grow) ref = ms;
+                dm::mbar_wait(&s.bar_d_full[b][0], (t >> 1) & 1, wc);      // also order the ring slot, written before the codes
+                dm::mbar_wait(&s.bar_d_full[b][1], (t >> 1) & 1, wc);
+                dm::tc_fence_after();
+                // sixteen 8-column pieces, two in flight (16-column pieces spill beside the 64 accumulators: 1904 against 1832 us at
+                // B1 N16384 H32); the first pair arrives while the weights are worked out, and group 1's under group 0's last additions
+                uint32_t sa[8], sb[8];
+                auto ld8 = [&](int pc, uint32_t* x) { dm::tmem_ld8(src + 8 * pc, x); };
+                ld8(0, sa);
+                ld8(1, sb);
+                float w0, w1;
+                {
+                    const float2 g0 = s.gp[rg][0][row], g1 = s.gp[rg][1][row];
+                    const float m_new = fmaxf(m_run, fmaxf(g0.x, g1.x));
+                    const float m_cur = (m_new == -INFINITY) ? 0.f : m_new;
+                    const float alpha = dm::ex2((m_run - m_cur) * dm::kLog2e);
+                    // M * l2 is not rounded on its own here (fma): the weight is the power of two of the basis' true distance
+                    const float s0 = dm::ex2(fmaf(-m_cur, dm::kLog2e, s.ms[rg][0][row]));
+                    const float s1 = dm::ex2(fmaf(-m_cur, dm::kLog2e, s.ms[rg][1][row]));
+                    l0 = fmaf(l0, alpha, __fmul_rn(s0, g0.y));
+                    l1 = fmaf(l1, alpha, __fmul_rn(s1, g1.y));
+                    w0 = s.vs[rg][0] * s0;
+                    w1 = s.vs[rg][1] * s1;
+                    m_run = m_new;
+                    if (__any_sync(0xffffffffu, alpha != 1.0f)) {
 #pragma unroll
                         for (int i = 0; i < 64; i += 2) dm::mul2(o_acc[i], o_acc[i + 1], o_acc[i], o_acc[i + 1], alpha, alpha);
                     }
-                    const float wg = ms == -INFINITY ? 0.f : vs * dm::ex2(ms - ref);      // (a group without a visible key)
+                }
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    const float wg = g ? w1 : w0;
                     auto add8 = [&](int pc, const uint32_t* x) {
 #pragma unroll
                         for (int i = 0; i < 8; i += 2)
@@ -276,46 +286,28 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                     for (int q = 0; q < 3; ++q) {
                         dm::tmem_ld_wait();
                         add8(2 * q, sa);
-                        ld8(2 * q + 2, sa);
+                        ld8(16 * g + 2 * q + 2, sa);
                         add8(2 * q + 1, sb);
-                        ld8(2 * q + 3, sb);
+                        ld8(16 * g + 2 * q + 3, sb);
                     }
                     dm::tmem_ld_wait();
                     dm::tc_fence_before();
                     dm::named_bar_arrive(kBarDFree + g, 256 + 32);
                     add8(6, sa);
+                    if (g == 0) ld8(16, sa);
                     add8(7, sb);
+                    if (g == 0) ld8(17, sb);
                 }
             }
             gt += n_tiles;
             int r_again = r;
             asm volatile("" : "+r"(r_again));
             const FwdItem w = fwd_item(p, r_again);
-            // ---- the item's epilogue: the softmax warps have left the denominator's four parts
-            dm::mbar_wait(&s.bar_l[r % kItems], (r / kItems) & 1, wc);
-            float2 lp[4];
-            float mp[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                lp[i] = s.lsum[r % kItems][i][row];
-                mp[i] = s.lmax[r % kItems][i][row];
-            }
-            const float m0 = fmaxf(mp[0], mp[1]), m = fmaxf(m0, fmaxf(mp[2], mp[3])), ml2 = __fmul_rn(m, dm::kLog2e);
-            float l = 0.f;
-            if (w.n_tiles == 2) {        // one tile per part: the running sum over the tiles, as a row's softmax in order would form it
-                const float alpha = dm::ex2((m0 - m) * dm::kLog2e), m0l2 = __fmul_rn(m0, dm::kLog2e);
-#pragma unroll
-                for (int g = 0; g < 2; ++g) {
-                    const float l0 = mp[g] == -INFINITY ? 0.f : __fmul_rn(dm::ex2(lp[g].y - m0l2), lp[g].x);
-                    l += fmaf(l0, alpha, __fmul_rn(dm::ex2(lp[2 + g].y - ml2), lp[2 + g].x));
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) l += mp[i] == -INFINITY ? 0.f : __fmul_rn(lp[i].x, dm::ex2(lp[i].y - ml2));
-            }
+            // ---- the item's epilogue
+            const float l = l0 + l1;
             const bool dead = (l == 0.f) || (l != l);
-            const float inv = dead ? 0.f : dm::ex2(ref - ml2) / l;
-            if (half == 0) p.lse[(int64_t)w.hc.bh * p.rm.nq + w.li * 128 + row] = dead ? -INFINITY : m + logf(l);
+            const float inv = dead ? 0.f : 1.0f / l;
+            if (half == 0) p.lse[(int64_t)w.hc.bh * p.rm.nq + w.li * 128 + row] = dead ? -INFINITY : m_run + logf(l);
             // The bf16 half rows leave through shared memory: stored directly every 16-byte store instruction would touch 32 different
             // rows; from the warp's staging slice each instruction writes four whole 128-byte half rows.  A warp's slice is its own, so
             // the hand-over needs no more than the warp.
@@ -372,9 +364,8 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             const float q8sc = q8sc_nx;
             const float* ksp = p.k8s + (int64_t)w.hc.bhk * (p.N / 64) + g;
             const float* vsp = p.v8s + (int64_t)w.hc.bhk * (p.N / 64) + g;
-            // The thread's own running maximum (its group, its team's tiles): it only places the floor of the basis, 12 binades below
-            // it.  The denominator's part is kept in a unit of its own that moves like the fold warps' basis.
-            float m_run = -INFINITY, l_part = 0.f, l_ref = -INFINITY;
+            // The thread's own running maximum (its group, its team's tiles): it only places the floor of the basis, 12 binades below it.
+            float m_run = -INFINITY;
             float ks_n = ks_nx, vs_n = vs_nx;
             w = fwd_item(p, r + 1);
             first_scales(w, gt + n_tiles);
@@ -421,7 +412,7 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 const bool some = m_run != -INFINITY;              // a key has been visible
                 const float ms = fmaxf(gm * dm::kLog2e, (some ? m_run * dm::kLog2e : 0.f) - dm::kPhatFloorB) - dm::kLog2_448;
                 // the ring slot of tile t - kRing has been read: its fold released the group's product before the product of tile t - 3,
-                // and S of this tile waited for the product of tile t - 2.  A group without a visible key weighs nothing.
+                // and S of this tile waited for the product of tile t - 2.  A group without a visible key weighs nothing (2^-inf).
                 s.ms[rg][g][row] = some ? ms : -INFINITY;
                 if (lane == 0) s.vs[rg][g] = vs;
                 float part0 = 0.f, part1 = 0.f;
@@ -441,26 +432,15 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                         codes[8 * h + (c >> 2)] = dm::cvt_e4m3x4(p0, p1, p2, p3);
                     }
                 }
+                s.gp[rg][g][row] = make_float2(gm, part0 + part1);
                 // the codes go back into tensor memory, over the first 16 columns of this thread's own 64 scores (all read by now): the
                 // P V products take them from there as their A operand, four e4m3 per column, lane = row
                 dm::tmem_st16(t_s, codes);
                 dm::tmem_st_wait();
                 dm::tc_fence_before();
                 dm::named_bar_arrive(kBarCodes + 2 * team + g, 128 + 32);
-                if (some) {
-                    if (ms > l_ref + 8.0f) {
-                        l_part *= dm::ex2(l_ref - ms);
-                        l_ref = ms;
-                    }
-                    l_part = fmaf(dm::ex2(ms - l_ref), part0 + part1, l_part);
-                }
             }
-            // ---- the item's epilogue: this part of the denominator to the fold warps, which write O and LSE.  The parts are numbered by
-            // the parity of the tile inside the item: the order of their sum does not depend on the CTA's walk.
-            s.lsum[r % kItems][2 * ((gt ^ team) & 1) + g][row] = make_float2(l_part, l_ref);
-            s.lmax[r % kItems][2 * ((gt ^ team) & 1) + g][row] = m_run;
             gt += n_tiles;
-            dm::mbar_arrive_warp(&s.bar_l[r % kItems]);
         }
     }
     dm::tc_fence_before();
