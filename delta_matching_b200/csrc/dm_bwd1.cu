@@ -102,6 +102,12 @@ constexpr int kThreads = 896;
 constexpr int kRegSoftmax = 72, kRegFold = 96, kRegService = 24;     // per thread after setmaxnreg: the sum is the launch pool
 constexpr int kRows = 3;               // ring of row constants
 constexpr int kGf = 4;                 // ring of product scales between softmax and fold warps
+// Tiles that dV's accumulator sums by itself.  The tensor pipe's fp32 additions drop what does not fit (they round towards zero), so the
+// sum of a long walk drifts: by 8.7e-7 of its size over 32 tiles, 3.5e-6 over 128, 1.9e-5 over 512, where rounded additions stay below
+// 2e-7; a drift of 1.9e-5 moves one bf16 value in two hundred.  So a walk of more than kWindow tiles moves the accumulator into an fp32
+// sum in memory every kWindow tiles, and starts it again: 1.6e-6 over 512 tiles.  Shorter windows drift less and cost more (pass 1 at
+// B1 N16384 H8, us: none 763, 64 tiles 769, 32 tiles 795); a shape of up to 64 row blocks never gets there.
+constexpr int kWindow = 64;
 
 // Named barriers.  Warp-to-warp hand-offs cost a quarter of an mbarrier's; an arriving side is never a whole round ahead, because
 // its next arrival on the same barrier needs a product that is issued behind the synchronising side's.
@@ -314,7 +320,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                             if (t > 0 || m > 0) dm::named_bar_sync(kBarDvFree, 256 + 32);
                             dm::tc_fence_after();
                             if (dm::elect_one()) {
-                                dm::umma_e4m3_lo_rt(t_dva, pa + 4 * m, dos + 512 * m, idesc_x, it > 0 || m > 0);
+                                dm::umma_e4m3_lo_rt(t_dva, pa + 4 * m, dos + 512 * m, idesc_x, (it >> 1) % kWindow != 0 || m > 0);
 #pragma unroll
                                 for (int k = 1; k < (kD == 128 ? 4 : 2); ++k)
                                     dm::umma_e4m3_lo<true>(t_dva, pa + 4 * m + 2 * k, dos + 512 * m + 256 * k, idesc_x);
@@ -437,12 +443,17 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         const uint32_t x_src = dm::tmem_addr(t_x, lane_base, 64 * half), dva = dm::tmem_addr(t_dva, lane_base, 64 * half);
         int t = 0;
         for (int r = 0;; ++r) {
-            const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
-            if (!w.valid) break;
+            int n_it;                                  // all that the tile loop keeps of the item: it has no registers to spare
+            float ik;                                  // for the epilogue; read early
+            {
+                const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
+                if (!w.valid) break;
+                n_it = w.n_it;
+                ik = 1.0f / p.k8s[(int64_t)w.hc.bhk * (p.N / G::kKeysPerScale) + G::kGrp * w.J + key / G::kKeysPerScale];
+            }
             float dk_acc[64];
 #pragma unroll
             for (int i = 0; i < 64; ++i) dk_acc[i] = 0.f;
-            const float ik = 1.0f / p.k8s[(int64_t)w.hc.bhk * (p.N / G::kKeysPerScale) + G::kGrp * w.J + key / G::kKeysPerScale];   // for the epilogue; read early
             auto fold_dk = [&](const float* g, int m) {             // two products a tile
                 dm::mbar_wait(&s.bar_x_full, m, wc);                // also orders the ring slot written before the codes
                 dm::tc_fence_after();
@@ -487,28 +498,77 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                 dm::tc_fence_before();
                 dm::named_bar_arrive(kBarDvFree, 256 + 32);
             };
-            for (int it = 0; it < w.n_it; it += 2, ++t) {
-                const float* g = s.gf[t % kGf] + (kD == 128 ? 0 : key >> 6);
-                fold_dk(g, 0);
-                if (kD == 256) {
-                    dm::mbar_wait(&s.bar_dv_full, 0, wc);            // two commits a tile, as for X
-                    dm::tc_fence_after();
-                    rescale_dv(s.sc[t % kRows][5]);
+            // The fp32 sum of dV's earlier windows lives in the item's own outputs, which are written at its end: a warp's 32 keys x 64
+            // columns of dK and dV are 8 KB, its share of the sum.  Unit u (16 columns) is in dV's (u even) or dK's half rows, at 64 bytes
+            // times u / 2: the epilogue's stores of a unit's columns then cover only what has been read.  (fp32 outputs: in dV itself.)  A
+            // slot is one thread's own; the lanes of a warp take whole 64-byte pieces.
+            struct DvSum {
+                uint8_t* at;                           // unit 0's slot of this lane
+                int64_t odd, even;                     // from there to units 1 and 2
+                int64_t step;                          // eight keys
+            };
+            auto dv_sum = [&]() {
+                int r_again = r;                       // (looked up again: the tile loop has no registers for it)
+                asm volatile("" : "+r"(r_again));
+                const dm::Bwd1Item v = dm::bwd1_item<kD>(p, r_again);
+                const int64_t at = (((int64_t)v.hc.b * p.N + v.J * 128 + lane_base + (lane >> 2)) * p.H + v.hc.h) * kD + 128 * v.zh + 64 * half;
+                const int64_t keys8 = (int64_t)p.H * (8 * kD);
+                uint8_t* dv = reinterpret_cast<uint8_t*>(p.dv) + 16 * (lane & 3);
+                if (kD == 128 && p.out_fp32) return DvSum{dv + 4 * at, 64, 128, 4 * keys8};
+                return DvSum{dv + 2 * at, reinterpret_cast<uint8_t*>(p.dk) - reinterpret_cast<uint8_t*>(p.dv), 64, 2 * keys8};
+            };
+            auto flush_dv = [&](float unit, bool first) {
+                DvSum m = dv_sum();
+#pragma unroll 1
+                for (int u = 0; u < 4; ++u) {
+                    uint8_t* to = m.at + ((u & 1) ? m.odd : 0) + ((u & 2) ? m.even : 0);
+#pragma unroll
+                    for (int c = 0; c < 16; c += 8) {
+                        uint32_t sa[8];
+                        dm::tmem_ld8(dva + 16 * u + c, sa);
+                        dm::tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 8; e += 4, to += m.step) {
+                            const float4 y = make_float4(__uint_as_float(sa[e]) * unit, __uint_as_float(sa[e + 1]) * unit,
+                                                         __uint_as_float(sa[e + 2]) * unit, __uint_as_float(sa[e + 3]) * unit);
+                            if (first) *reinterpret_cast<float4*>(to) = y;
+                            else dm::red_add_f32x4(to, y);
+                        }
+                    }
                 }
-                fold_dk(g, 1);                                       // (head_dim 128: its product was committed behind the tile's dV)
-                if (kD == 256) {
-                    dm::mbar_wait(&s.bar_dv_full, 1, wc);
-                    dm::tc_fence_after();
+                dm::tc_fence_before();
+                dm::named_bar_arrive(kBarDvFree, 256 + 32);
+            };
+            for (int it = 0; it < n_it;) {
+                const int end = min(n_it, it + 2 * kWindow);
+                for (; it < end; it += 2, ++t) {
+                    const float* g = s.gf[t % kGf] + (kD == 128 ? 0 : key >> 6);
+                    fold_dk(g, 0);
+                    if (kD == 256) {
+                        dm::mbar_wait(&s.bar_dv_full, 0, wc);            // two commits a tile, as for X
+                        dm::tc_fence_after();
+                        rescale_dv(s.sc[t % kRows][5]);
+                    }
+                    fold_dk(g, 1);                                       // (head_dim 128: its product was committed behind the tile's dV)
+                    if (kD == 256) {
+                        dm::mbar_wait(&s.bar_dv_full, 1, wc);
+                        dm::tc_fence_after();
+                    }
+                    if (it + 2 < end) {
+                        const int slot = (t + 1) % kRows;
+                        dm::mbar_wait(&s.bar_rows_full[slot], ((t + 1) / kRows) & 1, wc);
+                        rescale_dv(s.sc[slot][4]);
+                    }
                 }
-                if (it + 2 < w.n_it) {
-                    const int slot = (t + 1) % kRows;
-                    dm::mbar_wait(&s.bar_rows_full[slot], ((t + 1) / kRows) & 1, wc);
-                    rescale_dv(s.sc[slot][4]);
-                }
+                if (n_it > 2 * kWindow) flush_dv(s.fv[(t + kGf - 1) % kGf], it == 2 * kWindow);
             }
 
-            // ---- epilogue: dK *= 1 / k8s, dV from its accumulator, per query head
-            const bool have_dv = w.n_it > 0;
+            // ---- epilogue: dK *= 1 / k8s, dV from its accumulator, per query head.  After a long walk dV's accumulator has joined the sum of
+            // the windows, and dV leaves first: dK's rows hold a part of that sum.
+            const bool have_dv = n_it > 0, have_sum = (n_it >> 1) > kWindow;
+            int r_again = r;
+            asm volatile("" : "+r"(r_again));
+            const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r_again);
             const float fv = have_dv ? s.fv[(t + kGf - 1) % kGf] : 0.f;      // dV's last unit
             const int64_t row_stride = (int64_t)p.H * kD;            // elements between consecutive keys
             const int64_t off = (((int64_t)w.hc.b * p.N + w.J * 128) * p.H + w.hc.h) * kD + 128 * w.zh + 64 * half;   // key 0 of the block
@@ -521,19 +581,28 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                     for (int i = 0; i < 16; ++i) y[i] = 0.f;
                 }
             };
-            if (p.out_fp32) {
+            auto sum16 = [&](const DvSum& m, int u, float* y) {
+                const uint8_t* from = m.at + ((u & 1) ? m.odd : 0) + ((u & 2) ? m.even : 0);
+#pragma unroll
+                for (int j = 0; j < 4; ++j, from += m.step) *reinterpret_cast<float4*>(y + 4 * j) = __ldcg(reinterpret_cast<const float4*>(from));
+                __syncwarp();                                        // the warp has read the unit: its place may be written
+            };
+            if (kD == 128 && p.out_fp32) {                         // (refused at head_dim 256)
                 float4* ok = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dk) + off + key * row_stride);
                 float4* ov = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dv) + off + key * row_stride);
 #pragma unroll
                 for (int c = 0; c < 16; ++c)
                     ok[c] = make_float4(dk_acc[4 * c] * ik, dk_acc[4 * c + 1] * ik, dk_acc[4 * c + 2] * ik, dk_acc[4 * c + 3] * ik);
-#pragma unroll
+                const DvSum m = dv_sum();
+#pragma unroll 1
                 for (int pc = 0; pc < 4; ++pc) {
                     float y[16];
-                    dv16(pc, y);
+                    if (have_sum) sum16(m, pc, y);
+                    else dv16(pc, y);
+                    const float f = have_sum ? 1.0f : fv;
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
-                        ov[4 * pc + c] = make_float4(y[4 * c] * fv, y[4 * c + 1] * fv, y[4 * c + 2] * fv, y[4 * c + 3] * fv);
+                        ov[4 * pc + c] = make_float4(y[4 * c] * f, y[4 * c + 1] * f, y[4 * c + 2] * f, y[4 * c + 3] * f);
                 }
             } else {
                 // The bf16 rows leave through the warp's own staging slice, kStgCols columns at a time: a thread holds one key, so
@@ -562,25 +631,41 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                     }
                     __syncwarp();
                 };
+                if (have_sum) {
+                    const DvSum m = dv_sum();
+#pragma unroll 1
+                    for (int h = 0; h < 64 / G::kStgCols; ++h) {
+#pragma unroll
+                        for (int pc = 0; pc < kCh / 2; ++pc) {
+                            float y[16];
+                            sum16(m, (kCh / 2) * h + pc, y);
+                            put8(2 * pc, y, 1.0f);
+                            put8(2 * pc + 1, y + 8, 1.0f);
+                        }
+                        out(p.dv, h);
+                    }
+                }
 #pragma unroll
                 for (int h = 0; h < 64 / G::kStgCols; ++h) {
 #pragma unroll
                     for (int c = 0; c < kCh; ++c) put8(c, dk_acc + G::kStgCols * h + 8 * c, ik);
                     out(p.dk, h);
                 }
+                if (!have_sum) {
 #pragma unroll
-                for (int h = 0; h < 64 / G::kStgCols; ++h) {
+                    for (int h = 0; h < 64 / G::kStgCols; ++h) {
 #pragma unroll
-                    for (int pc = 0; pc < kCh / 2; ++pc) {
-                        float y[16];
-                        dv16((kCh / 2) * h + pc, y);
-                        put8(2 * pc, y, fv);
-                        put8(2 * pc + 1, y + 8, fv);
+                        for (int pc = 0; pc < kCh / 2; ++pc) {
+                            float y[16];
+                            dv16((kCh / 2) * h + pc, y);
+                            put8(2 * pc, y, fv);
+                            put8(2 * pc + 1, y + 8, fv);
+                        }
+                        out(p.dv, h);
                     }
-                    out(p.dv, h);
                 }
             }
-            if (have_dv) {
+            if (have_dv && !have_sum) {
                 dm::tc_fence_before();
                 dm::named_bar_arrive(kBarDvFree, 256 + 32);
             }

@@ -119,6 +119,11 @@ __device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// Four fp32 additions at one 16-byte address, performed in L2 (rounded to nearest); nothing is returned.
+__device__ __forceinline__ void red_add_f32x4(void* to, const float4& y) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(to), "f"(y.x), "f"(y.y), "f"(y.z), "f"(y.w) : "memory");
+}
+
 // Register re-allocation between warpgroups (all 128 threads of a warpgroup execute it): the issuer warpgroup gives
 // registers back, the compute warpgroups take them.  Counts are multiples of 8.
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
