@@ -148,12 +148,15 @@ def _kv_index(BH, H, Hk):
     return (bh // H) * Hk + (bh % H) // (H // Hk)
 
 
-def forward(Q8, Q8s, K8, K8s, V8, V8s, H, Hk, causal=True, tile_keys=None, pv="chain", acc=F32):
+def forward(Q8, Q8s, K8, K8s, V8, V8s, H, Hk, causal=True, tile_keys=None, pv="chain", acc=F32, floor="row"):
     """The faithful forward.  Codes [BH, N, D] / [BHk, N, D] e4m3, scales fp32.  Returns O (B, N, H, D) bf16 and
     LSE [BH, N] fp32 (natural log).  tile_keys = keys per online-softmax step (reference: 256 at D=128, 128 at D=256);
     pv = "chain" (the reference's zero-initialised tile temp with the rho chain and one promote per tile,
     mainloop_fwd_sm90_fp8f.hpp:1410-1418,1507-1515) or "group" (O += D_g * w_g per key group: the same sum in another
-    rounding order, softmax_fq8f.h kGroupsPerPromote == 1 form)."""
+    rounding order, softmax_fq8f.h kGroupsPerPromote == 1 form).  floor = what the 12-binade floor of a group's basis hangs on: "row" the
+    row's running maximum (the reference), "own" the running maximum of the groups at the same place of every other tile (the
+    head_dim-128 kernel, whose softmax threads see no others): never above the row's, so a basis is never higher and a code never
+    coarser than with "row"."""
     BH, N, D = Q8.shape
     rq, rk = blocks(D)
     if tile_keys is None:
@@ -174,6 +177,7 @@ def forward(Q8, Q8s, K8, K8s, V8, V8s, H, Hk, causal=True, tile_keys=None, pv="c
         l = torch.zeros(BH, BM, dtype=F32)
         Oacc = torch.zeros(BH, BM, D, dtype=F32)
         t_hi = ((r0 + BM - 1) // tile_keys) if causal else (N // tile_keys - 1)
+        own = {}
         for T in range(t_hi, -1, -1):
             S, gm = [], []
             for g in range(gpt):
@@ -195,7 +199,11 @@ def forward(Q8, Q8s, K8, K8s, V8, V8s, H, Hk, causal=True, tile_keys=None, pv="c
             accl = torch.zeros_like(l)
             ms_l, C_l = [], []
             for g in range(gpt):
-                ms = torch.maximum(gm[g] * l2, ml2 - _f32(PHAT_FLOOR_B)) - _f32(LOG2_448)
+                top = ml2
+                if floor == "own":
+                    own[T & 1, g] = torch.maximum(own.get((T & 1, g), gm[g]), gm[g])
+                    top = torch.where(own[T & 1, g] == -math.inf, torch.zeros_like(ml2), own[T & 1, g]) * l2
+                ms = torch.maximum(gm[g] * l2, top - _f32(PHAT_FLOOR_B)) - _f32(LOG2_448)
                 p = torch.exp2(S[g] * l2 - ms[..., None])
                 accl = accl + torch.exp2(ms - ml2) * p.sum(dim=-1)
                 ms_l.append(ms)

@@ -99,3 +99,25 @@ def test_rows_of_one_key_round_as_a_row_softmax(N, H, Hk, seed):
     rms = ref.square().mean().sqrt()
     off = ((dq - ref).abs() / ref.abs().clamp_min(rms))[:, 0].max().item()
     assert off <= 1 / 8 + 1 / 256, off                 # one e4m3 step of the row's single dS' code, one bf16 rounding
+
+
+@pytest.mark.parametrize("N,causal", [(512, True), (768, False)])
+def test_the_floor_of_a_basis_hangs_on_the_threads_own_maximum(N, causal):
+    """Every other 64-key group lies about 25 binades below its neighbours and carries values 2^24 times theirs.  Against the row's maximum,
+    12 binades up, most of its codes would be subnormal or zero; against the maximum of its own thread's groups they are whole."""
+    B, H, Hk, D = 1, 4, 2, 128
+    g = torch.Generator().manual_seed(9)
+    code = lambda h, f: torch.randn(B * h, N, D, generator=g).mul_(f).clamp_(-448, 448).to(torch.float8_e4m3fn)
+    Q8, K8, V8 = code(H, 100.0), code(Hk, 100.0), code(Hk, 100.0)
+    Q8s, V8s = torch.full((B * H, N // 128), 1.0 / 100), torch.full((B * Hk, N // 64), 2.0 ** -7)
+    K8s = torch.full((B * Hk, N // 64), 0.7 / 100)
+    K8s[:, 1::2] *= 0.05
+    V8s[:, 1::2] *= 2.0 ** 24
+    c = (Q8, Q8s, K8, K8s, V8, V8s)
+    own, lse_ref = O.forward(*c, H, Hk, causal, tile_keys=128, pv="group", floor="own")
+    row, _ = O.forward(*c, H, Hk, causal, tile_keys=128, pv="group")
+    o, lse = _lib.fwd_fp8(*(t.cuda() for t in (Q8, K8, V8, Q8s, K8s, V8s)), B, H, Hk, causal)
+    assert _lib.device_status() == 0
+    assert (lse.cpu() - lse_ref).abs().max() < 2e-4
+    assert O.rel(o.cpu(), own) < 2e-3, O.rel(o.cpu(), own)
+    assert O.rel(row, own) > 2e-2, O.rel(row, own)          # the inputs tell the two forms apart

@@ -94,6 +94,16 @@ def test_forward_realizations_agree(cfg1):
     assert O.rel(b["dQ"], a["dQ"]) < 1e-3
 
 
+def test_floor_forms_of_the_forward():
+    """The floor of a group's basis against the row's running maximum or the thread's own: the same codes at ordinary scores (no group lies
+    12 binades below another), single code steps of groups that weigh below 2^-12 at scores of 8 times that."""
+    q, k, v, _ = O.make_inputs(1, 512, 2, 2, 128, 3)
+    for scale, bound in ((1, 0.0), (8, 2.0 ** -12)):
+        c = O.quant_q((q * scale).transpose(1, 2)) + O.quant_k(k.transpose(1, 2))[:2] + O.quant_v(v.transpose(1, 2))
+        row, own = (O.forward(*c, 2, 2, True, tile_keys=128, pv="group", floor=f) for f in ("row", "own"))
+        assert O.rel(own[0], row[0]) <= bound and torch.equal(own[1], row[1])
+
+
 def test_fp64_accumulate_is_close_to_fp32(cfg1):
     q, k, v, dO, _ = cfg1
     a = O.attention_fwd_bwd(q, k, v, dO, True, "matched")
