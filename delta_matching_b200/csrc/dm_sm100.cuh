@@ -90,10 +90,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
 // One lane of a converged warp (always the same one).  Under this predicate the compiler knows that a single lane executes the
 // asynchronous instruction and feeds its descriptors from uniform registers; under `lane == 0` it cannot, and every
 // tcgen05.mma costs the issuing warp more.  Pass 1: 1268 -> 1211 us (B4 N4096 H32 Hk8 causal), 1638 -> 1418 us at head_dim 256
-// (B2 N4096 H16 Hk4 full); pass 2: 236 -> 225 us.  The forward and pass 0's role kernel, whose issuing warps wait most of
-// their time, did not gain and keep `lane == 0`.
-// A warp index taken through __shfl_sync tells the compiler the same about the role branch; it is used where it measured
-// faster (pass 2: 225 -> 217 us, forward at head_dim 256: 714 -> 699 us), not in pass 1 (1211 -> 1268 us).
+// (B2 N4096 H16 Hk4 full); pass 2: 236 -> 225 us.  Pass 0's role kernel, whose issuing warps wait most of their time, did not gain and
+// keeps `lane == 0`.  A warp index taken through __shfl_sync tells the compiler the same about the role branch (pass 2: 225 -> 217 us,
+// forward at head_dim 256: 714 -> 699 us).
 __device__ __forceinline__ bool elect_one() {
     uint32_t ok;
     asm volatile(
