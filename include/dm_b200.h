@@ -143,7 +143,8 @@ int dm_bwd_workspace_bytes(DmShape s, int32_t hcount, size_t* ds8_bytes, size_t*
 
 /* Pass 1: dK, dV (B, N, H, D) bf16 per QUERY head, the dS' code tiles and psi.  Pass 2: dQ (B, N, H, D) bf16.
  * Together they replace torch.ops.delta_matching.bwd_fp8_t (csrc/delta_matching_api.cpp:224-392, 429-438); the split
- * lets a caller run pass 2 of one head group on another stream (delta_matching/split.py:51-92). */
+ * lets a caller run pass 2 of one head group on another stream (delta_matching/split.py:51-92).  While pass 1 runs, the dK / dV
+ * rows of its heads hold partial sums of long walks: the two buffers must not overlap. */
 int dm_bwd_fp8_pass1(const void* q8, const void* k8, const void* v8, const void* do8, const float* q8s, const float* k8s,
                      const float* v8s, const float* do8s, const float* lse, const float* delta, DmShape s, int32_t h0,
                      int32_t hcount, void* dk_bf16, void* dv_bf16, void* ds8_ws, float* psi_ws, void* stream, char* err,
