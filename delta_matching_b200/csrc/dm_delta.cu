@@ -463,10 +463,11 @@ delta_roles_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                             sv[c] = dm::ex2(fminf(sv[c], dm::kMoE + 4.0f));
                             sv[c + 1] = dm::ex2(fminf(sv[c + 1], dm::kMoE + 4.0f));
                         }
-                        if (diag) {                                 // the diagonal tile only: keys above the row
+                        if (diag && 2 * g + half >= (warp & 3)) {   // the diagonal tile, 32 keys on or above the warp's 32 rows
+                            const int last = (2 * g + half == (warp & 3) ? lane : -1) - 16 * q;
 #pragma unroll
                             for (int c = 0; c < 16; ++c)
-                                if (g * 64 + c0 + c > row) sv[c] = 0.f;
+                                if (c > last) sv[c] = 0.f;
                         }
 #pragma unroll
                         for (int c = 0; c < 16; c += 2) {

@@ -353,8 +353,17 @@ __device__ __forceinline__ uint32_t cvt_e4m3x2(float lo, float hi) {
     asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
     return r;
 }
+// Four codes in one register: joined by a 16-bit pair move, which the second conversion does on the way (an `or` with a shift costs
+// an instruction of its own, one per four codes: forward at B4 N4096 H32 causal 504 -> 502 us).
 __device__ __forceinline__ uint32_t cvt_e4m3x4(float a, float b, float c, float d) {
-    return cvt_e4m3x2(a, b) | (cvt_e4m3x2(c, d) << 16);
+    uint32_t r;
+    asm("{\n\t.reg .b16 l, h;\n\t"
+        "cvt.rn.satfinite.e4m3x2.f32 l, %2, %1;\n\t"
+        "cvt.rn.satfinite.e4m3x2.f32 h, %4, %3;\n\t"
+        "mov.b32 %0, {l, h};\n\t}"
+        : "=r"(r)
+        : "f"(a), "f"(b), "f"(c), "f"(d));
+    return r;
 }
 
 }  // namespace dm
