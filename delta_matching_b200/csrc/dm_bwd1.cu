@@ -1,20 +1,20 @@
-// Pass 1 of the backward: dK and dV per query head, plus the e4m3 dS' code tiles and their psi scales for pass 2
+// Pass 1 of the backward at head_dim 128 (head_dim 256: dm_bwd1_d256.cu): dK and dV per query head, plus the e4m3 dS' code tiles and
+// their psi scales for pass 2
 // (csrc/mainloop_bwd_sm90_fp8r.hpp:695-952 of the reference, restated for tcgen05).
 //
 // One work item = one 128-key block of one (batch, query head), walked in tiles of 128 rows (two 64-row m-blocks) from the causal
-// start; at head_dim 256 one of its two d halves (Geo below).  The kernel is persistent: one CTA per SM walks its share of the items, every
+// start.  The kernel is persistent: one CTA per SM walks its share of the items, every
 // role keeps its own place in the list, and the next item starts under the tail of the current one.  896 threads:
 //   warps 0..15  softmax: P-hat, dS', the tile maxima, psi and both code tiles
 //   warps 16..23 fold: thread = (key, 64 d columns); dK in registers, and dV's accumulator kept in the unit of the next dO block
 //   warps 24..27 service, one per scheduler: the S / dP MMAs, the dK / dV MMAs and the dS' store, the TMA loads, the row constants
 // Per tile:
-//   S = Q K^T, dP = dO V^T   M128 N128 K32 x 4 each (x 8 at head_dim 256), tensor-memory lane = row, as soon as the softmax warps hold
+//   S = Q K^T, dP = dO V^T   M128 N128 K32 x 4 each, tensor-memory lane = row, as soon as the softmax warps hold
 //                            the previous pair
 //   softmax warps            codes P-hat8 = e4m3(P-hat), dS'8 = e4m3(dS' / psi), psi by the F2 / F2b rules from the tile maxima
 //   X = dS'8(m0)^T Q8        fold: dK += X * (psi 2^-8 q8sc)
 //   dV += P-hat8^T dO8       into the accumulator itself (tensor memory), which is in units of this block's dO scale
 //   X = dS'8(m1)^T Q8        fold: dK += X * (psi 2^-8 q8sc); then dV's accumulator times (this block's / the next one's dO scale)
-// (head_dim 256 has a dO scale per m-block: dV's product is formed m-block by m-block, its accumulator moved after each.)
 // Q8 / dO8 tiles serve twice: K-major as the A operand of S / dP and MN-major as the B operand of dK / dV.
 //
 // Why this shape.  The kernel before this one held S^T / dP^T (lane = key) for one 64-row m-block at a time: N = 64 MMAs run the
@@ -30,7 +30,6 @@
 // 16-column pieces (fewer spills in the fold warps, which need 64 accumulators and two 16-register pieces); 960 with 72 / 96 / 24
 // registers per role and a maximum barrier per row half; 900 with the hardware warps in the order service, fold, softmax; 875 with
 // the unit moved in 8-column pieces (28 instead of 88 bytes spilled).
-// head_dim 256 (B2 N4096 H16 full): 1350 us with the kernel before this one, 1109 with this.
 #include "dm_attn_common.cuh"
 #include "dm_host.h"
 
@@ -52,29 +51,26 @@ struct Bwd1Params {
     RowMap rm;                                    // which rows of the sequence the Q-side tensors hold
     int out_fp32;                                 // dK / dV leave as fp32 (partials that another rank's are added to)
     int n_heads;                                  // batch * hcount: (batch, query head) pairs of this call
-    FastDiv fd_heads, fd_hcount, fd_rep, fd_nbn;  // divisions by n_heads, hcount, H / Hk and N / 128
+    FastDiv fd_heads, fd_hcount, fd_rep;          // divisions by n_heads, hcount and H / Hk
 };
 
-// The work list: one item = one 128-key block J of one (batch, query head) (and one d half at head_dim 256), ordered by
+// The work list: one item = one 128-key block J of one (batch, query head), ordered by
 // key block, i.e. heaviest first when causal.  CTA c takes position c of the even rounds and G - 1 - c of the odd ones
 // (a snake), so the long and the short items of a round pair up.
 struct Bwd1Item {
     HeadCoord hc;
-    int J, zh, m_lo, n_it, bhl;                   // m_lo, n_it: first 64-row m-block and their count, both even
+    int J, m_lo, n_it, bhl;                   // m_lo, n_it: first 64-row m-block and their count, both even
     bool valid;
 };
-template <int kD>
 __device__ __forceinline__ Bwd1Item bwd1_item(const Bwd1Params& p, int round) {
     Bwd1Item w;
     const int G = gridDim.x, c = blockIdx.x;
     const int nbn = p.N / 128;
     const int idx = round * G + ((round & 1) ? G - 1 - c : c);
-    w.valid = idx < p.n_heads * nbn * (kD / 128);
-    const int jz = (int)fdiv((uint32_t)idx, p.fd_heads);
-    w.hc = head_coord(idx - jz * p.n_heads, p.h0, p.fd_hcount, p.H, p.Hk, p.fd_rep);
+    w.valid = idx < p.n_heads * nbn;
+    w.J = (int)fdiv((uint32_t)idx, p.fd_heads);
+    w.hc = head_coord(idx - w.J * p.n_heads, p.h0, p.fd_hcount, p.H, p.Hk, p.fd_rep);
     w.bhl = w.hc.b * p.hcount + (w.hc.h - p.h0);
-    w.zh = kD == 128 ? 0 : (int)fdiv((uint32_t)jz, p.fd_nbn);   // d half whose dK / dV columns the item keeps
-    w.J = jz - w.zh * nbn;
     // m-blocks are counted in the local rows; global position grows with the local index, and both chunks of a row map
     // start on a 128-row pair, so local and global m-block parity agree.  Causal: start at the first local m-block that is
     // not wholly above the diagonal of key block J; a rank may hold none (n_it == 0: dK = dV = 0 for this block).
@@ -112,65 +108,39 @@ constexpr int kWindow = 64;
 // Named barriers.  Warp-to-warp hand-offs cost a quarter of an mbarrier's; an arriving side is never a whole round ahead, because
 // its next arrival on the same barrier needs a product that is issued behind the synchronising side's.
 constexpr int kBarSpFree = 1;          // (S | dP) is in registers                          512 + 32
-constexpr int kBarAmax = 2;            // + psi tile: its warps' maxima are in shared memory  256 (head_dim 256: 128)
+constexpr int kBarAmax = 2;            // + m-block: its warps' maxima are in shared memory  256
 constexpr int kBarCodes = 6;           // + tile parity: the tile's codes are               512 + 32
 constexpr int kBarXFree = 8;           // the fold warps hold the dK product                256 + 32
 constexpr int kBarDvFree = 9;          // dV's accumulator is in the next block's unit      256 + 32
 
-// Geometry per head dim.  head_dim 256 (csrc/mainloop_bwd_sm90_fp8v10.hpp:1674-1761 of the reference): a code row is two
-// 128-byte sub-tiles, K / V scales per 32 keys, Q / dO scales per 64-row m-block (so dV's unit moves at every m-block), psi per
-// 64 rows x 64 keys.  The accumulators of 128 keys x 256 columns do not fit, so two work items (d half 0 and 1) share a key block:
-// both form S / dP, each keeps its 128 columns of dK / dV, and only d half 0 stores the dS' tiles and psi.  An item's own half of Q
-// and dO lives until the products have read it, the other half only until S / dP have: one stage of it is enough.  S of the next
-// tile is late behind the own half's two stages (the products end about 2000 clocks after the codes, a load takes 1300 more), and
-// there is no room for a third; Q and dO are released apart, each behind the last product that reads it, and S does not wait for dO
-// (B2 N4096 H16 full: 1217 -> 1141 us; 1109 with the other half loaded first and without a wait for the products before S; a stage
-// of both halves for S / dP and one of the own half for the products: 1292).
-template <int kD>
-struct Geo {
-    static constexpr int kDH = kD / 128;
-    static constexpr int kOwn = kD == 128 ? 3 : 2;       // ring of the tiles of Q / dO that the products read (the item's d half)
-    static constexpr int kOth = kD == 128 ? 0 : 1;       // stage of the other d half
-    static constexpr int kDs = kD == 128 ? 2 : 1;        // dS' code tiles
-    static constexpr int kStgCols = kD == 128 ? 32 : 16; // columns of the output staging
-    static constexpr int kKeysPerScale = kD == 128 ? 64 : 32;
-    static constexpr int kGrp = 128 / kKeysPerScale;     // K / V scales per key block
-    static constexpr int kPsiKeys = kD == 128 ? 1 : 2;   // psi tiles along the keys of a key block
-    static constexpr int kPsiWarps = 8 / kPsiKeys;       // softmax warps of a psi tile
-};
+constexpr int kStages = 3;             // ring of Q / dO tiles
+constexpr int kStgCols = 32;           // columns of the output staging
 
-template <int kD>
 struct Smem {
-    using G = Geo<kD>;
-    alignas(1024) uint8_t k[G::kDH][kTile];
-    alignas(1024) uint8_t v[G::kDH][kTile];
-    alignas(1024) uint8_t q[G::kOwn + G::kOth][kTile];      // the own half's stages, then the other half's
-    alignas(1024) uint8_t dO[G::kOwn + G::kOth][kTile];
+    alignas(1024) uint8_t k[kTile];
+    alignas(1024) uint8_t v[kTile];
+    alignas(1024) uint8_t q[kStages][kTile];
+    alignas(1024) uint8_t dO[kStages][kTile];
     alignas(1024) uint8_t pt[2][kTile];       // P-hat codes, [key][row], by tile parity
-    alignas(1024) uint8_t ds[G::kDs][kTile];  // dS' codes, same layout
-    alignas(16) uint8_t stg[8][32 * 2 * G::kStgCols];  // per fold warp: 32 keys of bf16 columns on their way out (chunks XOR-swizzled)
+    alignas(1024) uint8_t ds[2][kTile];       // dS' codes, same layout
+    alignas(16) uint8_t stg[8][32 * 2 * kStgCols];  // per fold warp: 32 keys of bf16 columns on their way out (chunks XOR-swizzled)
     alignas(16) float2 rd[kRows][128];        // per row: 8 - lse * log2e, -delta
-    alignas(16) float sc[kRows][8];                       // of m-block m: [m] q8sc, [2 + m] do8sc, [4 + m] what dV's accumulator is multiplied by
-                                              // before it, [6 + m] dV's unit
-    float gf[kGf][4];                         // dK scale of m-block m, 64-key half h at [2 m + h]
+    alignas(16) float sc[kRows][4];           // q8sc, do8sc, what dV's accumulator is multiplied by before the tile, dV's unit
+    float gf[kGf][2];                         // dK scale of m-block m
     float fv[kGf];                            // dV's unit after the tile
-    float psi[kGf][4];                        // psi of m-block m (psi tile h along the keys: [2 m + h]), on its way to pass 2
-    float amax[2][16];                        // [tile parity][psi tile, warp of it]
-    uint64_t bar_kv, bar_kv_free, bar_own[3], bar_own_free[3], bar_dov[2], bar_dov_free[2], bar_oth, bar_oth_free, bar_sp_full, bar_x_full,
-        bar_dv_full, bar_done[2], bar_ds_free[2], bar_rows_full[kRows], bar_rows_free[kRows];
+    float psi[kGf][2];                        // psi of m-block m, on its way to pass 2
+    float amax[2][16];                        // [tile parity][m-block, warp of it]
+    uint64_t bar_kv, bar_kv_free, bar_qdo[kStages], bar_qdo_free[kStages], bar_sp_full, bar_x_full, bar_done[2], bar_ds_free[2], bar_rows_full[kRows], bar_rows_free[kRows];
     uint32_t tmem_base;
     int abort_flag;
 };
 
-template <int kD>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
             const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
             const __grid_constant__ CUtensorMap tm_ds, const dm::Bwd1Params p) {
     extern __shared__ uint8_t smem_raw[];
-    using G = Geo<kD>;
-    constexpr int kDH = G::kDH, kOwn = G::kOwn;
-    Smem<kD>& s = *reinterpret_cast<Smem<kD>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    Smem& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     // The hardware warps are taken in the order service, fold, softmax (the role numbers below keep their tensor-memory quarter,
     // warp mod 4): 949 -> 900 us against softmax first (B4 N4096 H32 causal).
     const int tid = threadIdx.x, lane = tid & 31, hw_warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -186,12 +156,9 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         dm::mbar_init(&s.bar_kv_free, 1);
         dm::mbar_init(&s.bar_sp_full, 1);
         dm::mbar_init(&s.bar_x_full, 1);
-        dm::mbar_init(&s.bar_dv_full, 1);
-        dm::mbar_init(&s.bar_oth, 1);
-        dm::mbar_init(&s.bar_oth_free, 1);
-        for (int i = 0; i < kOwn; ++i) {
-            dm::mbar_init(&s.bar_own[i], 1);
-            dm::mbar_init(&s.bar_own_free[i], 1);
+        for (int i = 0; i < kStages; ++i) {
+            dm::mbar_init(&s.bar_qdo[i], 1);
+            dm::mbar_init(&s.bar_qdo_free[i], 1);
         }
         for (int i = 0; i < kRows; ++i) {
             dm::mbar_init(&s.bar_rows_full[i], 1);
@@ -199,9 +166,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         }
         for (int i = 0; i < 2; ++i) {
             dm::mbar_init(&s.bar_done[i], 1);
-            dm::mbar_init(&s.bar_dov[i], 1);
-            dm::mbar_init(&s.bar_dov_free[i], 1);
-            dm::mbar_init(&s.bar_ds_free[i], kD == 128 ? 1 : 2);
+            dm::mbar_init(&s.bar_ds_free[i], 1);
         }
         dm::fence_mbar_init();
     }
@@ -226,18 +191,16 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             const uint32_t q_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[0])), do_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.dO[0]));
             int t = 0, kvn = 0;
             for (int r = 0;; ++r) {
-                const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item(p, r);
                 if (!w.valid) break;
                 const int n = w.n_it >> 1;
                 if (n > 0) dm::mbar_wait(&s.bar_kv, kvn++ & 1, wc);
                 for (int it = 0; it < n; ++it, ++t) {
-                    const int st = t % kOwn;
-                    dm::mbar_wait(&s.bar_own[st], (t / kOwn) & 1, wc);
-                    if (kD == 256) dm::mbar_wait(&s.bar_oth, t & 1, wc);
+                    const int st = t % kStages;
+                    dm::mbar_wait(&s.bar_qdo[st], (t / kStages) & 1, wc);
                     // The softmax warps rewrite the code tiles of tile t - 2: its products and its dS' store must be done.  Gating the
-                    // products gates the softmax warps.  (head_dim 256: dO's stage was refilled behind the last product of tile t - 2, and
-                    // the softmax warps wait for the one dS' tile themselves.)
-                    if (kD == 128 && t >= 2) {
+                    // products gates the softmax warps.
+                    if (t >= 2) {
                         dm::mbar_wait(&s.bar_done[t & 1], ((t - 2) >> 1) & 1, wc);
                         dm::mbar_wait(&s.bar_ds_free[t & 1], ((t - 2) >> 1) & 1, wc);
                     }
@@ -246,21 +209,15 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                     dm::tc_fence_after();
                     if (dm::elect_one()) {
 #pragma unroll
-                        for (int m = 0; m < 2; ++m) {              // S, then dP; the d halves in order, whichever is the item's own
-                            if (kD == 256 && m == 1) dm::mbar_wait(&s.bar_dov[st], (t / kOwn) & 1, wc);
+                        for (int m = 0; m < 2; ++m) {              // S, then dP
+                            const uint32_t a = (m ? do_lo : q_lo) + st * kSub, b = m ? v_lo : k_lo, d = tmem + 128 * m;
 #pragma unroll
-                            for (int hh = 0; hh < kDH; ++hh) {
-                                const uint32_t a = (m ? do_lo : q_lo) + (kD == 128 || hh == w.zh ? st : kOwn) * kSub;
-                                const uint32_t b = (m ? v_lo : k_lo) + hh * kSub, d = tmem + 128 * m;
-#pragma unroll
-                                for (int k = 0; k < 4; ++k) {
-                                    if ((hh | k) == 0) dm::umma_e4m3_lo<false>(d, a, b, idesc_sp);
-                                    else dm::umma_e4m3_lo<true>(d, a + 2 * k, b + 2 * k, idesc_sp);
-                                }
+                            for (int k = 0; k < 4; ++k) {
+                                if (k == 0) dm::umma_e4m3_lo<false>(d, a, b, idesc_sp);
+                                else dm::umma_e4m3_lo<true>(d, a + 2 * k, b + 2 * k, idesc_sp);
                             }
                         }
                         dm::umma_commit(&s.bar_sp_full);
-                        if (kD == 256) dm::umma_commit(&s.bar_oth_free);
                         if (it == n - 1) dm::umma_commit(&s.bar_kv_free);     // the loader may bring the next item's K / V
                     }
                     __syncwarp();
@@ -274,16 +231,14 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             const uint32_t pt_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.pt[0])), ds_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.ds[0]));
             int t = 0;
             for (int r = 0;; ++r) {
-                const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item(p, r);
                 if (!w.valid) break;
                 int ds_row = (int)((((int64_t)w.bhl * nq_blk + (w.m_lo >> 1)) * nbn + w.J) * 128);   // dS' tile of the first row block
-                const int psi_stride = nbn * G::kPsiKeys;
-                float* psi_out = p.psi + ((int64_t)w.bhl * (2 * nq_blk) + w.m_lo + (lane >> 1)) * psi_stride + G::kPsiKeys * w.J + (lane & 1);
-                const bool psi_lane = w.zh == 0 && lane < 4 && (lane & 1) < G::kPsiKeys;
+                float* psi_out = p.psi + ((int64_t)w.bhl * (2 * nq_blk) + w.m_lo + lane) * nbn + w.J;
                 for (int it = 0; it < w.n_it; it += 2, ++t, ds_row += nbn * 128) {
-                    const int par = t & 1, st = t % kOwn, dt = kD == 128 ? par : 0;
-                    const uint32_t qs = q_lo + st * kSub, dos = do_lo + st * kSub, da = ds_lo + dt * kSub, pa = pt_lo + par * kSub;
-                    if (kD == 128 && t >= 1 && dm::elect_one()) {       // the previous tile has left shared memory
+                    const int par = t & 1, st = t % kStages;
+                    const uint32_t qs = q_lo + st * kSub, dos = do_lo + st * kSub, da = ds_lo + par * kSub, pa = pt_lo + par * kSub;
+                    if (t >= 1 && dm::elect_one()) {       // the previous tile has left shared memory
                         dm::tma_store_wait_read0();
                         dm::mbar_arrive(&s.bar_ds_free[par ^ 1]);
                     }
@@ -298,35 +253,25 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                             dm::umma_e4m3_lo<false>(t_x, da + 4 * m, qs + 512 * m, idesc_x);
                             dm::umma_e4m3_lo<true>(t_x, da + 4 * m + 2, qs + 512 * m + 256, idesc_x);
                             dm::umma_commit(&s.bar_x_full);
-                            if (m == 0 && w.zh == 0) {     // (d half 1 stores nothing but arrives all the same)
-                                dm::tma_store_2d(&tm_ds, 0, ds_row, s.ds[dt]);
+                            if (m == 0) {
+                                dm::tma_store_2d(&tm_ds, 0, ds_row, s.ds[par]);
                                 dm::tma_store_commit();
-                            }
-                            if (kD == 128 && m == 1) {
-                                dm::umma_commit(&s.bar_own_free[st]);       // the stage's Q / dO have been read for the last time
+                            } else {
+                                dm::umma_commit(&s.bar_qdo_free[st]);       // the stage's Q / dO have been read for the last time
                                 dm::umma_commit(&s.bar_done[par]);
-                            }
-                            if (kD == 256 && m == 1) {     // the one dS' tile has been read by both products, and has left
-                                dm::umma_commit(&s.bar_own_free[st]);
-                                dm::umma_commit(&s.bar_ds_free[0]);
-                                dm::tma_store_wait_read0();
-                                dm::mbar_arrive(&s.bar_ds_free[0]);
                             }
                         }
                         __syncwarp();
-                        if (m == 0 && psi_lane) psi_out[(int64_t)it * psi_stride] = s.psi[t % kGf][lane];
+                        if (m == 0 && lane < 2) psi_out[(int64_t)it * nbn] = s.psi[t % kGf][lane];
                         // dV += P-hat8^T dO8 of a whole dO scale block, in the accumulator itself
-                        if (kD == 256 || m == 0) {
-                            if (t > 0 || m > 0) dm::named_bar_sync(kBarDvFree, 256 + 32);
+                        if (m == 0) {
+                            if (t > 0) dm::named_bar_sync(kBarDvFree, 256 + 32);
                             dm::tc_fence_after();
                             if (dm::elect_one()) {
-                                dm::umma_e4m3_lo_rt(t_dva, pa + 4 * m, dos + 512 * m, idesc_x, (it >> 1) % kWindow != 0 || m > 0);
+                                dm::umma_e4m3_lo_rt(t_dva, pa, dos, idesc_x, (it >> 1) % kWindow != 0);
 #pragma unroll
-                                for (int k = 1; k < (kD == 128 ? 4 : 2); ++k)
-                                    dm::umma_e4m3_lo<true>(t_dva, pa + 4 * m + 2 * k, dos + 512 * m + 256 * k, idesc_x);
-                                if (kD == 256) dm::umma_commit(&s.bar_dv_full);
-                                if (kD == 128 || m == 1) dm::mbar_arrive(&s.bar_rows_free[t % kRows]);
-                                if (kD == 256 && m == 1) dm::umma_commit(&s.bar_dov_free[st]);
+                                for (int k = 1; k < 4; ++k) dm::umma_e4m3_lo<true>(t_dva, pa + 2 * k, dos + 256 * k, idesc_x);
+                                dm::mbar_arrive(&s.bar_rows_free[t % kRows]);
                             }
                             __syncwarp();
                         }
@@ -344,7 +289,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             // ahead as the ring allows
             int t = 0, kvn = 0;
             for (int r = 0;; ++r) {
-                const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item(p, r);
                 if (!w.valid) break;
                 const int n = w.n_it >> 1;
                 const int kv_row0 = w.hc.bhk * p.N + w.J * 128;
@@ -352,49 +297,29 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                 if (n > 0) {
                     if (kvn >= 1) dm::mbar_wait(&s.bar_kv_free, (kvn - 1) & 1, wc);
                     if (dm::elect_one()) {
-                        dm::mbar_expect_tx(&s.bar_kv, 2 * kDH * kTile);
-#pragma unroll
-                        for (int hh = 0; hh < kDH; ++hh) {
-                            dm::tma_load_2d(s.k[hh], &tm_k, 128 * hh, kv_row0, &s.bar_kv);
-                            dm::tma_load_2d(s.v[hh], &tm_v, 128 * hh, kv_row0, &s.bar_kv);
-                        }
+                        dm::mbar_expect_tx(&s.bar_kv, 2 * kTile);
+                        dm::tma_load_2d(s.k, &tm_k, 0, kv_row0, &s.bar_kv);
+                        dm::tma_load_2d(s.v, &tm_v, 0, kv_row0, &s.bar_kv);
                     }
                     __syncwarp();
                     ++kvn;
                 }
                 for (int it = 0; it < n; ++it, ++t) {
-                    const int st = t % kOwn;
-                    if (kD == 256) {
-                        if (t >= 1) dm::mbar_wait(&s.bar_oth_free, (t - 1) & 1, wc);
-                        if (dm::elect_one()) {
-                            dm::mbar_expect_tx(&s.bar_oth, 2 * kTile);
-                            dm::tma_load_2d(s.q[kOwn], &tm_q, 128 * (w.zh ^ 1), q_row0 + it * 128, &s.bar_oth);
-                            dm::tma_load_2d(s.dO[kOwn], &tm_do, 128 * (w.zh ^ 1), q_row0 + it * 128, &s.bar_oth);
-                        }
-                        __syncwarp();
-                    }
-                    if (t >= kOwn) dm::mbar_wait(&s.bar_own_free[st], (t / kOwn - 1) & 1, wc);
+                    const int st = t % kStages;
+                    if (t >= kStages) dm::mbar_wait(&s.bar_qdo_free[st], (t / kStages - 1) & 1, wc);
                     if (dm::elect_one()) {
-                        dm::mbar_expect_tx(&s.bar_own[st], kD == 128 ? 2 * kTile : kTile);
-                        dm::tma_load_2d(s.q[st], &tm_q, 128 * w.zh, q_row0 + it * 128, &s.bar_own[st]);
-                        if (kD == 128) dm::tma_load_2d(s.dO[st], &tm_do, 128 * w.zh, q_row0 + it * 128, &s.bar_own[st]);
+                        dm::mbar_expect_tx(&s.bar_qdo[st], 2 * kTile);
+                        dm::tma_load_2d(s.q[st], &tm_q, 0, q_row0 + it * 128, &s.bar_qdo[st]);
+                        dm::tma_load_2d(s.dO[st], &tm_do, 0, q_row0 + it * 128, &s.bar_qdo[st]);
                     }
                     __syncwarp();
-                    if (kD == 256) {
-                        if (t >= kOwn) dm::mbar_wait(&s.bar_dov_free[st], (t / kOwn - 1) & 1, wc);
-                        if (dm::elect_one()) {
-                            dm::mbar_expect_tx(&s.bar_dov[st], kTile);
-                            dm::tma_load_2d(s.dO[st], &tm_do, 128 * w.zh, q_row0 + it * 128, &s.bar_dov[st]);
-                        }
-                        __syncwarp();
-                    }
                 }
             }
         } else {
             // ---- the rows' constants (four per lane) and the Q / dO scales of the tile, kRows ahead
             int t = 0;
             for (int r = 0;; ++r) {
-                const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item(p, r);
                 if (!w.valid) break;
                 float unit = 0.f, top = 0.f;
                 for (int it = 0; it < w.n_it; it += 2, ++t) {
@@ -406,31 +331,21 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                         l4[i] = p.lse[gi + i];
                         d4[i] = p.delta[gi + i];
                     }
-                    // Q / dO scales: of the tile's 128-row block, or of its two m-blocks
-                    const int64_t sq = kD == 128 ? (int64_t)w.hc.bh * nq_blk + li : ((int64_t)w.hc.bh * nq_blk + li) * 2;
-                    float q8sc[2], do8sc[2], mult[2], un[2];
-#pragma unroll
-                    for (int m = 0; m < 2; ++m) {
-                        q8sc[m] = kD == 256 || m == 0 ? p.q8s[sq + m] : q8sc[0];
-                        do8sc[m] = kD == 256 || m == 0 ? p.do8s[sq + m] : do8sc[0];
-                        // dV's accumulator is kept in units of the current dO scale block's scale, so that the MMAs add to it directly.
-                        // A block more than 2^-80 below the item's largest so far (an all-zero one) takes the unit at that bound: the
-                        // accumulator stays finite, and zero codes add nothing whatever the unit is.
-                        top = fmaxf(top, do8sc[m]);
-                        const float unit_new = kD == 256 || m == 0 ? fmaxf(do8sc[m], top * 0x1p-80f) : unit;
-                        mult[m] = unit / unit_new;
-                        unit = unit_new;
-                        un[m] = dm::kMoInv * unit;
-                    }
+                    const int64_t sq = (int64_t)w.hc.bh * nq_blk + li;
+                    const float q8sc = p.q8s[sq], do8sc = p.do8s[sq];
+                    // dV's accumulator is kept in units of the current dO scale block's scale, so that the MMAs add to it directly.
+                    // A block more than 2^-80 below the item's largest so far (an all-zero one) takes the unit at that bound: the
+                    // accumulator stays finite, and zero codes add nothing whatever the unit is.
+                    top = fmaxf(top, do8sc);
+                    const float unit_new = fmaxf(do8sc, top * 0x1p-80f);
+                    const float mult = unit / unit_new;
+                    unit = unit_new;
                     if (t >= kRows) dm::mbar_wait(&s.bar_rows_free[slot], (t / kRows - 1) & 1, wc);
 #pragma unroll
                     for (int i = 0; i < 4; i += 2)
                         *reinterpret_cast<float4*>(&s.rd[slot][4 * lane + i]) =
                             make_float4(dm::phat_row_const(l4[i]), -d4[i], dm::phat_row_const(l4[i + 1]), -d4[i + 1]);
-                    if (lane == 0) {
-                        *reinterpret_cast<float4*>(s.sc[slot]) = make_float4(q8sc[0], q8sc[1], do8sc[0], do8sc[1]);
-                        *reinterpret_cast<float4*>(s.sc[slot] + 4) = make_float4(mult[0], mult[1], un[0], un[1]);
-                    }
+                    if (lane == 0) *reinterpret_cast<float4*>(s.sc[slot]) = make_float4(q8sc, do8sc, mult, dm::kMoInv * unit);
                     __syncwarp();
                     if (dm::elect_one()) dm::mbar_arrive(&s.bar_rows_full[slot]);
                 }
@@ -446,10 +361,10 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             int n_it;                                  // all that the tile loop keeps of the item: it has no registers to spare
             float ik;                                  // for the epilogue; read early
             {
-                const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item(p, r);
                 if (!w.valid) break;
                 n_it = w.n_it;
-                ik = 1.0f / p.k8s[(int64_t)w.hc.bhk * (p.N / G::kKeysPerScale) + G::kGrp * w.J + key / G::kKeysPerScale];
+                ik = 1.0f / p.k8s[(int64_t)w.hc.bhk * (p.N / 64) + 2 * w.J + key / 64];
             }
             float dk_acc[64];
 #pragma unroll
@@ -461,7 +376,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                 uint32_t sa[16], sb[16];
                 dm::tmem_ld16(x_src, sa);
                 dm::tmem_ld16(x_src + 16, sb);
-                const float gk = g[2 * m];
+                const float gk = g[m];
                 auto add16 = [&](int pc, const uint32_t* x) {
 #pragma unroll
                     for (int i = 0; i < 16; i += 2)
@@ -510,11 +425,11 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             auto dv_sum = [&]() {
                 int r_again = r;                       // (looked up again: the tile loop has no registers for it)
                 asm volatile("" : "+r"(r_again));
-                const dm::Bwd1Item v = dm::bwd1_item<kD>(p, r_again);
-                const int64_t at = (((int64_t)v.hc.b * p.N + v.J * 128 + lane_base + (lane >> 2)) * p.H + v.hc.h) * kD + 128 * v.zh + 64 * half;
-                const int64_t keys8 = (int64_t)p.H * (8 * kD);
+                const dm::Bwd1Item v = dm::bwd1_item(p, r_again);
+                const int64_t at = (((int64_t)v.hc.b * p.N + v.J * 128 + lane_base + (lane >> 2)) * p.H + v.hc.h) * 128 + 64 * half;
+                const int64_t keys8 = (int64_t)p.H * (8 * 128);
                 uint8_t* dv = reinterpret_cast<uint8_t*>(p.dv) + 16 * (lane & 3);
-                if (kD == 128 && p.out_fp32) return DvSum{dv + 4 * at, 64, 128, 4 * keys8};
+                if (p.out_fp32) return DvSum{dv + 4 * at, 64, 128, 4 * keys8};
                 return DvSum{dv + 2 * at, reinterpret_cast<uint8_t*>(p.dk) - reinterpret_cast<uint8_t*>(p.dv), 64, 2 * keys8};
             };
             auto flush_dv = [&](float unit, bool first) {
@@ -542,22 +457,13 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             for (int it = 0; it < n_it;) {
                 const int end = min(n_it, it + 2 * kWindow);
                 for (; it < end; it += 2, ++t) {
-                    const float* g = s.gf[t % kGf] + (kD == 128 ? 0 : key >> 6);
+                    const float* g = s.gf[t % kGf];
                     fold_dk(g, 0);
-                    if (kD == 256) {
-                        dm::mbar_wait(&s.bar_dv_full, 0, wc);            // two commits a tile, as for X
-                        dm::tc_fence_after();
-                        rescale_dv(s.sc[t % kRows][5]);
-                    }
-                    fold_dk(g, 1);                                       // (head_dim 128: its product was committed behind the tile's dV)
-                    if (kD == 256) {
-                        dm::mbar_wait(&s.bar_dv_full, 1, wc);
-                        dm::tc_fence_after();
-                    }
+                    fold_dk(g, 1);                                       // (its product was committed behind the tile's dV)
                     if (it + 2 < end) {
                         const int slot = (t + 1) % kRows;
                         dm::mbar_wait(&s.bar_rows_full[slot], ((t + 1) / kRows) & 1, wc);
-                        rescale_dv(s.sc[slot][4]);
+                        rescale_dv(s.sc[slot][2]);
                     }
                 }
                 if (n_it > 2 * kWindow) flush_dv(s.fv[(t + kGf - 1) % kGf], it == 2 * kWindow);
@@ -568,10 +474,10 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             const bool have_dv = n_it > 0, have_sum = (n_it >> 1) > kWindow;
             int r_again = r;
             asm volatile("" : "+r"(r_again));
-            const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r_again);
+            const dm::Bwd1Item w = dm::bwd1_item(p, r_again);
             const float fv = have_dv ? s.fv[(t + kGf - 1) % kGf] : 0.f;      // dV's last unit
-            const int64_t row_stride = (int64_t)p.H * kD;            // elements between consecutive keys
-            const int64_t off = (((int64_t)w.hc.b * p.N + w.J * 128) * p.H + w.hc.h) * kD + 128 * w.zh + 64 * half;   // key 0 of the block
+            const int64_t row_stride = (int64_t)p.H * 128;           // elements between consecutive keys
+            const int64_t off = (((int64_t)w.hc.b * p.N + w.J * 128) * p.H + w.hc.h) * 128 + 64 * half;   // key 0 of the block
             auto dv16 = [&](int pc, float* y) {
                 if (have_dv) {
                     dm::tmem_ld16(dva + 16 * pc, reinterpret_cast<uint32_t*>(y));
@@ -587,7 +493,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                 for (int j = 0; j < 4; ++j, from += m.step) *reinterpret_cast<float4*>(y + 4 * j) = __ldcg(reinterpret_cast<const float4*>(from));
                 __syncwarp();                                        // the warp has read the unit: its place may be written
             };
-            if (kD == 128 && p.out_fp32) {                         // (refused at head_dim 256)
+            if (p.out_fp32) {
                 float4* ok = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dk) + off + key * row_stride);
                 float4* ov = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.dv) + off + key * row_stride);
 #pragma unroll
@@ -606,11 +512,10 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                 }
             } else {
                 // The bf16 rows leave through the warp's own staging slice, kStgCols columns at a time: a thread holds one key, so
-                // stored directly every 16-byte store instruction would touch 32 rows; from the slice it writes 8 pieces of 64 bytes
-                // (head_dim 256: 16 of 32, whole sectors).
-                constexpr int kCh = G::kStgCols / 8;                   // 16-byte chunks per key
+                // stored directly every 16-byte store instruction would touch 32 rows; from the slice it writes 8 pieces of 64 bytes.
+                constexpr int kCh = kStgCols / 8;                   // 16-byte chunks per key
                 uint8_t* stg = s.stg[warp & 7];
-                auto chunk = [&](int row, int c) { return stg + row * (16 * kCh) + ((c ^ ((kCh == 4 ? row >> 1 : row >> 2) & (kCh - 1))) << 4); };
+                auto chunk = [&](int row, int c) { return stg + row * (16 * kCh) + ((c ^ ((row >> 1) & (kCh - 1))) << 4); };
                 auto put8 = [&](int c, const float* y, float f) {      // 8 columns = one 16-byte chunk
                     uint32_t w4[4];
 #pragma unroll
@@ -627,14 +532,14 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                     for (int i = 0; i < kCh; ++i) {
                         const int row = (32 / kCh) * i + lane / kCh;
                         const uint4 val = *reinterpret_cast<const uint4*>(chunk(row, c));
-                        *reinterpret_cast<uint4*>(dst + off + (lane_base + row) * row_stride + G::kStgCols * h + 8 * c) = val;
+                        *reinterpret_cast<uint4*>(dst + off + (lane_base + row) * row_stride + kStgCols * h + 8 * c) = val;
                     }
                     __syncwarp();
                 };
                 if (have_sum) {
                     const DvSum m = dv_sum();
 #pragma unroll 1
-                    for (int h = 0; h < 64 / G::kStgCols; ++h) {
+                    for (int h = 0; h < 64 / kStgCols; ++h) {
 #pragma unroll
                         for (int pc = 0; pc < kCh / 2; ++pc) {
                             float y[16];
@@ -646,14 +551,14 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                     }
                 }
 #pragma unroll
-                for (int h = 0; h < 64 / G::kStgCols; ++h) {
+                for (int h = 0; h < 64 / kStgCols; ++h) {
 #pragma unroll
-                    for (int c = 0; c < kCh; ++c) put8(c, dk_acc + G::kStgCols * h + 8 * c, ik);
+                    for (int c = 0; c < kCh; ++c) put8(c, dk_acc + kStgCols * h + 8 * c, ik);
                     out(p.dk, h);
                 }
                 if (!have_sum) {
 #pragma unroll
-                    for (int h = 0; h < 64 / G::kStgCols; ++h) {
+                    for (int h = 0; h < 64 / kStgCols; ++h) {
 #pragma unroll
                         for (int pc = 0; pc < kCh / 2; ++pc) {
                             float y[16];
@@ -675,8 +580,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         dm::reg_dec<kRegSoftmax>();
         const int rq = warp & 3, kq = warp >> 2;      // rows [32 rq, +32) and keys [32 kq, +32) of the tile
         const int rhalf = rq >> 1;                    // the 64-row m-block
-        const int psi_tile = kD == 128 ? rhalf : 2 * rhalf + (kq >> 1);
-        const bool leader = (warp & (kD == 128 ? 13 : 5)) == 0;      // one warp of each psi tile
+        const bool leader = (warp & 13) == 0;         // one warp of each m-block
         const int row_t = 32 * rq + (lane >> 2);      // the thread's rows: row_t + {0, 8, 16, 24}
         const int key_t = 32 * kq + 2 * (lane & 3);   // its keys: key_t + 8 j + {0, 1}
         const uint32_t t_s = dm::tmem_addr(tmem, lane_base, 32 * kq);
@@ -685,22 +589,22 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         const uint32_t ds_off = dm::smem_u32(s.ds[0]) - dm::smem_u32(s.pt[0]);
         int t = 0, rb = 0;                            // tiles so far; ring slot of the row constants
         for (int r = 0;; ++r) {
-            const dm::Bwd1Item w = dm::bwd1_item<kD>(p, r);
+            const dm::Bwd1Item w = dm::bwd1_item(p, r);
             if (!w.valid) break;
             const int n_it = w.n_it >> 1;
-            const float k8s_t = p.k8s[(int64_t)w.hc.bhk * (p.N / G::kKeysPerScale) + G::kGrp * w.J + 32 * kq / G::kKeysPerScale];
-            const float v8s_t = p.v8s[(int64_t)w.hc.bhk * (p.N / G::kKeysPerScale) + G::kGrp * w.J + 32 * kq / G::kKeysPerScale];
+            const float k8s_t = p.k8s[(int64_t)w.hc.bhk * (p.N / 64) + 2 * w.J + (kq >> 1)];
+            const float v8s_t = p.v8s[(int64_t)w.hc.bhk * (p.N / 64) + 2 * w.J + (kq >> 1)];
             const bool diag_item = p.causal && n_it > 0 && dm::global_block(p.rm, w.m_lo >> 1) == w.J;
             float g_max = 0.f;
 
             for (int it = 0; it < n_it; ++it, ++t, rb = rb == kRows - 1 ? 0 : rb + 1) {
                 const int par = t & 1;
                 dm::mbar_wait(&s.bar_sp_full, par, wc);
-                const float q8sc = s.sc[rb][rhalf], do8sc = s.sc[rb][2 + rhalf];
+                const float q8sc = s.sc[rb][0], do8sc = s.sc[rb][1];
                 const float dsc = dm::descale_log2(q8sc, k8s_t);
                 const float dpk = do8sc * v8s_t * k8s_t;
                 const float2* rd = &s.rd[rb][row_t];
-                const uint32_t addr = st_addr + par * kTile, ds_addr = st_addr + ds_off + (kD == 128 ? par * kTile : 0);
+                const uint32_t addr = st_addr + par * kTile, ds_addr = st_addr + ds_off + par * kTile;
                 dm::tc_fence_after();
 
                 // ---- phase 1: P-hat, dS', tile amax; P-hat codes to shared memory.  Two halves of 16 rows; S first: the
@@ -748,15 +652,14 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                 // the warp's maximum in one instruction: non-negative floats order like their bit patterns
                 const float am = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(am0, am1))));
                 if (lane == 0) s.amax[par][8 * rhalf + 2 * kq + (rq & 1)] = am;
-                if (kD == 256 && leader && t >= 1) dm::mbar_wait(&s.bar_ds_free[0], (t - 1) & 1, wc);   // one dS' tile: it is free
-                dm::named_bar_sync(kBarAmax + psi_tile, 32 * G::kPsiWarps);
+                dm::named_bar_sync(kBarAmax + rhalf, 256);
                 // psi of the tile: psi = max(psi_raw, g_max * 256e-8 / q8sc); the quotient can only win when its numerator
                 // exceeds psi_raw * q8sc, so the division is formed only then (the 1 % margin covers the rounding of both sides).
                 // g_max runs over the psi tiles of this row half: the floor acts only on a tile whose maximum lies eight decades
                 // below an earlier one's, and one barrier for both halves and both psi in every thread cost 3 %.
                 float psi_my;
                 {
-                    const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(s.amax[par][psi_tile * G::kPsiWarps + (lane & (G::kPsiWarps - 1))])));
+                    const float mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(s.amax[par][8 * rhalf + (lane & 7)])));
                     const float amx = mx * (1.0f / 448.0f);
                     psi_my = fmaxf(amx, 1e-30f);
                     const float fl_num = g_max * (256.0f * 1e-8f);
@@ -783,10 +686,9 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
                 // the scales of this tile's products for the fold warps (the ring slot was last read four tiles ago; S of this tile
                 // waited for the products of two tiles ago) and psi, which the product warp takes to global memory
                 if (leader && lane == 0) {
-                    const int i = kD == 128 ? 2 * rhalf : psi_tile;
-                    s.gf[t % kGf][i] = g_my;
-                    s.psi[t % kGf][i] = psi_my;
-                    if (warp == 0) s.fv[t % kGf] = s.sc[rb][7];
+                    s.gf[t % kGf][rhalf] = g_my;
+                    s.psi[t % kGf][rhalf] = psi_my;
+                    if (warp == 0) s.fv[t % kGf] = s.sc[rb][3];
                 }
                 dm::fence_proxy_async_smem();
                 dm::named_bar_arrive(kBarCodes + par, kSoftmaxThreads + 32);
@@ -809,15 +711,19 @@ namespace dmh {
 int prepare_bwd1(char* err, size_t errlen) {
     static DeviceOnce once;
     return device_once(once, err, errlen, [&]() -> int {
-        DM_CUDA(cudaFuncSetAttribute(bwd1_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<128>) + 1024));
-        DM_CUDA(cudaFuncSetAttribute(bwd1_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem<256>) + 1024));
+        DM_CUDA(cudaFuncSetAttribute(bwd1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem) + 1024));
         constexpr int kPool = kSoftmaxThreads * kRegSoftmax + 256 * kRegFold + 128 * kRegService;
         static_assert(kPool == kThreads * 72, "the roles' register requests must add up to the launch pool");
-        if (int rc = check_register_pool((const void*)bwd1_kernel<128>, kThreads, kPool, err, errlen)) return rc;
-        return check_register_pool((const void*)bwd1_kernel<256>, kThreads, kPool, err, errlen);
+        return check_register_pool((const void*)bwd1_kernel, kThreads, kPool, err, errlen);
     });
 }
 }  // namespace dmh
+
+namespace dmh {
+int launch_bwd1_d256(const void* q8, const void* k8, const void* v8, const void* do8, const float* q8s, const float* k8s, const float* v8s,
+                     const float* do8s, const float* lse, const float* delta, DmShape sh, int h0, int hcount, void* dk, void* dv, void* ds8_ws,
+                     float* psi_ws, void* stream, char* err, size_t errlen);
+}
 
 extern "C" int dm_bwd_workspace_bytes(DmShape sh, int32_t hcount, size_t* ds8_bytes, size_t* psi_bytes) {
     if (!ds8_bytes || !psi_bytes || sh.N <= 0 || sh.N % 128 || sh.B <= 0 || hcount <= 0) return DM_ERR_ARG;
@@ -860,6 +766,8 @@ extern "C" int dm_bwd_fp8_pass1_cp(const void* q8, const void* k8, const void* v
     const uint64_t ntiles = (uint64_t)sh.B * hcount * (cp.nq / 128) * (sh.N / 128);
     DM_REQUIRE(ntiles * 128 < ((uint64_t)1 << 31), DM_ERR_ARG, "dS' workspace too large for one call: split the heads (got %llu tiles)",
                (unsigned long long)ntiles);
+    if (sh.D == 256)
+        return dmh::launch_bwd1_d256(q8, k8, v8, do8, q8s, k8s, v8s, do8s, lse, delta, sh, h0, hcount, dk, dv, ds8_ws, psi_ws, stream, err, errlen);
     CUtensorMap tq, td, tk, tv, ts;
     if ((rc = dmh::make_tmap_u8(&tq, q8, sh.D, (uint64_t)sh.B * sh.H * cp.nq, 128, err, errlen))) return rc;
     if ((rc = dmh::make_tmap_u8(&td, do8, sh.D, (uint64_t)sh.B * sh.H * cp.nq, 128, err, errlen))) return rc;
@@ -870,15 +778,13 @@ extern "C" int dm_bwd_fp8_pass1_cp(const void* q8, const void* k8, const void* v
     if (!status) return DM_ERR_CUDA;
     dm::Bwd1Params p{q8s, k8s, v8s, do8s, lse, delta, static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), static_cast<uint8_t*>(ds8_ws), psi_ws,
                  sh.H, sh.Hk, sh.N, h0, hcount, sh.causal, status, dm::RowMap{cp.nq, cp.half_blocks, cp.off0, cp.off1}, out_fp32,
-                 sh.B * hcount, dm::make_fastdiv(sh.B * hcount), dm::make_fastdiv(hcount), dm::make_fastdiv(sh.H / sh.Hk),
-                 dm::make_fastdiv(sh.N / 128)};
-    // persistent: one CTA per SM walks the (key block, head[, d half]) items, heaviest first
+                 sh.B * hcount, dm::make_fastdiv(sh.B * hcount), dm::make_fastdiv(hcount), dm::make_fastdiv(sh.H / sh.Hk)};
+    // persistent: one CTA per SM walks the (key block, head) items, heaviest first
     if ((rc = dmh::prepare_bwd1(err, errlen))) return rc;
     int sms = 0;
     if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
-    const int64_t items = (int64_t)sh.B * hcount * (sh.N / 128) * (sh.D / 128);
+    const int64_t items = (int64_t)sh.B * hcount * (sh.N / 128);
     const int grid = (int)(items < sms ? items : sms);
-    if (sh.D == 128) DM_CUDA(dmh::launch_pdl(bwd1_kernel<128>, grid, kThreads, sizeof(Smem<128>) + 1024, stream, tq, td, tk, tv, ts, p));
-    else DM_CUDA(dmh::launch_pdl(bwd1_kernel<256>, grid, kThreads, sizeof(Smem<256>) + 1024, stream, tq, td, tk, tv, ts, p));
+    DM_CUDA(dmh::launch_pdl(bwd1_kernel, grid, kThreads, sizeof(Smem) + 1024, stream, tq, td, tk, tv, ts, p));
     return DM_OK;
 }

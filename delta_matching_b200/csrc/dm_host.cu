@@ -179,6 +179,7 @@ extern "C" int dm_init(char* err, size_t errlen) {
     if ((rc = dmh::prepare_fwd256(err, errlen))) return rc;
     if ((rc = dmh::prepare_delta(err, errlen))) return rc;
     if ((rc = dmh::prepare_bwd1(err, errlen))) return rc;
+    if ((rc = dmh::prepare_bwd1_d256(err, errlen))) return rc;
     return dmh::prepare_bwd2(err, errlen);
 }
 

@@ -96,6 +96,7 @@ int launch_gqa_fold(const void* x0, void* out0, const void* x1, void* out1, int 
                     size_t errlen);
 int prepare_delta(char* err, size_t errlen);
 int prepare_bwd1(char* err, size_t errlen);
+int prepare_bwd1_d256(char* err, size_t errlen);
 int prepare_bwd2(char* err, size_t errlen);
 
 // One int per device, zero-initialised: kernels write a non-zero value when a bounded wait gives up.

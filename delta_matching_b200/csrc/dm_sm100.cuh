@@ -203,6 +203,13 @@ __device__ __forceinline__ void tmem_ld16x256_x4(uint32_t taddr, uint32_t* r) {
         : "r"(taddr)
         : "memory");
 }
+// The same x 2 (16 columns): register 4 j + 2 a + e, j = 0, 1.
+__device__ __forceinline__ void tmem_ld16x256_x2(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
 // Four 16 x 8 byte matrices from that layout (register j = the four bytes of fragment j, in register order), stored transposed:
 // column i of matrix j becomes 16 consecutive bytes at the address that lane 8 j + i gives.
 __device__ __forceinline__ void stmatrix_t_b8_x4(uint32_t saddr, const uint32_t* r) {
