@@ -57,6 +57,7 @@ _SIGNATURES = {
     "dm_selftest_wait_timeout": (C.c_int, [_P, _P, *_ERR]),
     "dm_init": (C.c_int, [*_ERR]),
     "dm_register_pool_ok": (C.c_int, [C.c_int32] * 3),
+    "dm_walk_plan": (C.c_int, [C.c_int32] * 3 + [C.POINTER(C.c_int32)] * 2),
     "dm_quant_qv_kpartials": (C.c_int, [_P, DmStrides, _P, DmStrides, _P, DmStrides, DmShape] + [_P] * 5 + [_P, *_ERR]),
     "dm_kmean_partials": (C.c_int, [_P, DmStrides, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P, _P, *_ERR]),
     "dm_kmean_fold": (C.c_int, [_P, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P, _P, *_ERR]),

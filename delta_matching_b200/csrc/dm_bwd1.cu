@@ -55,18 +55,17 @@ struct Bwd1Params {
 };
 
 // The work list: one item = one 128-key block J of one (batch, query head), ordered by
-// key block, i.e. heaviest first when causal.  CTA c takes position c of the even rounds and G - 1 - c of the odd ones
-// (a snake), so the long and the short items of a round pair up.
+// key block, i.e. heaviest first when causal, and walked as walk_index says.
 struct Bwd1Item {
     HeadCoord hc;
     int J, m_lo, n_it, bhl;                   // m_lo, n_it: first 64-row m-block and their count, both even
     bool valid;
 };
-__device__ __forceinline__ Bwd1Item bwd1_item(const Bwd1Params& p, int round) {
+template <class Walk>
+__device__ __forceinline__ Bwd1Item bwd1_item(const Bwd1Params& p, const Walk& walk, int round) {
     Bwd1Item w;
-    const int G = gridDim.x, c = blockIdx.x;
     const int nbn = p.N / 128;
-    const int idx = round * G + ((round & 1) ? G - 1 - c : c);
+    const int idx = walk_index(walk, round);
     w.valid = idx < p.n_heads * nbn;
     w.J = (int)fdiv((uint32_t)idx, p.fd_heads);
     w.hc = head_coord(idx - w.J * p.n_heads, p.h0, p.fd_hcount, p.H, p.Hk, p.fd_rep);
@@ -135,10 +134,11 @@ struct Smem {
     int abort_flag;
 };
 
+template <class Walk>
 __global__ void __launch_bounds__(kThreads, 1)
 bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
             const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-            const __grid_constant__ CUtensorMap tm_ds, const dm::Bwd1Params p) {
+            const __grid_constant__ CUtensorMap tm_ds, const dm::Bwd1Params p, const __grid_constant__ Walk walk) {
     extern __shared__ uint8_t smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     // The hardware warps are taken in the order service, fold, softmax (the role numbers below keep their tensor-memory quarter,
@@ -191,7 +191,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             const uint32_t q_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[0])), do_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.dO[0]));
             int t = 0, kvn = 0;
             for (int r = 0;; ++r) {
-                const dm::Bwd1Item w = dm::bwd1_item(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item(p, walk, r);
                 if (!w.valid) break;
                 const int n = w.n_it >> 1;
                 if (n > 0) dm::mbar_wait(&s.bar_kv, kvn++ & 1, wc);
@@ -231,7 +231,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             const uint32_t pt_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.pt[0])), ds_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.ds[0]));
             int t = 0;
             for (int r = 0;; ++r) {
-                const dm::Bwd1Item w = dm::bwd1_item(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item(p, walk, r);
                 if (!w.valid) break;
                 int ds_row = (int)((((int64_t)w.bhl * nq_blk + (w.m_lo >> 1)) * nbn + w.J) * 128);   // dS' tile of the first row block
                 float* psi_out = p.psi + ((int64_t)w.bhl * (2 * nq_blk) + w.m_lo + lane) * nbn + w.J;
@@ -289,7 +289,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             // ahead as the ring allows
             int t = 0, kvn = 0;
             for (int r = 0;; ++r) {
-                const dm::Bwd1Item w = dm::bwd1_item(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item(p, walk, r);
                 if (!w.valid) break;
                 const int n = w.n_it >> 1;
                 const int kv_row0 = w.hc.bhk * p.N + w.J * 128;
@@ -319,7 +319,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             // ---- the rows' constants (four per lane) and the Q / dO scales of the tile, kRows ahead
             int t = 0;
             for (int r = 0;; ++r) {
-                const dm::Bwd1Item w = dm::bwd1_item(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item(p, walk, r);
                 if (!w.valid) break;
                 float unit = 0.f, top = 0.f;
                 for (int it = 0; it < w.n_it; it += 2, ++t) {
@@ -361,7 +361,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             int n_it;                                  // all that the tile loop keeps of the item: it has no registers to spare
             float ik;                                  // for the epilogue; read early
             {
-                const dm::Bwd1Item w = dm::bwd1_item(p, r);
+                const dm::Bwd1Item w = dm::bwd1_item(p, walk, r);
                 if (!w.valid) break;
                 n_it = w.n_it;
                 ik = 1.0f / p.k8s[(int64_t)w.hc.bhk * (p.N / 64) + 2 * w.J + key / 64];
@@ -425,7 +425,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             auto dv_sum = [&]() {
                 int r_again = r;                       // (looked up again: the tile loop has no registers for it)
                 asm volatile("" : "+r"(r_again));
-                const dm::Bwd1Item v = dm::bwd1_item(p, r_again);
+                const dm::Bwd1Item v = dm::bwd1_item(p, walk, r_again);
                 const int64_t at = (((int64_t)v.hc.b * p.N + v.J * 128 + lane_base + (lane >> 2)) * p.H + v.hc.h) * 128 + 64 * half;
                 const int64_t keys8 = (int64_t)p.H * (8 * 128);
                 uint8_t* dv = reinterpret_cast<uint8_t*>(p.dv) + 16 * (lane & 3);
@@ -474,7 +474,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
             const bool have_dv = n_it > 0, have_sum = (n_it >> 1) > kWindow;
             int r_again = r;
             asm volatile("" : "+r"(r_again));
-            const dm::Bwd1Item w = dm::bwd1_item(p, r_again);
+            const dm::Bwd1Item w = dm::bwd1_item(p, walk, r_again);
             const float fv = have_dv ? s.fv[(t + kGf - 1) % kGf] : 0.f;      // dV's last unit
             const int64_t row_stride = (int64_t)p.H * 128;           // elements between consecutive keys
             const int64_t off = (((int64_t)w.hc.b * p.N + w.J * 128) * p.H + w.hc.h) * 128 + 64 * half;   // key 0 of the block
@@ -589,7 +589,7 @@ bwd1_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CU
         const uint32_t ds_off = dm::smem_u32(s.ds[0]) - dm::smem_u32(s.pt[0]);
         int t = 0, rb = 0;                            // tiles so far; ring slot of the row constants
         for (int r = 0;; ++r) {
-            const dm::Bwd1Item w = dm::bwd1_item(p, r);
+            const dm::Bwd1Item w = dm::bwd1_item(p, walk, r);
             if (!w.valid) break;
             const int n_it = w.n_it >> 1;
             const float k8s_t = p.k8s[(int64_t)w.hc.bhk * (p.N / 64) + 2 * w.J + (kq >> 1)];
@@ -711,10 +711,13 @@ namespace dmh {
 int prepare_bwd1(char* err, size_t errlen) {
     static DeviceOnce once;
     return device_once(once, err, errlen, [&]() -> int {
-        DM_CUDA(cudaFuncSetAttribute(bwd1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem) + 1024));
         constexpr int kPool = kSoftmaxThreads * kRegSoftmax + 256 * kRegFold + 128 * kRegService;
         static_assert(kPool == kThreads * 72, "the roles' register requests must add up to the launch pool");
-        return check_register_pool((const void*)bwd1_kernel, kThreads, kPool, err, errlen);
+        for (auto kernel : {(const void*)bwd1_kernel<dm::SnakeWalk>, (const void*)bwd1_kernel<dm::PackedWalk>}) {
+            DM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem) + 1024));
+            if (int rc = check_register_pool(kernel, kThreads, kPool, err, errlen)) return rc;
+        }
+        return DM_OK;
     });
 }
 }  // namespace dmh
@@ -785,6 +788,10 @@ extern "C" int dm_bwd_fp8_pass1_cp(const void* q8, const void* k8, const void* v
     if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
     const int64_t items = (int64_t)sh.B * hcount * (sh.N / 128);
     const int grid = (int)(items < sms ? items : sms);
-    DM_CUDA(dmh::launch_pdl(bwd1_kernel, grid, kThreads, sizeof(Smem) + 1024, stream, tq, td, tk, tv, ts, p));
+    if (const dm::PackedWalk* walk = sh.causal && plain ? dmh::plan_walk(sh.B * hcount, sh.N / 128, grid) : nullptr) {
+        DM_CUDA(dmh::launch_pdl(bwd1_kernel<dm::PackedWalk>, grid, kThreads, sizeof(Smem) + 1024, stream, tq, td, tk, tv, ts, p, *walk));
+    } else {
+        DM_CUDA(dmh::launch_pdl(bwd1_kernel<dm::SnakeWalk>, grid, kThreads, sizeof(Smem) + 1024, stream, tq, td, tk, tv, ts, p, dm::SnakeWalk{}));
+    }
     return DM_OK;
 }

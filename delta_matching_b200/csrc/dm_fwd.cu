@@ -78,18 +78,17 @@ struct FwdParams {
 };
 
 // One work item of a persistent CTA.  Items are numbered rank-major (rank 0 = the row blocks with the most key tiles, all
-// heads, then rank 1, ...); CTA c of G takes item r G + c in even rounds r and r G + (G - 1 - c) in odd rounds, so a CTA that
-// got a long item in one round gets a short one in the next.
+// heads, then rank 1, ...) and walked as dm::walk_index says.
 struct FwdItem {
     dm::HeadCoord hc;
     int li, I, n_tiles;
     bool valid;
 };
-__device__ __forceinline__ FwdItem fwd_item(const FwdParams& p, int round) {
+template <class Walk>
+__device__ __forceinline__ FwdItem fwd_item(const FwdParams& p, const Walk& walk, int round) {
     FwdItem w;
-    const int G = gridDim.x, c = blockIdx.x;
     const int nq_blk = p.rm.nq / 128;
-    const int idx = round * G + ((round & 1) ? G - 1 - c : c);
+    const int idx = dm::walk_index(walk, round);
     w.valid = idx < p.n_heads * nq_blk;
     const int rank = (int)dm::fdiv((uint32_t)idx, p.fd_heads);
     w.hc = dm::head_coord(idx - rank * p.n_heads, p.h0, p.fd_hcount, p.H, p.Hk, p.fd_rep);
@@ -99,9 +98,10 @@ __device__ __forceinline__ FwdItem fwd_item(const FwdParams& p, int round) {
     return w;
 }
 
+template <class Walk>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
+                const __grid_constant__ CUtensorMap tm_v, const FwdParams p, const __grid_constant__ Walk walk) {
     extern __shared__ uint8_t smem_raw[];
     FwdSmem& s = *reinterpret_cast<FwdSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -148,7 +148,7 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             const uint32_t q_lo0 = dm::smem_desc_lo_sw128(dm::smem_u32(s.q[0])), k_lo = dm::smem_desc_lo_sw128(dm::smem_u32(s.k[0]));
             int gt = 0;
             for (int r = 0;; ++r) {
-                const FwdItem w = fwd_item(p, r);
+                const FwdItem w = fwd_item(p, walk, r);
                 if (!w.valid) break;
                 const int qb = r & 1;
                 const uint32_t q_lo = q_lo0 + qb * kSub;
@@ -182,7 +182,7 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             const uint32_t t_d = g ? t_d1 : t_d0;
             int t = 0, st = 0;
             for (int r = 0;; ++r) {
-                const FwdItem w = fwd_item(p, r);
+                const FwdItem w = fwd_item(p, walk, r);
                 if (!w.valid) break;
                 for (int it = 0; it < w.n_tiles; ++it, ++t) {
                     const int b = t & 1;
@@ -205,7 +205,7 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             // ---- TMA loads: every item's Q, then its K / V tiles, as far ahead as the rings allow (across items too)
             int gt = 0;
             for (int r = 0;; ++r) {
-                const FwdItem w = fwd_item(p, r);
+                const FwdItem w = fwd_item(p, walk, r);
                 if (!w.valid) break;
                 const int qb = r & 1;
                 const int q_row0 = w.hc.bh * p.rm.nq + w.li * 128, kv_row0 = w.hc.bhk * p.N;
@@ -236,7 +236,7 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         for (int r = 0;; ++r) {
             int n_tiles;                               // all that the tile loop keeps of the item: it has no registers to spare
             {
-                const FwdItem w = fwd_item(p, r);
+                const FwdItem w = fwd_item(p, walk, r);
                 if (!w.valid) break;
                 n_tiles = w.n_tiles;
             }
@@ -303,7 +303,7 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             gt += n_tiles;
             int r_again = r;
             asm volatile("" : "+r"(r_again));
-            const FwdItem w = fwd_item(p, r_again);
+            const FwdItem w = fwd_item(p, walk, r_again);
             // ---- the item's epilogue
             const float l = l0 + l1;
             const bool dead = (l == 0.f) || (l != l);
@@ -358,7 +358,7 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 vs_nx = p.v8s[ko];
             }
         };
-        FwdItem w = fwd_item(p, 0);
+        FwdItem w = fwd_item(p, walk, 0);
         first_scales(w, 0);
         for (int r = 0; w.valid; ++r) {
             const int n_tiles = w.n_tiles, I = w.I;
@@ -368,7 +368,7 @@ fwd_d128_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             // The thread's own running maximum (its group, its team's tiles): it only places the floor of the basis, 12 binades below it.
             float m_run = -INFINITY;
             float ks_n = ks_nx, vs_n = vs_nx;
-            w = fwd_item(p, r + 1);
+            w = fwd_item(p, walk, r + 1);
             first_scales(w, gt + n_tiles);
             for (int it = (gt ^ team) & 1; it < n_tiles; it += 2) {
                 const int t = gt + it, j = n_tiles - 1 - it, rg = t % kRing;
@@ -481,8 +481,11 @@ static_assert(kFwdRegPool == kThreads * 72, "the roles' register requests must a
 int prepare_fwd(char* err, size_t errlen) {
     static DeviceOnce once;
     return device_once(once, err, errlen, [&]() -> int {
-        DM_CUDA(cudaFuncSetAttribute(fwd_d128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem) + 1024));
-        return check_register_pool((const void*)fwd_d128_kernel, kThreads, kFwdRegPool, err, errlen);
+        for (auto kernel : {(const void*)fwd_d128_kernel<dm::SnakeWalk>, (const void*)fwd_d128_kernel<dm::PackedWalk>}) {
+            DM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem) + 1024));
+            if (int rc = check_register_pool(kernel, kThreads, kFwdRegPool, err, errlen)) return rc;
+        }
+        return DM_OK;
     });
 }
 
@@ -542,6 +545,10 @@ extern "C" int dm_fwd_fp8_cp(const void* q8, const void* k8, const void* v8, con
     // persistent: one CTA per SM walks the (head, row block) items, heaviest first
     const int64_t items = (int64_t)sh.B * hcount * (cp.nq / 128);
     const int grid = (int)(items < sms ? items : sms);
-    DM_CUDA(dmh::launch_pdl(fwd_d128_kernel, grid, kThreads, smem, stream, tq, tk, tv, p));
+    if (const dm::PackedWalk* walk = sh.causal && cp.nq == sh.N ? dmh::plan_walk(sh.B * hcount, sh.N / 128, grid) : nullptr) {
+        DM_CUDA(dmh::launch_pdl(fwd_d128_kernel<dm::PackedWalk>, grid, kThreads, smem, stream, tq, tk, tv, p, *walk));
+    } else {
+        DM_CUDA(dmh::launch_pdl(fwd_d128_kernel<dm::SnakeWalk>, grid, kThreads, smem, stream, tq, tk, tv, p, dm::SnakeWalk{}));
+    }
     return DM_OK;
 }

@@ -4,6 +4,9 @@
 #include <mutex>
 
 #include "dm_host.h"
+#include "dm_attn_common.cuh"
+
+#include <algorithm>
 
 namespace dmh {
 
@@ -160,6 +163,97 @@ int* device_status_word(char* err, size_t errlen) {
     return g_status[dev].load(std::memory_order_relaxed);
 }
 
+// In two to five rounds of causal items the snake leaves the busiest CTA 4 to 15 % above the mean (3.5 rounds of one head of 65536 rows:
+// 6 %; 8 heads of 5632: 11 %), and so does longest-first.  Packing comes to 1 or 2 %: the smallest capacity (by bisection) into which the
+// items fit when every CTA in turn takes the longest that still fits it (multifit).  An item costs its tiles and two more: with half a
+// tile the packings come out with CTAs of a dozen one-tile items, 83 against 67 us for pass 1 of B2 N2048 H16; with four or more the
+// gain of the packed calls shrinks.  Forward and pass 1 take it; pass 2, whose items cost six or more tiles besides their own, lost
+// as often as it won (B2 N3584 H8 24.1 -> 24.9 us).  Taken where the busiest CTA saves two tiles and 3 %: pass 1 / forward of one head
+// of 65536 1560 -> 1490 / 952 -> 905 us, B5 N11264 H1 254 -> 240 / 157 -> 146, B4 N5632 H2 111 -> 102 / 69.0 -> 64.8, B2 N3072 H9
+// 80.9 -> 77.4 / 50.4 -> 48.6, B10 N512 H12 31.1 -> 29.7 / 19.0 -> 18.5, B3 N2816 H7 78.2 -> 77.0 / 48.9 -> 48.5; with less to save
+// (B4 N1024 H14: one tile of 22) the longer walks cost what the balance gives, 24.5 -> 24.9 us, and beyond five rounds the snake is
+// within 3 %.
+namespace {
+struct WalkPlanner {
+    int heads, nblk, ctas;
+    int cost(int size) const { return size + 2; }
+    int snake() const {
+        const int n = heads * nblk;
+        int worst = 0;
+        for (int c = 0; c < ctas; ++c) {
+            int load = 0;
+            for (int r = 0;; ++r) {
+                const int i = r * ctas + ((r & 1) ? ctas - 1 - c : c);
+                if (r * ctas >= n) break;
+                if (i < n) load += cost(nblk - i / heads);
+            }
+            if (load > worst) worst = load;
+        }
+        return worst;
+    }
+    // Fills the CTAs up to `cap`; true if every item found a place.  `w` (may be null) takes the lists.
+    bool fill(int cap, dm::PackedWalk* w) const {
+        int used[dm::kWalkItems + 1] = {};           // items of a size that have a place
+        int left = heads * nblk, at = 0;
+        for (int c = 0; c < ctas; ++c) {
+            if (w) w->first[c] = (uint16_t)at;
+            int room = cap;
+            for (int size = nblk; size > 0 && left > 0;) {
+                if (used[size] == heads || cost(size) > room) {
+                    --size;
+                    continue;
+                }
+                if (w) w->item[at] = (uint16_t)((nblk - size) * heads + used[size]);
+                ++at;
+                ++used[size];
+                --left;
+                room -= cost(size);
+            }
+        }
+        if (w) w->first[ctas] = (uint16_t)at;
+        return left == 0;
+    }
+    bool plan(dm::PackedWalk* w) const {
+        int64_t total = 0;
+        for (int size = 1; size <= nblk; ++size) total += (int64_t)heads * cost(size);
+        int lo = std::max((int)((total + ctas - 1) / ctas), cost(nblk)), hi = snake();
+        const int limit = hi - std::max(2, (hi + 31) / 32);
+        while (lo < hi) {                       // the smallest capacity found to do (the fit is not quite monotone; any that does is right)
+            const int mid = (lo + hi) / 2;
+            if (fill(mid, nullptr)) hi = mid;
+            else lo = mid + 1;
+        }
+        if (hi > limit || !fill(hi, w)) return false;
+        for (int c = 1; c < ctas; ++c)          // an item for every CTA: those left without take the shortest, one each
+            w->first[c] = (uint16_t)std::min((int)w->first[c], heads * nblk - (ctas - c));
+        return true;
+    }
+};
+}  // namespace
+
+const dm::PackedWalk* plan_walk(int heads, int nblk, int ctas) {
+    const int64_t n = (int64_t)heads * nblk;
+    if (n <= ctas || n > dm::kWalkItems || ctas > dm::kWalkCtas) return nullptr;
+    // the last few shapes of the thread: a training step asks for the same ones again
+    struct Entry {
+        int heads, nblk, ctas;
+        bool taken;
+        dm::PackedWalk w;
+    };
+    constexpr unsigned kKept = 8;
+    static thread_local Entry kept[kKept] = {};
+    static thread_local unsigned next = 0;
+    for (const Entry& e : kept)
+        if (e.heads == heads && e.nblk == nblk && e.ctas == ctas) return e.taken ? &e.w : nullptr;
+    Entry& e = kept[next++ % kKept];
+    e.heads = 0;
+    e.taken = WalkPlanner{heads, nblk, ctas}.plan(&e.w);
+    e.heads = heads;
+    e.nblk = nblk;
+    e.ctas = ctas;
+    return e.taken ? &e.w : nullptr;
+}
+
 }  // namespace dmh
 
 extern "C" const char* dm_build_info(void) {
@@ -169,6 +263,15 @@ extern "C" const char* dm_build_info(void) {
 
 extern "C" int dm_register_pool_ok(int32_t compiled_regs_per_thread, int32_t threads, int32_t regs_needed) {
     return dmh::register_pool_ok(compiled_regs_per_thread, threads, regs_needed) ? 1 : 0;
+}
+
+extern "C" int dm_walk_plan(int32_t heads, int32_t nblk, int32_t ctas, int32_t* first, int32_t* items) {
+    if (heads <= 0 || nblk <= 0 || ctas <= 0 || !first || !items) return 0;
+    const dm::PackedWalk* w = dmh::plan_walk(heads, nblk, ctas);
+    if (!w) return 0;
+    for (int c = 0; c <= ctas; ++c) first[c] = w->first[c];
+    for (int i = 0; i < w->first[ctas]; ++i) items[i] = w->item[i];
+    return 1;
 }
 
 extern "C" int dm_init(char* err, size_t errlen) {

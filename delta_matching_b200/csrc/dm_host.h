@@ -13,6 +13,10 @@
 
 #include "../../include/dm_b200.h"
 
+namespace dm {
+struct PackedWalk;
+}
+
 namespace dmh {
 
 inline int fail(char* err, size_t errlen, int code, const char* fmt, ...) __attribute__((format(printf, 4, 5)));
@@ -86,6 +90,10 @@ int device_once(DeviceOnce& o, char* err, size_t errlen, F&& f) {
 }
 // Number of SMs of the current device (cached per device).
 int sm_count(int* sms, char* err, size_t errlen);
+
+// How `ctas` persistent CTAs walk heads x nblk items whose lengths fall by one tile a rank (nblk, .., 1), or null where the snake order is as
+// good (one round; many rounds).  The lists are the thread's own and hold until its next few calls.
+const dm::PackedWalk* plan_walk(int heads, int nblk, int ctas);
 
 // One-time set-up of each kernel family on the current device (also reached lazily from the entry points).
 int prepare_fwd(char* err, size_t errlen);

@@ -227,6 +227,12 @@ int dm_init(char* err, size_t errlen);
  * arithmetic, exported so it can be tested without a GPU.  No counterpart in the reference. */
 int dm_register_pool_ok(int32_t compiled_regs_per_thread, int32_t threads, int32_t regs_needed);
 
+/* The order in which `ctas` persistent thread blocks walk heads x nblk work items of a causal call (item = rank * heads + head, of
+ * nblk - rank tiles): 1 and the blocks' lists (block c: items[first[c]] .. items[first[c + 1] - 1]; `first` holds ctas + 1 numbers,
+ * `items` heads * nblk) where a packing is used, 0 where the kernels' fixed order is.  Pure host arithmetic, exported so it can be
+ * tested without a GPU.  No counterpart in the reference. */
+int dm_walk_plan(int32_t heads, int32_t nblk, int32_t ctas, int32_t* first, int32_t* items);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,70 @@
+"""The packed walk of the persistent kernels (causal calls of a few rounds): every item once, each block's longest first, and never worse than the
+fixed order it replaces."""
+import ctypes as C
+
+import pytest
+
+from delta_matching_b200 import _lib
+
+CTAS = 148
+
+
+def _plan(heads, nblk, ctas=CTAS):
+    first, items = (C.c_int32 * (ctas + 1))(), (C.c_int32 * (heads * nblk))()
+    if not _lib.lib().dm_walk_plan(heads, nblk, ctas, first, items):
+        return None
+    assert first[0] == 0 and first[ctas] == heads * nblk
+    return [list(items[first[c]:first[c + 1]]) for c in range(ctas)]
+
+
+def _cost(i, heads, nblk):
+    return nblk - i // heads + 2                             # its tiles, and two for what an item costs besides
+
+
+def _snake(heads, nblk, ctas=CTAS):
+    n = heads * nblk
+    walk = [[r * ctas + (ctas - 1 - c if r & 1 else c) for r in range((n + ctas - 1) // ctas)] for c in range(ctas)]
+    return [[i for i in w if i < n] for w in walk]
+
+
+# shapes of one item more than the blocks to the most that is packed; one head of many blocks; many heads of one block
+@pytest.mark.parametrize("heads,nblk,ctas", [(149, 1, 148), (75, 2, 148), (48, 6, 148), (32, 16, 148), (21, 22, 148), (16, 30, 148), (1, 512, 148),
+                                             (1, 800, 148), (2, 400, 148), (100, 8, 148), (11, 61, 148), (7, 9, 5), (1, 3, 2), (160, 5, 160)])
+def test_packed_walk(heads, nblk, ctas):
+    load = lambda walk: max(sum(_cost(i, heads, nblk) for i in w) for w in walk)
+    plan, snake = _plan(heads, nblk, ctas), _snake(heads, nblk, ctas)
+    if plan is None:
+        return
+    assert sorted(i for w in plan for i in w) == list(range(heads * nblk))
+    assert all(w and w == sorted(w) for w in plan)                 # rank-major: longest first
+    assert load(plan) < 0.97 * load(snake)
+
+
+def test_where_it_is_used():
+    assert all(_plan(h, n) for h, n in ((21, 22), (1, 512), (8, 44), (16, 28)))
+    assert _plan(8, 4) is None                               # one round
+    assert _plan(128, 32) is None                            # many rounds: the fixed order is as good
+    assert _plan(149, 1) is None                             # lengths that do not differ
+    worst = max(sum(_cost(i, 1, 512) for i in w) for w in _plan(1, 512))
+    assert worst <= 1.01 * sum(_cost(i, 1, 512) for i in range(512)) / CTAS
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,H", [(512, 75), (1536, 34), (2816, 21), (5632, 8)])
+def test_packed_calls_give_the_bits_of_one_round_calls(N, H):
+    import torch
+    from delta_matching_b200 import dm_attn_func
+    assert _plan(H, N // 128)
+    g = torch.Generator(device="cuda").manual_seed(N)
+    q, k, v, do = (torch.randn(1, N, H, 128, generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+
+    def run(lo, hi):
+        x = [t[:, :, lo:hi].contiguous().requires_grad_() for t in (q, k, v)]
+        o = dm_attn_func(*x, causal=True)
+        return (o.detach(), *torch.autograd.grad(o, x, do[:, :, lo:hi].contiguous()))
+
+    whole, step = run(0, H), CTAS // (N // 128)              # heads whose items are one round: the fixed order
+    for lo in range(0, H, step):
+        hi = min(H, lo + step)
+        for a, b in zip(whole, run(lo, hi)):
+            assert torch.equal(a[:, :, lo:hi], b)
