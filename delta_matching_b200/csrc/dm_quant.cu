@@ -90,6 +90,13 @@ __global__ void kmean_fold_kernel(const float* __restrict__ partials, int N, flo
     km[(int64_t)bh * D + d] = __fdiv_rn(acc, (float)N);
 }
 
+// max(a, |b|, |c|) for a >= 0; a NaN operand makes it a NaN (the positive canonical one)
+__device__ __forceinline__ float max3_abs_nan(float a, float b, float c) {
+    float d;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
 // ---- block quantizer ------------------------------------------------------------------------------------------------
 // MODE 0 = Q, 1 = K, 2 = V, 3 = dO, 4 = dO with the stale delta = rowsum(dO * O) (its own instantiation: the O loads
 // and the row sums cost registers the matched mode does not have to pay).
@@ -108,7 +115,7 @@ __device__ __forceinline__ void quant_block(int blk, int bh, const __nv_bfloat16
     constexpr int RPW = BLK / (8 * RW);   // steps per warp
     // Q, V and dO: the block maximum is a maximum of bf16 magnitudes (Q's multiply by a positive constant is monotone, so
     // it commutes with the maximum), which orders like their bit patterns: two elements per instruction, on the raw pairs.
-    // K subtracts a per-column mean first and takes the float route.
+    // K subtracts a per-column mean first: a float maximum, two elements per instruction.
     constexpr bool kPackedMax = MODE != 1;
     const int b = bh / heads, h = bh % heads;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -145,7 +152,7 @@ __device__ __forceinline__ void quant_block(int blk, int bh, const __nv_bfloat16
     };
 
     float amax = 0.f;
-    bool finite = false;                  // every element of the block is finite (known on the packed route only)
+    bool finite = false;                  // every element of the block is finite
     if (kPackedMax) {
         uint32_t m = 0;
 #pragma unroll
@@ -163,7 +170,21 @@ __device__ __forceinline__ void quant_block(int blk, int bh, const __nv_bfloat16
         amax = __uint_as_float(m << 16);
         if (MODE == 0) amax = __fmul_rn(amax, sm);
     }
-    if (!kPackedMax || !finite) {         // uniform over the block.  A NaN is skipped by the maximum, an infinity wins it.
+    if (MODE == 1) {                      // K: the maximum of the magnitudes that a NaN wins, two elements per instruction
+#pragma unroll
+        for (int r = 0; r < RPW; ++r)
+#pragma unroll
+            for (int e = 0; e < E; e += 2) amax = max3_abs_nan(amax, value(r, e), value(r, e + 1));
+        amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));     // non-negative floats and NaNs order like their bits
+        if (l == 0) s_bits[w] = __float_as_uint(amax);
+        __syncthreads();
+        uint32_t m = s_bits[0];
+#pragma unroll
+        for (int i = 1; i < 8; ++i) m = max(m, s_bits[i]);
+        finite = m < 0x7F800000u;
+        amax = __uint_as_float(m);
+    }
+    if (!finite) {                        // uniform over the block.  A NaN is skipped by the maximum, an infinity wins it.
         amax = 0.f;
 #pragma unroll
         for (int r = 0; r < RPW; ++r)
@@ -202,12 +223,13 @@ __device__ __forceinline__ void quant_block(int blk, int bh, const __nv_bfloat16
                         float q = __fmul_rn(xv, rcp);
                         q = __fmaf_rn(__fmaf_rn(-q, s, xv), rcp, q);
                         qv[e] = __fmaf_rn(__fmaf_rn(-q, s, xv), rcp, q);
+                        if (MODE == 1) qv[e] = copysignf(qv[e], xv);
                     } else {
                         qv[e] = fminf(fmaxf(quotient_rn<kExactRcp>(xv, s, rcp), -kE4M3Max), kE4M3Max);
                     }
                 }
                 c4[g] = e4m3x4(qv[0], qv[1], qv[2], qv[3]);
-                if (kFinite) {
+                if (kFinite && MODE != 1) {
                     const uint32_t sign = __byte_perm(u[r][2 * g], u[r][2 * g + 1], 0x7531);   // the high byte of each bf16
                     c4[g] = (c4[g] & 0x7F7F7F7Fu) | (sign & 0x80808080u);
                 }
@@ -242,7 +264,7 @@ __device__ __forceinline__ void quant_block(int blk, int bh, const __nv_bfloat16
         }
     };
     const bool in_range = s >= 0x1p-60f && s <= 0x1p60f;
-    if (kPackedMax && finite && in_range) emit(std::true_type{}, std::true_type{});
+    if (finite && in_range) emit(std::true_type{}, std::true_type{});
     else if (in_range) emit(std::true_type{}, std::false_type{});
     else emit(std::false_type{}, std::false_type{});
 }
@@ -258,11 +280,14 @@ __global__ void __launch_bounds__(256) quant_kernel(const __nv_bfloat16* __restr
 
 // The K quantizer with the K mean's fold in front of it, for short sequences: every block folds the head's chunk sums itself
 // (same order and division as kmean_fold_kernel, so the same bits; N / 64 additions per column, read from L2), which saves
-// the fold's launch; the first block of a head also writes the mean out.
+// the fold's launch; the first block of a head also writes the mean out.  From 64 chunk sums on, where the grid still gives every SM
+// two blocks, a block takes `per` = 4 key blocks: the 32 KB of chunk sums that it folds are read by a quarter as many (B4 N4096 Hk8:
+// 23.3 -> 20 us; at N 2048 9.4 -> 10.7, fewer blocks in flight).  Of the rest the instructions per element are the most: K's blocks
+// find out in their maximum whether they are finite and skip the clamps like the others (20 -> 17.1, at N 2048 9.4 -> 9.0).
 template <int D>
 __global__ void __launch_bounds__(256) quant_k_folded_kernel(const __nv_bfloat16* __restrict__ x, int64_t sb, int64_t sn, int64_t sh,
                                                              const float* __restrict__ partials, float* __restrict__ km_out,
-                                                             uint8_t* __restrict__ codes, float* __restrict__ scales, int heads, int N) {
+                                                             uint8_t* __restrict__ codes, float* __restrict__ scales, int heads, int N, int per) {
     dm::pdl_wait();
     __shared__ float s_km[D];
     const int bh = blockIdx.y;
@@ -275,12 +300,18 @@ __global__ void __launch_bounds__(256) quant_k_folded_kernel(const __nv_bfloat16
         if (blockIdx.x == 0) km_out[(int64_t)bh * D + threadIdx.x] = m;
     }
     __syncthreads();
-    quant_block<D, 1>(blockIdx.x, bh, x, sb, sn, sh, nullptr, 0, 0, 0, s_km - (int64_t)bh * D, codes, scales, nullptr, heads, N, 0.f);
+    for (int i = 0; i < per; ++i) {
+        if (i) __syncthreads();
+        quant_block<D, 1>(blockIdx.x * per + i, bh, x, sb, sn, sh, nullptr, 0, 0, 0, s_km - (int64_t)bh * D, codes, scales, nullptr, heads, N, 0.f);
+    }
 }
 
 // The three producers of the forward that depend on nothing but the inputs, in one launch: K's per-chunk column sums
 // (first in the grid: the K quantizer waits for them through the fold), the Q quantizer and the V quantizer.  A block
-// does exactly what a block of the separate kernels does, so the results carry the same bits.
+// does exactly what a block of the separate kernels does, so the results carry the same bits.  Bound by the bytes in flight: five blocks
+// per SM (48 registers, 24 bytes spilled) instead of the three that 79 registers leave take B4 N4096 H32 Hk8 from 63 to 54 us (5.3 TB/s),
+// B2 N2048 H16 from 18.3 to 15.7, B2 N4096 H16 head_dim 256 from 32 to 28; four blocks 56.5 / 17.1 / 30, six (64 bytes spilled) 60 / 17.4 / 30.
+// K's sums last, so that K would still be in L2 for its quantizer, end the launch on their latency (B4 N768 H12 11.6 -> 13.2 us).
 struct PrologueArgs {
     const __nv_bfloat16 *q, *k, *v;
     DmStrides qs, ks, vs;
@@ -291,7 +322,7 @@ struct PrologueArgs {
     float sm;
 };
 template <int D>
-__global__ void __launch_bounds__(256) prologue_kernel(const PrologueArgs a) {
+__global__ void __launch_bounds__(256, 5) prologue_kernel(const PrologueArgs a) {
     dm::pdl_wait();
     int i = blockIdx.x;
     if (i < a.n_p) {
@@ -593,8 +624,11 @@ int launch_kmean_fold_quant_k(const void* k, DmStrides ks, const float* partials
         if ((rc = check_device_ptr(ptrs[i], names[i], err, errlen))) return rc;
     if ((rc = check_strides(k, ks, s.D, "k", err, errlen))) return rc;
     DM_REQUIRE(aligned16(k8), DM_ERR_ARG, "codes is not 16-byte aligned");
-    DM_CUDA(launch_pdl(quant_k_folded_kernel<128>, dim3(s.N / 64, s.B * s.Hk), 256, 0, stream, static_cast<const __nv_bfloat16*>(k), ks.b, ks.n,
-                       ks.h, partials, km, static_cast<uint8_t*>(k8), k8s, s.Hk, s.N));
+    int sms = 0;
+    if ((rc = sm_count(&sms, err, errlen))) return rc;
+    const int nblk = s.N / 64, per = nblk >= 64 && (int64_t)nblk / 4 * s.B * s.Hk >= 2 * sms ? 4 : 1;      // (nblk is a multiple of 4)
+    DM_CUDA(launch_pdl(quant_k_folded_kernel<128>, dim3(s.N / 64 / per, s.B * s.Hk), 256, 0, stream, static_cast<const __nv_bfloat16*>(k), ks.b, ks.n,
+                       ks.h, partials, km, static_cast<uint8_t*>(k8), k8s, s.Hk, s.N, per));
     return DM_OK;
 }
 }  // namespace dmh
