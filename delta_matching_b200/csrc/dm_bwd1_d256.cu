@@ -64,7 +64,7 @@ struct Params {
 };
 
 // The work list: one item = 64 keys `zh` of one 128-key block J of one (batch, query head), ordered by key block, i.e. heaviest first when
-// causal, and walked in a snake over the rounds (dm_bwd1.cu).
+// causal, and walked in a snake over the rounds (as dm::SnakeWalk).
 struct Item {
     dm::HeadCoord hc;
     int J, zh, t_lo, n, bhl;                      // first 128-row tile and their count

@@ -50,7 +50,7 @@ struct Bwd2Params {
 };
 
 // One work item = one local 128-row block of one (batch, head); numbered rank-major (rank 0 = the row blocks with the most key
-// tiles, all heads, then rank 1, ...) and walked in a snake over the rounds, as in the forward.
+// tiles, all heads, then rank 1, ...) and walked in a snake over the rounds (as dm::SnakeWalk).
 struct Bwd2Item {
     dm::HeadCoord hc;
     int rb, n_it, bhl;

@@ -2,7 +2,7 @@
 // (csrc/flash_fwd_fp8f_launch.h:40, csrc/softmax_fq8f.h kGroups = 4): Q scales per 64 rows, K / V scales per 32 keys,
 // key tiles of 128 keys = FOUR 32-key P groups, each with its own per-row basis.
 //
-// One work item = 128 query rows of one (batch, head); the kernel is persistent, one CTA per SM walks its items (the walk of dm_fwd.cu),
+// One work item = 128 query rows of one (batch, head); the kernel is persistent, one CTA per SM walks its items (as dm::SnakeWalk),
 // and every role keeps its own place in the list.  A code row is 256 bytes = two 128-byte swizzled sub-tiles (d 0..127 and d 128..255).
 // 512 threads:
 //   warps 0..3   service (one elected lane issues): S; the products; the loads of Q and K; the loads of V
