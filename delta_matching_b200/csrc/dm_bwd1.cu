@@ -788,8 +788,9 @@ extern "C" int dm_bwd_fp8_pass1_cp(const void* q8, const void* k8, const void* v
     if ((rc = dmh::sm_count(&sms, err, errlen))) return rc;
     const int64_t items = (int64_t)sh.B * hcount * (sh.N / 128);
     const int grid = (int)(items < sms ? items : sms);
-    if (const dm::PackedWalk* walk = sh.causal && plain ? dmh::plan_walk(sh.B * hcount, sh.N / 128, grid) : nullptr) {
-        DM_CUDA(dmh::launch_pdl(bwd1_kernel<dm::PackedWalk>, grid, kThreads, sizeof(Smem) + 1024, stream, tq, td, tk, tv, ts, p, *walk));
+    dm::PackedWalk walk;
+    if (sh.causal && plain && dmh::plan_walk(sh.B * hcount, sh.N / 128, grid, &walk)) {
+        DM_CUDA(dmh::launch_pdl(bwd1_kernel<dm::PackedWalk>, grid, kThreads, sizeof(Smem) + 1024, stream, tq, td, tk, tv, ts, p, walk));
     } else {
         DM_CUDA(dmh::launch_pdl(bwd1_kernel<dm::SnakeWalk>, grid, kThreads, sizeof(Smem) + 1024, stream, tq, td, tk, tv, ts, p, dm::SnakeWalk{}));
     }

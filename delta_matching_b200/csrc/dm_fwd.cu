@@ -545,8 +545,9 @@ extern "C" int dm_fwd_fp8_cp(const void* q8, const void* k8, const void* v8, con
     // persistent: one CTA per SM walks the (head, row block) items, heaviest first
     const int64_t items = (int64_t)sh.B * hcount * (cp.nq / 128);
     const int grid = (int)(items < sms ? items : sms);
-    if (const dm::PackedWalk* walk = sh.causal && cp.nq == sh.N ? dmh::plan_walk(sh.B * hcount, sh.N / 128, grid) : nullptr) {
-        DM_CUDA(dmh::launch_pdl(fwd_d128_kernel<dm::PackedWalk>, grid, kThreads, smem, stream, tq, tk, tv, p, *walk));
+    dm::PackedWalk walk;
+    if (sh.causal && cp.nq == sh.N && dmh::plan_walk(sh.B * hcount, sh.N / 128, grid, &walk)) {
+        DM_CUDA(dmh::launch_pdl(fwd_d128_kernel<dm::PackedWalk>, grid, kThreads, smem, stream, tq, tk, tv, p, walk));
     } else {
         DM_CUDA(dmh::launch_pdl(fwd_d128_kernel<dm::SnakeWalk>, grid, kThreads, smem, stream, tq, tk, tv, p, dm::SnakeWalk{}));
     }

@@ -164,7 +164,7 @@ int* device_status_word(char* err, size_t errlen) {
 }
 
 // In two to five rounds of causal items the snake leaves the busiest CTA 4 to 15 % above the mean (3.5 rounds of one head of 65536 rows:
-// 6 %; 8 heads of 5632: 11 %), and so does longest-first.  Packing comes to 1 or 2 %: the smallest capacity (by bisection) into which the
+// 6 %; 8 heads of 5632: 11 %), and so does longest-first.  Packing comes to 1 or 2 %: the smallest capacity into which the
 // items fit when every CTA in turn takes the longest that still fits it (multifit).  An item costs its tiles and two more: with half a
 // tile the packings come out with CTAs of a dozen one-tile items, 83 against 67 us for pass 1 of B2 N2048 H16; with four or more the
 // gain of the packed calls shrinks.  Forward and pass 1 take it; pass 2, whose items cost six or more tiles besides their own, lost
@@ -176,82 +176,122 @@ int* device_status_word(char* err, size_t errlen) {
 namespace {
 struct WalkPlanner {
     int heads, nblk, ctas;
-    int cost(int size) const { return size + 2; }
-    int snake() const {
-        const int n = heads * nblk;
-        int worst = 0;
-        for (int c = 0; c < ctas; ++c) {
-            int load = 0;
-            for (int r = 0;; ++r) {
-                const int i = r * ctas + ((r & 1) ? ctas - 1 - c : c);
-                if (r * ctas >= n) break;
-                if (i < n) load += cost(nblk - i / heads);
+    static int cost(int size) { return size + 2; }
+    int snake() const {                              // tiles of the busiest CTA without a plan
+        int load[dm::kWalkCtas] = {};
+        int at = 0, step = 1;
+        for (int size = nblk; size > 0; --size)
+            for (int h = 0; h < heads; ++h) {
+                load[at] += cost(size);
+                if (at + step < 0 || at + step == ctas) step = -step;      // the round ends: the next one comes back
+                else at += step;
             }
-            if (load > worst) worst = load;
-        }
-        return worst;
+        return *std::max_element(load, load + ctas);
     }
-    // Fills the CTAs up to `cap`; true if every item found a place.  `w` (may be null) takes the lists.
+    // Fills the CTAs up to `cap`; true if every item found a place.  `w` takes the lists.  `largest` finds the largest size
+    // up to `s` of which an item is left (0: none) along links that skip the sizes used up and are shortened on the way, so that a
+    // fill costs items and CTAs and not sizes times CTAs.
     bool fill(int cap, dm::PackedWalk* w) const {
-        int used[dm::kWalkItems + 1] = {};           // items of a size that have a place
-        int left = heads * nblk, at = 0;
+        uint16_t used[dm::kWalkItems + 1], link[dm::kWalkItems + 1];
+        for (int s = 0; s <= nblk; ++s) {
+            used[s] = 0;
+            link[s] = (uint16_t)s;
+        }
+        const auto largest = [&link](int s) {
+            while (link[s] != s) s = link[s] = link[link[s]];
+            return s;
+        };
+        int at = 0;
         for (int c = 0; c < ctas; ++c) {
-            if (w) w->first[c] = (uint16_t)at;
+            w->first[c] = (uint16_t)at;
             int room = cap;
-            for (int size = nblk; size > 0 && left > 0;) {
-                if (used[size] == heads || cost(size) > room) {
-                    --size;
-                    continue;
-                }
-                if (w) w->item[at] = (uint16_t)((nblk - size) * heads + used[size]);
-                ++at;
-                ++used[size];
-                --left;
-                room -= cost(size);
+            for (int size = largest(std::min(nblk, room - cost(0))); size > 0; size = largest(std::min(size, std::max(room - cost(0), 0)))) {
+                const int n = std::min(heads - used[size], room / cost(size));
+                for (int i = 0; i < n; ++i) w->item[at + i] = (uint16_t)((nblk - size) * heads + used[size] + i);
+                at += n;
+                room -= n * cost(size);
+                used[size] = (uint16_t)(used[size] + n);
+                if (used[size] == heads) link[size] = (uint16_t)(size - 1);
             }
         }
-        if (w) w->first[ctas] = (uint16_t)at;
-        return left == 0;
+        w->first[ctas] = (uint16_t)at;
+        return at == heads * nblk;
     }
     bool plan(dm::PackedWalk* w) const {
         int64_t total = 0;
         for (int size = 1; size <= nblk; ++size) total += (int64_t)heads * cost(size);
-        int lo = std::max((int)((total + ctas - 1) / ctas), cost(nblk)), hi = snake();
-        const int limit = hi - std::max(2, (hi + 31) / 32);
-        while (lo < hi) {                       // the smallest capacity found to do (the fit is not quite monotone; any that does is right)
-            const int mid = (lo + hi) / 2;
-            if (fill(mid, nullptr)) hi = mid;
-            else lo = mid + 1;
+        const int busiest = snake(), limit = busiest - std::max(2, (busiest + 31) / 32);
+        // The smallest capacity that does is, but for a few shapes, what the mean CTA or the longest item asks for, so the search goes up from
+        // there in growing steps and halves the last one (the fit is not quite monotone; any capacity that does is right).
+        int fails = std::max((int)((total + ctas - 1) / ctas), cost(nblk)) - 1, fits = 0, held = 0;
+        for (int step = 1; !fits && fails < limit; step *= 2) {
+            held = std::min(fails + step, limit);
+            (fill(held, w) ? fits : fails) = held;
         }
-        if (hi > limit || !fill(hi, w)) return false;
+        if (!fits) return false;
+        while (fits - fails > 1) {
+            held = (fits + fails) / 2;
+            (fill(held, w) ? fits : fails) = held;
+        }
+        if (held != fits) fill(fits, w);
         for (int c = 1; c < ctas; ++c)          // an item for every CTA: those left without take the shortest, one each
             w->first[c] = (uint16_t)std::min((int)w->first[c], heads * nblk - (ctas - c));
         return true;
     }
 };
+
+// The answers for the shapes asked for last, the same for every thread and device (a plan is a pure function of the three numbers): forward and
+// backward run on different threads, and a program with bucketed lengths comes back to some dozens of shapes.  Shapes with and without a
+// plan have places of their own.  One that is not kept costs 2 to 10 us here (a fill that scanned every size for every CTA, once per step
+// of a bisection, took 20 to 1300), a kept one 0.1.  Evaluation of many lengths in turn, each call waited for, eight shapes per thread and
+// that fill / this: 15 lengths of one head of 38400 to 45568 rows 622 -> 409 us a call, 20 of two heads of 19456 to 24320 366 -> 244, 16 of
+// eight heads of 4864 to 8704 146 -> 125.
+struct WalkTable {
+    static constexpr unsigned kKept = 64;
+    std::mutex mu;
+    uint32_t planned[kKept] = {}, refused[kKept] = {};
+    dm::PackedWalk walk[kKept] = {};
+    unsigned next_planned = 0, next_refused = 0;
+};
+WalkTable g_walks;
+
+bool kept_walk(uint32_t key, dm::PackedWalk* out, bool* taken) {
+    std::lock_guard<std::mutex> lk(g_walks.mu);
+    for (unsigned i = 0; i < WalkTable::kKept; ++i) {
+        if (g_walks.planned[i] == key) {
+            *out = g_walks.walk[i];
+            return *taken = true;
+        }
+        if (g_walks.refused[i] == key) {
+            *taken = false;
+            return true;
+        }
+    }
+    return false;
+}
+void keep_walk(uint32_t key, const dm::PackedWalk& w, bool taken) {      // (two threads may keep the same answer twice)
+    std::lock_guard<std::mutex> lk(g_walks.mu);
+    if (taken) {
+        const unsigned i = g_walks.next_planned++ % WalkTable::kKept;
+        g_walks.planned[i] = key;
+        g_walks.walk[i] = w;
+    } else {
+        g_walks.refused[g_walks.next_refused++ % WalkTable::kKept] = key;
+    }
+}
 }  // namespace
 
-const dm::PackedWalk* plan_walk(int heads, int nblk, int ctas) {
+bool plan_walk(int heads, int nblk, int ctas, dm::PackedWalk* out) {
     const int64_t n = (int64_t)heads * nblk;
-    if (n <= ctas || n > dm::kWalkItems || ctas > dm::kWalkCtas) return nullptr;
-    // the last few shapes of the thread: a training step asks for the same ones again
-    struct Entry {
-        int heads, nblk, ctas;
-        bool taken;
-        dm::PackedWalk w;
-    };
-    constexpr unsigned kKept = 8;
-    static thread_local Entry kept[kKept] = {};
-    static thread_local unsigned next = 0;
-    for (const Entry& e : kept)
-        if (e.heads == heads && e.nblk == nblk && e.ctas == ctas) return e.taken ? &e.w : nullptr;
-    Entry& e = kept[next++ % kKept];
-    e.heads = 0;
-    e.taken = WalkPlanner{heads, nblk, ctas}.plan(&e.w);
-    e.heads = heads;
-    e.nblk = nblk;
-    e.ctas = ctas;
-    return e.taken ? &e.w : nullptr;
+    if (n <= ctas || n > dm::kWalkItems || ctas > dm::kWalkCtas) return false;
+    static_assert(dm::kWalkItems < 1024 && dm::kWalkCtas < 1024, "a key holds ten bits of each");
+    const uint32_t key = (uint32_t)heads | (uint32_t)nblk << 10 | (uint32_t)ctas << 20;
+    bool taken;
+    if (kept_walk(key, out, &taken)) return taken;
+    *out = {};
+    taken = WalkPlanner{heads, nblk, ctas}.plan(out);
+    keep_walk(key, *out, taken);
+    return taken;
 }
 
 }  // namespace dmh
@@ -267,10 +307,10 @@ extern "C" int dm_register_pool_ok(int32_t compiled_regs_per_thread, int32_t thr
 
 extern "C" int dm_walk_plan(int32_t heads, int32_t nblk, int32_t ctas, int32_t* first, int32_t* items) {
     if (heads <= 0 || nblk <= 0 || ctas <= 0 || !first || !items) return 0;
-    const dm::PackedWalk* w = dmh::plan_walk(heads, nblk, ctas);
-    if (!w) return 0;
-    for (int c = 0; c <= ctas; ++c) first[c] = w->first[c];
-    for (int i = 0; i < w->first[ctas]; ++i) items[i] = w->item[i];
+    dm::PackedWalk w;
+    if (!dmh::plan_walk(heads, nblk, ctas, &w)) return 0;
+    for (int c = 0; c <= ctas; ++c) first[c] = w.first[c];
+    for (int i = 0; i < w.first[ctas]; ++i) items[i] = w.item[i];
     return 1;
 }
 

@@ -91,9 +91,9 @@ int device_once(DeviceOnce& o, char* err, size_t errlen, F&& f) {
 // Number of SMs of the current device (cached per device).
 int sm_count(int* sms, char* err, size_t errlen);
 
-// How `ctas` persistent CTAs walk heads x nblk items whose lengths fall by one tile a rank (nblk, .., 1), or null where the snake order is as
-// good (one round; many rounds).  The lists are the thread's own and hold until its next few calls.
-const dm::PackedWalk* plan_walk(int heads, int nblk, int ctas);
+// How `ctas` persistent CTAs walk heads x nblk items whose lengths fall by one tile a rank (nblk, .., 1); false (and no lists) where the snake
+// order is as good (one round; many rounds).
+bool plan_walk(int heads, int nblk, int ctas, dm::PackedWalk* out);
 
 // One-time set-up of each kernel family on the current device (also reached lazily from the entry points).
 int prepare_fwd(char* err, size_t errlen);

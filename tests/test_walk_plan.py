@@ -1,6 +1,8 @@
 """The packed walk of the persistent kernels (causal calls of a few rounds): every item once, each block's longest first, and never worse than the
 fixed order it replaces."""
 import ctypes as C
+import threading
+import time
 
 import pytest
 
@@ -47,6 +49,44 @@ def test_where_it_is_used():
     assert _plan(149, 1) is None                             # lengths that do not differ
     worst = max(sum(_cost(i, 1, 512) for i in w) for w in _plan(1, 512))
     assert worst <= 1.01 * sum(_cost(i, 1, 512) for i in range(512)) / CTAS
+
+
+def _seconds_a_call(shapes):
+    """Of the entry point alone, over all shapes in turn; the best of several rounds."""
+    f, first, items = _lib.lib().dm_walk_plan, (C.c_int32 * (CTAS + 1))(), (C.c_int32 * 800)()
+    best = 1.0
+    for _ in range(6):
+        t = time.perf_counter()
+        for heads, nblk in shapes:
+            f(heads, nblk, CTAS, first, items)
+        best = min(best, (time.perf_counter() - t) / len(shapes))
+    return best
+
+
+def test_programs_of_many_lengths():
+    """Some dozens of shapes in turn are all kept, those with a plan beside those without, and a shape that is not kept costs about as much as a
+    launch: 1 and 5 to 10 us here, 200 to 600 where a fill scans every size for every block.  The limits leave an order for a busy machine."""
+    long = [(1, n) for n in range(300, 360)]
+    assert _seconds_a_call(long) < 20e-6
+    assert _seconds_a_call([s for n in range(60) for s in (long[n], (128 + n, 2))]) < 20e-6
+    assert _seconds_a_call([(1, n) for n in range(260, 400)]) < 80e-6
+
+
+def test_threads():
+    shapes = [(1, n) for n in range(250, 420, 2)] + [(h, n) for h in (2, 7, 8, 16, 21, 34) for n in range(150 // h + 1, 150 // h + 20, 2)]
+    want, got = [_plan(*s) for s in shapes], {}
+    assert sum(w is not None for w in want) > 64 and None in want           # more with a plan than are kept, and some without
+
+    def ask(i):
+        order = list(range(i, len(shapes))) + list(range(i))
+        got[i] = all([_plan(*shapes[j]) == want[j] for j in order])
+
+    threads = [threading.Thread(target=ask, args=(17 * i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(got) == 4 and all(got.values())
 
 
 @pytest.mark.gpu
