@@ -29,17 +29,27 @@ def _snake(heads, nblk, ctas=CTAS):
     return [[i for i in w if i < n] for w in walk]
 
 
-# shapes of one item more than the blocks to the most that is packed; one head of many blocks; many heads of one block
-@pytest.mark.parametrize("heads,nblk,ctas", [(149, 1, 148), (75, 2, 148), (48, 6, 148), (32, 16, 148), (21, 22, 148), (16, 30, 148), (1, 512, 148),
-                                             (1, 800, 148), (2, 400, 148), (100, 8, 148), (11, 61, 148), (7, 9, 5), (1, 3, 2), (160, 5, 160)])
+def _most(walk, heads, nblk):
+    return max(sum(_cost(i, heads, nblk) for i in w) for w in walk)
+
+
+# the fewest and the most items that are packed; one head of many blocks; many heads of two and three; other numbers of blocks to share among
+@pytest.mark.parametrize("heads,nblk,ctas", [(9, 33, 148), (99, 3, 148), (50, 16, 148), (160, 5, 148), (1, 512, 148), (1, 781, 148), (329, 2, 148),
+                                             (21, 22, 148), (16, 28, 148), (16, 30, 148), (100, 8, 148), (11, 61, 148), (1, 800, 160), (355, 2, 160),
+                                             (107, 3, 160), (1, 11, 5), (38, 2, 5)])
 def test_packed_walk(heads, nblk, ctas):
-    load = lambda walk: max(sum(_cost(i, heads, nblk) for i in w) for w in walk)
     plan, snake = _plan(heads, nblk, ctas), _snake(heads, nblk, ctas)
-    if plan is None:
-        return
+    assert plan is not None
     assert sorted(i for w in plan for i in w) == list(range(heads * nblk))
     assert all(w and w == sorted(w) for w in plan)                 # rank-major: longest first
-    assert load(plan) < 0.97 * load(snake)
+    assert _most(plan, heads, nblk) < 0.97 * _most(snake, heads, nblk)
+
+
+# where the mean block is above what a packing has to come down to; where the packing found is; more items or blocks than the lists hold
+@pytest.mark.parametrize("heads,nblk,ctas", [(48, 6, 148), (32, 16, 148), (1, 800, 148), (2, 400, 148), (7, 9, 5), (1, 3, 2), (160, 5, 160),
+                                             (149, 1, 148), (75, 2, 148), (1, 801, 148), (9, 89, 148), (21, 22, 161)])
+def test_fixed_order(heads, nblk, ctas):
+    assert _plan(heads, nblk, ctas) is None
 
 
 def test_where_it_is_used():
@@ -89,22 +99,28 @@ def test_threads():
     assert len(got) == 4 and all(got.values())
 
 
+# one group of one head; groups of four and seven query heads, batches, the stale delta; items of 1 to 88 tiles (dV in two windows)
 @pytest.mark.gpu
-@pytest.mark.parametrize("N,H", [(512, 75), (1536, 34), (2816, 21), (5632, 8)])
-def test_packed_calls_give_the_bits_of_one_round_calls(N, H):
+@pytest.mark.parametrize("B,N,H,Hk,mode", [(1, 512, 75, 75, "matched"), (1, 1536, 34, 34, "matched"), (1, 2816, 21, 21, "matched"),
+                                           (1, 5632, 8, 8, "matched"), (2, 3584, 8, 2, "matched"), (2, 3584, 8, 2, "stale"),
+                                           (3, 2816, 7, 1, "stale"), (5, 11264, 1, 1, "stale"), (5, 11264, 1, 1, "matched")])
+def test_packed_calls_give_the_bits_of_calls_in_the_fixed_order(B, N, H, Hk, mode):
     import torch
     from delta_matching_b200 import dm_attn_func
-    assert _plan(H, N // 128)
+    rep, nblk = H // Hk, N // 128
+    assert _plan(B * H, nblk)
     g = torch.Generator(device="cuda").manual_seed(N)
-    q, k, v, do = (torch.randn(1, N, H, 128, generator=g, device="cuda", dtype=torch.bfloat16) for _ in range(4))
+    q, k, v, do = (torch.randn(B, N, h, 128, generator=g, device="cuda", dtype=torch.bfloat16) for h in (H, Hk, Hk, H))
 
-    def run(lo, hi):
-        x = [t[:, :, lo:hi].contiguous().requires_grad_() for t in (q, k, v)]
-        o = dm_attn_func(*x, causal=True)
-        return (o.detach(), *torch.autograd.grad(o, x, do[:, :, lo:hi].contiguous()))
+    def run(b, lo, hi):                                      # KV groups lo .. hi - 1 of some sequences
+        x = [t[b, :, lo * r:hi * r].contiguous().requires_grad_() for t, r in ((q, rep), (k, 1), (v, 1))]
+        o = dm_attn_func(*x, causal=True, mode=mode)
+        return (o.detach(), *torch.autograd.grad(o, x, do[b, :, lo * rep:hi * rep].contiguous()))
 
-    whole, step = run(0, H), CTAS // (N // 128)              # heads whose items are one round: the fixed order
-    for lo in range(0, H, step):
-        hi = min(H, lo + step)
-        for a, b in zip(whole, run(lo, hi)):
-            assert torch.equal(a[:, :, lo:hi], b)
+    whole, step = run(slice(0, B), 0, Hk), max(1, CTAS // (nblk * rep))      # groups whose items are one round, or one group
+    assert _plan(step * rep, nblk) is None
+    for b in range(B):
+        for lo in range(0, Hk, step):
+            hi = min(Hk, lo + step)
+            for a, c, r in zip(whole, run(slice(b, b + 1), lo, hi), (rep, rep, 1, 1)):
+                assert torch.equal(a[b:b + 1, :, lo * r:hi * r], c)
