@@ -64,7 +64,7 @@ struct Params {
 };
 
 // The work list: one item = 64 keys `zh` of one 128-key block J of one (batch, query head), ordered by key block, i.e. heaviest first when
-// causal, and walked in a snake over the rounds (as dm::SnakeWalk).
+// causal, and walked in a snake over the rounds (dm::SnakeWalk).
 struct Item {
     dm::HeadCoord hc;
     int J, zh, t_lo, n, bhl;                      // first 128-row tile and their count
@@ -72,9 +72,8 @@ struct Item {
 };
 __device__ __forceinline__ Item item(const Params& p, int round) {
     Item w;
-    const int G = gridDim.x, c = blockIdx.x;
     const int nbn = p.N / 128;
-    const int idx = round * G + ((round & 1) ? G - 1 - c : c);
+    const int idx = dm::walk_index(dm::SnakeWalk{}, round);
     w.valid = idx < 2 * p.n_heads * nbn;
     const int jz = (int)dm::fdiv((uint32_t)idx, p.fd_heads);
     w.hc = dm::head_coord(idx - jz * p.n_heads, p.h0, p.fd_hcount, p.H, p.Hk, p.fd_rep);

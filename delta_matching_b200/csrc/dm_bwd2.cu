@@ -50,7 +50,7 @@ struct Bwd2Params {
 };
 
 // One work item = one local 128-row block of one (batch, head); numbered rank-major (rank 0 = the row blocks with the most key
-// tiles, all heads, then rank 1, ...) and walked in a snake over the rounds (as dm::SnakeWalk).
+// tiles, all heads, then rank 1, ...) and walked in a snake over the rounds (dm::SnakeWalk).
 struct Bwd2Item {
     dm::HeadCoord hc;
     int rb, n_it, bhl;
@@ -58,9 +58,8 @@ struct Bwd2Item {
 };
 __device__ __forceinline__ Bwd2Item bwd2_item(const Bwd2Params& p, int round) {
     Bwd2Item w;
-    const int G = gridDim.x, c = blockIdx.x;
     const int nq_blk = p.rm.nq / 128;
-    const int idx = round * G + ((round & 1) ? G - 1 - c : c);
+    const int idx = dm::walk_index(dm::SnakeWalk{}, round);
     w.valid = idx < p.n_heads * nq_blk;
     const int rank = (int)dm::fdiv((uint32_t)idx, p.fd_heads);
     w.hc = dm::head_coord(idx - rank * p.n_heads, p.h0, p.fd_hcount, p.H, p.Hk, p.fd_rep);

@@ -249,9 +249,8 @@ struct DeltaDivs {
 };
 __device__ __forceinline__ DeltaItem delta_item(const DeltaParams& p, const DeltaDivs& fd, int round) {
     DeltaItem w;
-    const int G = gridDim.x, c = blockIdx.x;
     const int nq_blk = p.rm.nq / 128, n_heads = (int)fd.heads.d;
-    const int idx = round * G + ((round & 1) ? G - 1 - c : c);
+    const int idx = dm::walk_index(dm::SnakeWalk{}, round);
     w.valid = idx < n_heads * nq_blk;
     const int rank = (int)dm::fdiv((uint32_t)idx, fd.heads);
     w.hc = dm::head_coord(idx - rank * n_heads, p.h0, fd.hcount, p.H, p.Hk, fd.rep);

@@ -2,7 +2,7 @@
 // (csrc/flash_fwd_fp8f_launch.h:40, csrc/softmax_fq8f.h kGroups = 4): Q scales per 64 rows, K / V scales per 32 keys,
 // key tiles of 128 keys = FOUR 32-key P groups, each with its own per-row basis.
 //
-// One work item = 128 query rows of one (batch, head); the kernel is persistent, one CTA per SM walks its items (as dm::SnakeWalk),
+// One work item = 128 query rows of one (batch, head); the kernel is persistent, one CTA per SM walks its items (dm::SnakeWalk),
 // and every role keeps its own place in the list.  A code row is 256 bytes = two 128-byte swizzled sub-tiles (d 0..127 and d 128..255).
 // 512 threads:
 //   warps 0..3   service (one elected lane issues): S; the products; the loads of Q and K; the loads of V
@@ -80,9 +80,8 @@ struct Fwd256Item {
 };
 __device__ __forceinline__ Fwd256Item fwd256_item(const Fwd256Params& p, int round) {
     Fwd256Item w;
-    const int G = gridDim.x, c = blockIdx.x;
     const int nblk = p.N / 128;
-    const int idx = round * G + ((round & 1) ? G - 1 - c : c);
+    const int idx = dm::walk_index(dm::SnakeWalk{}, round);
     w.valid = idx < p.n_heads * nblk;
     const int rank = (int)dm::fdiv((uint32_t)idx, p.fd_heads);
     w.hc = dm::head_coord(idx - rank * p.n_heads, p.h0, p.fd_hcount, p.H, p.Hk, p.fd_rep);
