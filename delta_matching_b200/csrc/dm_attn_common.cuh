@@ -1,6 +1,7 @@
 // Arithmetic shared by the attention kernels (forward, pass 0, pass 1): the numerics constants of the reference and
-// the single definition of P-hat that pass 0 and pass 1 must agree on bit for bit, so that the matched delta cancels
-// rowsum(P-hat * (dP - delta)) to fp32 round-off.
+// the two constants of P-hat's exponent.  Pass 0 and pass 1 must agree on P-hat = 2^min(S_raw * descale_log2 + phat_row_const, 12) (the F1
+// clamp of the reference, mainloop_bwd_sm90_fp8r.hpp:746) bit for bit: both form the exponent in one fma and take ex2 of it, so that the
+// matched delta cancels rowsum(P-hat * (dP - delta)) to fp32 round-off.
 #pragma once
 #include "dm_sm100.cuh"
 
@@ -16,10 +17,6 @@ constexpr float kMoInv = 1.0f / 256.0f;
 __device__ __forceinline__ float descale_log2(float q8sc, float k8sc) { return __fmul_rn(__fmul_rn(q8sc, k8sc), kLog2e); }
 // Per-row constant of the P-hat exponent: 8 - lse * log2(e), the product formed by one IEEE multiply.
 __device__ __forceinline__ float phat_row_const(float lse) { return kMoE - __fmul_rn(lse, kLog2e); }
-// P-hat = 2^min(S_raw * dsc - lse * log2e + 8, 12) (the F1 clamp of the reference, mainloop_bwd_sm90_fp8r.hpp:746).
-__device__ __forceinline__ float phat(float s_raw, float dsc, float row_const) {
-    return ex2(fminf(fmaf(s_raw, dsc, row_const), kMoE + 4.0f));
-}
 
 // Row map of the Q-side tensors (Q8, dO8, O, LSE, delta, dQ, dS' tiles): normally all N rows in order; under context
 // parallelism a rank holds two chunks of the sequence (zig-zag), `half` 128-row blocks starting at global block off0

@@ -217,16 +217,6 @@ __device__ __forceinline__ void stmatrix_t_b8_x4(uint32_t saddr, const uint32_t*
                  ::"r"(saddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
                  : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-          "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-          "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
-}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
@@ -354,14 +344,9 @@ __device__ __forceinline__ float fmax3_abs(float a, float b, float c) {
     asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
-// two fp32 -> two e4m3 (round-to-nearest-even, saturate-to-finite), lo in bits 0..7
-__device__ __forceinline__ uint32_t cvt_e4m3x2(float lo, float hi) {
-    uint16_t r;
-    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
-    return r;
-}
-// Four codes in one register: joined by a 16-bit pair move, which the second conversion does on the way (an `or` with a shift costs
-// an instruction of its own, one per four codes: forward at B4 N4096 H32 causal 504 -> 502 us).
+// Four fp32 -> four e4m3 (round-to-nearest-even, saturate-to-finite), the first in bits 0..7.  Joined by a 16-bit pair move, which the
+// second conversion does on the way (an `or` with a shift costs an instruction of its own, one per four codes: forward at B4 N4096 H32
+// causal 504 -> 502 us).
 __device__ __forceinline__ uint32_t cvt_e4m3x4(float a, float b, float c, float d) {
     uint32_t r;
     asm("{\n\t.reg .b16 l, h;\n\t"
