@@ -25,6 +25,7 @@
 
 #include "dm_host.h"
 #include "dm_launch.cuh"
+#include "dm_sm100.cuh"
 
 namespace {
 
@@ -33,13 +34,6 @@ constexpr float kTiny = 1e-30f;
 
 __device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t u) { return __uint_as_float(u & 0xFFFF0000u); }
-
-__device__ __forceinline__ uint32_t e4m3x4(float a, float b, float c, float d) {
-    uint16_t lo, hi;
-    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(lo) : "f"(b), "f"(a));
-    asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(hi) : "f"(d), "f"(c));
-    return (uint32_t)lo | ((uint32_t)hi << 16);
-}
 
 // RN(x / s).  kExactRcp: r = RN(1 / s), 2^-60 <= s <= 2^60 and |x| <= 449 s (see the contract at the top of the file).
 // Scalar on purpose: the same steps on packed fp32 pairs measured slower in the Q quantizer (59.5 against 53.4 us on
@@ -289,7 +283,7 @@ __device__ __forceinline__ void quant_block(int blk, int bh, const __nv_bfloat16
                         qv[e] = fminf(fmaxf(quotient_rn<kExactRcp>(xv, s, rcp), -kE4M3Max), kE4M3Max);
                     }
                 }
-                c4[g] = e4m3x4(qv[0], qv[1], qv[2], qv[3]);
+                c4[g] = dm::cvt_e4m3x4(qv[0], qv[1], qv[2], qv[3]);
                 if (kFinite && MODE != 1) {
                     const uint32_t sign = __byte_perm(u[r][2 * g], u[r][2 * g + 1], 0x7531);   // the high byte of each bf16
                     c4[g] = (c4[g] & 0x7F7F7F7Fu) | (sign & 0x80808080u);
