@@ -31,7 +31,7 @@
 // rounds as a plain row softmax does, and it costs nothing: the softmax warps lose their share of the denominator and the fold its
 // epilogue, which pays for the multiplications of O (lazy basis -> this, us: B4 N4096 H32 causal 508 -> 506, B1 N16384 H32
 // 1788 -> 1792, B2 N2048 H16 49.2 -> 47.2, B4 N768 H12 22.5 -> 20.6, B64 N256 H16 59.5 -> 53.3).
-// What bounds it: the issue rate more than any pipe (ncu at B1 N4096 H32 causal: issue slots 71 % active, MUFU 53 %, tensor pipe 25 %).  Of
+// What bounds it: the issue rate more than any pipe (ncu at B1 N4096 H32 causal: issue slots 70 % active, MUFU 54 %, tensor pipe 26 %).  Of
 // the lazy form's 531 us at B4 N4096 H32 (on a slower clock) 526 were left without the exponentials, 508 without three quarters of the
 // fold's loads and 497 without the second read of the scores.
 #include "dm_attn_common.cuh"

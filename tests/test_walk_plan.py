@@ -45,7 +45,7 @@ def test_packed_walk(heads, nblk, ctas):
     assert _most(plan, heads, nblk) < 0.97 * _most(snake, heads, nblk)
 
 
-# where the mean block is above what a packing has to come down to; where the packing found is; more items or blocks than the lists hold
+# where the mean block is above the load that a packing has to come down to; where every packing found is; more items or blocks than the lists hold
 @pytest.mark.parametrize("heads,nblk,ctas", [(48, 6, 148), (32, 16, 148), (1, 800, 148), (2, 400, 148), (7, 9, 5), (1, 3, 2), (160, 5, 160),
                                              (149, 1, 148), (75, 2, 148), (1, 801, 148), (9, 89, 148), (21, 22, 161)])
 def test_fixed_order(heads, nblk, ctas):
