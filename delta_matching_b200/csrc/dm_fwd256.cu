@@ -353,13 +353,14 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const uint32_t c_row = dm::smem_u32(s.c[0]) + row * 128;
         int t = 0, sl = 0;
         // What an item's first tile needs from global memory is read one item ahead, a tile's K scales one tile ahead: read in place they
-        // would be exposed loads.
+        // would be exposed loads.  The four scales of a tile are read one by one: a caller's scale tensor may start at any multiple of 4 bytes.
+        auto scales4 = [](const float* at) { return make_float4(at[0], at[1], at[2], at[3]); };
         float q8sc_nx = 0.f;
         float4 ks_nx = make_float4(0.f, 0.f, 0.f, 0.f);
         auto first_scales = [&](const Fwd256Item& wi) {
             if (!wi.valid) return;
             q8sc_nx = p.q8s[(int64_t)wi.hc.bh * (p.N / 64) + 2 * wi.I + (row >> 6)];
-            ks_nx = *reinterpret_cast<const float4*>(p.k8s + (int64_t)wi.hc.bhk * (p.N / 32) + 4 * (wi.n_tiles - 1));
+            ks_nx = scales4(p.k8s + (int64_t)wi.hc.bhk * (p.N / 32) + 4 * (wi.n_tiles - 1));
         };
         Fwd256Item w = fwd256_item(p, 0);
         first_scales(w);
@@ -375,8 +376,8 @@ fwd_d256_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             for (int it = 0; it < n_tiles; ++it, ++t, sl = sl == kRing - 1 ? 0 : sl + 1) {
                 const int j = n_tiles - 1 - it;
                 const float dsc[4] = {q8sc * ks_n.x, q8sc * ks_n.y, q8sc * ks_n.z, q8sc * ks_n.w};
-                const float4 vs4 = *reinterpret_cast<const float4*>(vsp + 4 * j);
-                if (it + 1 < n_tiles) ks_n = *reinterpret_cast<const float4*>(ksp + 4 * (j - 1));
+                const float4 vs4 = scales4(vsp + 4 * j);
+                if (it + 1 < n_tiles) ks_n = scales4(ksp + 4 * (j - 1));
                 const bool diag = p.causal && j == I;
 
                 dm::mbar_wait(&s.bar_s, t & 1, wc);

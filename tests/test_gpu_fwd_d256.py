@@ -31,3 +31,24 @@ def test_forward_d256(B, N, H, Hk, causal, scale):
     for h0 in range(H):
         _lib.fwd_fp8(*d, B, H, Hk, causal, h0=h0, hcount=1, out=(o2, lse2))
     assert torch.equal(o, o2) and torch.equal(lse, lse2), "the walk over several items changed the bits"
+
+
+@pytest.mark.parametrize("off", [1, 2, 3])
+def test_scales_at_any_multiple_of_4_bytes(off):
+    """Codes are promised to be 16-byte aligned, scales only to be fp32: views into one buffer give the bits of tensors of their own."""
+    B, N, H, Hk = 1, 640, 3, 1
+    q, k, v, _ = O.make_inputs(B, N, H, Hk, 256, 2032)
+    Q8, Q8s = O.quant_q(q.transpose(1, 2))
+    K8, K8s, _ = O.quant_k(k.transpose(1, 2))
+    V8, V8s = O.quant_v(v.transpose(1, 2))
+    codes, scales = [t.cuda() for t in (Q8, K8, V8)], [t.float().cuda() for t in (Q8s, K8s, V8s)]
+    views = []
+    for t in scales:
+        buf = torch.full((t.numel() + 8,), float("nan"), device="cuda")
+        assert buf.data_ptr() % 16 == 0
+        views.append(buf[off:off + t.numel()].view(t.shape))
+        views[-1].copy_(t)
+    o, lse = _lib.fwd_fp8(*codes, *scales, B, H, Hk, True)
+    o2, lse2 = _lib.fwd_fp8(*codes, *views, B, H, Hk, True)
+    assert _lib.device_status() == 0
+    assert torch.equal(o, o2) and torch.equal(lse, lse2)
