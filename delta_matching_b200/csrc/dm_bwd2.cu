@@ -327,15 +327,19 @@ bwd2_d256_kernel(const __grid_constant__ CUtensorMap tm_ds, const __grid_constan
             const Bwd2Item w = bwd2_item(p, r);
             if (!w.valid) break;
             const int mb = 2 * w.rb + (row >> 6);
-            const float2* psi_row = reinterpret_cast<const float2*>(p.psi + ((int64_t)w.bhl * nbm_l + mb) * (2 * nbn));   // [heads, N/64, N/64]
+            // [heads, N/64, N/64]; one value at a time, as psi may start at any multiple of 4 bytes
+            const float* psi_row = p.psi + ((int64_t)w.bhl * nbm_l + mb) * (2 * nbn);
             float psi_max = 0.f;
             float dq[128];
 #pragma unroll
             for (int i = 0; i < 128; ++i) dq[i] = 0.f;
-            float2 psi_n = psi_row[0];                                     // read a tile ahead
+            float psi_n[2] = {psi_row[0], psi_row[1]};                     // read a tile ahead
             for (int it = 0; it < w.n_it; ++it, ++t) {
-                const float psi2[2] = {psi_n.x, psi_n.y};
-                if (it + 1 < w.n_it) psi_n = psi_row[it + 1];
+                const float psi2[2] = {psi_n[0], psi_n[1]};
+                if (it + 1 < w.n_it) {
+                    psi_n[0] = psi_row[2 * it + 2];
+                    psi_n[1] = psi_row[2 * it + 3];
+                }
 #pragma unroll
                 for (int kh = 0; kh < 2; ++kh) {
                     const float psi_cur = psi2[kh];
