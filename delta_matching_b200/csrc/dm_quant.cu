@@ -413,6 +413,8 @@ int check_geometry(int B, int heads, int N, int D, char* err, size_t errlen) {
     return DM_OK;
 }
 
+bool aligned8(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; }      // chunk sums are written as pairs
+
 int check_strides(const void* p, DmStrides s, int D, const char* name, char* err, size_t errlen) {
     DM_REQUIRE((reinterpret_cast<uintptr_t>(p) & 15u) == 0, DM_ERR_ARG, "%s is not 16-byte aligned", name);
     DM_REQUIRE(s.b % 8 == 0 && s.n % 8 == 0 && s.h % 8 == 0, DM_ERR_ARG,
@@ -436,6 +438,7 @@ extern "C" int dm_kmean(const void* k, DmStrides ks, int32_t B, int32_t Hk, int3
     if ((rc = dmh::check_device_ptr(km, "km", err, errlen))) return rc;
     if ((rc = dmh::check_device_ptr(partials, "partials", err, errlen))) return rc;
     if ((rc = check_strides(k, ks, D, "k", err, errlen))) return rc;
+    DM_REQUIRE(aligned8(partials), DM_ERR_ARG, "partials is not 8-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const __nv_bfloat16* kp = static_cast<const __nv_bfloat16*>(k);
     if (D == 128) {
@@ -462,6 +465,7 @@ extern "C" int dm_quant_qv_kpartials(const void* q, DmStrides qs, const void* k,
     if ((rc = check_strides(k, ks, s.D, "k", err, errlen))) return rc;
     if ((rc = check_strides(v, vs, s.D, "v", err, errlen))) return rc;
     DM_REQUIRE(dmh::aligned16(q8) && dmh::aligned16(v8), DM_ERR_ARG, "codes are not 16-byte aligned");
+    DM_REQUIRE(aligned8(partials), DM_ERR_ARG, "partials is not 8-byte aligned");
     const int qblk = s.D == 128 ? 128 : 64, kblk = s.D == 128 ? 64 : 32, cpb = s.D == 128 ? 4 : 2;
     PrologueArgs a;
     a.q = static_cast<const __nv_bfloat16*>(q); a.k = static_cast<const __nv_bfloat16*>(k); a.v = static_cast<const __nv_bfloat16*>(v);
@@ -489,6 +493,7 @@ extern "C" int dm_kmean_partials(const void* k, DmStrides ks, int32_t B, int32_t
     if ((rc = dmh::check_device_ptr(k, "k", err, errlen))) return rc;
     if ((rc = dmh::check_device_ptr(partials, "partials", err, errlen))) return rc;
     if ((rc = check_strides(k, ks, D, "k", err, errlen))) return rc;
+    DM_REQUIRE(aligned8(partials), DM_ERR_ARG, "partials is not 8-byte aligned");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const __nv_bfloat16* kp = static_cast<const __nv_bfloat16*>(k);
     if (D == 128) DM_CUDA(dmh::launch_pdl(kmean_partial_kernel<128>, dim3(N / 64 / 4, B * Hk), 256, 0, stream, kp, ks.b, ks.n, ks.h, Hk, N, partials));

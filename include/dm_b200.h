@@ -8,7 +8,8 @@
  * Layouts.  bf16 tensors use the flash-attention layout (batch, seqlen, heads, head_dim) with explicit element strides
  * for batch / seqlen / head (the head_dim stride must be 1).  fp8 code tensors are [batch*heads, seqlen, head_dim]
  * e4m3, contiguous, 16-byte aligned; scales are contiguous fp32 [batch*heads, seqlen / rows_per_scale] with
- * rows_per_scale = (128, 64) for (Q / dO, K / V) at head_dim 128 and (64, 32) at head_dim 256.  Query head h reads KV
+ * rows_per_scale = (128, 64) for (Q / dO, K / V) at head_dim 128 and (64, 32) at head_dim 256.  Scales, LSE, delta, psi and the K
+ * mean may start at any multiple of 4 bytes; every other tensor is 16-byte aligned unless its call says less.  Query head h reads KV
  * head h / (H / Hk).
  *
  * Each declaration cites the reference interface it replaces (paths inside the haok1402/delta-matching project).
@@ -57,7 +58,8 @@ typedef struct DmCp {
 const char* dm_build_info(void);
 
 /* Per-head K mean over the sequence, fp32 [B*Hk, D], bit-exact fold order: 64-row chunk sums (rows ascending), chunks
- * folded serially, one IEEE division by N.  `partials` is caller-provided scratch of dm_kmean_scratch_bytes() bytes.
+ * folded serially, one IEEE division by N.  `partials` is caller-provided scratch of dm_kmean_scratch_bytes() bytes, 8-byte
+ * aligned in every call that writes it.
  * Replaces _kmean_kernel (delta_matching/quant.py:17-29) and kmean_m17 (delta_matching/producers.py:75-94). */
 size_t dm_kmean_scratch_bytes(int32_t B, int32_t Hk, int32_t N, int32_t D);
 int dm_kmean(const void* k_bf16, DmStrides ks, int32_t B, int32_t Hk, int32_t N, int32_t D, float* km, float* partials,

@@ -227,6 +227,14 @@ def test_library_checks_its_inputs():
     buf = torch.empty(Q8.numel() + 16, dtype=torch.uint8, device="cuda")
     shifted = buf[1:1 + Q8.numel()].view(torch.float8_e4m3fn).view(Q8.shape)
     _raises(RuntimeError, "aligned", lambda: _lib.fwd_fp8(shifted, K8, V8, Q8s, K8s, V8s, 1, 4, 2, True))
+    # the K mean's chunk sums are written as pairs of fp32
+    part = torch.empty(2 * 8 * 128 + 2, device="cuda")[1:]
+    km, st, stream = torch.empty(2, 128, device="cuda"), _lib._strides_bnhd, _lib._stream(q.device)
+    _raises(RuntimeError, "aligned", lambda: _lib._call("dm_kmean", _lib._ptr(k), st(k), 1, 2, 512, 128, _lib._ptr(km), _lib._ptr(part), stream))
+    _raises(RuntimeError, "aligned", lambda: _lib._call("dm_kmean_partials", _lib._ptr(k), st(k), 1, 2, 512, 128, _lib._ptr(part), stream))
+    _raises(RuntimeError, "aligned", lambda: _lib._call("dm_quant_qv_kpartials", _lib._ptr(q), st(q), _lib._ptr(k), st(k), _lib._ptr(v), st(v),
+                                                        _lib._shape(1, 4, 2, 512, 128, True), _lib._ptr(Q8), _lib._ptr(Q8s), _lib._ptr(V8),
+                                                        _lib._ptr(V8s), _lib._ptr(part), stream))
     _raises(RuntimeError, "seqlen", lambda: _lib.delta_fp8(Q8[:, :192], K8, V8, Q8, Q8s, K8s, V8s, Q8s, lse, 1, 4, 2, True))
     _raises(RuntimeError, "nheads", lambda: _lib.fwd_fp8(Q8, K8, V8, Q8s, K8s, V8s, 1, 4, 3, True))
     assert _lib.device_status() == 0
