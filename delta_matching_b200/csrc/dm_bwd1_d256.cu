@@ -19,10 +19,10 @@
 // the keys each form their own scores only.  The price is that every MMA is N = 64 wide, which takes as long as 128 (2100 clocks of
 // tensor pipe a tile), but of the softmax warps' work, which bounded that kernel, each item has half.  Q and dO share a ring of five 32 KB
 // units, so that Q (and S) run half a tile further ahead than dO; Q is released behind dK's last product, dO behind dV's.
-// Measured, us at B2 N4096 H16 full / causal / B1 N1920 H8 causal: 1055 / 617 / 68.5 with the d halves, 834 / 448 / 35.6 with this.  What bounds
+// Measured, us at B2 N4096 H16 full / causal / B1 N1920 H8 causal: 1056 / 625 / 68.7 with the d halves, 840 / 455 / 36.0 with this.  What bounds
 // it: two chains of about 3400 clocks a tile, the fold's (each product's wait, loads and additions, twice; the unit moved twice) and the one
 // dS' tile's (codes, both products, free again); shared memory is half busy with operands (280 KB a tile).  On the way: 72 / 96 / 24
-// registers for softmax, fold and service 864, 56 / 128 / 24 906 and 56 / 120 / 40 831 (the service warps spilled at 24); the m-blocks'
+// registers for softmax, fold and service 864, 56 / 128 / 24 906 (the service warps spill at 24); the m-blocks'
 // loops unrolled 862 (the instruction cache missed one request in nine); two X buffers and one of S / dP instead 855.
 #include "dm_attn_common.cuh"
 #include "dm_host.h"

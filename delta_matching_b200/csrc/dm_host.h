@@ -92,7 +92,7 @@ int device_once(DeviceOnce& o, char* err, size_t errlen, F&& f) {
 int sm_count(int* sms, char* err, size_t errlen);
 
 // How `ctas` persistent CTAs walk heads x nblk items whose lengths fall by one tile a rank (nblk, .., 1); false (and no lists) where the snake
-// order is as good (one round; many rounds).
+// order is taken: one round, little to save, or more items than the list holds.
 bool plan_walk(int heads, int nblk, int ctas, dm::PackedWalk* out);
 
 // One-time set-up of each kernel family on the current device (also reached lazily from the entry points).

@@ -100,8 +100,7 @@ def test_config3_gqa_and_logit_range(scale):
 
 
 def test_config4_head_dim_256_full_stale():
-    """B2 N4096 H16 Hk4 D256, non-causal, stale delta: 1024 forward items and 2048 pass-1 items (two d halves per key
-    block)."""
+    """B2 N4096 H16 Hk4 D256, non-causal, stale delta: 1024 forward items and 2048 pass-1 items (64 keys each)."""
     B, N, H, Hk = 2, 4096, 16, 4
     q, k, v, do = O.make_inputs(B, N, H, Hk, 256, 1004)
     got = _run(q, k, v, do, "stale", causal=False)
